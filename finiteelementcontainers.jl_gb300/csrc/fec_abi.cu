@@ -1198,14 +1198,15 @@ int fec_assemble(fec_ctx* c, int want, int precision, double t, double dt, const
   ga.R_u = want_r ? R_u : nullptr;
   ga.acc_stride = c->acc_stride;
   cudaError_t e;
-  // meshes of mixed element sizes: one gather launch per group of nodes of one size
+  // meshes of mixed element sizes: with the tangent, one gather launch per group of nodes of one size
   bool mixed_sizes = false;
   for (const Block& B : c->blocks) mixed_sizes = mixed_sizes || B.nnpe != c->blocks[0].nnpe;
-  if (mixed_sizes && !gather_runs_generic() && !c->groups_ready)
+  const bool groups = mixed_sizes && want_k && !gather_runs_generic();
+  if (groups && !c->groups_ready)
     if (int rc = build_node_groups(c)) return rc;
   {
     LaunchTimer timer(c, s, "node_gather");
-    if (mixed_sizes && !gather_runs_generic())
+    if (groups)
       e = fec::launch_gather_groups(precision, c->nf, ga, static_cast<const int32_t*>(c->d_node_groups.p),
                                     c->node_groups.data(), int(c->node_groups.size()), s, &c->last_launches);
     else

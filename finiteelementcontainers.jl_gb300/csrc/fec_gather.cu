@@ -90,6 +90,12 @@ cudaError_t go_pipe(const GatherArgs& g, cudaStream_t s, int* launches) {
 
 template <typename Real, int NF>
 cudaError_t by_size(const GatherArgs& g, cudaStream_t s, int* launches) {
+  if (g.nzval == nullptr) {  // residual alone
+    if (g.nn <= 0 || g.R_u == nullptr) return cudaSuccess;
+    residual_gather_kernel<Real, NF><<<unsigned((g.nn * NF + 255) / 256), 256, 0, s>>>(g);
+    ++*launches;
+    return cudaGetLastError();
+  }
   if (NF == 3 && g.nn > 0 && g.nblocks == 1 && g.blk[0].nnpe == 8 && g.nzval != nullptr && gather_pipe_enabled()) {
     if (g.blk[0].layout == KE_NODE_ROWS) return go_pipe<Real>(g, s, launches);
     if constexpr (sizeof(Real) == 8)
