@@ -97,6 +97,7 @@ struct fec_ctx {
   DevBuf d_cl_img, d_cl_table;  // tensor-core closure: packed parameters, per-point table
   DevBuf d_V;                   // matrix-free action: the direction as a full field
   DevBuf d_colptr0, d_rowval32, d_cg;  // linear solve: 0-based CSC pattern, CG scratch
+  fec::PcgHost cg_host;                // linear solve: where the host reads the stopping test
   DevBuf d_flag;                       // non-finite scan result
   DevBuf d_nbr_ptr, d_nbr;             // neighbour lists on the device (device symbolic phase, CSC fill)
   DevBuf d_tile_counter;               // single launch of mixed element blocks: next work tile
@@ -395,6 +396,7 @@ int fec_ctx_destroy(fec_ctx* c) {
                     &c->d_cg, &c->d_flag, &c->d_nbr_ptr, &c->d_nbr, &c->d_tile_counter, &c->d_node_groups})
     b->release();
   for (DevBuf& b : c->d_affine) b.release();
+  c->cg_host.release();
   delete c;
   return FEC_OK;
 }
@@ -1359,7 +1361,7 @@ int fec_cg_solve(fec_ctx* c, const double* nzval, const double* b, double* x, in
   int it = 0;
   double rr = 0.0;
   const cudaError_t e = fec::pcg(A, b, x, static_cast<double*>(c->d_cg.p), max_iter, rtol, 10, preconditioner == 1,
-                                 &it, &rr, s);
+                                 c->cg_host, &it, &rr, s);
   if (iterations) *iterations = it;
   if (rel_residual) *rel_residual = rr;
   if (e != cudaSuccess) return fail(c, FEC_ERR_CUDA, "conjugate gradients: %s", cudaGetErrorString(e));

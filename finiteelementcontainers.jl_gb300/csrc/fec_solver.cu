@@ -3,167 +3,431 @@
 // IterativeLinearSolver, src/Solvers.jl:88-152, which hands K and R to a Krylov
 // CG), on the device.
 //
-// K is symmetric, so its CSC columns are its rows: y = K x takes one warp per
-// column j, y_j = sum_p val[p] x[row[p]], reduced by a fixed shuffle tree.  Dot
-// products reduce in two fixed-shape stages (per-block partials in a fixed grid,
-// then one block), so a solve is bitwise repeatable.  The CG scalars live on the
-// device; the host reads the residual norm every few iterations only.
+// K is symmetric, so its CSC columns are its rows.  An iteration is three
+// kernels: y = K p with the partial sums of p.y, x and r updated with the
+// partial sums of r.z and r.r, and the new direction.  The partial sums of a
+// kernel (one per CTA) are added by every CTA of the next one in the same fixed
+// order, so there is no reduction kernel, the scalars never leave the device and
+// a solve is bitwise repeatable.
+//
+// What bounds it: up to some 100k unknowns launches, the latency of dependent
+// loads and the FP64 pipe, which takes an SM 16 clocks per warp instruction
+// however few lanes are active (the matrix of a 36 x 32 x 34 box, 11 MB, stays in
+// L2); beyond, the matrix from memory.  Hence three launches an iteration instead
+// of eight, chained by programmatic dependent launch; a product with one FP64
+// instruction per entry and no shuffle tree (a warp copies the entries of its
+// next 32 rows to shared memory, coalesced and asynchronous, while each lane adds
+// a row of the last 32, whose x entries are mostly neighbours' too); sums
+// through shared memory and one warp; and the stopping test on the device, which
+// the host reads one batch of iterations behind, so the stream never runs dry and
+// the kernels of a batch that follow the converged iteration return at once.
+// Per iteration, Poisson: 36 x 32 x 34 elements 55 -> 15 us (product 7, update 4,
+// direction 4), 70^3 elements 59 us (product 44: 2.5 TB/s of matrix).
 #include <cmath>
-#include <vector>
+#include <cstring>
+#include "fec_launch.h"
 #include "fec_solver.h"
 
 namespace fec {
 namespace {
 
-constexpr int DOT_BLOCKS = 608, DOT_THREADS = 256;
+constexpr int THREADS = 256;
+constexpr int MAX_CTAS = 304;  // the partial sums of one kernel
+constexpr int WARPS = THREADS / 32;
+constexpr int CAP = 896;       // entries a warp stages at once (32 rows of 27 fit; longer rows take more rounds)
+constexpr size_t ROWS_SMEM = size_t(WARPS) * 2 * CAP * 12;  // (value, row) double-buffered
 
-__global__ void spmv_sym_kernel(CscSym A, const double* __restrict__ x, double* __restrict__ y) {
-  const int64_t j = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+// scalars on the device
+struct CgScalars {
+  double rz[2];      // r.z of the iteration, by parity
+  double bb, rr;     // b.b; r.r of the last stopping test
+  int it;            // iterations of the last stopping test
+  int done;          // 1: converged (or b = 0); the iteration kernels return
+};
+
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Sums over the CTA of a and b (fixed order), to thread 0 (a) and thread 32 (b).
+// Through shared memory: a shuffle tree in every warp would issue three times the
+// FP64 instructions.
+struct SumBuf {
+  double a[THREADS], b[THREADS];
+};
+__device__ __forceinline__ double warp_total(const double* v) {
   const int lane = threadIdx.x & 31;
-  if (j >= A.n) return;
-  double s = 0.0;
-  for (int64_t p = A.colptr[j] + lane; p < A.colptr[j + 1]; p += 32) s = fma(A.val[p], x[A.rowval[p]], s);
+  double t = v[lane];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if (lane == 0) y[j] = s;
-}
-
-__global__ void inv_diag_kernel(CscSym A, double* __restrict__ inv_diag) {
-  const int64_t j = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (j >= A.n) return;
-  double d = 0.0;
-  for (int64_t p = A.colptr[j] + lane; p < A.colptr[j + 1]; p += 32)
-    if (A.rowval[p] == j) d = A.val[p];
+  for (int k = 1; k < THREADS / 32; ++k) t += v[lane + 32 * k];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
-  if (lane == 0) inv_diag[j] = d != 0.0 ? 1.0 / d : 1.0;
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
 }
-
-__global__ void __launch_bounds__(DOT_THREADS) dot_partial_kernel(int64_t n, const double* __restrict__ a,
-                                                                  const double* __restrict__ b,
-                                                                  double* __restrict__ partial) {
-  __shared__ double red[DOT_THREADS];
-  const int64_t chunk = (n + DOT_BLOCKS - 1) / DOT_BLOCKS;
-  const int64_t lo = int64_t(blockIdx.x) * chunk, hi = lo + chunk < n ? lo + chunk : n;
-  double s = 0.0;
-  for (int64_t i = lo + threadIdx.x; i < hi; i += DOT_THREADS) s = fma(a[i], b[i], s);
-  red[threadIdx.x] = s;
+__device__ __forceinline__ void cta_sums(SumBuf& buf, double a, double b, double* out_a, double* out_b) {
+  buf.a[threadIdx.x] = a;
+  buf.b[threadIdx.x] = b;
   __syncthreads();
-  for (int w = DOT_THREADS / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
+  if (threadIdx.x < 32) {
+    const double t = warp_total(buf.a);
+    if (threadIdx.x == 0) *out_a = t;
+  } else if (threadIdx.x < 64) {
+    const double t = warp_total(buf.b);
+    if (threadIdx.x == 32) *out_b = t;
   }
-  if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
 }
-
-__global__ void __launch_bounds__(1024) dot_final_kernel(const double* __restrict__ partial, double* out) {
-  __shared__ double red[1024];
-  red[threadIdx.x] = threadIdx.x < DOT_BLOCKS ? partial[threadIdx.x] : 0.0;
+// The partial sums part[0 .. count), added in the same order by every CTA, on
+// every thread.
+__device__ __forceinline__ double total(const double* part, int count, double* slot) {
+  if (threadIdx.x < 32) {
+    double s = 0.0;
+    for (int i = threadIdx.x; i < count; i += 32) s += __ldcg(part + i);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) *slot = s;
+  }
   __syncthreads();
-  for (int w = 512; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
+  return *slot;
+}
+
+// Entries [c0, c0 + CAP) of the 32 rows 32 rc .. of a warp; this lane's row is
+// 32 rc + lane and has the entries [lo, hi).
+struct Round {
+  int64_t rc, lo, hi, c0, end;
+};
+
+// f(j, (K x)_j, K_jj) for the rows of this warp (WANT_DIAG, else 0): a lane adds a
+// row in its order; the entries of the next round are on their way meanwhile.
+template <bool WANT_DIAG, class F>
+__device__ __forceinline__ void rows_product(const CscSym& A, const double* x, unsigned char* sm, F f) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double* val = reinterpret_cast<double*>(sm) + warp * 2 * CAP;
+  int32_t* row = reinterpret_cast<int32_t*>(sm + size_t(WARPS) * 2 * CAP * 8) + warp * 2 * CAP;
+  const int64_t GW = int64_t(gridDim.x) * WARPS, n = A.n;
+  auto ptr = [&](int64_t j) { return __ldg(A.colptr + (j < n ? j : n)); };
+  auto start = [&](int64_t rc, int64_t lo, int64_t hi) {
+    Round r;
+    r.rc = rc;
+    r.lo = lo;
+    r.hi = hi;
+    r.c0 = __shfl_sync(0xffffffffu, lo, 0);
+    r.end = __shfl_sync(0xffffffffu, hi, 31);
+    return r;
+  };
+  auto issue = [&](const Round& r, int st) {
+    if (r.rc * 32 < n) {
+      const int cnt = int(r.end - r.c0 < CAP ? r.end - r.c0 : CAP);
+      for (int i = lane; i < cnt; i += 32) {
+        gp::cp_small<8>(val + st * CAP + i, A.val + r.c0 + i);
+        gp::cp_small<4>(row + st * CAP + i, A.rowval + r.c0 + i);
+      }
+    }
+    gp::commit();
+  };
+  int64_t rc = int64_t(blockIdx.x) * WARPS + warp;
+  Round cur = start(rc, ptr(rc * 32 + lane), ptr(rc * 32 + lane + 1));
+  issue(cur, 0);
+  int64_t rc1 = rc + GW, lo1 = ptr(rc1 * 32 + lane), hi1 = ptr(rc1 * 32 + lane + 1);  // the chunk after
+  double s = 0.0, d = 0.0;
+  for (int it = 0; cur.rc * 32 < n; ++it) {
+    const int st = it & 1;
+    Round nxt = cur;
+    const bool last = cur.c0 + CAP >= cur.end;  // of these 32 rows
+    if (last) {
+      nxt = start(rc1, lo1, hi1);
+      rc1 += GW;
+      lo1 = ptr(rc1 * 32 + lane);
+      hi1 = ptr(rc1 * 32 + lane + 1);
+    } else {
+      nxt.c0 += CAP;
+    }
+    issue(nxt, st ^ 1);
+    gp::wait_prev();
+    __syncwarp();
+    const int64_t j = cur.rc * 32 + lane;
+    const int b = int((cur.lo > cur.c0 ? cur.lo : cur.c0) - cur.c0);
+    const int e = int((cur.hi < cur.c0 + CAP ? cur.hi : cur.c0 + CAP) - cur.c0);
+    const double* v = val + st * CAP;
+    const int32_t* c = row + st * CAP;
+    constexpr int U = 9;
+    for (int i = b; i < e; i += U) {
+      double xv[U];
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        const int cc = i + k < e ? c[i + k] : -1;
+        xv[k] = cc >= 0 ? x[cc] : 0.0;
+        if (WANT_DIAG && cc == j) d = v[i + k];
+      }
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        if (i + k < e) s = fma(v[i + k], xv[k], s);
+    }
+    if (last) {
+      if (j < n) f(j, s, d);
+      s = d = 0.0;
+    }
+    __syncwarp();  // every lane has read this stage
+    cur = nxt;
   }
-  if (threadIdx.x == 0) *out = red[0];
+  asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-// r = b - r (r holds K x on entry); z = M^-1 r; p = z
-__global__ void cg_init_kernel(int64_t n, const double* b, double* r, double* z, double* p, const double* inv_diag) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double ri = b[i] - r[i];
-  r[i] = ri;
-  const double zi = inv_diag ? inv_diag[i] * ri : ri;
-  z[i] = zi;
-  p[i] = zi;
+// r = b - K x; z = M^-1 r; p = z; partial sums of r.z and b.b.  inv_diag: filled
+// here when the preconditioner is Jacobi's, else null (M = 1).
+__global__ void __launch_bounds__(THREADS) cg_init_kernel(CscSym A, const double* __restrict__ b, const double* x,
+                                                          double* r, double* z, double* p, double* inv_diag,
+                                                          double* part_rz, double* part_bb) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ SumBuf buf;
+  double rz = 0.0, bb = 0.0;
+  auto put = [&](int64_t j, double s, double d) {
+    const double bj = b[j], rj = bj - s;
+    double zj = rj;
+    if (inv_diag) {
+      const double m = d != 0.0 ? 1.0 / d : 1.0;
+      inv_diag[j] = m;
+      zj = m * rj;
+    }
+    r[j] = rj;
+    z[j] = zj;
+    p[j] = zj;
+    rz = fma(rj, zj, rz);
+    bb = fma(bj, bj, bb);
+  };
+  if (inv_diag)
+    rows_product<true>(A, x, sm, put);
+  else
+    rows_product<false>(A, x, sm, put);
+  cta_sums(buf, rz, bb, part_rz + blockIdx.x, part_bb + blockIdx.x);
 }
 
-// alpha = rz / pAp; x += alpha p; r -= alpha Ap; z = M^-1 r
-__global__ void cg_update_kernel(int64_t n, const double* sc, double* x, double* r, double* z, const double* p,
-                                 const double* Ap, const double* inv_diag) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double alpha = sc[0] / sc[1];
-  x[i] = fma(alpha, p[i], x[i]);
-  const double ri = fma(-alpha, Ap[i], r[i]);
-  r[i] = ri;
-  z[i] = inv_diag ? inv_diag[i] * ri : ri;
+// b.b and whether it is zero (one CTA)
+__global__ void __launch_bounds__(THREADS) cg_start_kernel(const double* part_rz, const double* part_bb, int count,
+                                                           CgScalars* sc) {
+  __shared__ double slot[2];
+  const double rz = total(part_rz, count, slot), bb = total(part_bb, count, slot + 1);
+  if (threadIdx.x == 0) {
+    sc->rz[0] = rz;
+    sc->bb = bb;
+    sc->rr = 0.0;
+    sc->it = 0;
+    sc->done = bb == 0.0 ? 1 : 0;
+  }
 }
 
-// beta = rz_new / rz; p = z + beta p
-__global__ void cg_direction_kernel(int64_t n, const double* sc, const double* z, double* p) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  p[i] = fma(sc[2] / sc[0], p[i], z[i]);
+// y = K p; partial sums of p.y
+__global__ void __launch_bounds__(THREADS) cg_product_kernel(CscSym A, const double* p, double* y, double* part,
+                                                             const CgScalars* sc) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ SumBuf buf;
+  grid_wait();
+  grid_next();
+  if (__ldcg(&sc->done)) return;
+  double py = 0.0;
+  rows_product<false>(A, p, sm, [&](int64_t j, double s, double) {
+    y[j] = s;
+    py = fma(p[j], s, py);
+  });
+  buf.a[threadIdx.x] = py;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const double t = warp_total(buf.a);
+    if (threadIdx.x == 0) part[blockIdx.x] = t;
+  }
 }
 
-__global__ void copy_scalar_kernel(double* sc) { sc[0] = sc[2]; }
+// alpha = r.z / p.y; x += alpha p; r -= alpha y; z = M^-1 r; partial sums of the
+// new r.z and r.r.  (A thread's next entries are loaded before it waits for the
+// sum or uses those it has.)
+__global__ void __launch_bounds__(THREADS) cg_update_kernel(int64_t n, const CgScalars* sc, int parity,
+                                                            const double* part_py, int count, double* x, double* r,
+                                                            double* z, const double* p, const double* y,
+                                                            const double* inv_diag, double* part_rz, double* part_rr) {
+  __shared__ SumBuf buf;
+  __shared__ double slot;
+  grid_wait();
+  grid_next();
+  if (__ldcg(&sc->done)) return;
+  int64_t i = int64_t(blockIdx.x) * THREADS + threadIdx.x;
+  double pi = 0.0, yi = 0.0, xi = 0.0, ri = 0.0, mi = 1.0;
+  auto load = [&] {
+    if (i >= n) return;
+    pi = p[i];
+    yi = y[i];
+    xi = x[i];
+    ri = r[i];
+    if (inv_diag) mi = inv_diag[i];
+  };
+  load();
+  const double alpha = __ldcg(&sc->rz[parity]) / total(part_py, count, &slot);
+  double rz = 0.0, rr = 0.0;
+  while (i < n) {
+    const int64_t k = i;
+    const double xk = fma(alpha, pi, xi), rk = fma(-alpha, yi, ri), zk = mi * rk;
+    i += int64_t(gridDim.x) * THREADS;
+    load();
+    x[k] = xk;
+    r[k] = rk;
+    z[k] = zk;
+    rz = fma(rk, zk, rz);
+    rr = fma(rk, rk, rr);
+  }
+  cta_sums(buf, rz, rr, part_rz + blockIdx.x, part_rr + blockIdx.x);
+}
+
+// beta = new r.z / r.z; p = z + beta p; the new r.z for the next iteration
+__global__ void __launch_bounds__(THREADS) cg_direction_kernel(int64_t n, CgScalars* sc, int parity,
+                                                               const double* part_rz, int count, const double* z,
+                                                               double* p) {
+  __shared__ double slot;
+  grid_wait();
+  grid_next();
+  if (__ldcg(&sc->done)) return;
+  int64_t i = int64_t(blockIdx.x) * THREADS + threadIdx.x;
+  double zi = 0.0, pi = 0.0;
+  auto load = [&] {
+    if (i >= n) return;
+    zi = z[i];
+    pi = p[i];
+  };
+  load();
+  const double rz = total(part_rz, count, &slot);
+  const double beta = rz / __ldcg(&sc->rz[parity]);
+  if (blockIdx.x == 0 && threadIdx.x == 0) sc->rz[parity ^ 1] = rz;
+  while (i < n) {
+    const int64_t k = i;
+    const double pk = fma(beta, pi, zi);
+    i += int64_t(gridDim.x) * THREADS;
+    load();
+    p[k] = pk;
+  }
+}
+
+// The stopping test after `it` iterations: sqrt(r.r) / sqrt(b.b) <= rtol (one CTA).
+__global__ void __launch_bounds__(THREADS) cg_test_kernel(CgScalars* sc, const double* part_rr, int count, int it,
+                                                          double rtol) {
+  __shared__ double slot;
+  grid_wait();
+  grid_next();
+  if (__ldcg(&sc->done)) return;
+  const double rr = total(part_rr, count, &slot);
+  if (threadIdx.x == 0) {
+    sc->rr = rr;
+    sc->it = it;
+    if (sqrt(rr) / sqrt(sc->bb) <= rtol) sc->done = 1;
+  }
+}
+
+// A launch that may start while the kernel before it on the stream drains; its
+// kernels wait (grid_wait) before they read what that one wrote.
+template <typename... P, typename... Q>
+cudaError_t launch_next(void (*kern)(P...), unsigned grid, size_t smem, cudaStream_t s, Q... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
+constexpr size_t SC_DOUBLES = (sizeof(CgScalars) + 7) / 8;
 
 }  // namespace
 
-size_t pcg_scratch_doubles(int64_t n) { return size_t(5) * size_t(n) + DOT_BLOCKS + 8; }
-
-cudaError_t spmv_sym(const CscSym& A, const double* x, double* y, cudaStream_t s) {
-  const int64_t threads = A.n * 32;
-  spmv_sym_kernel<<<unsigned((threads + 255) / 256), 256, 0, s>>>(A, x, y);
-  return cudaGetLastError();
+cudaError_t PcgHost::ensure() {
+  cudaError_t e;
+  if (!pinned && (e = cudaMallocHost(&pinned, 2 * SLOT)) != cudaSuccess) return e;
+  for (cudaEvent_t& d : done)
+    if (!d && (e = cudaEventCreateWithFlags(&d, cudaEventDisableTiming)) != cudaSuccess) return e;
+  return cudaSuccess;
 }
 
+void PcgHost::release() {
+  if (pinned) cudaFreeHost(pinned);
+  pinned = nullptr;
+  for (cudaEvent_t& d : done) {
+    if (d) cudaEventDestroy(d);
+    d = nullptr;
+  }
+}
+
+size_t pcg_scratch_doubles(int64_t n) { return size_t(5) * size_t(n) + 3 * MAX_CTAS + SC_DOUBLES; }
+
 cudaError_t pcg(const CscSym& A, const double* b, double* x, double* scratch, int max_iter, double rtol,
-                int check_every, bool jacobi, int* iterations, double* rel_residual, cudaStream_t s) {
+                int check_every, bool jacobi, PcgHost& host, int* iterations, double* rel_residual, cudaStream_t s) {
+  static_assert(sizeof(CgScalars) <= PcgHost::SLOT, "host slot");
+  *iterations = 0;
+  *rel_residual = 0.0;
+  if (A.n == 0) return cudaSuccess;
   const int64_t n = A.n;
   double* r = scratch;
   double* z = r + n;
   double* p = z + n;
-  double* Ap = p + n;
-  double* inv_diag = Ap + n;
-  double* partial = inv_diag + n;
-  double* sc = partial + DOT_BLOCKS;  // [0] rz, [1] pAp, [2] rz_new, [3] rr, [4] bb
-  const unsigned gv = unsigned((n + 255) / 256);
-  const unsigned gw = unsigned((n * 32 + 255) / 256);
-  auto dot = [&](const double* a, const double* bb, double* out) {
-    dot_partial_kernel<<<DOT_BLOCKS, DOT_THREADS, 0, s>>>(n, a, bb, partial);
-    dot_final_kernel<<<1, 1024, 0, s>>>(partial, out);
+  double* y = p + n;
+  double* inv_diag = jacobi ? y + n : nullptr;
+  double* part_py = y + 2 * n;
+  double* part_rz = part_py + MAX_CTAS;
+  double* part_rr = part_rz + MAX_CTAS;
+  CgScalars* sc = reinterpret_cast<CgScalars*>(part_rr + MAX_CTAS);
+  const int64_t groups = (n + THREADS - 1) / THREADS, sms = num_sms() < MAX_CTAS ? num_sms() : MAX_CTAS;
+  const unsigned gm = unsigned(groups < sms ? groups : sms);  // one CTA of the product per SM (shared memory)
+  const unsigned gv = unsigned(groups < MAX_CTAS ? groups : MAX_CTAS);
+  cudaError_t e;
+  if ((e = host.ensure()) != cudaSuccess || (e = ensure_smem<cg_init_kernel>(ROWS_SMEM)) != cudaSuccess ||
+      (e = ensure_smem<cg_product_kernel>(ROWS_SMEM)) != cudaSuccess)
+    return e;
+  cg_init_kernel<<<gm, THREADS, ROWS_SMEM, s>>>(A, b, x, r, z, p, inv_diag, part_rz, part_py);
+  cg_start_kernel<<<1, THREADS, 0, s>>>(part_rz, part_py, int(gm), sc);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  // the scalars after batch k land in host slot k & 1
+  auto read_back = [&](int k) {
+    const cudaError_t e1 = cudaMemcpyAsync(static_cast<char*>(host.pinned) + (k & 1) * PcgHost::SLOT, sc,
+                                           sizeof(CgScalars), cudaMemcpyDeviceToHost, s);
+    return e1 != cudaSuccess ? e1 : cudaEventRecord(host.done[k & 1], s);
   };
-  *iterations = 0;
-  *rel_residual = 0.0;
-  if (n == 0) return cudaSuccess;
-  if (jacobi) inv_diag_kernel<<<gw, 256, 0, s>>>(A, inv_diag);
-  spmv_sym_kernel<<<gw, 256, 0, s>>>(A, x, r);
-  cg_init_kernel<<<gv, 256, 0, s>>>(n, b, r, z, p, jacobi ? inv_diag : nullptr);
-  dot(r, z, sc + 0);
-  dot(b, b, sc + 4);
-  double host[2] = {0.0, 0.0};
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  if ((e = cudaMemcpyAsync(&host[1], sc + 4, sizeof(double), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
-  if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-  const double bnorm = std::sqrt(host[1]);
-  if (bnorm == 0.0) {
-    cudaMemsetAsync(x, 0, sizeof(double) * size_t(n), s);
-    return cudaGetLastError();
-  }
-  int it = 0;
-  for (; it < max_iter;) {
-    spmv_sym_kernel<<<gw, 256, 0, s>>>(A, p, Ap);
-    dot(p, Ap, sc + 1);
-    cg_update_kernel<<<gv, 256, 0, s>>>(n, sc, x, r, z, p, Ap, jacobi ? inv_diag : nullptr);
-    ++it;
-    if (it % check_every == 0 || it == max_iter) {
-      dot(r, r, sc + 3);
-      if ((e = cudaMemcpyAsync(&host[0], sc + 3, sizeof(double), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
-      if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-      *rel_residual = std::sqrt(host[0]) / bnorm;
-      if (*rel_residual <= rtol) break;
+  auto scalars = [&](int k, CgScalars* out) {
+    const cudaError_t e1 = cudaEventSynchronize(host.done[k & 1]);
+    if (e1 == cudaSuccess) memcpy(out, static_cast<char*>(host.pinned) + (k & 1) * PcgHost::SLOT, sizeof(CgScalars));
+    return e1;
+  };
+  CgScalars st;
+  int it = 0, batch = 0;
+  while (it < max_iter) {
+    const int end = max_iter - it < check_every ? max_iter : it + check_every;
+    while (it < end) {
+      const int par = it & 1;
+      if ((e = launch_next(cg_product_kernel, gm, ROWS_SMEM, s, A, p, y, part_py, sc)) != cudaSuccess) return e;
+      if ((e = launch_next(cg_update_kernel, gv, 0, s, n, sc, par, part_py, int(gm), x, r, z, p, y, inv_diag, part_rz,
+                           part_rr)) != cudaSuccess)
+        return e;
+      ++it;
+      if (it == end && (e = launch_next(cg_test_kernel, 1u, 0, s, sc, part_rr, int(gv), it, rtol)) != cudaSuccess)
+        return e;
+      if ((e = launch_next(cg_direction_kernel, gv, 0, s, n, sc, par, part_rz, int(gv), z, p)) != cudaSuccess) return e;
     }
-    dot(r, z, sc + 2);
-    cg_direction_kernel<<<gv, 256, 0, s>>>(n, sc, z, p);
-    copy_scalar_kernel<<<1, 1, 0, s>>>(sc);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = read_back(batch)) != cudaSuccess) return e;
+    if (batch > 0) {  // the test of the batch before, while this one runs
+      if ((e = scalars(batch - 1, &st)) != cudaSuccess) return e;
+      if (st.done) break;
+    }
+    ++batch;
   }
-  *iterations = it;
-  return cudaGetLastError();
+  // (after a break the batch just enqueued changed nothing)
+  if ((e = cudaMemcpyAsync(host.pinned, sc, sizeof(CgScalars), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+  if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+  memcpy(&st, host.pinned, sizeof st);
+  if (st.bb == 0.0) {  // x = 0 solves it
+    *iterations = 0;
+    *rel_residual = 0.0;
+    return cudaMemsetAsync(x, 0, sizeof(double) * size_t(n), s);
+  }
+  *iterations = st.it;
+  *rel_residual = max_iter > 0 ? std::sqrt(st.rr) / std::sqrt(st.bb) : 0.0;
+  return cudaSuccess;
 }
 
 }  // namespace fec

@@ -14,12 +14,21 @@ struct CscSym {
   const double* val;      // nnz
 };
 
+// Page-locked memory and events a solve reads its stopping test through; kept by
+// the caller between solves (one solve at a time).
+struct PcgHost {
+  static constexpr size_t SLOT = 64;
+  void* pinned = nullptr;
+  cudaEvent_t done[2] = {nullptr, nullptr};
+  cudaError_t ensure();
+  void release();
+};
+
 size_t pcg_scratch_doubles(int64_t n);
-cudaError_t spmv_sym(const CscSym& A, const double* x, double* y, cudaStream_t s);
 // Conjugate gradients for A x = b from the x passed in (Jacobi-preconditioned if
-// asked); stops when ||b - A x|| <= rtol ||b|| (checked every check_every
-// iterations) or after max_iter.  Synchronises the stream at the checks.
+// asked); stops when ||b - A x|| <= rtol ||b|| (tested every check_every
+// iterations) or after max_iter.  Synchronises the stream.
 cudaError_t pcg(const CscSym& A, const double* b, double* x, double* scratch, int max_iter, double rtol,
-                int check_every, bool jacobi, int* iterations, double* rel_residual, cudaStream_t s);
+                int check_every, bool jacobi, PcgHost& host, int* iterations, double* rel_residual, cudaStream_t s);
 
 }  // namespace fec
