@@ -55,6 +55,7 @@ struct Block {
   // within 1e-13 of the element size): x0 = the first element's coordinates
   bool congruent = false;
   double x0[24] = {0};
+  bool tensor_rule = false;  // hex8: the reference tables are a symmetric 2x2x2 rule's (hex8_tensor_rule)
   // tet10/hex27 block whose element e is a translate of element e mod nclass
   // (nclass <= 8, 0: none): xc = the first nclass elements' node coordinates
   int nclass = 0;
@@ -173,7 +174,9 @@ int build_affine(fec_ctx* c, size_t b) {
   if (c->d_affine.size() != c->blocks.size()) c->d_affine.resize(c->blocks.size());
   DevBuf& d = c->d_affine[b];
   d.release();
-  const Block& B = c->blocks[b];
+  Block& B = c->blocks[b];
+  double t[3];
+  B.tensor_rule = B.elem_type == FEC_HEX8 && fec::hex8_tensor_rule(c->ref_host.data() + c->ref_off[b], t);
   if (c->device < 0) return FEC_OK;
   std::vector<unsigned char> tab;
   if (B.congruent) {
@@ -189,13 +192,19 @@ int build_affine(fec_ctx* c, size_t b) {
 
 // The table a launch of block b may use: FP64 assemblies of congruent hex8
 // blocks on their own launch (the single launch across blocks keeps the
-// per-element kernels), unless FEC_HEX8_AFFINE=0.
+// per-element kernels), unless FEC_HEX8_AFFINE=0.  The mechanics kernel also
+// wants the tables of a symmetric rule; `gradients`: a kernel that only reads the
+// block's gradients and JxW (Poisson, the action) takes any.
 // Assemblies of tet10/hex27 blocks of translation classes get theirs: FP32-element
 // and FP64 (tet10: the tensor-core kernels; hex27 FP64: the class gradients).
-const void* affine_table(const fec_ctx* c, size_t b, int precision, bool mixed) {
+const void* affine_table(const fec_ctx* c, size_t b, int precision, bool mixed, bool gradients = false) {
   if (mixed || b >= c->d_affine.size()) return nullptr;
-  if (c->blocks[b].elem_type == FEC_HEX8)
-    return precision == FEC_FP64 && fec::hex8_affine_enabled() ? c->d_affine[b].p : nullptr;
+  const Block& B = c->blocks[b];
+  if (B.elem_type == FEC_HEX8)
+    return precision == FEC_FP64 && fec::hex8_affine_enabled() &&
+                   (B.tensor_rule || gradients || B.physics == FEC_PHYS_POISSON)
+               ? c->d_affine[b].p
+               : nullptr;
   return (precision == FEC_FP32_ELEMENT || precision == FEC_FP64) ? c->d_affine[b].p : nullptr;
 }
 
@@ -1282,7 +1291,7 @@ int fec_assemble_action(fec_ctx* c, int precision, double t, double dt, const do
     ea.Re = static_cast<char*>(c->d_Re.p) + rsz * size_t(re_off);
     // FP64 blocks of translated hex8 elements: the block's constant gradients and JxW
     if (B.elem_type == FEC_HEX8 && precision == FEC_FP64 && B.congruent)
-      if (const void* tab = affine_table(c, b, precision, false))
+      if (const void* tab = affine_table(c, b, precision, false, true))
         ea.affine = static_cast<const unsigned char*>(tab) + fec::hex8_affine_grad_offset();
     cudaError_t e;
     {

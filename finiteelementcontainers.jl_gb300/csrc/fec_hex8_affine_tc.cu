@@ -67,18 +67,20 @@ constexpr int T_W = 0;
 constexpr int T_SIG = ND * W_SLICE;
 constexpr int T_G = T_SIG + NPAD * 4;
 constexpr int T_JXW = T_G + NQ * 24 * 8;
-constexpr int T_BYTES = T_JXW + NQ * 8;
+constexpr int T_TEN = T_JXW + NQ * 8;           // TEN_N doubles, see tensor_gradient
+constexpr int TEN_N = 10 + 2 + NQ * 9;          // coefficients, diagonal flag (+ pad), Ji [q][k][j]
+constexpr int T_BYTES = T_TEN + TEN_N * 8;
 static_assert(T_BYTES % 16 == 0 && T_G % 8 == 0, "table layout");
 constexpr int TMEM_COLS = 512;
 constexpr int TM_ENT = NLEV * NPAD;  // 2 x 48 columns after the accumulators: the slicers' scaled tangent entries (hi, lo)
 static_assert(TM_ENT + 2 * 48 <= TMEM_COLS, "tensor memory columns");
 constexpr long long WAIT_BUDGET = 2000000000LL;
 
-constexpr int PROD_W = 3, SL_W = 6, R_W = 1, EP_W = 4, MMA_W = 1;
+constexpr int PROD_W = 3, SL_W = 6, R_W = 2, EP_W = 4, MMA_W = 1;
 constexpr int NTHR = 32 * (PROD_W + SL_W + R_W + EP_W + MMA_W);
 constexpr int T_SL = 32 * PROD_W, T_R = T_SL + 32 * SL_W, T_EP = T_R + 32 * R_W, T_MMA = T_EP + 32 * EP_W;
 constexpr int NSL = 32 * SL_W;
-static_assert(32 * PROD_W == NPT && NSL == 2 * NPT && (T_EP / 32) % 4 == 2, "roles");
+static_assert(32 * PROD_W == NPT && NSL == 2 * NPT, "roles");
 // named barriers (0 is __syncthreads)
 constexpr int BAR_FULL = 1;   // producers arrive, slicers + residual warp sync
 constexpr int BAR_EMPTY = 2;  // slicers + residual warp arrive, producers sync
@@ -95,14 +97,119 @@ __device__ __constant__ int8_t kGroups[NGROUP][3] = {{0, 0, 4}, {0, 4, 3}, {1, 0
 // MMA row of (element el of the tile, ik = 3 i + k)
 __host__ __device__ __forceinline__ int row_of(int el, int ik) { return 32 * (el / 3) + 9 * (el % 3) + ik; }
 
+// The Neo-Hookean update as the tensor-core kernel takes it: with H = F^-T and
+//   Z = a1/2 H - 2/3 c2 F,   Y = a2 H,
+// the tangent entry is three products, A_iJkL = H_iJ Z_kL + Z_iJ H_kL + Y_iL H_kJ
+// + c2 d_ik d_JL, and the stress P = c2 F - Y (a1, a2, c2 times JxW; see
+// NeoHookean).  The slicers' entries were four products of products: a third of
+// the FP32 instructions.  Every product that feeds a sum is an explicit FMA or
+// rounded on its own, so the residual-only kernel gives the same bits.
+struct AffNeoHookean {
+  static constexpr int NS = 0, SCR2 = 28;  // H, Z, Y, c2
+  struct Mid {
+    double F[9], H[9], a1h, a2, c2;
+  };
+  // J^(-1/3): CUDA's FP32 rcbrtf and one third-order step from the expansion of
+  // (1 - e)^(-1/3), e = 1 - J r^3 (e is below 2^-20, the dropped term below
+  // 2^-62); the library function outside FP32's range.
+  __device__ static double inv_cbrt(double J) {
+    if (!(J > 1e-30 && J < 1e30)) return rcbrt(J);
+    const double r = double(rcbrtf(float(J)));
+    const double e = fma(-J * r, r * r, 1.0);
+    return fma(r * e, fma(e, 2.0 / 9.0, 1.0 / 3.0), r);
+  }
+  __device__ static void point(const double* props, const double (&gu)[3][3], double jxw, const double*, double*,
+                               Mid& m) {
+    const double Kj = props[0] * jxw, Gj = props[1] * jxw;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) m.F[i] = gu[i / 3][i % 3] + (i % 4 == 0 ? 1.0 : 0.0);
+    const double* F = m.F;
+    double c[9];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {  // cofactors (cyclic indices: no signs)
+        const int i1 = (i + 1) % 3, i2 = (i + 2) % 3, j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+        c[i * 3 + j] = fma(F[i1 * 3 + j1], F[i2 * 3 + j2], -mul_rn(F[i1 * 3 + j2], F[i2 * 3 + j1]));
+      }
+    const double J = fma(F[0], c[0], fma(F[1], c[1], mul_rn(F[2], c[2])));
+    const double rJ = 1.0 / J;
+    double I1 = mul_rn(F[0], F[0]);
+#pragma unroll
+    for (int i = 1; i < 9; ++i) I1 = fma(F[i], F[i], I1);
+    const double r3 = inv_cbrt(J);
+    const double I13 = mul_rn(I1, 1.0 / 3.0);
+    const double JJ = mul_rn(J, J), d = JJ - J;
+    m.c2 = mul_rn(mul_rn(r3, r3), Gj);
+    m.a2 = fma(m.c2, I13, -mul_rn(0.5 * Kj, d - 1.0));
+    m.a1h = fma(m.c2, mul_rn(I13, 1.0 / 3.0), mul_rn(0.25 * Kj, JJ + d));
+#pragma unroll
+    for (int i = 0; i < 9; ++i) m.H[i] = mul_rn(c[i], rJ);
+  }
+  __device__ static void stress(const Mid& m, float2* P) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) P[i] = df64_split(fma(m.c2, m.F[i], -mul_rn(m.a2, m.H[i])));
+  }
+  // the point's split stress and tangent scratch; returns a bound of |A_iJkL|
+  __device__ static float stage(const Mid& m, float2* P, float2* scr) {
+    const double m23 = mul_rn(-2.0 / 3.0, m.c2);
+    float hm = 0.f, zm = 0.f, ym = 0.f;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      const double y = mul_rn(m.a2, m.H[i]);
+      const float2 h = df64_split(m.H[i]), z = df64_split(fma(m23, m.F[i], mul_rn(m.a1h, m.H[i]))), ys = df64_split(y);
+      P[i] = df64_split(fma(m.c2, m.F[i], -y));
+      scr[i] = h;
+      scr[9 + i] = z;
+      scr[18 + i] = ys;
+      hm = fmaxf(hm, fabsf(h.x));
+      zm = fmaxf(zm, fabsf(z.x));
+      ym = fmaxf(ym, fabsf(ys.x));
+    }
+    const float2 c = df64_split(m.c2);
+    scr[27] = c;
+    return (2.f * zm + ym) * hm + fabsf(c.x);
+  }
+  __device__ static float2 entry(const float2* s, int i, int J, int k, int L) {
+    const float2* Z = s + 9;
+    const float2* Y = s + 18;
+    float2 v = df64_dot3(s[i * 3 + J], Z[k * 3 + L], Z[i * 3 + J], s[k * 3 + L], Y[i * 3 + L], s[k * 3 + J]);
+    if (i == k && J == L) v = df64_add(v, s[27]);
+    return v;
+  }
+};
+
+struct AffJ2 {
+  static constexpr int NS = J2::NS, SCR2 = J2::SCR2;
+  struct Mid {
+    double P[9], scr[J2::SCR];
+  };
+  __device__ static void point(const double* props, double (&gu)[3][3], double jxw, const double* so, double* sn,
+                               Mid& m) {
+    J2::point(props, gu, jxw, so, sn, m.P, m.scr);
+  }
+  __device__ static void stress(const Mid& m, float2* P) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) P[i] = df64_split(m.P[i]);
+  }
+  __device__ static float stage(const Mid& m, float2* P, float2* scr) {
+    stress(m, P);
+    J2::split_scratch(m.scr, scr);
+    return J2::abound(scr);
+  }
+  __device__ static float2 entry(const float2* s, int i, int J, int k, int L) {
+    return J2::aentry_df64(s, i, J, k, L);
+  }
+};
+
 template <class Model>
 struct Layout {
   static constexpr int W = 0;
   static constexpr int A = W + ND * W_SLICE;
   static constexpr int P = A + ND * A_SLICE;                      // float2 [96][9]
   static constexpr int SCR = P + NPT * 9 * 8;                     // float2 [96][SCR2]
-  static constexpr int G = (SCR + NPT * Model::SCR2 * 8 + 15) / 16 * 16;  // double [8][24]
-  static constexpr int G2 = G + NQ * 24 * 8;                      // float2 [8][24]
+  static constexpr int TEN = (SCR + NPT * Model::SCR2 * 8 + 15) / 16 * 16;  // double [TEN_N]
+  static constexpr int G2 = TEN + TEN_N * 8;                      // float2 [8][24]
   static constexpr int JXW = G2 + NQ * 24 * 8;                    // double [8]
   static constexpr int SIG = JXW + NQ * 8;                        // int [48]
   static constexpr int TAU = SIG + NPAD * 4;                      // int [2][12]: per tile parity
@@ -172,53 +279,81 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 
-// Point phase of quadrature point q of element e (FP64): the eight lanes of an
-// element (consecutive, aligned to 8) each load one node's displacement and
-// share it; gu = sum_a u_a (x) dNX_qa; the constitutive update.  Every lane of
-// the warp calls it (the shuffles); `live` lanes get P9 and scr.
-template <class Model>
-__device__ __forceinline__ void point_phase(const ElemArgs& g, const double* s_g, const double* s_jxw, int64_t e, int q,
-                                            bool live, double* P9, double* scr) {
-  const int lane = threadIdx.x & 31;
-  double uo[3] = {0.0, 0.0, 0.0};
-  if (live) {
-    const int64_t node = g.conn[e * 8 + q];
+// Node of an element at the corner in point q's octant (bits x, y, z of q).
+__device__ __forceinline__ int corner_node(int q) { return q ^ ((q >> 1) & 1); }
+
+// -d where the bit is clear
+__device__ __forceinline__ double signed_by(double d, unsigned bit) {
+  return __hiloint2double(__double2hiint(d) ^ int(bit ? 0u : 0x80000000u), __double2loint(d));
+}
+
+// Gradient at point q of the nodal values of an element, shared by its eight
+// lanes (consecutive, aligned to 8): lane q holds v = the value at corner q minus
+// node 0's.  The point rule is symmetric (points at -t_d, t_d per direction), so a
+// trilinear value is interpolated (I) or differenced (D) one direction at a time,
+// the other value coming from the lane across: gx = I_z I_y D_x v, gy = I_z D_y
+// I_x v, gz = D_z I_y I_x v.  13 FP64 operations per component instead of the 24 of
+// sum_a v_a dN_a, which is what counts: the FP64 pipe takes a sub-partition 64
+// clocks per warp instruction.  Differences of values come first, so the
+// result is no further from the exact gradient.  co: I_x (own, across), I_y, then
+// I_y, I_z, I_z with the scales of gz, gy, gx folded in.
+__device__ __forceinline__ void tensor_gradient(const double* co, int q, const double (&v)[3], double (&g)[3][3]) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) uo[d] = __ldg(&g.U[node * 3 + d]);
+  for (int i = 0; i < 3; ++i) {
+    const double vx = __shfl_xor_sync(0xffffffffu, v[i], 1);
+    const double A = fma(co[0], v[i], mul_rn(co[1], vx)), B = signed_by(v[i] - vx, q & 1);
+    const double Ay = __shfl_xor_sync(0xffffffffu, A, 2), By = __shfl_xor_sync(0xffffffffu, B, 2);
+    const double C = fma(co[4], A, mul_rn(co[5], Ay)), D = signed_by(A - Ay, q & 2);
+    const double E = fma(co[2], B, mul_rn(co[3], By));
+    const double Cz = __shfl_xor_sync(0xffffffffu, C, 4), Dz = __shfl_xor_sync(0xffffffffu, D, 4),
+                 Ez = __shfl_xor_sync(0xffffffffu, E, 4);
+    g[i][0] = fma(co[8], E, mul_rn(co[9], Ez));
+    g[i][1] = fma(co[6], D, mul_rn(co[7], Dz));
+    g[i][2] = signed_by(C - Cz, q & 4);
   }
-  double gu[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-  const double* gq = s_g + q * 24;
+}
+
+// Point phase of quadrature point q of element e (FP64): the displacement gradient
+// and the constitutive update.  Every lane of the warp calls it (the shuffles);
+// uo: the displacement of the lane's corner node (0 where not live).
+template <class Model>
+__device__ __forceinline__ void point_phase(const ElemArgs& g, const double* s_ten, const double* s_jxw, int64_t e,
+                                            int q, bool live, const double (&uo)[3], typename Model::Mid& m) {
+  const int lane = threadIdx.x & 31;
+  double st[Model::NS ? Model::NS : 1];
+  double* sn = nullptr;
+  if (Model::NS && live) {  // (the state on its way during the gradient)
+    const double* so = g.state_old + (e * NQ + q) * Model::NS;
 #pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const int src = (lane & ~7) | a;
-    const double u0 = __shfl_sync(0xffffffffu, uo[0], src), u1 = __shfl_sync(0xffffffffu, uo[1], src),
-                 u2 = __shfl_sync(0xffffffffu, uo[2], src);
+    for (int k = 0; k < Model::NS; ++k) st[k] = so[k];
+    if (g.state_new) sn = g.state_new + (e * NQ + q) * Model::NS;
+  }
+  double v[3], gu[3][3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const double gj = gq[a * 3 + j];
-      gu[0][j] = fma(u0, gj, gu[0][j]);
-      gu[1][j] = fma(u1, gj, gu[1][j]);
-      gu[2][j] = fma(u2, gj, gu[2][j]);
+  for (int d = 0; d < 3; ++d) v[d] = uo[d] - __shfl_sync(0xffffffffu, uo[d], lane & ~7);
+  tensor_gradient(s_ten, q, v, gu);
+  if (s_ten[10] == 0.0) {  // not an axis-aligned box: reference gradient times dxi/dX
+    const double* Ji = s_ten + 12 + q * 9;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double r0 = gu[i][0], r1 = gu[i][1], r2 = gu[i][2];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) gu[i][j] = fma(r0, Ji[j], fma(r1, Ji[3 + j], mul_rn(r2, Ji[6 + j])));
     }
   }
-  if (live) {
-    const double* so = Model::NS ? g.state_old + (e * NQ + q) * Model::NS : nullptr;
-    double* sn = (Model::NS && g.state_new) ? g.state_new + (e * NQ + q) * Model::NS : nullptr;
-    Model::point(g.props, gu, s_jxw[q], so, sn, P9, scr);
-  }
+  if (live) Model::point(g.props, gu, s_jxw[q], st, sn, m);
 }
 
 // node pair n = (a, b), a <= b, as a << 4 | b
 __constant__ unsigned char kPairNodes[NPAIR] = {0x00, 0x01, 0x02, 0x03, 0x04, 0x05, 0x06, 0x07, 0x11, 0x12, 0x13, 0x14, 0x15, 0x16, 0x17, 0x22, 0x23, 0x24, 0x25, 0x26, 0x27, 0x33, 0x34, 0x35, 0x36, 0x37, 0x44, 0x45, 0x46, 0x47, 0x55, 0x56, 0x57, 0x66, 0x67, 0x77};
 
-// sum_L v_L[j] 2^(-8L) of the seven level accumulators of one pair: levels 6..4
-// in FP32 (their rounding is below 2^-55 of level 0), then 3..0 in double-float
+// The sum of the seven level accumulators of one pair: levels 6..4 in FP32 (their
+// rounding is below 2^-55 of level 0), then 3..0 in double-float
 __device__ __forceinline__ float2 combine_levels(const float (&v)[NLEV][4], int j) {
-  float hi = fmaf(fmaf(v[6][j], 0.00390625f, v[5][j]), 0.00390625f, v[4][j]), lo = 0.f;
+  float hi = (v[6][j] + v[5][j]) + v[4][j], lo = 0.f;
 #pragma unroll
   for (int L = 3; L >= 0; --L) {
-    const float a = v[L][j], b = hi * 0.00390625f;
-    lo *= 0.00390625f;
+    const float a = v[L][j], b = hi;
     const float s = a + b, bb = s - a;
     lo += (a - (s - bb)) + (b - bb);
     hi = s + lo;
@@ -247,7 +382,7 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
   extern __shared__ __align__(1024) unsigned char sm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t s0 = smem_u32(sm);
-  double* s_g = reinterpret_cast<double*>(sm + Lay::G);
+  double* s_ten = reinterpret_cast<double*>(sm + Lay::TEN);
   float2* s_g2 = reinterpret_cast<float2*>(sm + Lay::G2);
   double* s_jxw = reinterpret_cast<double*>(sm + Lay::JXW);
   int* s_sig = reinterpret_cast<int*>(sm + Lay::SIG);
@@ -265,11 +400,9 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
     reinterpret_cast<uint4*>(sm + Lay::A)[i] = make_uint4(0u, 0u, 0u, 0u);
   for (int i = tid; i < ND * W_SLICE / 16; i += NTHR)
     reinterpret_cast<uint4*>(sm + Lay::W)[i] = __ldg(reinterpret_cast<const uint4*>(tab + T_W) + i);
-  for (int i = tid; i < NQ * 24; i += NTHR) {
-    const double v = __ldg(reinterpret_cast<const double*>(tab + T_G) + i);
-    s_g[i] = v;
-    s_g2[i] = df64_split(v);
-  }
+  for (int i = tid; i < NQ * 24; i += NTHR)
+    s_g2[i] = df64_split(__ldg(reinterpret_cast<const double*>(tab + T_G) + i));
+  for (int i = tid; i < TEN_N; i += NTHR) s_ten[i] = __ldg(reinterpret_cast<const double*>(tab + T_TEN) + i);
   if (tid < NQ) s_jxw[tid] = __ldg(reinterpret_cast<const double*>(tab + T_JXW) + tid);
   if (tid < NPAD) s_sig[tid] = __ldg(reinterpret_cast<const int*>(tab + T_SIG) + tid);
   if (tid < 45) {
@@ -310,22 +443,32 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
   if (tid < T_SL) {
     // ---------------- producers: thread (el, q) ----------------
     const int el = tid >> 3, q = tid & 7;
+    // the nodes of tile k+1 and the displacements of tile k+1 are fetched while tile
+    // k is computed (a load latency each, once per tile)
+    auto node_of = [&](int64_t tile) {
+      const int64_t e = tile * EPT + el;
+      return tile < ntiles && e < g.ne ? g.conn[e * 8 + corner_node(q)] : -1;
+    };
+    double un[3] = {0.0, 0.0, 0.0};
+    auto fetch = [&](int node) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) un[d] = node >= 0 ? __ldg(&g.U[int64_t(node) * 3 + d]) : 0.0;
+    };
+    fetch(node_of(blockIdx.x));
+    int next = node_of(blockIdx.x + int64_t(gridDim.x));
     for (int k = 0;; ++k) {
       const int64_t tile = blockIdx.x + int64_t(k) * gridDim.x;
       if (tile >= ntiles) break;
       const int64_t e = tile * EPT + el;
       const bool live = e < g.ne;
-      double P9[9], scr[Model::SCR];
-      point_phase<Model>(g, s_g, s_jxw, e, q, live, P9, scr);
+      const double uo[3] = {un[0], un[1], un[2]};
+      fetch(next);
+      next = node_of(tile + 2 * int64_t(gridDim.x));
+      typename Model::Mid mid;
+      point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
       if (k >= 1) named_sync(BAR_EMPTY, N_FULL);  // tile k-1's staging has been read
       float bnd = 0.f;
-      if (live) {
-        float2* pP = s_P + tid * 9;
-#pragma unroll
-        for (int m = 0; m < 9; ++m) pP[m] = df64_split(P9[m]);
-        Model::split_scratch(scr, s_scr + tid * SCR2);
-        bnd = Model::abound(s_scr + tid * SCR2) * 1.0001f;
-      }
+      if (live) bnd = Model::stage(mid, s_P + tid * 9, s_scr + tid * SCR2) * 1.0001f;
       // the element's scale 2^tau > |every tangent entry| (its eight points are
       // lanes 8j .. 8j+7 of this warp)
 #pragma unroll
@@ -361,9 +504,9 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
         const uint32_t code0 = s_code[w0 + (c < cnt ? c : 0)], code1 = s_code[w0 + (c1 < cnt ? c1 : 0)];
         float2 a0 = make_float2(0.f, 0.f), a1 = a0;
         if (live && c < cnt)
-          a0 = Model::aentry_df64(sc, code0 & 15, (code0 >> 4) & 15, (code0 >> 8) & 15, (code0 >> 12) & 15);
+          a0 = Model::entry(sc, code0 & 15, (code0 >> 4) & 15, (code0 >> 8) & 15, (code0 >> 12) & 15);
         if (live && c1 < cnt)
-          a1 = Model::aentry_df64(sc, code1 & 15, (code1 >> 4) & 15, (code1 >> 8) & 15, (code1 >> 12) & 15);
+          a1 = Model::entry(sc, code1 & 15, (code1 >> 4) & 15, (code1 >> 8) & 15, (code1 >> 12) & 15);
         tmem_st2(ent + uint32_t(2 * c), a0.x * fs, a0.y * fs);
         if (c + 1 < 23) tmem_st2(ent + uint32_t(2 * c + 2), a1.x * fs, a1.y * fs);
       }
@@ -386,12 +529,20 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
           unsigned char* p2 = As + op_off(rbase + int((code >> 24) & 15), q * 9 + int(code >> 28));
           const bool twin = p1 != p2;
           float xh = x[2 * j], xl = x[2 * j + 1];
+          // digit s: the part of x at or above 2^(-8s), by adding and subtracting
+          // 1.5 2^(23-8s) (a rounding instruction issues at an eighth of the rate);
+          // |xl| <= ulp(xh) / 2 <= 2^-18 has no digits before the third
 #pragma unroll
           for (int s = 0; s < ND; ++s) {
-            const float dh = rintf(xh), dl = rintf(xl);
-            xh = (xh - dh) * 256.f;
-            xl = (xl - dl) * 256.f;
-            const unsigned short bits = static_cast<unsigned short>(__float_as_uint(dh + dl) >> 16);
+            const float big = pow2f(23 - 8 * s) * 1.5f;
+            float d = __fsub_rn(__fadd_rn(xh, big), big);
+            xh = __fsub_rn(xh, d);
+            if (s >= 3) {
+              const float dl = __fsub_rn(__fadd_rn(xl, big), big);
+              xl = __fsub_rn(xl, dl);
+              d = __fadd_rn(d, dl);
+            }
+            const unsigned short bits = static_cast<unsigned short>(__float_as_uint(d) >> 16);
             *reinterpret_cast<unsigned short*>(p1 + s * A_SLICE) = bits;
             if (twin) *reinterpret_cast<unsigned short*>(p2 + s * A_SLICE) = bits;
           }
@@ -401,16 +552,17 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
       mbar_arrive(bar_sl);
     }
   } else if (tid < T_EP) {
-    // ---------------- residual warp ----------------
+    // ---------------- residual warps ----------------
     for (int k = 0;; ++k) {
       const int64_t tile = blockIdx.x + int64_t(k) * gridDim.x;
       if (tile >= ntiles) break;
       named_sync(BAR_FULL, N_FULL);
       if (WANT_R) {
-        static_assert(EPT * 24 % 32 == 0, "residual entries per lane");
-#pragma unroll 3
-        for (int j = 0; j < EPT * 24 / 32; ++j) {
-          const int idx = lane + 32 * j, el = idx / 24, ai = idx % 24;
+        constexpr int RT = 32 * R_W, NE = (EPT * 24 + RT - 1) / RT;
+#pragma unroll
+        for (int j = 0; j < NE; ++j) {
+          const int idx = tid - T_R + RT * j, el = idx / 24, ai = idx % 24;
+          if (idx >= EPT * 24) break;
           const int64_t e = tile * EPT + el;
           const double r = residual_entry(s_g2, s_P + el * NQ * 9, ai / 3, ai % 3);
           if (e < g.ne) static_cast<double*>(g.Re)[e * 24 + ai] = r;
@@ -514,24 +666,25 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
 constexpr int R_EPB = 16;
 template <class Model>
 __global__ void __launch_bounds__(R_EPB * NQ) hex8_affine_r_kernel(ElemArgs g, const unsigned char* __restrict__ tab) {
-  __shared__ double s_g[NQ * 24], s_jxw[NQ];
+  __shared__ double s_ten[TEN_N], s_jxw[NQ];
   __shared__ float2 s_g2[NQ * 24], s_P[R_EPB * NQ * 9];
   const int tid = threadIdx.x, el = tid >> 3, q = tid & 7;
-  for (int i = tid; i < NQ * 24; i += blockDim.x) {
-    const double v = __ldg(reinterpret_cast<const double*>(tab + T_G) + i);
-    s_g[i] = v;
-    s_g2[i] = df64_split(v);
-  }
+  for (int i = tid; i < NQ * 24; i += blockDim.x)
+    s_g2[i] = df64_split(__ldg(reinterpret_cast<const double*>(tab + T_G) + i));
+  for (int i = tid; i < TEN_N; i += blockDim.x) s_ten[i] = __ldg(reinterpret_cast<const double*>(tab + T_TEN) + i);
   if (tid < NQ) s_jxw[tid] = __ldg(reinterpret_cast<const double*>(tab + T_JXW) + tid);
   __syncthreads();
   const int64_t e0 = int64_t(blockIdx.x) * R_EPB, e = e0 + el;
   const bool live = e < g.ne;
-  double P9[9], scr[Model::SCR];
-  point_phase<Model>(g, s_g, s_jxw, e, q, live, P9, scr);
+  double uo[3] = {0.0, 0.0, 0.0};
   if (live) {
+    const int64_t node = g.conn[e * 8 + corner_node(q)];
 #pragma unroll
-    for (int m = 0; m < 9; ++m) s_P[tid * 9 + m] = df64_split(P9[m]);
+    for (int d = 0; d < 3; ++d) uo[d] = __ldg(&g.U[node * 3 + d]);
   }
+  typename Model::Mid mid;
+  point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
+  if (live) Model::stress(mid, s_P + tid * 9);
   __syncthreads();
   for (int idx = tid; idx < R_EPB * 24; idx += blockDim.x) {
     const int ee = idx / 24, ai = idx % 24;
@@ -584,14 +737,59 @@ cudaError_t launch_hex8_affine_tc(int physics, bool want_r, bool want_k, const E
   if (!a.affine || (want_k && !a.Ke) || (want_r && !a.Re)) return cudaErrorInvalidValue;
   if (!want_k) {
     if (!want_r) return cudaSuccess;
-    if (physics == 2) return aff::launch_r<NeoHookean>(a, s, launches);
-    if (physics == 3) return aff::launch_r<J2>(a, s, launches);
+    if (physics == 2) return aff::launch_r<aff::AffNeoHookean>(a, s, launches);
+    if (physics == 3) return aff::launch_r<aff::AffJ2>(a, s, launches);
     return cudaErrorNotSupported;
   }
   if (physics == 2)
-    return want_r ? aff::launch1<NeoHookean, true>(a, s, launches) : aff::launch1<NeoHookean, false>(a, s, launches);
-  if (physics == 3) return want_r ? aff::launch1<J2, true>(a, s, launches) : aff::launch1<J2, false>(a, s, launches);
+    return want_r ? aff::launch1<aff::AffNeoHookean, true>(a, s, launches) : aff::launch1<aff::AffNeoHookean, false>(a, s, launches);
+  if (physics == 3) return want_r ? aff::launch1<aff::AffJ2, true>(a, s, launches) : aff::launch1<aff::AffJ2, false>(a, s, launches);
   return cudaErrorNotSupported;
+}
+
+// Whether the reference tables are trilinear gradients at points (-+t_0, -+t_1,
+// -+t_2), x fastest (2 x 2 x 2 Gauss, Lobatto): c[d] = (1 + t_d) / 2 then.
+bool hex8_tensor_rule(const double* ref, double c[3]) {
+  using L = RefLayout<1>;
+  const double* dN = ref + L::DN_OFF;
+  auto corner = [](int a) { return a ^ ((a >> 1) & 1); };  // bits x, y, z of node a
+  for (int d = 0; d < 3; ++d) {
+    // at the last point, the derivative along k summed over the direction that is neither k nor d
+    const int k = (d + 1) % 3;
+    double s = 0.0;
+    for (int a = 0; a < 8; ++a)
+      if ((corner(a) >> d & 1) && (corner(a) >> k & 1)) s += dN[(7 * 8 + a) * 3 + k];
+    c[d] = 2.0 * s;
+  }
+  for (int q = 0; q < 8; ++q)
+    for (int a = 0; a < 8; ++a)
+      for (int k = 0; k < 3; ++k) {
+        double v = (corner(a) >> k & 1) ? 0.5 : -0.5;
+        for (int d = 0; d < 3; ++d)
+          if (d != k) v *= (corner(a) >> d & 1) == (q >> d & 1) ? c[d] : 1.0 - c[d];
+        if (!(std::fabs(v - dN[(q * 8 + a) * 3 + k]) <= 1e-15)) return false;
+      }
+  return true;
+}
+
+// Half the inverse edge lengths of an axis-aligned box in node order; false for
+// any other element (edges to 1e-13 of the largest, as in the congruence test).
+static bool box_scales(const double* x0, double sc[3]) {
+  double h = 0.0, len[3];
+  for (int d = 0; d < 3; ++d) {
+    len[d] = x0[6 * 3 + d] - x0[d];  // node 6 is opposite node 0
+    h = std::fmax(h, std::fabs(len[d]));
+  }
+  for (int a = 0; a < 8; ++a)
+    for (int d = 0; d < 3; ++d) {
+      const int bit = (a ^ ((a >> 1) & 1)) >> d & 1;
+      if (!(std::fabs(x0[a * 3 + d] - x0[d] - (bit ? len[d] : 0.0)) <= 1e-13 * h)) return false;
+    }
+  for (int d = 0; d < 3; ++d) {
+    if (!(len[d] > 0.0)) return false;
+    sc[d] = 1.0 / len[d];
+  }
+  return true;
 }
 
 // Host: the constant operand of a block whose elements are translates of its
@@ -602,7 +800,7 @@ cudaError_t launch_hex8_affine_tc(int physics, bool want_r, bool want_k, const E
 bool hex8_affine_table(const double* x0, const double* ref, std::vector<unsigned char>& out) {
   using L = RefLayout<1>;
   out.assign(aff::T_BYTES, 0);
-  double dNX[8][8][3], jxw[8];
+  double dNX[8][8][3], jxw[8], ten[aff::TEN_N] = {0.0};
   for (int q = 0; q < 8; ++q) {
     const double* dN = ref + L::DN_OFF + q * 24;
     double J[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
@@ -624,6 +822,8 @@ bool hex8_affine_table(const double* x0, const double* ref, std::vector<unsigned
     Ji[2][0] = c02 * r;
     Ji[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * r;
     Ji[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * r;
+    for (int k = 0; k < 3; ++k)
+      for (int d = 0; d < 3; ++d) ten[12 + q * 9 + k * 3 + d] = Ji[k][d];
     for (int a = 0; a < 8; ++a)
       for (int d = 0; d < 3; ++d) {
         double s = 0.0;
@@ -652,7 +852,7 @@ bool hex8_affine_table(const double* x0, const double* ref, std::vector<unsigned
         for (int s = 0; s < aff::ND; ++s) {
           const double d = std::nearbyint(y);
           y = (y - d) * 256.0;
-          const float fd = float(d);
+          const float fd = float(std::ldexp(d, -8 * s));  // digits at their place value
           uint32_t u;
           std::memcpy(&u, &fd, 4);
           const uint16_t bits = uint16_t(u >> 16);
@@ -660,6 +860,20 @@ bool hex8_affine_table(const double* x0, const double* ref, std::vector<unsigned
         }
       }
     }
+  // tensor_gradient's coefficients, with the scales dxi/dX folded in for a box
+  double cI[3] = {1.0, 1.0, 1.0}, sc[3];
+  hex8_tensor_rule(ref, cI);
+  const bool box = box_scales(x0, sc);
+  ten[10] = box ? 1.0 : 0.0;
+  if (!box) sc[0] = sc[1] = sc[2] = 0.5;
+  const double own[5] = {cI[0], cI[1], cI[1] * sc[2], cI[2] * sc[1], cI[2] * sc[0]};
+  const double across[5] = {1.0 - cI[0], 1.0 - cI[1], (1.0 - cI[1]) * sc[2], (1.0 - cI[2]) * sc[1],
+                            (1.0 - cI[2]) * sc[0]};
+  for (int k = 0; k < 5; ++k) {
+    ten[2 * k] = own[k];
+    ten[2 * k + 1] = across[k];
+  }
+  std::memcpy(out.data() + aff::T_TEN, ten, sizeof ten);
   std::memcpy(out.data() + aff::T_SIG, sig, sizeof sig);
   std::memcpy(out.data() + aff::T_G, dNX, sizeof dNX);
   std::memcpy(out.data() + aff::T_JXW, jxw, sizeof jxw);

@@ -76,6 +76,10 @@ cudaError_t launch_hex8_affine_tc(int physics, bool want_r, bool want_k, const E
 // Host: that table from the first element's node coordinates x0[8][3] and the
 // block's reference tables (RefLayout<1>); false for a degenerate element.
 bool hex8_affine_table(const double* x0, const double* ref, std::vector<unsigned char>& out);
+// Host: whether a hex8 block's reference tables are trilinear gradients at the
+// points (-+t_0, -+t_1, -+t_2) of a symmetric 2 x 2 x 2 rule (that kernel's point
+// phase); c[d] = (1 + t_d) / 2 then.
+bool hex8_tensor_rule(const double* ref, double c[3]);
 // FEC_HEX8_AFFINE=0 keeps such blocks on the per-element kernels.
 bool hex8_affine_enabled();
 // Byte offset, in that table, of the block's spatial gradients dNX [8 points][8
