@@ -55,7 +55,7 @@ namespace aff {
 constexpr int EPT = 12;              // elements per tile (three per 32-row quarter)
 constexpr int NQ = 8;
 constexpr int NPT = EPT * NQ;        // quadrature points per tile (96)
-constexpr int KR = 72, KP = 80;      // reduction length r = (q, J, L), padded to 5 K steps
+constexpr int KR = 72, KP = 80;      // reduction length r = (J, L, q), q fastest, padded to 5 K steps
 constexpr int NPAIR = 36, NPAD = 48; // node pairs a <= b, padded N
 constexpr int ND = 7;                // digits per operand
 constexpr int NLEV = 7;              // accumulated levels s + t = 0..6
@@ -97,15 +97,17 @@ __device__ __constant__ int8_t kGroups[NGROUP][3] = {{0, 0, 4}, {0, 4, 3}, {1, 0
 // MMA row of (element el of the tile, ik = 3 i + k)
 __host__ __device__ __forceinline__ int row_of(int el, int ik) { return 32 * (el / 3) + 9 * (el % 3) + ik; }
 
-// The Neo-Hookean update as the tensor-core kernel takes it: with H = F^-T and
-//   Z = a1/2 H - 2/3 c2 F,   Y = a2 H,
-// the tangent entry is three products, A_iJkL = H_iJ Z_kL + Z_iJ H_kL + Y_iL H_kJ
-// + c2 d_ik d_JL, and the stress P = c2 F - Y (a1, a2, c2 times JxW; see
-// NeoHookean).  The slicers' entries were four products of products: a third of
-// the FP32 instructions.  Every product that feeds a sum is an explicit FMA or
-// rounded on its own, so the residual-only kernel gives the same bits.
+// The Neo-Hookean update as the tensor-core kernel takes it.  With H = F^-T and the
+// stress P = c2 F - a2 H (a1, a2, c2, P times JxW; see NeoHookean) the tangent entry
+// is three products of per-point vectors,
+//   A_iJkL = H_iJ Z_kL + Z_iJ H_kL + Y_iL H_kJ + c2 d_ik d_JL,
+//   Z = a1/2 H - 2/3 c2 F = -2/3 P + b H,  b = a1/2 - 2/3 a2,   Y = a2 H,
+// instead of four products of products, and a point hands on H, P (which the
+// residual needs anyway) and three scalars.  Every product that feeds a sum is an
+// explicit FMA or rounded on its own, so the residual-only kernel gives the same
+// bits.
 struct AffNeoHookean {
-  static constexpr int NS = 0, SCR2 = 28;  // H, Z, Y, c2
+  static constexpr int NS = 0, SCR2 = 12;  // H, b, a2, c2
   struct Mid {
     double F[9], H[9], a1h, a2, c2;
   };
@@ -152,29 +154,40 @@ struct AffNeoHookean {
   }
   // the point's split stress and tangent scratch; returns a bound of |A_iJkL|
   __device__ static float stage(const Mid& m, float2* P, float2* scr) {
-    const double m23 = mul_rn(-2.0 / 3.0, m.c2);
-    float hm = 0.f, zm = 0.f, ym = 0.f;
+    float hm = 0.f, pm = 0.f;
 #pragma unroll
     for (int i = 0; i < 9; ++i) {
-      const double y = mul_rn(m.a2, m.H[i]);
-      const float2 h = df64_split(m.H[i]), z = df64_split(fma(m23, m.F[i], mul_rn(m.a1h, m.H[i]))), ys = df64_split(y);
-      P[i] = df64_split(fma(m.c2, m.F[i], -y));
+      const float2 h = df64_split(m.H[i]), p = df64_split(fma(m.c2, m.F[i], -mul_rn(m.a2, m.H[i])));
+      P[i] = p;
       scr[i] = h;
-      scr[9 + i] = z;
-      scr[18 + i] = ys;
       hm = fmaxf(hm, fabsf(h.x));
-      zm = fmaxf(zm, fabsf(z.x));
-      ym = fmaxf(ym, fabsf(ys.x));
+      pm = fmaxf(pm, fabsf(p.x));
     }
-    const float2 c = df64_split(m.c2);
-    scr[27] = c;
-    return (2.f * zm + ym) * hm + fabsf(c.x);
+    const float2 b = df64_split(fma(-2.0 / 3.0, m.a2, m.a1h)), a2 = df64_split(m.a2), c2 = df64_split(m.c2);
+    scr[9] = b;
+    scr[10] = a2;
+    scr[11] = c2;
+    return (2.f * (0.67f * pm + fabsf(b.x) * hm) + fabsf(a2.x) * hm) * hm + fabsf(c2.x);
   }
-  __device__ static float2 entry(const float2* s, int i, int J, int k, int L) {
-    const float2* Z = s + 9;
-    const float2* Y = s + 18;
-    float2 v = df64_dot3(s[i * 3 + J], Z[k * 3 + L], Z[i * 3 + J], s[k * 3 + L], Y[i * 3 + L], s[k * 3 + J]);
-    if (i == k && J == L) v = df64_add(v, s[27]);
+  // what a slicer thread keeps of its point
+  struct Tangent {
+    float2 H[9], Z[9], Y[9], c2;
+  };
+  __device__ static void load(const float2* scr, const float2* P, Tangent& t) {
+    const float2 m23 = make_float2(-0.666666686534881591796875f, 1.98682155172491e-08f);  // -2/3 to 2^-50
+    const float2 b = scr[9], a2 = scr[10];
+    t.c2 = scr[11];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      t.H[i] = scr[i];
+      t.Z[i] = df64_fma(b, t.H[i], df64_mul(m23, P[i]));
+      t.Y[i] = df64_mul(a2, t.H[i]);
+    }
+  }
+  __device__ static float2 entry(const Tangent& t, int i, int J, int k, int L) {
+    float2 v = df64_dot3(t.H[i * 3 + J], t.Z[k * 3 + L], t.Z[i * 3 + J], t.H[k * 3 + L], t.Y[i * 3 + L],
+                         t.H[k * 3 + J]);
+    if (i == k && J == L) v = df64_add(v, t.c2);
     return v;
   }
 };
@@ -197,8 +210,15 @@ struct AffJ2 {
     J2::split_scratch(m.scr, scr);
     return J2::abound(scr);
   }
-  __device__ static float2 entry(const float2* s, int i, int J, int k, int L) {
-    return J2::aentry_df64(s, i, J, k, L);
+  struct Tangent {
+    float2 s[SCR2];
+  };
+  __device__ static void load(const float2* scr, const float2*, Tangent& t) {
+#pragma unroll
+    for (int i = 0; i < SCR2; ++i) t.s[i] = scr[i];
+  }
+  __device__ static float2 entry(const Tangent& t, int i, int J, int k, int L) {
+    return J2::aentry_df64(t.s, i, J, k, L);
   }
 };
 
@@ -214,8 +234,8 @@ struct Layout {
   static constexpr int SIG = JXW + NQ * 8;                        // int [48]
   static constexpr int TAU = SIG + NPAD * 4;                      // int [2][12]: per tile parity
   static constexpr int TAUST = TAU + 2 * 16 * 4;                  // int [12]: the staged tile's scales
-  static constexpr int CODE = TAUST + 16 * 4;                     // uint32 [45] entry codes (+pad)
-  static constexpr int BAR = (CODE + 48 * 4 + 15) / 16 * 16;      // mbarriers: slices, MMAs, TMEM read
+  static constexpr int CODE = TAUST + 16 * 4;                     // uint32 [3][48] where an entry's digits go
+  static constexpr int BAR = (CODE + 3 * 48 * 4 + 15) / 16 * 16;  // mbarriers: slices, MMAs, TMEM read
   static constexpr int TSLOT = BAR + 32;
   static constexpr int SMEM = TSLOT + 16;
   static_assert(SMEM <= 232448, "shared memory");
@@ -260,9 +280,11 @@ __device__ __forceinline__ void tmem_ld4x7(uint32_t taddr, float (*v)[4]) {
     for (int j = 0; j < 4; ++j) v[L][j] = __uint_as_float(r[L * 4 + j]);
 }
 
-__device__ __forceinline__ void tmem_st2(uint32_t taddr, float a, float b) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(__float_as_uint(a)),
-               "r"(__float_as_uint(b))
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
+               "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+               "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
+               "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
                : "memory");
 }
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
@@ -362,6 +384,27 @@ __device__ __forceinline__ float2 combine_levels(const float (&v)[NLEV][4], int 
   return make_float2(hi, lo);
 }
 
+// The unique tangent entries (r1, r2), r1 <= r2, of a point in two halves, each by
+// a warp of its own: with the point's vectors in registers and the entry a
+// constant an entry is its arithmetic and no more.
+constexpr int N_HALF = 23;
+template <class Model, int HALF>
+__device__ __forceinline__ void park_entries(const typename Model::Tangent& t, float fs, uint32_t ent) {
+  constexpr int W0 = HALF ? N_HALF : 0, CNT = HALF ? 45 - N_HALF : N_HALF;
+  float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int r1 = 0; r1 < 9; ++r1)
+#pragma unroll
+    for (int r2 = r1; r2 < 9; ++r2) {
+      const int c = r1 * 9 - r1 * (r1 - 1) / 2 + r2 - r1 - W0;
+      if (c < 0 || c >= CNT) continue;
+      const float2 a = Model::entry(t, r1 / 3, r1 % 3, r2 / 3, r2 % 3);
+      v[2 * (c & 3)] = a.x * fs;
+      v[2 * (c & 3) + 1] = a.y * fs;
+      if ((c & 3) == 3 || c == CNT - 1) tmem_st8(ent + uint32_t(2 * (c & ~3)), v);
+    }
+}
+
 // R_(a,i) of one element from its points' split JxW P [8][9] (double-float, q in order)
 __device__ __forceinline__ double residual_entry(const float2* s_g2, const float2* P8, int a, int i) {
   float2 R = make_float2(0.f, 0.f);
@@ -405,17 +448,18 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
   for (int i = tid; i < TEN_N; i += NTHR) s_ten[i] = __ldg(reinterpret_cast<const double*>(tab + T_TEN) + i);
   if (tid < NQ) s_jxw[tid] = __ldg(reinterpret_cast<const double*>(tab + T_JXW) + tid);
   if (tid < NPAD) s_sig[tid] = __ldg(reinterpret_cast<const int*>(tab + T_SIG) + tid);
-  if (tid < 45) {
-    // unique entry w = (r1, r2), r1 <= r2, r1 = 3i + J, r2 = 3k + L: i, J, k, L and
-    // the operand positions (row ik = 3i + k, column 3J + L) and (row 3k + i, column 3L + J)
-    int m = tid, r = 0;
+  if (tid < 3 * 45) {
+    // unique entry w = (r1, r2), r1 <= r2, r1 = 3i + J, r2 = 3k + L, of the j-th element
+    // of a lane quarter: the operand positions (row 9j + 3i + k, column group 3J + L)
+    // and (row 9j + 3k + i, column group 3L + J) as byte offsets, low and high half
+    const int el = tid / 45;
+    int m = tid % 45, r = 0;
     for (int c = 0; c < 9; ++c)
       if (m >= 9 - r) { m -= 9 - r; ++r; }
     const int r1 = r, r2 = r + m;
     const int i = r1 / 3, J = r1 % 3, k = r2 / 3, L = r2 % 3;
-    s_code[tid] = uint32_t(i) | uint32_t(J) << 4 | uint32_t(k) << 8 | uint32_t(L) << 12 |
-                  uint32_t(i * 3 + k) << 16 | uint32_t(J * 3 + L) << 20 | uint32_t(k * 3 + i) << 24 |
-                  uint32_t(L * 3 + J) << 28;
+    s_code[el * 48 + tid % 45] = op_off(9 * el + i * 3 + k, (J * 3 + L) * 8) |
+                                 op_off(9 * el + k * 3 + i, (L * 3 + J) * 8) << 16;
   }
   if (tid == 0) {
     mbar_init(bar_sl, NSL);
@@ -481,41 +525,32 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
       named_arrive(BAR_FULL, N_FULL);
     }
   } else if (tid < T_R) {
-    // ---------------- slicers: thread (point p, half h) ----------------
-    const int ts = tid - T_SL, p = ts >> 1, h = ts & 1, el = p >> 3, q = p & 7;
-    const int w0 = h ? 23 : 0, cnt = h ? 22 : 23;
-    const int rbase = row_of(el, 0);
+    // ---------------- slicers: warps 0-2 half 0 of the entries, 3-5 half 1; lane = point ----------------
+    const int ts = tid - T_SL, h = ts >= NPT ? 1 : 0, p = ts - h * NPT, el = p >> 3, q = p & 7;
+    const int w0 = h ? N_HALF : 0, cnt = h ? 45 - N_HALF : N_HALF;
     // this warp's TMEM lanes (quarter warp % 4) and entry columns (two slicer warps share quarters 0 and 3)
     const uint32_t ent = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(TM_ENT + (warp >= 7 ? 48 : 0));
+    const uint32_t* code = s_code + (el % 3) * 48 + w0;
+    unsigned char* As = sm + Lay::A + (el / 3) * 4 * SBO + q * 2;
     for (int k = 0;; ++k) {
       const int64_t tile = blockIdx.x + int64_t(k) * gridDim.x;
       if (tile >= ntiles) break;
-      const bool live = tile * EPT + el < g.ne;
       named_sync(BAR_FULL, N_FULL);
-      const float2* sc = s_scr + p * SCR2;
       const int tau = s_taust[el];
-      const float fs = pow2f(7 - tau);  // entries scaled to |x| < 128
+      const float fs = tile * EPT + el < g.ne ? pow2f(7 - tau) : 0.f;  // entries scaled to |x| < 128
       // pass 1 (overlaps the previous tile's MMAs): the scaled entries into this
-      // lane's TMEM columns ent + 2c (hi), + 2c + 1 (lo); 23 steps on every lane
-      // (the .sync.aligned stores), the 23rd a zero on the half with 22
-#pragma unroll 1
-      for (int c = 0; c < 23; c += 2) {
-        const int c1 = c + 1 < 23 ? c + 1 : c;
-        const uint32_t code0 = s_code[w0 + (c < cnt ? c : 0)], code1 = s_code[w0 + (c1 < cnt ? c1 : 0)];
-        float2 a0 = make_float2(0.f, 0.f), a1 = a0;
-        if (live && c < cnt)
-          a0 = Model::entry(sc, code0 & 15, (code0 >> 4) & 15, (code0 >> 8) & 15, (code0 >> 12) & 15);
-        if (live && c1 < cnt)
-          a1 = Model::entry(sc, code1 & 15, (code1 >> 4) & 15, (code1 >> 8) & 15, (code1 >> 12) & 15);
-        tmem_st2(ent + uint32_t(2 * c), a0.x * fs, a0.y * fs);
-        if (c + 1 < 23) tmem_st2(ent + uint32_t(2 * c + 2), a1.x * fs, a1.y * fs);
-      }
+      // lane's TMEM columns ent + 2c (hi), + 2c + 1 (lo)
+      typename Model::Tangent tan;
+      Model::load(s_scr + p * SCR2, s_P + p * 9, tan);
+      if (h == 0)
+        park_entries<Model, 0>(tan, fs, ent);
+      else
+        park_entries<Model, 1>(tan, fs, ent);
       tmem_wait_st();
       named_arrive(BAR_EMPTY, N_FULL);  // the staging may be refilled
       // pass 2: the digits, once tile k-1's MMAs have read the slices
       if (k >= 1) wait_or_report(bar_mma, uint32_t((k - 1) & 1));
-      if ((ts & 15) == 0) s_tau[(k & 1) * 16 + el] = tau;
-      unsigned char* As = sm + Lay::A;
+      if (h == 0 && q == 0) s_tau[(k & 1) * 16 + el] = tau;
 #pragma unroll 1
       for (int c0 = 0; c0 < 24; c0 += 4) {
         float x[8];
@@ -524,9 +559,9 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
         for (int j = 0; j < 4; ++j) {
           const int c = c0 + j;
           if (c >= cnt) break;
-          const uint32_t code = s_code[w0 + c];
-          unsigned char* p1 = As + op_off(rbase + int((code >> 16) & 15), q * 9 + int((code >> 20) & 15));
-          unsigned char* p2 = As + op_off(rbase + int((code >> 24) & 15), q * 9 + int(code >> 28));
+          const uint32_t at = code[c];
+          unsigned char* p1 = As + (at & 0xffffu);
+          unsigned char* p2 = As + (at >> 16);
           const bool twin = p1 != p2;
           float xh = x[2 * j], xl = x[2 * j + 1];
           // digit s: the part of x at or above 2^(-8s), by adding and subtracting
@@ -856,7 +891,7 @@ bool hex8_affine_table(const double* x0, const double* ref, std::vector<unsigned
           uint32_t u;
           std::memcpy(&u, &fd, 4);
           const uint16_t bits = uint16_t(u >> 16);
-          std::memcpy(out.data() + aff::T_W + s * aff::W_SLICE + aff::op_off(n, r), &bits, 2);
+          std::memcpy(out.data() + aff::T_W + s * aff::W_SLICE + aff::op_off(n, r % 9 * 8 + r / 9), &bits, 2);
         }
       }
     }
