@@ -26,16 +26,17 @@
 // holds (element 3 w + j, ik = 3 i + k): every element's nine rows lie in one
 // warp's TMEM lanes, lanes 27-31 of each warp are padding rows.
 //   warps 0-2   FP64 point phase (displacement gradient, constitutive update),
-//               one thread per quadrature point, into a staging area;
+//               one thread per quadrature point, into a staging area (the
+//               stresses double-buffered for the residual warps);
 //   warps 3-8   tangent entries (45 unique per point, double-float), parked in
 //               TMEM, then (once the previous tile's MMAs read the slices) their
 //               digits into the seven A slices;
-//   warp 9      the residual R = sum_q dNX P in double-float;
-//   warps 10-13 the epilogue: TMEM -> double-float values (row (e, i, k) holds
+//   warps 9-10  the residual R = sum_q dNX P in double-float;
+//   warps 11-14 the epilogue: TMEM -> double-float values (row (e, i, k) holds
 //               K_(a,i),(b,k) for a <= b), stored as they leave tensor memory:
 //               the symmetric half (KE_PAIRS, entry 9n + 3i + k of pair n), or
 //               each value at its two places in the node rows of the whole K_e;
-//   warp 14     issues the tile's 50 MMAs (10 groups of digit pairs x 5 K steps).
+//   warp 15     issues the tile's 50 MMAs (10 groups of digit pairs x 5 K steps).
 // The A slices are rewritten as soon as the MMAs that read them completed; the
 // next MMAs wait only for the epilogue's reads of the accumulators.
 #include <cstdint>
@@ -82,9 +83,11 @@ constexpr int T_SL = 32 * PROD_W, T_R = T_SL + 32 * SL_W, T_EP = T_R + 32 * R_W,
 constexpr int NSL = 32 * SL_W;
 static_assert(32 * PROD_W == NPT && NSL == 2 * NPT, "roles");
 // named barriers (0 is __syncthreads)
-constexpr int BAR_FULL = 1;   // producers arrive, slicers + residual warp sync
-constexpr int BAR_EMPTY = 2;  // slicers + residual warp arrive, producers sync
-constexpr int N_FULL = 32 * (PROD_W + SL_W + R_W);
+constexpr int BAR_FULL = 1;    // producers arrive, slicers sync: a tile staged
+constexpr int BAR_EMPTY = 2;   // slicers arrive, producers sync: the tangent scratch read
+constexpr int BAR_RFULL = 3;   // + parity: producers arrive, residual warps sync
+constexpr int BAR_REMPTY = 5;  // + parity: residual warps arrive, producers sync: that stress buffer read
+constexpr int N_SL = 32 * (PROD_W + SL_W), N_RES = 32 * (PROD_W + R_W);
 
 // The MMAs of a tile: A slice t against W slices s0 .. s0+ns-1 at once (consecutive
 // W slices are consecutive 48-row blocks, one N = 48 ns operand), accumulating
@@ -226,11 +229,11 @@ template <class Model>
 struct Layout {
   static constexpr int W = 0;
   static constexpr int A = W + ND * W_SLICE;
-  static constexpr int P = A + ND * A_SLICE;                      // float2 [96][9]
-  static constexpr int SCR = P + NPT * 9 * 8;                     // float2 [96][SCR2]
+  static constexpr int P = A + ND * A_SLICE;                      // float2 [2][96][9]: per tile parity
+  static constexpr int SCR = P + 2 * NPT * 9 * 8;                 // float2 [96][SCR2]
   static constexpr int TEN = (SCR + NPT * Model::SCR2 * 8 + 15) / 16 * 16;  // double [TEN_N]
-  static constexpr int G2 = TEN + TEN_N * 8;                      // float2 [8][24]
-  static constexpr int JXW = G2 + NQ * 24 * 8;                    // double [8]
+  static constexpr int TEN2 = TEN + TEN_N * 8;                    // float2 [TEN_N]: the same split
+  static constexpr int JXW = TEN2 + TEN_N * 8;                    // double [8]
   static constexpr int SIG = JXW + NQ * 8;                        // int [48]
   static constexpr int TAU = SIG + NPAD * 4;                      // int [2][12]: per tile parity
   static constexpr int TAUST = TAU + 2 * 16 * 4;                  // int [12]: the staged tile's scales
@@ -405,15 +408,47 @@ __device__ __forceinline__ void park_entries(const typename Model::Tangent& t, f
     }
 }
 
-// R_(a,i) of one element from its points' split JxW P [8][9] (double-float, q in order)
-__device__ __forceinline__ double residual_entry(const float2* s_g2, const float2* P8, int a, int i) {
-  float2 R = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    const float2* gq = s_g2 + q * 24 + a * 3;
-    const float2* P = P8 + q * 9 + i * 3;
-    R = df64_dot3_acc(R, gq[0], P[0], gq[1], P[1], gq[2], P[2]);
+// a0 b0 + a1 b1 in double-float
+__device__ __forceinline__ float2 df64_dot2(float2 a0, float2 b0, float2 a1, float2 b1) {
+  const float p0 = __fmul_rn(a0.x, b0.x), p1 = __fmul_rn(a1.x, b1.x);
+  float e = __fmaf_rn(a0.x, b0.x, -p0);
+  e = __fmaf_rn(a0.x, b0.y, e);
+  e = __fmaf_rn(a0.y, b0.x, e);
+  e = __fadd_rn(__fmaf_rn(a1.x, b1.x, -p1), e);
+  e = __fmaf_rn(a1.x, b1.y, e);
+  e = __fmaf_rn(a1.y, b1.x, e);
+  const float t = __fadd_rn(p0, p1), v = __fsub_rn(t, p0);
+  return df64_fast2sum(t, __fadd_rn(e, __fadd_rn(__fsub_rn(p0, __fsub_rn(t, v)), __fsub_rn(p1, v))));
+}
+__device__ __forceinline__ float2 df64_across(float2 v, int bit) {
+  return make_float2(__shfl_xor_sync(0xffffffffu, v.x, bit), __shfl_xor_sync(0xffffffffu, v.y, bit));
+}
+// (v + across) where the lane's bit is set, its negative else: the transpose of a difference
+__device__ __forceinline__ float2 df64_spread(float2 v, int q, int bit) {
+  const float2 t = df64_add(v, df64_across(v, bit));
+  return (q & bit) ? t : df64_neg(t);
+}
+
+// R_(a,i) = sum_q sum_J dNX_qaJ JxW P_iJ at node a = corner_node(q), from the row i of
+// JxW P of the lane's point q (double-float): the transpose of tensor_gradient, one
+// direction at a time across the element's eight lanes -- 150 FP32 operations per
+// entry instead of the 290 of the sum over points, and no gradient table.  Every
+// lane of the warp calls it.
+__device__ __forceinline__ double residual_entry(const float2* ten2, bool box, int q, float2 p0, float2 p1, float2 p2) {
+  if (!box) {  // to the reference element
+    const float2* Ji = ten2 + 12 + q * 9;
+    const float2 x = df64_dot3(Ji[0], p0, Ji[1], p1, Ji[2], p2), y = df64_dot3(Ji[3], p0, Ji[4], p1, Ji[5], p2),
+                 z = df64_dot3(Ji[6], p0, Ji[7], p1, Ji[8], p2);
+    p0 = x;
+    p1 = y;
+    p2 = z;
   }
+  const float2 E = df64_dot2(ten2[8], p0, ten2[9], df64_across(p0, 4));
+  const float2 D = df64_dot2(ten2[6], p1, ten2[7], df64_across(p1, 4));
+  const float2 C = df64_spread(p2, q, 4);
+  const float2 A = df64_add(df64_dot2(ten2[4], C, ten2[5], df64_across(C, 2)), df64_spread(D, q, 2));
+  const float2 B = df64_dot2(ten2[2], E, ten2[3], df64_across(E, 2));
+  const float2 R = df64_add(df64_dot2(ten2[0], A, ten2[1], df64_across(A, 1)), df64_spread(B, q, 1));
   return widen(R.x) + widen(R.y);
 }
 
@@ -426,7 +461,7 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t s0 = smem_u32(sm);
   double* s_ten = reinterpret_cast<double*>(sm + Lay::TEN);
-  float2* s_g2 = reinterpret_cast<float2*>(sm + Lay::G2);
+  float2* s_ten2 = reinterpret_cast<float2*>(sm + Lay::TEN2);
   double* s_jxw = reinterpret_cast<double*>(sm + Lay::JXW);
   int* s_sig = reinterpret_cast<int*>(sm + Lay::SIG);
   int* s_tau = reinterpret_cast<int*>(sm + Lay::TAU);
@@ -443,9 +478,11 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
     reinterpret_cast<uint4*>(sm + Lay::A)[i] = make_uint4(0u, 0u, 0u, 0u);
   for (int i = tid; i < ND * W_SLICE / 16; i += NTHR)
     reinterpret_cast<uint4*>(sm + Lay::W)[i] = __ldg(reinterpret_cast<const uint4*>(tab + T_W) + i);
-  for (int i = tid; i < NQ * 24; i += NTHR)
-    s_g2[i] = df64_split(__ldg(reinterpret_cast<const double*>(tab + T_G) + i));
-  for (int i = tid; i < TEN_N; i += NTHR) s_ten[i] = __ldg(reinterpret_cast<const double*>(tab + T_TEN) + i);
+  for (int i = tid; i < TEN_N; i += NTHR) {
+    const double v = __ldg(reinterpret_cast<const double*>(tab + T_TEN) + i);
+    s_ten[i] = v;
+    s_ten2[i] = df64_split(v);
+  }
   if (tid < NQ) s_jxw[tid] = __ldg(reinterpret_cast<const double*>(tab + T_JXW) + tid);
   if (tid < NPAD) s_sig[tid] = __ldg(reinterpret_cast<const int*>(tab + T_SIG) + tid);
   if (tid < 3 * 45) {
@@ -510,9 +547,11 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
       next = node_of(tile + 2 * int64_t(gridDim.x));
       typename Model::Mid mid;
       point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
-      if (k >= 1) named_sync(BAR_EMPTY, N_FULL);  // tile k-1's staging has been read
+      const int buf = k & 1;
+      if (k >= 1) named_sync(BAR_EMPTY, N_SL);                     // tile k-1's scratch has been read
+      if (WANT_R && k >= 2) named_sync(BAR_REMPTY + buf, N_RES);   // and tile k-2's stresses
       float bnd = 0.f;
-      if (live) bnd = Model::stage(mid, s_P + tid * 9, s_scr + tid * SCR2) * 1.0001f;
+      if (live) bnd = Model::stage(mid, s_P + (buf * NPT + tid) * 9, s_scr + tid * SCR2) * 1.0001f;
       // the element's scale 2^tau > |every tangent entry| (its eight points are
       // lanes 8j .. 8j+7 of this warp)
 #pragma unroll
@@ -522,7 +561,8 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
         if (bnd > 0.f) frexpf(bnd, &tau);
         s_taust[el] = tau < -119 ? -119 : (tau > 126 ? 126 : tau);
       }
-      named_arrive(BAR_FULL, N_FULL);
+      named_arrive(BAR_FULL, N_SL);
+      if (WANT_R) named_arrive(BAR_RFULL + buf, N_RES);
     }
   } else if (tid < T_R) {
     // ---------------- slicers: warps 0-2 half 0 of the entries, 3-5 half 1; lane = point ----------------
@@ -535,19 +575,19 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
     for (int k = 0;; ++k) {
       const int64_t tile = blockIdx.x + int64_t(k) * gridDim.x;
       if (tile >= ntiles) break;
-      named_sync(BAR_FULL, N_FULL);
+      named_sync(BAR_FULL, N_SL);
       const int tau = s_taust[el];
       const float fs = tile * EPT + el < g.ne ? pow2f(7 - tau) : 0.f;  // entries scaled to |x| < 128
       // pass 1 (overlaps the previous tile's MMAs): the scaled entries into this
       // lane's TMEM columns ent + 2c (hi), + 2c + 1 (lo)
       typename Model::Tangent tan;
-      Model::load(s_scr + p * SCR2, s_P + p * 9, tan);
+      Model::load(s_scr + p * SCR2, s_P + ((k & 1) * NPT + p) * 9, tan);
       if (h == 0)
         park_entries<Model, 0>(tan, fs, ent);
       else
         park_entries<Model, 1>(tan, fs, ent);
       tmem_wait_st();
-      named_arrive(BAR_EMPTY, N_FULL);  // the staging may be refilled
+      named_arrive(BAR_EMPTY, N_SL);  // the staging may be refilled
       // pass 2: the digits, once tile k-1's MMAs have read the slices
       if (k >= 1) wait_or_report(bar_mma, uint32_t((k - 1) & 1));
       if (h == 0 && q == 0) s_tau[(k & 1) * 16 + el] = tau;
@@ -587,23 +627,23 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
       mbar_arrive(bar_sl);
     }
   } else if (tid < T_EP) {
-    // ---------------- residual warps ----------------
-    for (int k = 0;; ++k) {
-      const int64_t tile = blockIdx.x + int64_t(k) * gridDim.x;
-      if (tile >= ntiles) break;
-      named_sync(BAR_FULL, N_FULL);
-      if (WANT_R) {
-        constexpr int RT = 32 * R_W, NE = (EPT * 24 + RT - 1) / RT;
-#pragma unroll
-        for (int j = 0; j < NE; ++j) {
-          const int idx = tid - T_R + RT * j, el = idx / 24, ai = idx % 24;
-          if (idx >= EPT * 24) break;
-          const int64_t e = tile * EPT + el;
-          const double r = residual_entry(s_g2, s_P + el * NQ * 9, ai / 3, ai % 3);
-          if (e < g.ne) static_cast<double*>(g.Re)[e * 24 + ai] = r;
+    // ---------------- residual warps: (four elements, component) units; lane = point ----------------
+    if (WANT_R) {
+      const bool box = s_ten[10] != 0.0;
+      for (int k = 0;; ++k) {
+        const int64_t tile = blockIdx.x + int64_t(k) * gridDim.x;
+        if (tile >= ntiles) break;
+        named_sync(BAR_RFULL + (k & 1), N_RES);
+#pragma unroll 1
+        for (int u = warp - T_R / 32; u < PROD_W * 3; u += R_W) {
+          const int p = (u / 3) * 32 + lane, i = u % 3, q = p & 7;
+          const int64_t e = tile * EPT + (p >> 3);
+          const float2* P = s_P + ((k & 1) * NPT + p) * 9 + i * 3;
+          const double r = residual_entry(s_ten2, box, q, P[0], P[1], P[2]);
+          if (e < g.ne) static_cast<double*>(g.Re)[e * 24 + corner_node(q) * 3 + i] = r;
         }
+        named_arrive(BAR_REMPTY + (k & 1), N_RES);
       }
-      named_arrive(BAR_EMPTY, N_FULL);
     }
   } else if (tid < T_MMA) {
     // ---------------- epilogue: thread = TMEM lane = row (el, i, k) ----------------
@@ -702,14 +742,16 @@ constexpr int R_EPB = 16;
 template <class Model>
 __global__ void __launch_bounds__(R_EPB * NQ) hex8_affine_r_kernel(ElemArgs g, const unsigned char* __restrict__ tab) {
   __shared__ double s_ten[TEN_N], s_jxw[NQ];
-  __shared__ float2 s_g2[NQ * 24], s_P[R_EPB * NQ * 9];
+  __shared__ float2 s_ten2[TEN_N];
   const int tid = threadIdx.x, el = tid >> 3, q = tid & 7;
-  for (int i = tid; i < NQ * 24; i += blockDim.x)
-    s_g2[i] = df64_split(__ldg(reinterpret_cast<const double*>(tab + T_G) + i));
-  for (int i = tid; i < TEN_N; i += blockDim.x) s_ten[i] = __ldg(reinterpret_cast<const double*>(tab + T_TEN) + i);
+  for (int i = tid; i < TEN_N; i += blockDim.x) {
+    const double v = __ldg(reinterpret_cast<const double*>(tab + T_TEN) + i);
+    s_ten[i] = v;
+    s_ten2[i] = df64_split(v);
+  }
   if (tid < NQ) s_jxw[tid] = __ldg(reinterpret_cast<const double*>(tab + T_JXW) + tid);
   __syncthreads();
-  const int64_t e0 = int64_t(blockIdx.x) * R_EPB, e = e0 + el;
+  const int64_t e = int64_t(blockIdx.x) * R_EPB + el;
   const bool live = e < g.ne;
   double uo[3] = {0.0, 0.0, 0.0};
   if (live) {
@@ -719,12 +761,15 @@ __global__ void __launch_bounds__(R_EPB * NQ) hex8_affine_r_kernel(ElemArgs g, c
   }
   typename Model::Mid mid;
   point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
-  if (live) Model::stress(mid, s_P + tid * 9);
-  __syncthreads();
-  for (int idx = tid; idx < R_EPB * 24; idx += blockDim.x) {
-    const int ee = idx / 24, ai = idx % 24;
-    if (e0 + ee < g.ne)
-      static_cast<double*>(g.Re)[(e0 + ee) * 24 + ai] = residual_entry(s_g2, s_P + ee * NQ * 9, ai / 3, ai % 3);
+  float2 P[9];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) P[i] = make_float2(0.f, 0.f);
+  if (live) Model::stress(mid, P);
+  const bool box = s_ten[10] != 0.0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const double r = residual_entry(s_ten2, box, q, P[i * 3], P[i * 3 + 1], P[i * 3 + 2]);
+    if (live) static_cast<double*>(g.Re)[e * 24 + corner_node(q) * 3 + i] = r;
   }
 }
 
