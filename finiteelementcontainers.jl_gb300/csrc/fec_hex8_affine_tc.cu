@@ -22,23 +22,32 @@
 // (contributions below 2^-56 of the scales); the epilogue sums the seven levels
 // in double-float and scales by 2^(tau_e + sigma_n - 14).
 //
-// One persistent CTA per SM, tiles of 12 elements.  MMA row m = 32 w + 9 j + ik
-// holds (element 3 w + j, ik = 3 i + k): every element's nine rows lie in one
-// warp's TMEM lanes, lanes 27-31 of each warp are padding rows.
-//   warps 0-2   FP64 point phase (displacement gradient, constitutive update),
-//               one thread per quadrature point, into a staging area (the
-//               stresses double-buffered for the residual warps);
-//   warps 3-8   tangent entries (45 unique per point, double-float), parked in
-//               TMEM, then (once the previous tile's MMAs read the slices) their
-//               digits into the seven A slices;
-//   warps 9-10  the residual R = sum_q dNX P in double-float;
-//   warps 11-14 the epilogue: TMEM -> double-float values (row (e, i, k) holds
+// One persistent CTA per SM, tiles of 12 elements.  MMA row 32 w + 9 j + ik (3 more
+// where w is odd, see quarter_start) holds (element 3 w + j, ik = 3 i + k): every
+// element's nine rows lie in one warp's TMEM lanes, the other five are padding.
+//   producers   FP64 point phase (displacement gradient, constitutive update),
+//               one thread per quadrature point: two or three groups of three warps
+//               take the tiles in turn, each with a staging buffer of its own; then,
+//               while the slicers read it, the residual R = sum_q dNX P in
+//               double-float;
+//   6 slicers   two threads per point: tangent entries (45 unique, double-float),
+//               parked in TMEM, then (once the previous tile's MMAs read the
+//               slices) their digits into the seven A slices;
+//   4 warps     the epilogue: TMEM -> double-float values (row (e, i, k) holds
 //               K_(a,i),(b,k) for a <= b), stored as they leave tensor memory:
 //               the symmetric half (KE_PAIRS, entry 9n + 3i + k of pair n), or
 //               each value at its two places in the node rows of the whole K_e;
-//   warp 15     issues the tile's 50 MMAs (10 groups of digit pairs x 5 K steps).
+//   1 warp      issues the tile's 45 MMAs.
 // The A slices are rewritten as soon as the MMAs that read them completed; the
 // next MMAs wait only for the epilogue's reads of the accumulators.
+//
+// What bounds it: every role is near the tile period (about 14k SM clocks a tile of
+// 12 elements), and straight-line code is what they all pay for -- five warps of a
+// sub-partition run different code, which does not fit the instruction cache, at
+// about five clocks an instruction (ncu: no-instruction stalls 3.3 per issue against
+// 1.2 for memory).  So the loops that can be small are kept small: one entry's digits
+// (four at once: 9.0 ms instead of 8.05), the MMA issue (unrolled: 9.4), one residual
+// component (three: 8.7).  128^3 Neo-Hookean: 8.05 ms; 64 x 56 x 60 J2: 0.84 ms.
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -63,9 +72,11 @@ constexpr int NLEV = 7;              // accumulated levels s + t = 0..6
 constexpr int SBO = KP * 16;         // bytes between 8-row groups of an operand tile
 constexpr int A_SLICE = 128 * KP * 2;
 constexpr int W_SLICE = NPAD * KP * 2;
+constexpr int MAXS = 256 / NPAD;     // W digits in one MMA (N <= 256)
+constexpr int W_BYTES = ND * W_SLICE;
 // table built on the host (hex8_affine_table): W digits, sigma, dNX, JxW
 constexpr int T_W = 0;
-constexpr int T_SIG = ND * W_SLICE;
+constexpr int T_SIG = W_BYTES;
 constexpr int T_G = T_SIG + NPAD * 4;
 constexpr int T_JXW = T_G + NQ * 24 * 8;
 constexpr int T_TEN = T_JXW + NQ * 8;           // TEN_N doubles, see tensor_gradient
@@ -73,32 +84,39 @@ constexpr int TEN_N = 10 + 2 + NQ * 9;          // coefficients, diagonal flag (
 constexpr int T_BYTES = T_TEN + TEN_N * 8;
 static_assert(T_BYTES % 16 == 0 && T_G % 8 == 0, "table layout");
 constexpr int TMEM_COLS = 512;
-constexpr int TM_ENT = NLEV * NPAD;  // 2 x 48 columns after the accumulators: the slicers' scaled tangent entries (hi, lo)
-static_assert(TM_ENT + 2 * 48 <= TMEM_COLS, "tensor memory columns");
+constexpr int TM_ENT = NLEV * NPAD;  // 96 columns after the accumulators: the slicers' scaled tangent entries (hi, lo)
+static_assert(TM_ENT + 96 <= TMEM_COLS, "tensor memory columns");
 constexpr long long WAIT_BUDGET = 2000000000LL;
 
-constexpr int PROD_W = 3, SL_W = 6, R_W = 2, EP_W = 4, MMA_W = 1;
-constexpr int NTHR = 32 * (PROD_W + SL_W + R_W + EP_W + MMA_W);
-constexpr int T_SL = 32 * PROD_W, T_R = T_SL + 32 * SL_W, T_EP = T_R + 32 * R_W, T_MMA = T_EP + 32 * EP_W;
-constexpr int NSL = 32 * SL_W;
-static_assert(32 * PROD_W == NPT && NSL == 2 * NPT, "roles");
-// named barriers (0 is __syncthreads)
-constexpr int BAR_FULL = 1;    // producers arrive, slicers sync: a tile staged
-constexpr int BAR_EMPTY = 2;   // slicers arrive, producers sync: the tangent scratch read
-constexpr int BAR_RFULL = 3;   // + parity: producers arrive, residual warps sync
-constexpr int BAR_REMPTY = 5;  // + parity: residual warps arrive, producers sync: that stress buffer read
-constexpr int N_SL = 32 * (PROD_W + SL_W), N_RES = 32 * (PROD_W + R_W);
+// Warps.  Five warps a sub-partition leave 96 registers a thread.  Two or three
+// groups of producers, by what the physics costs them; a slicer thread takes half of
+// a point's entries.
+constexpr int PROD_W = 3, EP_W = 4, MMA_W = 1, NSL = 2 * NPT;
+template <class Model>
+struct Roles {
+  static constexpr int PG = Model::PROD_GROUPS;
+  static constexpr int T_SL = 32 * PROD_W * PG, T_EP = T_SL + NSL, T_MMA = T_EP + 32 * EP_W, NTHR = T_MMA + 32 * MMA_W;
+  static constexpr int N_SL = 32 * PROD_W + NSL;  // a producer group and the slicers
+  static constexpr int EMPTY = 1 + PG;            // first EMPTY barrier
+  static_assert(32 * PROD_W == NPT && NTHR <= 640, "roles");
+};
+// named barriers (0 is __syncthreads), each + the tile's producer group and buffer k % PG
+constexpr int BAR_FULL = 1;  // producers arrive, slicers sync: a tile staged
+                             // Roles::EMPTY: slicers arrive, producers sync: that buffer read
 
-// The MMAs of a tile: A slice t against W slices s0 .. s0+ns-1 at once (consecutive
-// W slices are consecutive 48-row blocks, one N = 48 ns operand), accumulating
-// into levels s0+t .. s0+t+ns-1 (consecutive 48-column blocks).  Every pair
-// s + t <= 6 once; the t = 0 groups write each level first.
-constexpr int NGROUP = 10;
-__device__ __constant__ int8_t kGroups[NGROUP][3] = {{0, 0, 4}, {0, 4, 3}, {1, 0, 4}, {1, 4, 2}, {2, 0, 4},
-                                                      {2, 4, 1}, {3, 0, 4}, {4, 0, 3}, {5, 0, 2}, {6, 0, 1}};
+// The MMAs of a tile: A digit t against up to five W digits s0 .. at once
+// (consecutive W slices are consecutive 48-row blocks, one N = 48 ns operand),
+// accumulating into levels s0+t .. (consecutive 48-column blocks).  Every pair s + t <=
+// 6 once; the t = 0 ones write each level first.  (The pairs in three subsets of 16
+// with barriers of their own, so that the epilogue of one overlaps the MMAs of the
+// next, were slower: 105 MMAs read A from shared memory 105 instead of 45 times,
+// 9-10k against 5k clocks a tile.)
 
-// MMA row of (element el of the tile, ik = 3 i + k)
-__host__ __device__ __forceinline__ int row_of(int el, int ik) { return 32 * (el / 3) + 9 * (el % 3) + ik; }
+// MMA row of (element el of the tile, ik = 3 i + k) within its quarter of 32 rows.
+// The odd quarters start at row 3: the four elements of a slicer warp then lie in
+// different eighths of the 128-byte core matrices, so their digit stores hit
+// different banks (the stores share the shared-memory pipe with the MMAs' reads).
+__host__ __device__ __forceinline__ int quarter_start(int quarter) { return 3 * (quarter & 1); }
 
 // The Neo-Hookean update as the tensor-core kernel takes it.  With H = F^-T and the
 // stress P = c2 F - a2 H (a1, a2, c2, P times JxW; see NeoHookean) the tangent entry
@@ -111,6 +129,8 @@ __host__ __device__ __forceinline__ int row_of(int el, int ik) { return 32 * (el
 // bits.
 struct AffNeoHookean {
   static constexpr int NS = 0, SCR2 = 12;  // H, b, a2, c2
+  static constexpr bool TANGENT_P = true;  // the slicers read the stress
+  static constexpr int PROD_GROUPS = 2;
   struct Mid {
     double F[9], H[9], a1h, a2, c2;
   };
@@ -172,7 +192,7 @@ struct AffNeoHookean {
     scr[11] = c2;
     return (2.f * (0.67f * pm + fabsf(b.x) * hm) + fabsf(a2.x) * hm) * hm + fabsf(c2.x);
   }
-  // what a slicer thread keeps of its point
+  // what a slicer thread keeps of its point (of these, the vectors its entries read)
   struct Tangent {
     float2 H[9], Z[9], Y[9], c2;
   };
@@ -197,6 +217,8 @@ struct AffNeoHookean {
 
 struct AffJ2 {
   static constexpr int NS = J2::NS, SCR2 = J2::SCR2;
+  static constexpr bool TANGENT_P = false;
+  static constexpr int PROD_GROUPS = 3;
   struct Mid {
     double P[9], scr[J2::SCR];
   };
@@ -228,17 +250,18 @@ struct AffJ2 {
 template <class Model>
 struct Layout {
   static constexpr int W = 0;
-  static constexpr int A = W + ND * W_SLICE;
-  static constexpr int P = A + ND * A_SLICE;                      // float2 [2][96][9]: per tile parity
-  static constexpr int SCR = P + 2 * NPT * 9 * 8;                 // float2 [96][SCR2]
-  static constexpr int TEN = (SCR + NPT * Model::SCR2 * 8 + 15) / 16 * 16;  // double [TEN_N]
-  static constexpr int TEN2 = TEN + TEN_N * 8;                    // float2 [TEN_N]: the same split
-  static constexpr int JXW = TEN2 + TEN_N * 8;                    // double [8]
-  static constexpr int SIG = JXW + NQ * 8;                        // int [48]
+  static constexpr int A = W + W_BYTES;
+  static constexpr int PG = Model::PROD_GROUPS;
+  static constexpr int P = A + ND * A_SLICE;                      // float2 [PG][96][9] (where the slicers read it)
+  static constexpr int SCR = P + (Model::TANGENT_P ? PG * NPT * 9 * 8 : 0);  // float2 [PG][96][SCR2]
+  static constexpr int TEN = (SCR + PG * NPT * Model::SCR2 * 8 + 15) / 16 * 16;  // double [TEN_N]
+  static constexpr int TEN2 = TEN + TEN_N * 8;                    // float2 [10]: the coefficients split
+  static constexpr int JXW = TEN2 + 10 * 8;                    // double [8]
+  static constexpr int SIG = JXW + NQ * 8;                        // float [48]: 2^(sigma - 7)
   static constexpr int TAU = SIG + NPAD * 4;                      // int [2][12]: per tile parity
-  static constexpr int TAUST = TAU + 2 * 16 * 4;                  // int [12]: the staged tile's scales
-  static constexpr int CODE = TAUST + 16 * 4;                     // uint32 [3][48] where an entry's digits go
-  static constexpr int BAR = (CODE + 3 * 48 * 4 + 15) / 16 * 16;  // mbarriers: slices, MMAs, TMEM read
+  static constexpr int TAUST = TAU + 2 * 16 * 4;                  // int [PG][12]: the staged tiles' scales
+  static constexpr int CODE = TAUST + PG * 16 * 4;                     // uint32 [6][48] where an entry's digits go
+  static constexpr int BAR = (CODE + 6 * 48 * 4 + 15) / 16 * 16;  // mbarriers: slices, MMAs, TMEM read
   static constexpr int TSLOT = BAR + 32;
   static constexpr int SMEM = TSLOT + 16;
   static_assert(SMEM <= 232448, "shared memory");
@@ -274,8 +297,8 @@ __device__ __forceinline__ void tmem_ld4x7(uint32_t taddr, float (*v)[4]) {
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
         "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
         "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27])
-      : "r"(taddr), "r"(taddr + 48u), "r"(taddr + 96u), "r"(taddr + 144u), "r"(taddr + 192u), "r"(taddr + 240u),
-        "r"(taddr + 288u)
+      : "r"(taddr), "r"(taddr + 1u * NPAD), "r"(taddr + 2u * NPAD), "r"(taddr + 3u * NPAD), "r"(taddr + 4u * NPAD),
+        "r"(taddr + 5u * NPAD), "r"(taddr + 6u * NPAD)
       : "memory");
 #pragma unroll
   for (int L = 0; L < NLEV; ++L)
@@ -290,16 +313,14 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8]) {
                "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
                : "memory");
 }
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
-  uint32_t r[8];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-      : "r"(taddr)
-      : "memory");
-#pragma unroll
-  for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
+__device__ __forceinline__ void tmem_ld2(uint32_t taddr, float& a, float& b) {
+  uint32_t r[2];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];\n\ttcgen05.wait::ld.sync.aligned;"
+               : "=r"(r[0]), "=r"(r[1])
+               : "r"(taddr)
+               : "memory");
+  a = __uint_as_float(r[0]);
+  b = __uint_as_float(r[1]);
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -389,11 +410,14 @@ __device__ __forceinline__ float2 combine_levels(const float (&v)[NLEV][4], int 
 
 // The unique tangent entries (r1, r2), r1 <= r2, of a point in two halves, each by
 // a warp of its own: with the point's vectors in registers and the entry a
-// constant an entry is its arithmetic and no more.
-constexpr int N_HALF = 23;
+// constant an entry is its arithmetic and no more.  The first half are the 24 entries
+// with i = 0, the second the 21 with i, k in {1, 2}: neither reads every vector.
+constexpr int N_HALF = 24;
 template <class Model, int HALF>
-__device__ __forceinline__ void park_entries(const typename Model::Tangent& t, float fs, uint32_t ent) {
+__device__ __forceinline__ void park_entries(const float2* scr, const float2* P, float fs, uint32_t ent) {
   constexpr int W0 = HALF ? N_HALF : 0, CNT = HALF ? 45 - N_HALF : N_HALF;
+  typename Model::Tangent t;
+  Model::load(scr, P, t);
   float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int r1 = 0; r1 < 9; ++r1)
@@ -434,9 +458,11 @@ __device__ __forceinline__ float2 df64_spread(float2 v, int q, int bit) {
 // direction at a time across the element's eight lanes -- 150 FP32 operations per
 // entry instead of the 290 of the sum over points, and no gradient table.  Every
 // lane of the warp calls it.
-__device__ __forceinline__ double residual_entry(const float2* ten2, bool box, int q, float2 p0, float2 p1, float2 p2) {
-  if (!box) {  // to the reference element
-    const float2* Ji = ten2 + 12 + q * 9;
+__device__ __forceinline__ double residual_entry(const double* ten, const float2* ten2, int q, float2 p0, float2 p1, float2 p2) {
+  if (ten[10] == 0.0) {  // not a box: to the reference element
+    float2 Ji[9];
+#pragma unroll
+    for (int m = 0; m < 9; ++m) Ji[m] = df64_split(ten[12 + q * 9 + m]);
     const float2 x = df64_dot3(Ji[0], p0, Ji[1], p1, Ji[2], p2), y = df64_dot3(Ji[3], p0, Ji[4], p1, Ji[5], p2),
                  z = df64_dot3(Ji[6], p0, Ji[7], p1, Ji[8], p2);
     p0 = x;
@@ -453,17 +479,19 @@ __device__ __forceinline__ double residual_entry(const float2* ten2, bool box, i
 }
 
 template <class Model, bool WANT_R>
-__global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, const unsigned char* __restrict__ tab) {
+__global__ void __launch_bounds__(Roles<Model>::NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, const unsigned char* __restrict__ tab) {
   using namespace tc;
   using Lay = Layout<Model>;
-  constexpr int SCR2 = Model::SCR2;
+  using Ro = Roles<Model>;
+  constexpr int SCR2 = Model::SCR2, PG = Ro::PG, NTHR = Ro::NTHR, N_SL = Ro::N_SL;
+  constexpr int T_SL = Ro::T_SL, T_EP = Ro::T_EP, T_MMA = Ro::T_MMA;
   extern __shared__ __align__(1024) unsigned char sm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t s0 = smem_u32(sm);
   double* s_ten = reinterpret_cast<double*>(sm + Lay::TEN);
   float2* s_ten2 = reinterpret_cast<float2*>(sm + Lay::TEN2);
   double* s_jxw = reinterpret_cast<double*>(sm + Lay::JXW);
-  int* s_sig = reinterpret_cast<int*>(sm + Lay::SIG);
+  float* s_sig = reinterpret_cast<float*>(sm + Lay::SIG);
   int* s_tau = reinterpret_cast<int*>(sm + Lay::TAU);
   int* s_taust = reinterpret_cast<int*>(sm + Lay::TAUST);
   uint32_t* s_code = reinterpret_cast<uint32_t*>(sm + Lay::CODE);
@@ -476,27 +504,27 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
   // ---- setup: A slices zero (padding rows and columns stay zero), W digits, tables ----
   for (int i = tid; i < ND * A_SLICE / 16; i += NTHR)
     reinterpret_cast<uint4*>(sm + Lay::A)[i] = make_uint4(0u, 0u, 0u, 0u);
-  for (int i = tid; i < ND * W_SLICE / 16; i += NTHR)
+  for (int i = tid; i < W_BYTES / 16; i += NTHR)
     reinterpret_cast<uint4*>(sm + Lay::W)[i] = __ldg(reinterpret_cast<const uint4*>(tab + T_W) + i);
   for (int i = tid; i < TEN_N; i += NTHR) {
     const double v = __ldg(reinterpret_cast<const double*>(tab + T_TEN) + i);
     s_ten[i] = v;
-    s_ten2[i] = df64_split(v);
+    if (i < 10) s_ten2[i] = df64_split(v);
   }
   if (tid < NQ) s_jxw[tid] = __ldg(reinterpret_cast<const double*>(tab + T_JXW) + tid);
-  if (tid < NPAD) s_sig[tid] = __ldg(reinterpret_cast<const int*>(tab + T_SIG) + tid);
-  if (tid < 3 * 45) {
+  if (tid < NPAD) s_sig[tid] = pow2f(__ldg(reinterpret_cast<const int*>(tab + T_SIG) + tid) - 7);
+  if (tid < 6 * 45) {
     // unique entry w = (r1, r2), r1 <= r2, r1 = 3i + J, r2 = 3k + L, of the j-th element
     // of a lane quarter: the operand positions (row 9j + 3i + k, column group 3J + L)
-    // and (row 9j + 3k + i, column group 3L + J) as byte offsets, low and high half
-    const int el = tid / 45;
+    // and (row 9j + 3k + i, column group 3L + J) as byte offsets, low and high half; the
+    // quarter's start is 0 or 3: table 3 (quarter & 1) + j
+    const int el = tid / 45, r0 = quarter_start(el / 3) + 9 * (el % 3);
     int m = tid % 45, r = 0;
     for (int c = 0; c < 9; ++c)
       if (m >= 9 - r) { m -= 9 - r; ++r; }
     const int r1 = r, r2 = r + m;
     const int i = r1 / 3, J = r1 % 3, k = r2 / 3, L = r2 % 3;
-    s_code[el * 48 + tid % 45] = op_off(9 * el + i * 3 + k, (J * 3 + L) * 8) |
-                                 op_off(9 * el + k * 3 + i, (L * 3 + J) * 8) << 16;
+    s_code[el * 48 + tid % 45] = op_off(r0 + i * 3 + k, (J * 3 + L) * 8) | op_off(r0 + k * 3 + i, (L * 3 + J) * 8) << 16;
   }
   if (tid == 0) {
     mbar_init(bar_sl, NSL);
@@ -522,36 +550,37 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
   };
 
   if (tid < T_SL) {
-    // ---------------- producers: thread (el, q) ----------------
-    const int el = tid >> 3, q = tid & 7;
-    // the nodes of tile k+1 and the displacements of tile k+1 are fetched while tile
-    // k is computed (a load latency each, once per tile)
+    // ---------------- producers: the group of tiles k = buf, buf + PG, ...; thread (el, q) ----------------
+    const int buf = tid / NPT, pt = tid - buf * NPT, el = pt >> 3, q = pt & 7;
+    const int64_t G = gridDim.x;
+    // the node of the group's next tile is fetched while it computes this one
     auto node_of = [&](int64_t tile) {
       const int64_t e = tile * EPT + el;
       return tile < ntiles && e < g.ne ? g.conn[e * 8 + corner_node(q)] : -1;
     };
-    double un[3] = {0.0, 0.0, 0.0};
-    auto fetch = [&](int node) {
-#pragma unroll
-      for (int d = 0; d < 3; ++d) un[d] = node >= 0 ? __ldg(&g.U[int64_t(node) * 3 + d]) : 0.0;
-    };
-    fetch(node_of(blockIdx.x));
-    int next = node_of(blockIdx.x + int64_t(gridDim.x));
-    for (int k = 0;; ++k) {
-      const int64_t tile = blockIdx.x + int64_t(k) * gridDim.x;
+    int node = node_of(blockIdx.x + buf * G);
+    for (int k = buf;; k += PG) {
+      const int64_t tile = blockIdx.x + k * G;
       if (tile >= ntiles) break;
       const int64_t e = tile * EPT + el;
       const bool live = e < g.ne;
-      const double uo[3] = {un[0], un[1], un[2]};
-      fetch(next);
-      next = node_of(tile + 2 * int64_t(gridDim.x));
+      double uo[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) uo[d] = live ? __ldg(&g.U[int64_t(node) * 3 + d]) : 0.0;
+      node = node_of(tile + PG * G);
       typename Model::Mid mid;
       point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
-      const int buf = k & 1;
-      if (k >= 1) named_sync(BAR_EMPTY, N_SL);                     // tile k-1's scratch has been read
-      if (WANT_R && k >= 2) named_sync(BAR_REMPTY + buf, N_RES);   // and tile k-2's stresses
+      if (k >= PG) named_sync(Ro::EMPTY + buf, N_SL);  // tile k-PG's staging has been read
       float bnd = 0.f;
-      if (live) bnd = Model::stage(mid, s_P + (buf * NPT + tid) * 9, s_scr + tid * SCR2) * 1.0001f;
+      float2 P[9];
+#pragma unroll
+      for (int i = 0; i < 9; ++i) P[i] = make_float2(0.f, 0.f);
+      if (live) {
+        bnd = Model::stage(mid, P, s_scr + tid * SCR2) * 1.0001f;
+        if (Model::TANGENT_P)
+#pragma unroll
+          for (int i = 0; i < 9; ++i) s_P[tid * 9 + i] = P[i];
+      }
       // the element's scale 2^tau > |every tangent entry| (its eight points are
       // lanes 8j .. 8j+7 of this warp)
 #pragma unroll
@@ -559,143 +588,122 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
       if (q == 0) {
         int tau = 0;
         if (bnd > 0.f) frexpf(bnd, &tau);
-        s_taust[el] = tau < -119 ? -119 : (tau > 126 ? 126 : tau);
+        s_taust[buf * 16 + el] = tau < -119 ? -119 : (tau > 126 ? 126 : tau);
       }
-      named_arrive(BAR_FULL, N_SL);
-      if (WANT_R) named_arrive(BAR_RFULL + buf, N_RES);
+      named_arrive(BAR_FULL + buf, N_SL);
+      if (WANT_R) {  // while the slicers work on the staging
+#pragma unroll 1
+        for (int i = 0; i < 3; ++i) {
+          const double r = residual_entry(s_ten, s_ten2, q, P[0], P[1], P[2]);
+          if (live) static_cast<double*>(g.Re)[e * 24 + corner_node(q) * 3 + i] = r;
+#pragma unroll
+          for (int j = 0; j < 6; ++j) P[j] = P[j + 3];
+        }
+      }
     }
-  } else if (tid < T_R) {
-    // ---------------- slicers: warps 0-2 half 0 of the entries, 3-5 half 1; lane = point ----------------
-    const int ts = tid - T_SL, h = ts >= NPT ? 1 : 0, p = ts - h * NPT, el = p >> 3, q = p & 7;
-    const int w0 = h ? N_HALF : 0, cnt = h ? 45 - N_HALF : N_HALF;
-    // this warp's TMEM lanes (quarter warp % 4) and entry columns (two slicer warps share quarters 0 and 3)
-    const uint32_t ent = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(TM_ENT + (warp >= 7 ? 48 : 0));
-    const uint32_t* code = s_code + (el % 3) * 48 + w0;
+  } else if (tid < T_EP) {
+    // ---------------- slicers: three warps (96 points) per half of the entries; lane = point ----------------
+    const int ts = tid - T_SL, half = ts / NPT, p = ts - half * NPT, el = p >> 3, q = p & 7;
+    const int w0 = half ? N_HALF : 0, cnt = half ? 45 - N_HALF : N_HALF;
+    // this warp's TMEM lanes (quarter warp % 4) and entry columns (every fourth slicer warp has the same lanes)
+    const uint32_t ent = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(TM_ENT + ((ts >> 5) >> 2) * 48);
+    const uint32_t* code = s_code + ((el / 3 & 1) * 3 + el % 3) * 48 + w0;
     unsigned char* As = sm + Lay::A + (el / 3) * 4 * SBO + q * 2;
     for (int k = 0;; ++k) {
       const int64_t tile = blockIdx.x + int64_t(k) * gridDim.x;
       if (tile >= ntiles) break;
-      named_sync(BAR_FULL, N_SL);
-      const int tau = s_taust[el];
+      const int buf = k % PG;
+      named_sync(BAR_FULL + buf, N_SL);
+      const int tau = s_taust[buf * 16 + el];
       const float fs = tile * EPT + el < g.ne ? pow2f(7 - tau) : 0.f;  // entries scaled to |x| < 128
       // pass 1 (overlaps the previous tile's MMAs): the scaled entries into this
       // lane's TMEM columns ent + 2c (hi), + 2c + 1 (lo)
-      typename Model::Tangent tan;
-      Model::load(s_scr + p * SCR2, s_P + ((k & 1) * NPT + p) * 9, tan);
-      if (h == 0)
-        park_entries<Model, 0>(tan, fs, ent);
+      const float2* scr = s_scr + (buf * NPT + p) * SCR2;
+      const float2* P = s_P + (buf * NPT + p) * 9;
+      if (half == 0)
+        park_entries<Model, 0>(scr, P, fs, ent);
       else
-        park_entries<Model, 1>(tan, fs, ent);
+        park_entries<Model, 1>(scr, P, fs, ent);
       tmem_wait_st();
-      named_arrive(BAR_EMPTY, N_SL);  // the staging may be refilled
+      named_arrive(Ro::EMPTY + buf, N_SL);  // the staging may be refilled
       // pass 2: the digits, once tile k-1's MMAs have read the slices
       if (k >= 1) wait_or_report(bar_mma, uint32_t((k - 1) & 1));
-      if (h == 0 && q == 0) s_tau[(k & 1) * 16 + el] = tau;
+      if (half == 0 && q == 0) s_tau[(k & 1) * 16 + el] = tau;
 #pragma unroll 1
-      for (int c0 = 0; c0 < 24; c0 += 4) {
-        float x[8];
-        tmem_ld8(ent + uint32_t(2 * c0), x);
+      for (int c = 0; c < cnt; ++c) {
+        float xh, xl;
+        tmem_ld2(ent + uint32_t(2 * c), xh, xl);
+        const uint32_t at = code[c];
+        unsigned char* p1 = As + (at & 0xffffu);
+        unsigned char* p2 = As + (at >> 16);
+        const bool twin = p1 != p2;
+        // digit s: the part of x at or above 2^(-8s), by adding and subtracting
+        // 1.5 2^(23-8s) (a rounding instruction issues at an eighth of the rate);
+        // |xl| <= ulp(xh) / 2 <= 2^-18 has no digits before the third
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int c = c0 + j;
-          if (c >= cnt) break;
-          const uint32_t at = code[c];
-          unsigned char* p1 = As + (at & 0xffffu);
-          unsigned char* p2 = As + (at >> 16);
-          const bool twin = p1 != p2;
-          float xh = x[2 * j], xl = x[2 * j + 1];
-          // digit s: the part of x at or above 2^(-8s), by adding and subtracting
-          // 1.5 2^(23-8s) (a rounding instruction issues at an eighth of the rate);
-          // |xl| <= ulp(xh) / 2 <= 2^-18 has no digits before the third
-#pragma unroll
-          for (int s = 0; s < ND; ++s) {
-            const float big = pow2f(23 - 8 * s) * 1.5f;
-            float d = __fsub_rn(__fadd_rn(xh, big), big);
-            xh = __fsub_rn(xh, d);
-            if (s >= 3) {
-              const float dl = __fsub_rn(__fadd_rn(xl, big), big);
-              xl = __fsub_rn(xl, dl);
-              d = __fadd_rn(d, dl);
-            }
-            const unsigned short bits = static_cast<unsigned short>(__float_as_uint(d) >> 16);
-            *reinterpret_cast<unsigned short*>(p1 + s * A_SLICE) = bits;
-            if (twin) *reinterpret_cast<unsigned short*>(p2 + s * A_SLICE) = bits;
+        for (int s = 0; s < ND; ++s) {
+          const float big = pow2f(23 - 8 * s) * 1.5f;
+          float d = __fsub_rn(__fadd_rn(xh, big), big);
+          xh = __fsub_rn(xh, d);
+          if (s >= 3) {
+            const float dl = __fsub_rn(__fadd_rn(xl, big), big);
+            xl = __fsub_rn(xl, dl);
+            d = __fadd_rn(d, dl);
           }
+          const unsigned short bits = static_cast<unsigned short>(__float_as_uint(d) >> 16);
+          *reinterpret_cast<unsigned short*>(p1 + s * A_SLICE) = bits;
+          if (twin) *reinterpret_cast<unsigned short*>(p2 + s * A_SLICE) = bits;
         }
       }
       fence_async_smem();
       mbar_arrive(bar_sl);
     }
-  } else if (tid < T_EP) {
-    // ---------------- residual warps: (four elements, component) units; lane = point ----------------
-    if (WANT_R) {
-      const bool box = s_ten[10] != 0.0;
-      for (int k = 0;; ++k) {
-        const int64_t tile = blockIdx.x + int64_t(k) * gridDim.x;
-        if (tile >= ntiles) break;
-        named_sync(BAR_RFULL + (k & 1), N_RES);
-#pragma unroll 1
-        for (int u = warp - T_R / 32; u < PROD_W * 3; u += R_W) {
-          const int p = (u / 3) * 32 + lane, i = u % 3, q = p & 7;
-          const int64_t e = tile * EPT + (p >> 3);
-          const float2* P = s_P + ((k & 1) * NPT + p) * 9 + i * 3;
-          const double r = residual_entry(s_ten2, box, q, P[0], P[1], P[2]);
-          if (e < g.ne) static_cast<double*>(g.Re)[e * 24 + corner_node(q) * 3 + i] = r;
-        }
-        named_arrive(BAR_REMPTY + (k & 1), N_RES);
-      }
-    }
   } else if (tid < T_MMA) {
     // ---------------- epilogue: thread = TMEM lane = row (el, i, k) ----------------
     const int qw = warp & 3;
-    const int el = qw * 3 + (lane < 27 ? lane / 9 : 0), ik = lane % 9, i = ik / 3, kc = ik % 3;
+    const int row = lane - quarter_start(qw);  // of the quarter's 27
+    const bool used = row >= 0 && row < 27;
+    const int el = qw * 3 + (used ? row / 9 : 0), ik = used ? row % 9 : 0, i = ik / 3, kc = ik % 3;
     const uint32_t lane_addr = tmem + (uint32_t(qw * 32) << 16);
     for (int k = 0;; ++k) {
       const int64_t tile = blockIdx.x + int64_t(k) * gridDim.x;
       if (tile >= ntiles) break;
       const uint32_t par = uint32_t(k & 1);
       wait_or_report(bar_sl, par);
-      wait_or_report(bar_mma, par);
-      tc_fence_after();
       const int64_t e0 = tile * EPT;
-      const bool live = lane < 27 && e0 + el < g.ne;
+      const bool live = used && e0 + el < g.ne;
       const int tau = s_tau[(k & 1) * 16 + el];
       const float f1 = pow2f(tau - 7);
-      if (g.ke_pairs) {
-        // the symmetric half straight from the levels: pair n = (a, b) of row
-        // (el, i, k) is K_(a,i),(b,k), entry 9n + 3i + k of the element's KE_PAIRS block
-        float2* dst = static_cast<float2*>(g.Ke) + (e0 + el) * (NPAIR * 9) + ik;
+      wait_or_report(bar_mma, par);
+      tc_fence_after();
 #pragma unroll 1
-        for (int c = 0; c < NPAIR / 4; ++c) {
-          float v[NLEV][4];
-          tmem_ld4x7(lane_addr + uint32_t(c * 4), v);
+      for (int n0 = 0; n0 < NPAIR; n0 += 4) {
+        float v[NLEV][4];
+        tmem_ld4x7(lane_addr + uint32_t(n0), v);
+        if (g.ke_pairs) {
+          // the symmetric half straight from the levels: pair n = (a, b) of row
+          // (el, i, k) is K_(a,i),(b,k), entry 9n + 3i + k of the element's KE_PAIRS block
+          float2* dst = static_cast<float2*>(g.Ke) + (e0 + el) * (NPAIR * 9) + ik + n0 * 9;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const float2 hl = combine_levels(v, j);
-            const float f = f1 * pow2f(s_sig[c * 4 + j] - 7);
-            if (live) dst[(c * 4 + j) * 9] = make_float2(hl.x * f, hl.y * f);
+            const float f = f1 * s_sig[n0 + j];
+            if (live) dst[j * 9] = make_float2(hl.x * f, hl.y * f);
           }
-        }
-        tc_fence_before();
-        mbar_arrive(bar_tfree);  // the accumulators may be overwritten
-        continue;
-      }
-      // node rows of the whole K_e: pair n = (a, b) of row (el, i, k), K_(a,i),(b,k), is
-      // entry b of node row (a, i, k) and, by symmetry, entry a of node row (b, k, i)
-      float2* dst = static_cast<float2*>(g.Ke) + (e0 + el) * 576;
-#pragma unroll 1
-      for (int c = 0; c < NPAIR / 4; ++c) {
-        float v[NLEV][4];
-        tmem_ld4x7(lane_addr + uint32_t(c * 4), v);
+        } else {
+          // node rows of the whole K_e: pair n = (a, b) of row (el, i, k), K_(a,i),(b,k), is
+          // entry b of node row (a, i, k) and, by symmetry, entry a of node row (b, k, i)
+          float2* dst = static_cast<float2*>(g.Ke) + (e0 + el) * 576;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 hl = combine_levels(v, j);
-          const float f = f1 * pow2f(s_sig[c * 4 + j] - 7);
-          const int ab = kPairNodes[c * 4 + j], a = ab >> 4, b = ab & 15;
-          const float2 val = make_float2(hl.x * f, hl.y * f);
-          if (live) {
-            dst[((a * 3 + i) * 3 + kc) * 8 + b] = val;
-            if (a != b) dst[((b * 3 + kc) * 3 + i) * 8 + a] = val;
+          for (int j = 0; j < 4; ++j) {
+            const float2 hl = combine_levels(v, j);
+            const float f = f1 * s_sig[n0 + j];
+            const int ab = kPairNodes[n0 + j], a = ab >> 4, b = ab & 15;
+            const float2 val = make_float2(hl.x * f, hl.y * f);
+            if (live) {
+              dst[((a * 3 + i) * 3 + kc) * 8 + b] = val;
+              if (a != b) dst[((b * 3 + kc) * 3 + i) * 8 + a] = val;
+            }
           }
         }
       }
@@ -709,19 +717,25 @@ __global__ void __launch_bounds__(NTHR, 1) hex8_affine_tc_kernel(ElemArgs g, con
     for (int k = 0;; ++k) {
       const int64_t tile = blockIdx.x + int64_t(k) * gridDim.x;
       if (tile >= ntiles) break;
-      if (k >= 1) wait_or_report(bar_tfree, uint32_t((k - 1) & 1));  // the accumulators are free
-      wait_or_report(bar_sl, uint32_t(k & 1));                       // the tile's slices are written
+      wait_or_report(bar_sl, uint32_t(k & 1));  // the tile's slices are written
       tc_fence_after();
+      if (k >= 1) {
+        wait_or_report(bar_tfree, uint32_t((k - 1) & 1));  // the accumulators are free
+        tc_fence_after();
+      }
       if (lane == 0) {
 #pragma unroll 1
-        for (int gi = 0; gi < NGROUP; ++gi) {
-          const int t = kGroups[gi][0], s0g = kGroups[gi][1], ns = kGroups[gi][2];
-          const uint32_t idesc = tc::idesc_bf16(128, NPAD * ns), d = tmem + uint32_t((s0g + t) * NPAD);
-          const uint64_t a0 = dA + uint64_t((t * A_SLICE) >> 4), w0d = dW + uint64_t((s0g * W_SLICE) >> 4);
+        for (int t = 0; t < ND; ++t)
+#pragma unroll 1
+          for (int s = 0; s < ND - t; s += MAXS) {
+            const int ns = ND - t - s < MAXS ? ND - t - s : MAXS;
+            const uint32_t idesc = tc::idesc_bf16(128, NPAD * ns);
+            const uint64_t a0 = dA + uint64_t((t * A_SLICE) >> 4), ws = dW + uint64_t((s * W_SLICE) >> 4);
 #pragma unroll
-          for (int kk = 0; kk < KP / 16; ++kk)
-            mma_bf16(d, a0 + uint64_t(kk * 16), w0d + uint64_t(kk * 16), idesc, (t == 0 && kk == 0) ? 0u : 1u);
-        }
+            for (int kk = 0; kk < KP / 16; ++kk)
+              mma_bf16(tmem + uint32_t((s + t) * NPAD), a0 + uint64_t(kk * 16), ws + uint64_t(kk * 16), idesc,
+                       (t == 0 && kk == 0) ? 0u : 1u);
+          }
         mma_commit(bar_mma);
       }
       __syncwarp();
@@ -742,12 +756,12 @@ constexpr int R_EPB = 16;
 template <class Model>
 __global__ void __launch_bounds__(R_EPB * NQ) hex8_affine_r_kernel(ElemArgs g, const unsigned char* __restrict__ tab) {
   __shared__ double s_ten[TEN_N], s_jxw[NQ];
-  __shared__ float2 s_ten2[TEN_N];
+  __shared__ float2 s_ten2[10];
   const int tid = threadIdx.x, el = tid >> 3, q = tid & 7;
   for (int i = tid; i < TEN_N; i += blockDim.x) {
     const double v = __ldg(reinterpret_cast<const double*>(tab + T_TEN) + i);
     s_ten[i] = v;
-    s_ten2[i] = df64_split(v);
+    if (i < 10) s_ten2[i] = df64_split(v);
   }
   if (tid < NQ) s_jxw[tid] = __ldg(reinterpret_cast<const double*>(tab + T_JXW) + tid);
   __syncthreads();
@@ -765,10 +779,9 @@ __global__ void __launch_bounds__(R_EPB * NQ) hex8_affine_r_kernel(ElemArgs g, c
 #pragma unroll
   for (int i = 0; i < 9; ++i) P[i] = make_float2(0.f, 0.f);
   if (live) Model::stress(mid, P);
-  const bool box = s_ten[10] != 0.0;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const double r = residual_entry(s_ten2, box, q, P[i * 3], P[i * 3 + 1], P[i * 3 + 2]);
+    const double r = residual_entry(s_ten, s_ten2, q, P[i * 3], P[i * 3 + 1], P[i * 3 + 2]);
     if (live) static_cast<double*>(g.Re)[e * 24 + corner_node(q) * 3 + i] = r;
   }
 }
@@ -781,7 +794,7 @@ cudaError_t launch1(const ElemArgs& a, cudaStream_t s, int* launches) {
   const int64_t ntiles = (a.ne + EPT - 1) / EPT;
   if (ntiles == 0) return cudaSuccess;
   const int grid = int(ntiles < num_sms() ? ntiles : num_sms());
-  hex8_affine_tc_kernel<Model, WANT_R><<<grid, NTHR, SMEM, s>>>(a, static_cast<const unsigned char*>(a.affine));
+  hex8_affine_tc_kernel<Model, WANT_R><<<grid, Roles<Model>::NTHR, SMEM, s>>>(a, static_cast<const unsigned char*>(a.affine));
   if (launches) ++*launches;
   return cudaGetLastError();
 }
