@@ -179,7 +179,9 @@ int build_affine(fec_ctx* c, size_t b) {
   B.tensor_rule = B.elem_type == FEC_HEX8 && fec::hex8_tensor_rule(c->ref_host.data() + c->ref_off[b], t);
   if (c->device < 0) return FEC_OK;
   std::vector<unsigned char> tab;
-  if (B.congruent) {
+  if (B.elem_type == FEC_HEX8 && !B.congruent) {
+    if (!B.tensor_rule || !fec::hex8_general_table(c->ref_host.data() + c->ref_off[b], tab)) return FEC_OK;
+  } else if (B.congruent) {
     if (!fec::hex8_affine_table(B.x0, c->ref_host.data() + c->ref_off[b], tab)) return FEC_OK;
   } else if (B.nclass > 0) {
     if (!fec::class_tc_table(B.elem_type, B.nclass, B.xc.data(), c->ref_host.data() + c->ref_off[b], tab))
@@ -201,11 +203,23 @@ const void* affine_table(const fec_ctx* c, size_t b, int precision, bool mixed, 
   if (mixed || b >= c->d_affine.size()) return nullptr;
   const Block& B = c->blocks[b];
   if (B.elem_type == FEC_HEX8)
-    return precision == FEC_FP64 && fec::hex8_affine_enabled() &&
+    return B.congruent && precision == FEC_FP64 && fec::hex8_affine_enabled() &&
                    (B.tensor_rule || gradients || B.physics == FEC_PHYS_POISSON)
                ? c->d_affine[b].p
                : nullptr;
   return (precision == FEC_FP32_ELEMENT || precision == FEC_FP64) ? c->d_affine[b].p : nullptr;
+}
+
+// The table of a Neo-Hookean hex8 block of elements of any shape on its own launch
+// (FP64, a symmetric rule), unless FEC_HEX8_GENERAL=0 or FEC_HEX8_DF64=tile.  A block
+// of translated elements has its own; with FEC_HEX8_AFFINE=0 it takes the per-element
+// kernels.
+const void* general_table(const fec_ctx* c, size_t b, int precision, bool mixed) {
+  const Block& B = c->blocks[b];
+  if (mixed || b >= c->d_affine.size() || B.elem_type != FEC_HEX8 || B.congruent || precision != FEC_FP64 ||
+      B.physics != FEC_PHYS_NEOHOOKEAN || fec::hex8_df64_tile_kernel() || !fec::hex8_general_enabled())
+    return nullptr;
+  return c->d_affine[b].p;
 }
 
 int ensure(fec_ctx* c, DevBuf& b, size_t bytes) {
@@ -236,7 +250,8 @@ bool fp64_pairs(const fec_ctx* c, size_t b, int precision, bool want_k, bool mix
       !(B.physics == FEC_PHYS_NEOHOOKEAN || B.physics == FEC_PHYS_J2))
     return false;
   if (B.elem_type == FEC_HEX27) return !mixed && hex27_pairs_enabled();
-  return B.elem_type == FEC_HEX8 && fec::hex8_pairs_enabled() && affine_table(c, b, precision, mixed) != nullptr;
+  return B.elem_type == FEC_HEX8 && fec::hex8_pairs_enabled() &&
+         (affine_table(c, b, precision, mixed) || general_table(c, b, precision, mixed));
 }
 
 // Workspace entries of block b's element matrices: the class tensor-core kernels
@@ -1117,6 +1132,7 @@ int fec_assemble(fec_ctx* c, int want, int precision, double t, double dt, const
     ea.Re = want_r ? static_cast<char*>(c->d_Re.p) + rsz * size_t(re_off) : nullptr;
     ea.closure = c->d_cl_args.p;
     ea.affine = affine_table(c, b, precision, mixed);
+    ea.hex8_general = general_table(c, b, precision, mixed);
     ea.ke_pairs = fp64_pairs(c, b, precision, want_k, mixed) ? 1 : 0;
     if (B.physics == FEC_PHYS_J2_MLP && !ea.closure)
       return fail(c, FEC_ERR_STATE, "block %d uses the learned closure but fec_closure_set was not called", int(b) + 1);
@@ -1647,14 +1663,19 @@ int fec_assemble_noalloc(fec_ctx* c, int want, int precision, double t, double d
   if (any_state && !state_old) return fail(c, FEC_ERR_ARG, "state_old is NULL for a physics with state");
   // workspace: element matrices, then (256-byte aligned) element residuals
   const size_t rsz = precision == FEC_FP64 ? sizeof(double) : sizeof(float);
-  int64_t ke_total = 0, re_total = 0;
+  int64_t ke_total = 0, ke_limit = 0, re_total = 0;
   for (size_t b = 0; b < c->blocks.size(); ++b) {
     ke_total += ke_entries(c, b, precision, want_k, false);
+    // (hex8 blocks of any shape count their whole element matrices against the limit,
+    // which the per-element kernels they may run write)
+    if (general_table(c, b, precision, false)) ke_limit += pad4(c->blocks[b].ne * 576);
+    else ke_limit += ke_entries(c, b, precision, want_k, false);
     re_total += c->blocks[b].ne * c->nf * c->blocks[b].nnpe;
   }
+  const size_t limit_off = ((want_k ? rsz * size_t(ke_limit) : 0) + 255) & ~size_t(255);
   const size_t ke_bytes = want_k ? rsz * size_t(ke_total) : 0;
   const size_t re_off_bytes = (ke_bytes + 255) & ~size_t(255);
-  const size_t need = re_off_bytes + (want_r ? rsz * size_t(re_total) : 0);
+  const size_t need = limit_off + (want_r ? rsz * size_t(re_total) : 0);
   if (need > FEC_NOALLOC_SCRATCH_BYTES)
     return fail(c, FEC_ERR_ARG,
                 "fec_assemble_noalloc needs %zu bytes of element workspace but the static scratch holds %zu "
@@ -1693,6 +1714,7 @@ int fec_assemble_noalloc(fec_ctx* c, int want, int precision, double t, double d
     ea.Re = want_r ? static_cast<char*>(Re) + rsz * size_t(re_off) : nullptr;
     ea.closure = c->d_cl_args.p;
     ea.affine = affine_table(c, b, precision, false);
+    ea.hex8_general = general_table(c, b, precision, false);
     ea.ke_pairs = fp64_pairs(c, b, precision, want_k, false) ? 1 : 0;
     if (B.physics == FEC_PHYS_J2_MLP && !ea.closure)
       return fail(c, FEC_ERR_STATE, "block %d uses the learned closure but fec_closure_set was not called", int(b) + 1);

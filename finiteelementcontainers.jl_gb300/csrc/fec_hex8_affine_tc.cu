@@ -100,9 +100,9 @@ struct Roles {
   static constexpr int EMPTY = 1 + PG;            // first EMPTY barrier
   static_assert(32 * PROD_W == NPT && NTHR <= 640, "roles");
 };
-// named barriers (0 is __syncthreads), each + the tile's producer group and buffer k % PG
-constexpr int BAR_FULL = 1;  // producers arrive, slicers sync: a tile staged
-                             // Roles::EMPTY: slicers arrive, producers sync: that buffer read
+// named barriers (0 is __syncthreads), each + the producer group
+constexpr int BAR_FULL = 1;  // the group arrives, slicers sync: a tile staged
+                             // Roles::EMPTY: slicers arrive, the group syncs: the buffer of its next tile read
 
 // The MMAs of a tile: A digit t against up to five W digits s0 .. at once
 // (consecutive W slices are consecutive 48-row blocks, one N = 48 ns operand),
@@ -130,7 +130,8 @@ __host__ __device__ __forceinline__ int quarter_start(int quarter) { return 3 * 
 struct AffNeoHookean {
   static constexpr int NS = 0, SCR2 = 12;  // H, b, a2, c2
   static constexpr bool TANGENT_P = true;  // the slicers read the stress
-  static constexpr int PROD_GROUPS = 2;
+  static constexpr bool GENERAL = false;
+  static constexpr int PROD_GROUPS = 2, STAGES = 2;
   struct Mid {
     double F[9], H[9], a1h, a2, c2;
   };
@@ -215,10 +216,120 @@ struct AffNeoHookean {
   }
 };
 
+// Neo-Hookean on any hex8 mesh: the same contraction in reference coordinates.  With
+// G = dX/dxi and g = dx/dxi (x = X + u) at a point, F = g G^-1, and pulled back to the
+// reference element (indices J -> alpha through G^-1) the update reads
+//   H_ia = (g^-T)_ia,   Q_ia = (g M)_ia,  M = G^-1 G^-T,   P_ia = c2 Q - a2 H,
+//   A_iakb = H_ia Z_kb + Z_ia H_kb + Y_ib H_ka + c2 d_ik M_ab,
+// so the constant operand is that of the reference element's own gradients, whatever
+// the element's shape.  M and Q are carried times det G squared.
+struct GenNeoHookean {
+  static constexpr int NS = 0, SCR2 = 17;  // H, b, a2, c2 M (6)
+  static constexpr bool GENERAL = true, TANGENT_P = true;
+  static constexpr int PROD_GROUPS = 3, STAGES = 1;
+  struct Mid {
+    double Q[9], H[9], M[6], a1h, a2, c2s;  // c2s: c2 / det G^2
+  };
+  __device__ static void cofactors(const double (&F)[3][3], double (&c)[9]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const int i1 = (i + 1) % 3, i2 = (i + 2) % 3, j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+        c[i * 3 + j] = fma(F[i1][j1], F[i2][j2], -mul_rn(F[i1][j2], F[i2][j1]));
+      }
+  }
+  // det G and M det G^2 (xx, yy, zz, yz, xz, xy)
+  __device__ static double metric(const double (&G)[3][3], double (&M)[6]) {
+    double c[9];
+    cofactors(G, c);
+    constexpr int A[6] = {0, 1, 2, 1, 0, 0}, B[6] = {0, 1, 2, 2, 2, 1};
+#pragma unroll
+    for (int m = 0; m < 6; ++m)
+      M[m] = fma(c[A[m]], c[B[m]], fma(c[3 + A[m]], c[3 + B[m]], mul_rn(c[6 + A[m]], c[6 + B[m]])));
+    return fma(G[0][0], c[0], fma(G[0][1], c[1], mul_rn(G[0][2], c[2])));
+  }
+  __device__ static void point(const double* props, const double (&g)[3][3], double detG, double w, Mid& m) {
+    double c[9];
+    cofactors(g, c);
+    const double detg = fma(g[0][0], c[0], fma(g[0][1], c[1], mul_rn(g[0][2], c[2])));
+    const double rG = 1.0 / detG, rg = 1.0 / detg;
+    constexpr int S[9] = {0, 5, 4, 5, 1, 3, 4, 3, 2};
+    double I1 = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const double q = fma(g[i][0], m.M[S[a]], fma(g[i][1], m.M[S[3 + a]], mul_rn(g[i][2], m.M[S[6 + a]])));
+        m.Q[i * 3 + a] = q;
+        I1 = fma(q, g[i][a], I1);
+      }
+    const double rG2 = mul_rn(rG, rG), J = mul_rn(detg, rG), jxw = mul_rn(detG, w);
+    const double Kj = mul_rn(props[0], jxw), Gj = mul_rn(props[1], jxw);
+    const double r3 = AffNeoHookean::inv_cbrt(J);
+    const double I13 = mul_rn(mul_rn(I1, rG2), 1.0 / 3.0);
+    const double JJ = mul_rn(J, J), d = JJ - J;
+    const double c2 = mul_rn(mul_rn(r3, r3), Gj);
+    m.a2 = fma(c2, I13, -mul_rn(0.5 * Kj, d - 1.0));
+    m.a1h = fma(c2, mul_rn(I13, 1.0 / 3.0), mul_rn(0.25 * Kj, JJ + d));
+    m.c2s = mul_rn(c2, rG2);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) m.H[i] = mul_rn(c[i], rg);
+  }
+  __device__ static void stress(const Mid& m, float2* P) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) P[i] = df64_split(fma(m.c2s, m.Q[i], -mul_rn(m.a2, m.H[i])));
+  }
+  __device__ static float stage(const Mid& m, float2* P, float2* scr) {
+    float hm = 0.f, pm = 0.f, cm = 0.f;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      const float2 h = df64_split(m.H[i]), p = df64_split(fma(m.c2s, m.Q[i], -mul_rn(m.a2, m.H[i])));
+      P[i] = p;
+      scr[i] = h;
+      hm = fmaxf(hm, fabsf(h.x));
+      pm = fmaxf(pm, fabsf(p.x));
+    }
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      const float2 c = df64_split(mul_rn(m.c2s, m.M[i]));
+      scr[11 + i] = c;
+      cm = fmaxf(cm, fabsf(c.x));
+    }
+    const float2 b = df64_split(fma(-2.0 / 3.0, m.a2, m.a1h)), a2 = df64_split(m.a2);
+    scr[9] = b;
+    scr[10] = a2;
+    return (2.f * (0.67f * pm + fabsf(b.x) * hm) + fabsf(a2.x) * hm) * hm + cm;
+  }
+  struct Tangent {
+    float2 H[9], Z[9], Y[9], cM[6];
+  };
+  __device__ static void load(const float2* scr, const float2* P, Tangent& t) {
+    AffNeoHookean::Tangent u;
+    AffNeoHookean::load(scr, P, u);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      t.H[i] = u.H[i];
+      t.Z[i] = u.Z[i];
+      t.Y[i] = u.Y[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 6; ++i) t.cM[i] = scr[11 + i];
+  }
+  __device__ static float2 entry(const Tangent& t, int i, int J, int k, int L) {
+    constexpr int S[9] = {0, 5, 4, 5, 1, 3, 4, 3, 2};
+    float2 v = df64_dot3(t.H[i * 3 + J], t.Z[k * 3 + L], t.Z[i * 3 + J], t.H[k * 3 + L], t.Y[i * 3 + L],
+                         t.H[k * 3 + J]);
+    if (i == k) v = df64_add(v, t.cM[S[J * 3 + L]]);
+    return v;
+  }
+};
+
 struct AffJ2 {
   static constexpr int NS = J2::NS, SCR2 = J2::SCR2;
   static constexpr bool TANGENT_P = false;
-  static constexpr int PROD_GROUPS = 3;
+  static constexpr bool GENERAL = false;
+  static constexpr int PROD_GROUPS = 3, STAGES = 3;
   struct Mid {
     double P[9], scr[J2::SCR];
   };
@@ -251,16 +362,16 @@ template <class Model>
 struct Layout {
   static constexpr int W = 0;
   static constexpr int A = W + W_BYTES;
-  static constexpr int PG = Model::PROD_GROUPS;
-  static constexpr int P = A + ND * A_SLICE;                      // float2 [PG][96][9] (where the slicers read it)
-  static constexpr int SCR = P + (Model::TANGENT_P ? PG * NPT * 9 * 8 : 0);  // float2 [PG][96][SCR2]
-  static constexpr int TEN = (SCR + PG * NPT * Model::SCR2 * 8 + 15) / 16 * 16;  // double [TEN_N]
+  static constexpr int NB = Model::STAGES;                        // staging buffers
+  static constexpr int P = A + ND * A_SLICE;                      // float2 [NB][96][9] (where the slicers read it)
+  static constexpr int SCR = P + (Model::TANGENT_P ? NB * NPT * 9 * 8 : 0);  // float2 [NB][96][SCR2]
+  static constexpr int TEN = (SCR + NB * NPT * Model::SCR2 * 8 + 15) / 16 * 16;  // double [TEN_N]
   static constexpr int TEN2 = TEN + TEN_N * 8;                    // float2 [10]: the coefficients split
   static constexpr int JXW = TEN2 + 10 * 8;                    // double [8]
   static constexpr int SIG = JXW + NQ * 8;                        // float [48]: 2^(sigma - 7)
   static constexpr int TAU = SIG + NPAD * 4;                      // int [2][12]: per tile parity
-  static constexpr int TAUST = TAU + 2 * 16 * 4;                  // int [PG][12]: the staged tiles' scales
-  static constexpr int CODE = TAUST + PG * 16 * 4;                     // uint32 [6][48] where an entry's digits go
+  static constexpr int TAUST = TAU + 2 * 16 * 4;                  // int [NB][12]: the staged tiles' scales
+  static constexpr int CODE = TAUST + NB * 16 * 4;                     // uint32 [6][48] where an entry's digits go
   static constexpr int BAR = (CODE + 6 * 48 * 4 + 15) / 16 * 16;  // mbarriers: slices, MMAs, TMEM read
   static constexpr int TSLOT = BAR + 32;
   static constexpr int SMEM = TSLOT + 16;
@@ -390,6 +501,22 @@ __device__ __forceinline__ void point_phase(const ElemArgs& g, const double* s_t
   if (live) Model::point(g.props, gu, s_jxw[q], st, sn, m);
 }
 
+// The same on an element of any shape, X: its corner node's coordinates; s_ten: the
+// reference element's coefficients, w: the quadrature weight.
+__device__ __forceinline__ void general_point(const ElemArgs& g, const double* s_ten, double w, int q, bool live,
+                                              const double (&X)[3], const double (&uo)[3], GenNeoHookean::Mid& m) {
+  const int lane = threadIdx.x & 31;
+  double v[3], G[3][3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) v[d] = X[d] - __shfl_sync(0xffffffffu, X[d], lane & ~7);
+  tensor_gradient(s_ten, q, v, G);
+  const double detG = GenNeoHookean::metric(G, m.M);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) v[d] += uo[d] - __shfl_sync(0xffffffffu, uo[d], lane & ~7);
+  tensor_gradient(s_ten, q, v, G);
+  if (live) GenNeoHookean::point(g.props, G, detG, w, m);
+}
+
 // node pair n = (a, b), a <= b, as a << 4 | b
 __constant__ unsigned char kPairNodes[NPAIR] = {0x00, 0x01, 0x02, 0x03, 0x04, 0x05, 0x06, 0x07, 0x11, 0x12, 0x13, 0x14, 0x15, 0x16, 0x17, 0x22, 0x23, 0x24, 0x25, 0x26, 0x27, 0x33, 0x34, 0x35, 0x36, 0x37, 0x44, 0x45, 0x46, 0x47, 0x55, 0x56, 0x57, 0x66, 0x67, 0x77};
 
@@ -483,7 +610,7 @@ __global__ void __launch_bounds__(Roles<Model>::NTHR, 1) hex8_affine_tc_kernel(E
   using namespace tc;
   using Lay = Layout<Model>;
   using Ro = Roles<Model>;
-  constexpr int SCR2 = Model::SCR2, PG = Ro::PG, NTHR = Ro::NTHR, N_SL = Ro::N_SL;
+  constexpr int SCR2 = Model::SCR2, PG = Ro::PG, NB = Model::STAGES, NTHR = Ro::NTHR, N_SL = Ro::N_SL;
   constexpr int T_SL = Ro::T_SL, T_EP = Ro::T_EP, T_MMA = Ro::T_MMA;
   extern __shared__ __align__(1024) unsigned char sm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -550,16 +677,17 @@ __global__ void __launch_bounds__(Roles<Model>::NTHR, 1) hex8_affine_tc_kernel(E
   };
 
   if (tid < T_SL) {
-    // ---------------- producers: the group of tiles k = buf, buf + PG, ...; thread (el, q) ----------------
-    const int buf = tid / NPT, pt = tid - buf * NPT, el = pt >> 3, q = pt & 7;
+    // ---------------- producers: the group of tiles k = grp, grp + PG, ...; thread (el, q) ----------------
+    const int grp = tid / NPT, pt = tid - grp * NPT, el = pt >> 3, q = pt & 7;
+    const int sp = (NB == 1 ? 0 : grp) * NPT + pt;  // the staged point
     const int64_t G = gridDim.x;
     // the node of the group's next tile is fetched while it computes this one
     auto node_of = [&](int64_t tile) {
       const int64_t e = tile * EPT + el;
       return tile < ntiles && e < g.ne ? g.conn[e * 8 + corner_node(q)] : -1;
     };
-    int node = node_of(blockIdx.x + buf * G);
-    for (int k = buf;; k += PG) {
+    int node = node_of(blockIdx.x + grp * G);
+    for (int k = grp;; k += PG) {
       const int64_t tile = blockIdx.x + k * G;
       if (tile >= ntiles) break;
       const int64_t e = tile * EPT + el;
@@ -567,19 +695,27 @@ __global__ void __launch_bounds__(Roles<Model>::NTHR, 1) hex8_affine_tc_kernel(E
       double uo[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) uo[d] = live ? __ldg(&g.U[int64_t(node) * 3 + d]) : 0.0;
-      node = node_of(tile + PG * G);
       typename Model::Mid mid;
-      point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
-      if (k >= PG) named_sync(Ro::EMPTY + buf, N_SL);  // tile k-PG's staging has been read
+      if constexpr (Model::GENERAL) {
+        double X[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) X[d] = live ? __ldg(&g.coords[int64_t(node) * 3 + d]) : 0.0;
+        node = node_of(tile + PG * G);
+        general_point(g, s_ten, s_jxw[q], q, live, X, uo, mid);
+      } else {
+        node = node_of(tile + PG * G);
+        point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
+      }
+      if (k >= NB) named_sync(Ro::EMPTY + grp, N_SL);  // the buffer's last tile has been read
       float bnd = 0.f;
       float2 P[9];
 #pragma unroll
       for (int i = 0; i < 9; ++i) P[i] = make_float2(0.f, 0.f);
       if (live) {
-        bnd = Model::stage(mid, P, s_scr + tid * SCR2) * 1.0001f;
+        bnd = Model::stage(mid, P, s_scr + sp * SCR2) * 1.0001f;
         if (Model::TANGENT_P)
 #pragma unroll
-          for (int i = 0; i < 9; ++i) s_P[tid * 9 + i] = P[i];
+          for (int i = 0; i < 9; ++i) s_P[sp * 9 + i] = P[i];
       }
       // the element's scale 2^tau > |every tangent entry| (its eight points are
       // lanes 8j .. 8j+7 of this warp)
@@ -588,9 +724,9 @@ __global__ void __launch_bounds__(Roles<Model>::NTHR, 1) hex8_affine_tc_kernel(E
       if (q == 0) {
         int tau = 0;
         if (bnd > 0.f) frexpf(bnd, &tau);
-        s_taust[buf * 16 + el] = tau < -119 ? -119 : (tau > 126 ? 126 : tau);
+        s_taust[(NB == 1 ? 0 : grp) * 16 + el] = tau < -119 ? -119 : (tau > 126 ? 126 : tau);
       }
-      named_arrive(BAR_FULL + buf, N_SL);
+      named_arrive(BAR_FULL + grp, N_SL);
       if (WANT_R) {  // while the slicers work on the staging
 #pragma unroll 1
         for (int i = 0; i < 3; ++i) {
@@ -612,8 +748,8 @@ __global__ void __launch_bounds__(Roles<Model>::NTHR, 1) hex8_affine_tc_kernel(E
     for (int k = 0;; ++k) {
       const int64_t tile = blockIdx.x + int64_t(k) * gridDim.x;
       if (tile >= ntiles) break;
-      const int buf = k % PG;
-      named_sync(BAR_FULL + buf, N_SL);
+      const int buf = k % NB;
+      named_sync(BAR_FULL + k % PG, N_SL);
       const int tau = s_taust[buf * 16 + el];
       const float fs = tile * EPT + el < g.ne ? pow2f(7 - tau) : 0.f;  // entries scaled to |x| < 128
       // pass 1 (overlaps the previous tile's MMAs): the scaled entries into this
@@ -625,7 +761,7 @@ __global__ void __launch_bounds__(Roles<Model>::NTHR, 1) hex8_affine_tc_kernel(E
       else
         park_entries<Model, 1>(scr, P, fs, ent);
       tmem_wait_st();
-      named_arrive(Ro::EMPTY + buf, N_SL);  // the staging may be refilled
+      named_arrive(Ro::EMPTY + (k + NB) % PG, N_SL);  // the staging may be refilled (by tile k + NB's group)
       // pass 2: the digits, once tile k-1's MMAs have read the slices
       if (k >= 1) wait_or_report(bar_mma, uint32_t((k - 1) & 1));
       if (half == 0 && q == 0) s_tau[(k & 1) * 16 + el] = tau;
@@ -767,14 +903,20 @@ __global__ void __launch_bounds__(R_EPB * NQ) hex8_affine_r_kernel(ElemArgs g, c
   __syncthreads();
   const int64_t e = int64_t(blockIdx.x) * R_EPB + el;
   const bool live = e < g.ne;
-  double uo[3] = {0.0, 0.0, 0.0};
+  double uo[3] = {0.0, 0.0, 0.0}, X[3] = {0.0, 0.0, 0.0};
   if (live) {
     const int64_t node = g.conn[e * 8 + corner_node(q)];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) uo[d] = __ldg(&g.U[node * 3 + d]);
+    for (int d = 0; d < 3; ++d) {
+      uo[d] = __ldg(&g.U[node * 3 + d]);
+      if (Model::GENERAL) X[d] = __ldg(&g.coords[node * 3 + d]);
+    }
   }
   typename Model::Mid mid;
-  point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
+  if constexpr (Model::GENERAL)
+    general_point(g, s_ten, s_jxw[q], q, live, X, uo, mid);
+  else
+    point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
   float2 P[9];
 #pragma unroll
   for (int i = 0; i < 9; ++i) P[i] = make_float2(0.f, 0.f);
@@ -883,6 +1025,29 @@ static bool box_scales(const double* x0, double sc[3]) {
     sc[d] = 1.0 / len[d];
   }
   return true;
+}
+
+// FEC_HEX8_GENERAL=0 keeps hex8 blocks of any shape on the per-element kernels.
+bool hex8_general_enabled() {
+  const char* v = std::getenv("FEC_HEX8_GENERAL");
+  return !(v && v[0] == '0');
+}
+
+cudaError_t launch_hex8_general_tc(bool want_r, bool want_k, const ElemArgs& a, cudaStream_t s, int* launches) {
+  if (!a.hex8_general || (want_k && !a.Ke) || (want_r && !a.Re)) return cudaErrorInvalidValue;
+  ElemArgs b = a;
+  b.affine = a.hex8_general;
+  if (!want_k) return want_r ? aff::launch_r<aff::GenNeoHookean>(b, s, launches) : cudaSuccess;
+  return want_r ? aff::launch1<aff::GenNeoHookean, true>(b, s, launches)
+                : aff::launch1<aff::GenNeoHookean, false>(b, s, launches);
+}
+
+// The operand of the reference element itself (the cube [-1, 1]^3).
+bool hex8_general_table(const double* ref, std::vector<unsigned char>& out) {
+  double x[24];
+  for (int a = 0; a < 8; ++a)
+    for (int d = 0; d < 3; ++d) x[a * 3 + d] = (a ^ ((a >> 1) & 1)) >> d & 1 ? 1.0 : -1.0;
+  return hex8_affine_table(x, ref, out);
 }
 
 // Host: the constant operand of a block whose elements are translates of its
