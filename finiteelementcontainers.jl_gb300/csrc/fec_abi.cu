@@ -1305,14 +1305,19 @@ int fec_assemble_action(fec_ctx* c, int precision, double t, double dt, const do
     const int ns = num_states_of(B.physics);
     ea.state_old = ns ? state_old + st_off : nullptr;
     ea.Re = static_cast<char*>(c->d_Re.p) + rsz * size_t(re_off);
-    // FP64 blocks of translated hex8 elements: the block's constant gradients and JxW
-    if (B.elem_type == FEC_HEX8 && precision == FEC_FP64 && B.congruent)
+    // FP64 hex8 mechanics with the tables of a symmetric rule: the tensor-core kernel's
+    // point phase; else blocks of translated elements: their constant gradients and JxW
+    if (B.elem_type == FEC_HEX8 && B.physics != FEC_PHYS_POISSON) ea.affine = affine_table(c, b, precision, false);
+    ea.hex8_general = general_table(c, b, precision, false);
+    const bool tensor = ea.affine || ea.hex8_general;
+    if (!tensor && B.elem_type == FEC_HEX8 && precision == FEC_FP64 && B.congruent)
       if (const void* tab = affine_table(c, b, precision, false, true))
         ea.affine = static_cast<const unsigned char*>(tab) + fec::hex8_affine_grad_offset();
     cudaError_t e;
     {
       LaunchTimer timer(c, s, "element_action");
-      e = fec::launch_action(B.physics, B.elem_type, precision, ea, V, s, &c->last_launches);
+      e = tensor ? fec::launch_hex8_action(B.physics, ea, V, s, &c->last_launches)
+                 : fec::launch_action(B.physics, B.elem_type, precision, ea, V, s, &c->last_launches);
     }
     if (e == cudaErrorNotSupported)
       return fail(c, FEC_ERR_UNSUPPORTED, "block %d: matrix-free action of physics %d on element type %d is not built",

@@ -176,6 +176,37 @@ struct AffNeoHookean {
 #pragma unroll
     for (int i = 0; i < 9; ++i) P[i] = df64_split(fma(m.c2, m.F[i], -mul_rn(m.a2, m.H[i])));
   }
+  // (A : D)_iJ = (a1 h + m f) H + m h F + a2 H D^T H + c2 D, h = H : D, f = F : D, m = -2/3 c2
+  __device__ static void action(const Mid& m, const double (&D)[3][3], double (&out)[3][3]) {
+    const double m23 = mul_rn(-2.0 / 3.0, m.c2);
+    action_terms(m.H, m.F, D, D, 2.0 * m.a1h, m.a2, m23, m.c2, out);
+  }
+  // (a1 h + m f) H + m h Q + a2 H D^T H + c E, h = H : D, f = Q : D
+  __device__ static void action_terms(const double* H, const double* Q, const double (&D)[3][3],
+                                      const double (&E)[3][3], double a1, double a2, double m, double c,
+                                      double (&out)[3][3]) {
+    double h = 0.0, f = 0.0;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      h = fma(H[k], D[k / 3][k % 3], h);
+      f = fma(Q[k], D[k / 3][k % 3], f);
+    }
+    const double s1 = fma(a1, h, mul_rn(m, f)), s2 = mul_rn(m, h);
+    double M[3][3];  // a2 (D^T H)
+#pragma unroll
+    for (int l = 0; l < 3; ++l)
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        M[l][j] = mul_rn(a2, fma(D[0][l], H[j], fma(D[1][l], H[3 + j], mul_rn(D[2][l], H[6 + j]))));
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        out[i][j] = fma(H[i * 3], M[0][j],
+                        fma(H[i * 3 + 1], M[1][j],
+                            fma(H[i * 3 + 2], M[2][j],
+                                fma(c, E[i][j], fma(s2, Q[i * 3 + j], mul_rn(s1, H[i * 3 + j]))))));
+  }
   // the point's split stress and tangent scratch; returns a bound of |A_iJkL|
   __device__ static float stage(const Mid& m, float2* P, float2* scr) {
     float hm = 0.f, pm = 0.f;
@@ -280,6 +311,20 @@ struct GenNeoHookean {
 #pragma unroll
     for (int i = 0; i < 9; ++i) P[i] = df64_split(fma(m.c2s, m.Q[i], -mul_rn(m.a2, m.H[i])));
   }
+  __device__ static void action(const Mid& m, const double (&D)[3][3], double (&out)[3][3]) {
+    constexpr int S[9] = {0, 5, 4, 5, 1, 3, 4, 3, 2};
+    double E[3][3], Q[9];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        E[i][a] = fma(D[i][0], m.M[S[a]], fma(D[i][1], m.M[S[3 + a]], mul_rn(D[i][2], m.M[S[6 + a]])));
+        Q[i * 3 + a] = m.Q[i * 3 + a];
+      }
+    // (Q and M are carried times det G^2: c2s Q and c2s E are c2 Q and c2 E; f and h Q
+    // come with m23 c2s)
+    AffNeoHookean::action_terms(m.H, Q, D, E, 2.0 * m.a1h, m.a2, mul_rn(-2.0 / 3.0, m.c2s), m.c2s, out);
+  }
   __device__ static float stage(const Mid& m, float2* P, float2* scr) {
     float hm = 0.f, pm = 0.f, cm = 0.f;
 #pragma unroll
@@ -340,6 +385,9 @@ struct AffJ2 {
   __device__ static void stress(const Mid& m, float2* P) {
 #pragma unroll
     for (int i = 0; i < 9; ++i) P[i] = df64_split(m.P[i]);
+  }
+  __device__ static void action(const Mid& m, const double (&D)[3][3], double (&out)[3][3]) {
+    J2::action(m.scr, D, out);
   }
   __device__ static float stage(const Mid& m, float2* P, float2* scr) {
     stress(m, P);
@@ -928,6 +976,89 @@ __global__ void __launch_bounds__(R_EPB * NQ) hex8_affine_r_kernel(ElemArgs g, c
   }
 }
 
+// The transpose of tensor_gradient for one component in FP64: the value at node
+// corner_node(q) from the row p of the lane's point q.
+__device__ __forceinline__ double tensor_spread(const double* co, int q, double p0, double p1, double p2) {
+  auto across = [](double v, int bit) { return __shfl_xor_sync(0xffffffffu, v, bit); };
+  const double E = fma(co[8], p0, mul_rn(co[9], across(p0, 4)));
+  const double D = fma(co[6], p1, mul_rn(co[7], across(p1, 4)));
+  const double C = signed_by(p2 + across(p2, 4), q & 4);
+  const double A = fma(co[4], C, fma(co[5], across(C, 2), signed_by(D + across(D, 2), q & 2)));
+  const double B = fma(co[2], E, mul_rn(co[3], across(E, 2)));
+  return fma(co[0], A, fma(co[1], across(A, 1), signed_by(B + across(B, 1), q & 1)));
+}
+
+// Matrix-free tangent action K_e v_e (see fec_action.cu) with the point phase and
+// gradients of the kernels above, in FP64 throughout: the FP64 pipe bounds it, and
+// the sum-factorised gradients and their transpose take 13 operations a component
+// where the sums over nodes take 24 (about 300 a point instead of 500).  16
+// elements per CTA, one thread per point.
+template <class Model>
+__global__ void __launch_bounds__(R_EPB * NQ) hex8_action_kernel(ElemArgs g, const unsigned char* __restrict__ tab,
+                                                                 const double* __restrict__ V) {
+  __shared__ double s_ten[TEN_N], s_jxw[NQ];
+  const int tid = threadIdx.x, el = tid >> 3, q = tid & 7, lane = tid & 31;
+  for (int i = tid; i < TEN_N; i += blockDim.x) s_ten[i] = __ldg(reinterpret_cast<const double*>(tab + T_TEN) + i);
+  if (tid < NQ) s_jxw[tid] = __ldg(reinterpret_cast<const double*>(tab + T_JXW) + tid);
+  __syncthreads();
+  const int64_t e = int64_t(blockIdx.x) * R_EPB + el;
+  const bool live = e < g.ne;
+  double uo[3] = {0.0, 0.0, 0.0}, X[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0};
+  if (live) {
+    const int64_t node = g.conn[e * 8 + corner_node(q)];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      uo[d] = __ldg(&g.U[node * 3 + d]);
+      v[d] = __ldg(&V[node * 3 + d]);
+      if (Model::GENERAL) X[d] = __ldg(&g.coords[node * 3 + d]);
+    }
+  }
+  typename Model::Mid mid;
+  if constexpr (Model::GENERAL)
+    general_point(g, s_ten, s_jxw[q], q, live, X, uo, mid);
+  else
+    point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
+  double D[3][3], out[3][3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) v[d] -= __shfl_sync(0xffffffffu, v[d], lane & ~7);
+  tensor_gradient(s_ten, q, v, D);
+  const bool box = s_ten[10] != 0.0;
+  const double* Ji = s_ten + 12 + q * 9;
+  if (!box) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double r0 = D[i][0], r1 = D[i][1], r2 = D[i][2];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) D[i][j] = fma(r0, Ji[j], fma(r1, Ji[3 + j], mul_rn(r2, Ji[6 + j])));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 9; ++i) out[i / 3][i % 3] = 0.0;
+  if (live) Model::action(mid, D, out);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    double p0 = out[i][0], p1 = out[i][1], p2 = out[i][2];
+    if (!box) {
+      const double x = fma(Ji[0], p0, fma(Ji[1], p1, mul_rn(Ji[2], p2))),
+                   y = fma(Ji[3], p0, fma(Ji[4], p1, mul_rn(Ji[5], p2)));
+      p2 = fma(Ji[6], p0, fma(Ji[7], p1, mul_rn(Ji[8], p2)));
+      p0 = x;
+      p1 = y;
+    }
+    const double r = tensor_spread(s_ten, q, p0, p1, p2);
+    if (live) static_cast<double*>(g.Re)[e * 24 + corner_node(q) * 3 + i] = r;
+  }
+}
+
+template <class Model>
+cudaError_t launch_act(const ElemArgs& a, const void* tab, const double* V, cudaStream_t s, int* launches) {
+  const int64_t nb = (a.ne + R_EPB - 1) / R_EPB;
+  if (nb == 0) return cudaSuccess;
+  hex8_action_kernel<Model><<<unsigned(nb), R_EPB * NQ, 0, s>>>(a, static_cast<const unsigned char*>(tab), V);
+  if (launches) ++*launches;
+  return cudaGetLastError();
+}
+
 template <class Model, bool WANT_R>
 cudaError_t launch1(const ElemArgs& a, cudaStream_t s, int* launches) {
   constexpr int SMEM = Layout<Model>::SMEM;
@@ -1040,6 +1171,14 @@ cudaError_t launch_hex8_general_tc(bool want_r, bool want_k, const ElemArgs& a, 
   if (!want_k) return want_r ? aff::launch_r<aff::GenNeoHookean>(b, s, launches) : cudaSuccess;
   return want_r ? aff::launch1<aff::GenNeoHookean, true>(b, s, launches)
                 : aff::launch1<aff::GenNeoHookean, false>(b, s, launches);
+}
+
+cudaError_t launch_hex8_action(int physics, const ElemArgs& a, const double* V, cudaStream_t s, int* launches) {
+  if (!a.Re) return cudaErrorInvalidValue;
+  if (physics == 2 && a.affine) return aff::launch_act<aff::AffNeoHookean>(a, a.affine, V, s, launches);
+  if (physics == 3 && a.affine) return aff::launch_act<aff::AffJ2>(a, a.affine, V, s, launches);
+  if (physics == 2 && a.hex8_general) return aff::launch_act<aff::GenNeoHookean>(a, a.hex8_general, V, s, launches);
+  return cudaErrorNotSupported;
 }
 
 // The operand of the reference element itself (the cube [-1, 1]^3).

@@ -94,6 +94,9 @@ bool hex8_pairs_enabled();
 // coordinates, whose constant operand is the reference element's.  Needs the tables
 // of a symmetric 2 x 2 x 2 rule.  FEC_HEX8_GENERAL=0 keeps the per-element kernels.
 cudaError_t launch_hex8_general_tc(bool want_r, bool want_k, const ElemArgs& args, cudaStream_t stream, int* launches);
+// The FP64 matrix-free action on such blocks (args.affine: Neo-Hookean and J2;
+// args.hex8_general: Neo-Hookean), as launch_action.
+cudaError_t launch_hex8_action(int physics, const ElemArgs& args, const double* V, cudaStream_t stream, int* launches);
 bool hex8_general_table(const double* ref, std::vector<unsigned char>& out);
 bool hex8_general_enabled();
 // Tet10 (7) / hex27 (8) Neo-Hookean (2) or J2 (3) for a block whose element e is

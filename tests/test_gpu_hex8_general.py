@@ -121,3 +121,49 @@ def test_tables_of_another_rule_keep_the_per_element_kernels(fec):
     with environment(FEC_HEX8_GENERAL="0"):
         R2, K2 = fec.assemble_residual_and_stiffness(asm, Uu, p)
         assert torch.equal(R2, R) and torch.equal(K2.nzval, nz)
+
+
+@pytest.mark.parametrize("cells, stretch, rotate, fixed", [
+    ((2, 1, 1), (1.0, 1.0, 1.0), False, False), ((17, 1, 1), (1.0, 1.0, 1.0), True, False),   # one over a CTA's 16
+    ((5, 6, 7), (1.0, 0.02, 0.3), True, True), ((4, 5, 3), (1e-5, 1e-5, 1e-5), False, False)])
+def test_action_matches_assembled_matrix_and_per_element_kernel(fec, cells, stretch, rotate, fixed):
+    import torch
+    mesh = _mesh(fec, cells, 8, stretch, rotate)
+    asm, p, _, Uu = _setup(fec, mesh, fixed)
+    _, K = fec.assemble_residual_and_stiffness(asm, Uu, p)
+    V = np.random.default_rng(3).standard_normal(asm.dof.unknown_dofs.size)
+    Vd = torch.from_numpy(V).cuda()
+    A = fec.assemble_matrix_free_action(asm, fec.stiffness_action, Uu, Vd, p).cpu().numpy().copy()
+    with environment(FEC_HEX8_GENERAL="0"):
+        B = fec.assemble_matrix_free_action(asm, fec.stiffness_action, Uu, Vd, p).cpu().numpy().copy()
+    ref = K.to_scipy().T @ V
+    scale = abs(K.to_scipy()).T @ np.abs(V)   # the terms of each entry
+    assert np.all(np.abs(A - B) <= TOL64 * scale)
+    assert np.all(np.abs(A - ref) <= TOL64 * scale)
+
+
+@pytest.mark.parametrize("phys_name", ["neohookean", "j2"])
+def test_action_on_a_skewed_block_of_translates(fec, phys_name):
+    """A block of translated parallelepipeds (not boxes): gradients through dxi/dX."""
+    import torch
+    mesh = fec.StructuredMesh("hex", (0.0,) * 3, (1.0,) * 3, (6, 6, 6))
+    X = mesh.nodal_coords @ np.array([[1.0, 0.2, 0.0], [0.1, 0.9, 0.3], [0.0, -0.2, 1.1]])
+    mesh = fec.UnstructuredMesh(X, {"b": ("HEX8", mesh.element_conns["block_1"])})
+    u = fec.VectorFunction(fec.FunctionSpace(mesh), "u")
+    asm = fec.SparseMatrixAssembler(u)
+    phys = fec.NeoHookean.from_youngs(1.0, 0.3) if phys_name == "neohookean" else fec.J2Plasticity(200.0, 0.3, 0.25, 2.0)
+    p = fec.create_parameters(mesh, asm, phys)
+    rng = np.random.default_rng(5)
+    U = X * np.array([0.004, -0.001, 0.002]) + 1e-4 * rng.standard_normal(X.shape)
+    Uu, V = torch.from_numpy(U.ravel()).cuda(), rng.standard_normal(U.size)
+    R, K = fec.assemble_residual_and_stiffness(asm, Uu, p)
+    A = fec.assemble_matrix_free_action(asm, fec.stiffness_action, Uu, torch.from_numpy(V).cuda(), p).cpu().numpy()
+    M = K.to_scipy()
+    assert np.all(np.abs(A - M.T @ V) <= TOL64 * (abs(M).T @ np.abs(V)))
+    fused = R.clone()
+    fec.assemble_vector(asm, fec.residual, Uu, p)
+    assert torch.equal(fec.residual(asm), fused)
+    with environment(FEC_HEX8_AFFINE="0"):
+        R2, K2 = fec.assemble_residual_and_stiffness(asm, Uu, p)
+        assert max(rel_err(fused.cpu().numpy(), R2.cpu().numpy())[:2]) <= TOL64
+        assert rel_err(M.data, K2.nzval.cpu().numpy())[2] <= TOL64
