@@ -107,6 +107,11 @@ struct fec_ctx {
   DevBuf d_node_groups;
   std::vector<fec::NodeGroup> node_groups;
   bool groups_ready = false;
+  // per block: the plan of the gather by output entry (built on first use, per pattern);
+  // plan_state 0: not tried, 1: built, 2: the mesh has none
+  std::vector<DevBuf> d_plan;
+  std::vector<int64_t> plan_nslots;
+  std::vector<int> plan_state;
   std::vector<DevBuf> d_affine;        // per block: the tensor-core operand table of a congruent hex8 block
                                        // or of a tet10/hex27 block of translation classes
   bool single_launch = false;          // FP64 mechanics: every element block in one launch
@@ -365,10 +370,106 @@ int build_node_groups(fec_ctx* c) {
   return FEC_OK;
 }
 
+// Whether block b's element matrices of this assembly are stored as symmetric halves.
+bool stores_pairs(const fec_ctx* c, size_t b, int precision, bool want_r, bool want_k, bool mixed) {
+  const Block& B = c->blocks[b];
+  return fp64_pairs(c, b, precision, want_k, mixed) ||
+         (want_k && fec::class_tc_runs(B.physics, B.elem_type, precision, want_r, want_k,
+                                       affine_table(c, b, precision, mixed) != nullptr));
+}
+
+// The plan of block b's gather by output entry (fec_pairgather.cu), built on first use
+// on stream s, before the element kernels: their workspace is its scratch.  slots null
+// where the block has none: nodes shared with other blocks or with very many elements,
+// indices that do not fit, no memory for it, or a first use under stream capture (the
+// per-node gathers then give the same bits).
+int pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s, fec::PairPlan* out) {
+  *out = fec::PairPlan{nullptr, nullptr, nullptr, 0};
+  if (c->plan_state.size() != c->blocks.size()) {
+    c->plan_state.assign(c->blocks.size(), 0);
+    c->plan_nslots.assign(c->blocks.size(), 0);
+    for (DevBuf& x : c->d_plan) x.release();
+    c->d_plan.assign(c->blocks.size(), DevBuf());
+  }
+  const Block& B = c->blocks[b];
+  // at most: a pair of neighbours once, a pair of element nodes once
+  const int64_t np = int64_t(B.nnpe) * (B.nnpe + 1) / 2, max_list = B.ne * np;
+  const int64_t max_slots = std::min(max_list, (c->nbr_ptr.empty() ? max_list : (c->nbr_ptr.back() + c->nn) / 2));
+  const size_t slot_bytes = sizeof(int4) * size_t(max_slots), count_bytes = (2 * size_t(max_slots) + 15) / 16 * 16;
+  DevBuf& d = c->d_plan[b];  // slots, counts, list
+  if (c->plan_state[b] == 0) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+      cudaGetLastError();
+      return FEC_OK;
+    }
+    if (cs != cudaStreamCaptureStatusNone) return FEC_OK;
+    c->plan_state[b] = 2;
+    if (max_list <= 0 || max_list >= (int64_t(1) << 31) || c->nn >= (int64_t(1) << 31)) return FEC_OK;
+    // scratch: sums, counts per node, flags, slots and counts in node order
+    const size_t n1 = size_t(c->nn) + 1, scan_n = fec::pattern_scan_scratch(c->nn + 1);
+    const size_t need = 8 * (2 * n1 + scan_n) + 4 * 2 * n1 + 16 + 16 + slot_bytes + count_bytes;
+    DevBuf own;
+    struct Free {
+      DevBuf* b;
+      ~Free() { b->release(); }
+    } free_own{&own};
+    void* t = c->d_Ke.p;
+    if (c->d_Ke.bytes < need) {
+      if (cudaMalloc(&own.p, need) != cudaSuccess) {
+        cudaGetLastError();
+        return FEC_OK;
+      }
+      t = own.p;
+    }
+    d.release();
+    if (cudaMalloc(&d.p, slot_bytes + count_bytes + sizeof(uint32_t) * size_t(max_list)) != cudaSuccess) {
+      cudaGetLastError();
+      d.p = nullptr;
+      return FEC_OK;
+    }
+    int4* slots2 = static_cast<int4*>(t);
+    uint16_t* count2 = reinterpret_cast<uint16_t*>(slots2 + max_slots);
+    int64_t* slot0 = reinterpret_cast<int64_t*>(reinterpret_cast<char*>(count2) + count_bytes);
+    int64_t* list0 = slot0 + n1;
+    int64_t* scan = list0 + n1;
+    int32_t* nslot = reinterpret_cast<int32_t*>(scan + scan_n);
+    int32_t* nlist = nslot + n1;
+    int* flags = nlist + n1;
+    char* base = static_cast<char*>(d.p);
+    FEC_CUDA(c, cudaMemsetAsync(flags, 0, 2 * sizeof(int), s));
+    FEC_CUDA(c, fec::pair_plan_count(ga, int(b), B.ne, nslot, nlist, flags, s));
+    FEC_CUDA(c, fec::pattern_scan(nslot, nullptr, c->nn, slot0, scan, s));
+    FEC_CUDA(c, fec::pattern_scan(nlist, nullptr, c->nn, list0, scan, s));
+    FEC_CUDA(c, fec::pair_plan_fill(ga, int(b), B.ne, slot0, list0, slots2, base, count2,
+                                    reinterpret_cast<uint16_t*>(base + slot_bytes),
+                                    reinterpret_cast<uint32_t*>(base + slot_bytes + count_bytes), flags, s));
+    int64_t total = 0;
+    int h[2];
+    FEC_CUDA(c, cudaMemcpyAsync(&total, slot0 + c->nn, 8, cudaMemcpyDeviceToHost, s));
+    FEC_CUDA(c, cudaMemcpyAsync(h, flags, sizeof h, cudaMemcpyDeviceToHost, s));
+    FEC_CUDA(c, cudaStreamSynchronize(s));
+    if (h[0] || h[1] || total == 0) {
+      d.release();
+      return FEC_OK;
+    }
+    c->plan_nslots[b] = total;
+    c->plan_state[b] = 1;
+  }
+  if (c->plan_state[b] == 1) {
+    const char* base = static_cast<const char*>(d.p);
+    *out = fec::PairPlan{reinterpret_cast<const int4*>(base), reinterpret_cast<const uint16_t*>(base + slot_bytes),
+                         reinterpret_cast<const uint32_t*>(base + slot_bytes + count_bytes), c->plan_nslots[b]};
+  }
+  return FEC_OK;
+}
+
 void invalidate_pattern(fec_ctx* c) {
   c->pattern_ready = false;
   c->groups_ready = false;
   c->d_node_groups.release();
+  for (DevBuf& b : c->d_plan) b.release();
+  c->plan_state.assign(c->plan_state.size(), 0);
   c->nnz = 0;
   c->d_colptr0.release();
   c->d_rowval32.release();
@@ -420,6 +521,7 @@ int fec_ctx_destroy(fec_ctx* c) {
                     &c->d_cg, &c->d_flag, &c->d_nbr_ptr, &c->d_nbr, &c->d_tile_counter, &c->d_node_groups})
     b->release();
   for (DevBuf& b : c->d_affine) b.release();
+  for (DevBuf& b : c->d_plan) b.release();
   c->cg_host.release();
   delete c;
   return FEC_OK;
@@ -1111,6 +1213,36 @@ int fec_assemble(fec_ctx* c, int want, int precision, double t, double dt, const
   if (want_r && (rc = ensure(c, c->d_Re, rsz * size_t(re_total)))) return rc;
   GatherArgs ga;
   memset(&ga, 0, sizeof ga);
+  ga.nn = c->nn;
+  ga.nf = c->nf;
+  ga.nblocks = int(c->blocks.size());
+  ga.nadj_ptr = static_cast<const int64_t*>(c->d_nadj_ptr.p);
+  ga.nadj = static_cast<const uint32_t*>(c->d_nadj.p);
+  ga.conn = static_cast<const int32_t*>(c->d_conn.p);
+  ga.epos = static_cast<const uint16_t*>(c->d_epos.p);
+  ga.umask = static_cast<const uint8_t*>(c->d_umask.p);
+  ga.col_base = static_cast<const int64_t*>(c->d_col_base.p);
+  ga.col_len = static_cast<const int32_t*>(c->d_col_len.p);
+  ga.dof_to_unknown = static_cast<const int64_t*>(c->d_dtu.p);
+  // meshes of mixed element sizes: with the tangent, one gather launch per group of nodes of one size
+  bool mixed_sizes = false;
+  for (const Block& B : c->blocks) mixed_sizes = mixed_sizes || B.nnpe != c->blocks[0].nnpe;
+  const bool groups = mixed_sizes && want_k && !gather_runs_generic();
+  // FP64 blocks stored as symmetric halves, alone of their element size: gathered by output entry
+  std::vector<fec::PairPlan> plans(c->blocks.size(), fec::PairPlan{nullptr, nullptr, nullptr, 0});
+  if (want_k && precision == FEC_FP64 && c->nf == 3 && (groups || c->blocks.size() == 1) && fec::gather_pairs_enabled())
+    for (size_t b = 0; b < c->blocks.size(); ++b) {
+      const Block& B = c->blocks[b];
+      bool alone = stores_pairs(c, b, precision, want_r, want_k, mixed);
+      for (size_t o = 0; o < c->blocks.size(); ++o) alone = alone && (o == b || c->blocks[o].nnpe != B.nnpe);
+      if (!alone) continue;
+      BlockInfo& bi = ga.blk[b];
+      bi.elem_start = B.elem_start;
+      bi.conn_off = B.conn_off;
+      bi.epos_off = B.epos_off;
+      bi.nnpe = B.nnpe;
+      if (int rc = pair_plan(c, ga, b, s, &plans[b])) return rc;
+    }
   int64_t ke_off = 0, re_off = 0, st_off = 0;
   for (size_t b = 0; b < c->blocks.size(); ++b) {
     const Block& B = c->blocks[b];
@@ -1187,10 +1319,9 @@ int fec_assemble(fec_ctx* c, int want, int precision, double t, double dt, const
     bi.ndof = ndof;
     // the hex8 mechanics kernels write the node-rows layout (the FP64 tensor-core
     // kernel the symmetric half), the class tensor-core kernels the symmetric half
-    const bool pairs = ea.ke_pairs ||
-                       (want_k && fec::class_tc_runs(B.physics, B.elem_type, precision, want_r, want_k, ea.affine != nullptr));
-    bi.layout = pairs ? fec::KE_PAIRS
-                      : (B.elem_type == FEC_HEX8 && (B.physics == FEC_PHYS_NEOHOOKEAN || B.physics == FEC_PHYS_J2 ||
+    bi.layout = stores_pairs(c, b, precision, want_r, want_k, mixed)
+                    ? fec::KE_PAIRS
+                    : (B.elem_type == FEC_HEX8 && (B.physics == FEC_PHYS_NEOHOOKEAN || B.physics == FEC_PHYS_J2 ||
                                                      tc_closure(B, precision)))
                             ? fec::KE_NODE_ROWS
                             : fec::KE_ROW_MAJOR;
@@ -1208,34 +1339,22 @@ int fec_assemble(fec_ctx* c, int want, int precision, double t, double dt, const
     }
     if (e != cudaSuccess) return fail(c, FEC_ERR_CUDA, "element kernel launch: %s", cudaGetErrorString(e));
   }
-  ga.nn = c->nn;
-  ga.nf = c->nf;
-  ga.nblocks = int(c->blocks.size());
-  ga.nadj_ptr = static_cast<const int64_t*>(c->d_nadj_ptr.p);
-  ga.nadj = static_cast<const uint32_t*>(c->d_nadj.p);
-  ga.conn = static_cast<const int32_t*>(c->d_conn.p);
-  ga.epos = static_cast<const uint16_t*>(c->d_epos.p);
-  ga.umask = static_cast<const uint8_t*>(c->d_umask.p);
-  ga.col_base = static_cast<const int64_t*>(c->d_col_base.p);
-  ga.col_len = static_cast<const int32_t*>(c->d_col_len.p);
-  ga.dof_to_unknown = static_cast<const int64_t*>(c->d_dtu.p);
   ga.Ke = c->d_Ke.p;
   ga.Re = c->d_Re.p;
   ga.nzval = want_k ? nzval : nullptr;
   ga.R_u = want_r ? R_u : nullptr;
   ga.acc_stride = c->acc_stride;
   cudaError_t e;
-  // meshes of mixed element sizes: with the tangent, one gather launch per group of nodes of one size
-  bool mixed_sizes = false;
-  for (const Block& B : c->blocks) mixed_sizes = mixed_sizes || B.nnpe != c->blocks[0].nnpe;
-  const bool groups = mixed_sizes && want_k && !gather_runs_generic();
   if (groups && !c->groups_ready)
     if (int rc = build_node_groups(c)) return rc;
   {
     LaunchTimer timer(c, s, "node_gather");
     if (groups)
       e = fec::launch_gather_groups(precision, c->nf, ga, static_cast<const int32_t*>(c->d_node_groups.p),
-                                    c->node_groups.data(), int(c->node_groups.size()), s, &c->last_launches);
+                                    c->node_groups.data(), int(c->node_groups.size()), plans.data(), s,
+                                    &c->last_launches);
+    else if (plans[0].slots)
+      e = fec::launch_pair_gather(ga, 0, plans[0], s, &c->last_launches);
     else
       e = fec::launch_gather(precision, c->nf, ga, s, &c->last_launches);
   }

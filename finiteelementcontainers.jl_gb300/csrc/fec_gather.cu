@@ -73,6 +73,13 @@ bool gather_pipe_enabled() {
   return !(e && e[0] == '0');
 }
 
+}  // namespace
+bool gather_pairs_enabled() {
+  const char* e = getenv("FEC_GATHER_PAIRS");
+  return !(e && e[0] == '0');
+}
+namespace {
+
 template <typename Real, bool PAIRS = false>
 cudaError_t go_pipe(const GatherArgs& g, cudaStream_t s, int* launches) {
   constexpr int MINB = 2;
@@ -113,13 +120,21 @@ cudaError_t by_size(const GatherArgs& g, cudaStream_t s, int* launches) {
   }
 }
 template <typename Real, int NF>
-cudaError_t groups(const GatherArgs& g0, const int32_t* nodes, const NodeGroup* grp, int ngroups, cudaStream_t s,
-                   int* launches) {
+cudaError_t groups(const GatherArgs& g0, const int32_t* nodes, const NodeGroup* grp, int ngroups,
+                   const PairPlan* plans, cudaStream_t s, int* launches) {
   for (int i = 0; i < ngroups; ++i) {
     GatherArgs g = g0;
     g.nodes = nodes + grp[i].off;
     g.nnodes = grp[i].count;
     cudaError_t e;
+    // the block whose plan covers the group (the only one of its element size)
+    int pb = -1;
+    for (int b = 0; plans && b < g.nblocks; ++b)
+      if (plans[b].slots && g.blk[b].nnpe == grp[i].A) pb = b;
+    if (pb >= 0) {
+      if ((e = launch_pair_gather(g, pb, plans[pb], s, launches)) != cudaSuccess) return e;
+      continue;
+    }
     switch (grp[i].A) {
       case 4: e = go<Real, NF, 4>(g, s, launches); break;
       case 8: e = go<Real, NF, 8>(g, s, launches); break;
@@ -134,13 +149,14 @@ cudaError_t groups(const GatherArgs& g0, const int32_t* nodes, const NodeGroup* 
 }  // namespace
 
 cudaError_t launch_gather_groups(int precision, int nf, const GatherArgs& g, const int32_t* nodes,
-                                 const NodeGroup* grp, int ngroups, cudaStream_t s, int* launches) {
+                                 const NodeGroup* grp, int ngroups, const PairPlan* plans, cudaStream_t s,
+                                 int* launches) {
   if (precision == 0) {
-    if (nf == 1) return groups<float2, 1>(g, nodes, grp, ngroups, s, launches);
-    if (nf == 3) return groups<float2, 3>(g, nodes, grp, ngroups, s, launches);
+    if (nf == 1) return groups<float2, 1>(g, nodes, grp, ngroups, plans, s, launches);
+    if (nf == 3) return groups<float2, 3>(g, nodes, grp, ngroups, plans, s, launches);
   } else if (precision == 1) {
-    if (nf == 1) return groups<float, 1>(g, nodes, grp, ngroups, s, launches);
-    if (nf == 3) return groups<float, 3>(g, nodes, grp, ngroups, s, launches);
+    if (nf == 1) return groups<float, 1>(g, nodes, grp, ngroups, plans, s, launches);
+    if (nf == 3) return groups<float, 3>(g, nodes, grp, ngroups, plans, s, launches);
   }
   return cudaErrorNotSupported;
 }

@@ -1270,12 +1270,17 @@ __global__ void __launch_bounds__(WPB * 32, MINB) node_gather_kernel(GatherArgs 
 // of element residuals); 313k elements of the action: 399 -> 30 us.
 constexpr int RCH = 8;  // elements whose loads are in flight per thread
 template <typename Real, int NF>
-__global__ void __launch_bounds__(256) residual_gather_kernel(GatherArgs g) {
+__device__ __forceinline__ void residual_gather_entry(const GatherArgs& g, int64_t t) {
   using RT = typename RE<Real>::T;
-  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t n = t / NF;
+  int64_t n = t / NF;
   const int i = int(t - n * NF);
-  if (n >= g.nn) return;
+  if (g.nodes) {
+    if (n >= g.nnodes) return;
+    n = g.nodes[n];
+    t = n * NF + i;
+  } else if (n >= g.nn) {
+    return;
+  }
   const unsigned um = g.umask[n];
   int64_t p = g.nadj_ptr[n];
   const int64_t p1 = g.nadj_ptr[n + 1];
@@ -1302,6 +1307,10 @@ __global__ void __launch_bounds__(256) residual_gather_kernel(GatherArgs g) {
       if (p + c < p1) racc += to_double(v[c]);
   }
   g.R_u[dtu] = racc;
+}
+template <typename Real, int NF>
+__global__ void __launch_bounds__(256) residual_gather_kernel(GatherArgs g) {
+  residual_gather_entry<Real, NF>(g, int64_t(blockIdx.x) * blockDim.x + threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------

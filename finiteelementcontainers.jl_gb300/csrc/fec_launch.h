@@ -39,8 +39,34 @@ struct NodeGroup {
   int A;
   int64_t off, count;
 };
+// plans: per block, or null; a block with a plan (slots set, alone of its element
+// size) is gathered by it.
+struct PairPlan;
 cudaError_t launch_gather_groups(int precision, int nf, const GatherArgs& args, const int32_t* nodes,
-                                 const NodeGroup* groups, int ngroups, cudaStream_t stream, int* launches);
+                                 const NodeGroup* groups, int ngroups, const PairPlan* plans, cudaStream_t stream,
+                                 int* launches);
+// The gather of one block's symmetric-half element matrices (KE_PAIRS, double-float
+// entries) by output entry (fec_pairgather.cu): its plan on the device and the launch,
+// which writes the CSC values of every node of the block and, when R_u is set, the
+// residual of g.nodes (all nodes when null).  Bitwise launch_gather's results.
+struct PairPlan {
+  const int4* slots;
+  const uint16_t* count;
+  const uint32_t* list;
+  int64_t nslots;
+};
+// Pairs and list entries per node (int32, nn); flags (int[2], zeroed by the caller):
+// [0] a node with too many rows or elements, [1] a node shared with another block.
+// unordered, unordered_count: scratch of the sizes of slots and count.
+cudaError_t pair_plan_count(const GatherArgs& g, int block, int64_t ne, int32_t* nslot, int32_t* nlist, int* flags,
+                            cudaStream_t stream);
+cudaError_t pair_plan_fill(const GatherArgs& g, int block, int64_t ne, const int64_t* slot0, const int64_t* list0,
+                           void* unordered, void* slots, uint16_t* unordered_count, uint16_t* count, uint32_t* list,
+                           int* flags, cudaStream_t stream);
+cudaError_t launch_pair_gather(const GatherArgs& g, int block, const PairPlan& plan, cudaStream_t stream,
+                               int* launches);
+// FEC_GATHER_PAIRS=0 keeps the per-node gathers.
+bool gather_pairs_enabled();
 // Matrix-free tangent action: element contributions K_e v_e (summed over points
 // in point order) into the residual workspace args.Re; V is the full direction
 // field (zero on Dirichlet dofs).  The state is read only.

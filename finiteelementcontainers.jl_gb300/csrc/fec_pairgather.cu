@@ -1,0 +1,294 @@
+// fec_pairgather.cu -- the gather of element matrices stored as symmetric halves
+// (KE_PAIRS) by output entry instead of by node.
+//
+// Two nodes n <= m share a block of nine entries in every element that has both.
+// The plan lists, for every such node pair, where those blocks are, in increasing
+// element order; a thread adds a row (three entries) of one pair over its list -- the
+// same additions in the same order as the per-node gathers (fec_kernels.cuh), so
+// bitwise their results -- and stores it at its two places, columns (n, k) and rows
+// (m, i), columns (m, i) and row (n, k).  Every stored block is read once (the
+// per-node gathers read it for both nodes), nothing goes through shared memory, and
+// the loads of a thread do not depend on one another.  Nodes with Dirichlet dofs need
+// no path of their own.
+//
+// Bound: latency and issue, then DRAM.  A hex8 node of a box has 14 pairs with lists
+// of 8, 4, 2 or 1; the pairs of GROUP consecutive nodes are ordered by the length of
+// their lists, so that the lanes of a warp have the same (in node order a warp runs
+// its longest list, and an entry per thread, not a row, spends most of its
+// instructions on addresses: 1,014 warp instructions a node).
+#include <type_traits>
+#include "fec_launch.h"
+#include "fec_pattern.h"
+
+namespace fec {
+namespace {
+
+constexpr int WPB = 8;      // warps per CTA of the plan kernel
+constexpr int MAXL = 1024;  // rows per column of a node
+constexpr int GROUP = 32;   // nodes whose pairs are ordered together
+constexpr int CLASSES = 64; // list lengths told apart
+
+// One warp per node n: its elements' nodes m >= n with an unknown component, told
+// apart by their row offset in n's columns.  FILL = false: how many pairs and list
+// entries n has; FILL = true: writes them.  flags[0]: a node with too many rows or
+// elements; flags[1]: a node of this block shared with another.
+struct PlanArgs {
+  int64_t nn, elem_start, ne, conn_off, epos_off;
+  int A;
+  bool shared;                     // several blocks: nodes may be shared
+  const int64_t* nadj_ptr;
+  const uint32_t* nadj;
+  const int32_t* conn;
+  const uint16_t* epos;
+  const uint8_t* umask;
+  const int32_t* col_len;
+  int32_t *nslot, *nlist;          // per node (FILL = false)
+  const int64_t *slot0, *list0;    // their exclusive sums (FILL = true)
+  int4* slots;                     // n, m, first list entry, row offsets of m in n's and of n in m's columns
+  uint16_t* count;                 // list entries of a slot
+  uint32_t* list;                  // (element * pairs + pair) << 1 | transposed
+  int* flags;
+};
+
+__device__ __forceinline__ bool owned(const PlanArgs& a, int64_t n) {
+  const int64_t p0 = a.nadj_ptr[n], p1 = a.nadj_ptr[n + 1];
+  return p1 > p0 && int64_t(a.nadj[p0] >> 5) >= a.elem_start && int64_t(a.nadj[p1 - 1] >> 5) < a.elem_start + a.ne;
+}
+
+template <bool FILL>
+__global__ void __launch_bounds__(WPB * 32) plan_kernel(PlanArgs a) {
+  __shared__ uint16_t s_cnt[WPB][MAXL], s_at[WPB][FILL ? MAXL : 1], s_rank[WPB][FILL ? MAXL : 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t n = int64_t(blockIdx.x) * WPB + warp;
+  if (n >= a.nn) return;
+  uint16_t* cnt = s_cnt[warp];
+  const int64_t p0 = a.nadj_ptr[n], p1 = a.nadj_ptr[n + 1];
+  const int L = a.col_len[n];
+  bool use = (a.umask[n] & 7u) != 0 && (!a.shared || owned(a, n));
+  if (use && (L > MAXL || (p1 - p0) * a.A > 65535)) {
+    if (lane == 0) a.flags[0] = 1;
+    use = false;
+  }
+  if (!use) {
+    if (!FILL && lane == 0) a.nslot[n] = a.nlist[n] = 0;
+    return;
+  }
+  for (int i = lane; i < L; i += 32) cnt[i] = 0;
+  __syncwarp();
+  // elements in order; an element's nodes are distinct, so its lanes are
+  for (int64_t p = p0; p < p1; ++p) {
+    const uint32_t packed = a.nadj[p];
+    const int64_t le = int64_t(packed >> 5) - a.elem_start;
+    if (lane < a.A) {
+      const int64_t m = a.conn[a.conn_off + le * a.A + lane];
+      if (!FILL && a.shared && !owned(a, m)) a.flags[1] = 1;
+      if (m >= n && (a.umask[m] & 7u)) ++cnt[a.epos[a.epos_off + (le * a.A + int(packed & 31u)) * a.A + lane]];
+    }
+    __syncwarp();
+  }
+  // pairs and list entries before each row offset
+  int slots = 0, entries = 0;
+  for (int i0 = 0; i0 < L; i0 += 32) {
+    const int i = i0 + lane, c = i < L ? cnt[i] : 0;
+    const unsigned mask = __ballot_sync(0xffffffffu, c > 0);
+    int inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (FILL && i < L) {
+      s_rank[warp][i] = uint16_t(slots + __popc(mask & ((1u << lane) - 1u)));
+      s_at[warp][i] = uint16_t(entries + inc - c);
+    }
+    slots += __popc(mask);
+    entries += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  if (!FILL) {
+    if (lane == 0) {
+      a.nslot[n] = slots;
+      a.nlist[n] = entries;
+    }
+    return;
+  }
+  __syncwarp();
+  const int np = a.A * (a.A + 1) / 2;
+  for (int64_t p = p0; p < p1; ++p) {
+    const uint32_t packed = a.nadj[p];
+    const int64_t le = int64_t(packed >> 5) - a.elem_start;
+    const int la = int(packed & 31u), lb = lane;
+    if (lb < a.A) {
+      const int32_t m = a.conn[a.conn_off + le * a.A + lb];
+      if (m >= n && (a.umask[m] & 7u)) {
+        const uint16_t* ep = a.epos + a.epos_off + le * a.A * a.A;
+        const int off = ep[la * a.A + lb];
+        const int c = cnt[off];
+        const int x = la < lb ? la : lb, y = la < lb ? lb : la;
+        const int64_t at = a.list0[n] + s_at[warp][off];
+        const int64_t block = le * np + x * (2 * a.A - x + 1) / 2 + y - x;
+        a.list[at] = uint32_t(block) << 1 | (la > lb ? 1u : 0u);
+        ++s_at[warp][off];
+        if (c != 0xffff) {  // the pair's first element (at is its first list entry)
+          const int64_t s = a.slot0[n] + s_rank[warp][off];
+          a.slots[s] = make_int4(int(n), m, int(uint32_t(at)), off | int(uint32_t(ep[lb * a.A + la]) << 16));
+          a.count[s] = uint16_t(c);
+          cnt[off] = 0xffff;
+        }
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// The slots of GROUP consecutive nodes by descending list length (a CTA per group).
+__global__ void __launch_bounds__(256) order_kernel(int64_t nn, const int64_t* slot0, const int4* in,
+                                                    const uint16_t* cin, int4* out, uint16_t* cout) {
+  __shared__ int hist[CLASSES];
+  const int64_t n0 = int64_t(blockIdx.x) * GROUP, n1 = n0 + GROUP < nn ? n0 + GROUP : nn;
+  const int64_t s0 = slot0[n0], s1 = slot0[n1];
+  auto cls = [](int c) { return c < CLASSES ? CLASSES - 1 - c : 0; };
+  for (int i = threadIdx.x; i < CLASSES; i += 256) hist[i] = 0;
+  __syncthreads();
+  for (int64_t s = s0 + threadIdx.x; s < s1; s += 256) atomicAdd(&hist[cls(cin[s])], 1);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int sum = 0;
+    for (int i = 0; i < CLASSES; ++i) {
+      const int h = hist[i];
+      hist[i] = sum;
+      sum += h;
+    }
+  }
+  __syncthreads();
+  for (int64_t s = s0 + threadIdx.x; s < s1; s += 256) {
+    const int c = cin[s];
+    const int64_t at = s0 + atomicAdd(&hist[cls(c)], 1);
+    out[at] = in[s];
+    cout[at] = uint16_t(c);
+  }
+}
+
+// Row k of pair slot s per thread (85 slots a CTA); the first nbr CTAs form the residual.
+constexpr int SLOTS = 85;
+__global__ void __launch_bounds__(256) pair_gather_kernel(GatherArgs g, PairPlan plan, int block, unsigned nbr) {
+  if (blockIdx.x < nbr) {
+    residual_gather_entry<float2, 3>(g, int64_t(blockIdx.x) * 256 + threadIdx.x);
+    return;
+  }
+  const int sl = int(threadIdx.x) / 3, k = int(threadIdx.x) - 3 * sl;
+  const int64_t s = int64_t(blockIdx.x - nbr) * SLOTS + sl;
+  if (sl >= SLOTS || s >= plan.nslots) return;
+  const int4 r = __ldg(plan.slots + s);
+  int left = __ldg(plan.count + s);
+  const uint32_t* lp = plan.list + uint32_t(r.z);
+  const unsigned un = g.umask[r.x], um = g.umask[r.y];
+  const int64_t cn = g.col_base[r.x], cm = g.col_base[r.y];
+  const int Ln = g.col_len[r.x], Lm = g.col_len[r.y];
+  const float2* Ke = static_cast<const float2*>(g.Ke) + g.blk[block].ke_off;
+  float2 acc[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+  auto add = [&](auto num) {  // the next `num` elements, loads first
+    constexpr int N = decltype(num)::value;
+    uint32_t at[N];
+    float2 v[N][3];
+#pragma unroll
+    for (int c = 0; c < N; ++c) at[c] = __ldg(lp + c);
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+      const bool tr = at[c] & 1u;
+      const float2* e = Ke + int64_t(at[c] >> 1) * 9 + (tr ? k : 3 * k);
+      const int d = tr ? 3 : 1;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) v[c][i] = __ldg(e + i * d);
+    }
+#pragma unroll
+    for (int c = 0; c < N; ++c)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) acc[i] = GatherAcc::plus(acc[i], v[c][i]);
+    lp += N;
+    left -= N;
+  };
+  while (left >= 4) add(std::integral_constant<int, 4>());
+  if (left >= 2) add(std::integral_constant<int, 2>());
+  if (left >= 1) add(std::integral_constant<int, 1>());
+  if (!((un >> k) & 1u)) return;
+  const int kk = __popc(un & ((1u << k) - 1u));
+  double* col = g.nzval + cn + int64_t(kk) * Ln + (r.w & 0xffff);
+  double* row = g.nzval + cm + int(uint32_t(r.w) >> 16) + kk;
+  int ii = 0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if ((um >> i) & 1u) {
+      const double v = GatherAcc::value(acc[i]);
+      col[ii] = v;
+      if (r.x != r.y) row[int64_t(ii) * Lm] = v;
+      ++ii;
+    }
+}
+
+}  // namespace
+
+cudaError_t pair_plan_count(const GatherArgs& g, int block, int64_t ne, int32_t* nslot, int32_t* nlist, int* flags,
+                            cudaStream_t s) {
+  PlanArgs a{};
+  const BlockInfo& B = g.blk[block];
+  a.nn = g.nn;
+  a.elem_start = B.elem_start;
+  a.ne = ne;
+  a.conn_off = B.conn_off;
+  a.epos_off = B.epos_off;
+  a.A = B.nnpe;
+  a.shared = g.nblocks > 1;
+  a.nadj_ptr = g.nadj_ptr;
+  a.nadj = g.nadj;
+  a.conn = g.conn;
+  a.epos = g.epos;
+  a.umask = g.umask;
+  a.col_len = g.col_len;
+  a.nslot = nslot;
+  a.nlist = nlist;
+  a.flags = flags;
+  plan_kernel<false><<<unsigned((g.nn + WPB - 1) / WPB), WPB * 32, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t pair_plan_fill(const GatherArgs& g, int block, int64_t ne, const int64_t* slot0, const int64_t* list0,
+                           void* unordered, void* slots, uint16_t* count2, uint16_t* count, uint32_t* list, int* flags,
+                           cudaStream_t s) {
+  PlanArgs a{};
+  const BlockInfo& B = g.blk[block];
+  a.nn = g.nn;
+  a.elem_start = B.elem_start;
+  a.ne = ne;
+  a.conn_off = B.conn_off;
+  a.epos_off = B.epos_off;
+  a.A = B.nnpe;
+  a.shared = g.nblocks > 1;
+  a.nadj_ptr = g.nadj_ptr;
+  a.nadj = g.nadj;
+  a.conn = g.conn;
+  a.epos = g.epos;
+  a.umask = g.umask;
+  a.col_len = g.col_len;
+  a.slot0 = slot0;
+  a.list0 = list0;
+  a.slots = static_cast<int4*>(unordered);
+  a.count = count2;
+  a.list = list;
+  a.flags = flags;
+  plan_kernel<true><<<unsigned((g.nn + WPB - 1) / WPB), WPB * 32, 0, s>>>(a);
+  order_kernel<<<unsigned((g.nn + GROUP - 1) / GROUP), 256, 0, s>>>(g.nn, slot0, a.slots, count2,
+                                                                     static_cast<int4*>(slots), count);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pair_gather(const GatherArgs& g, int block, const PairPlan& plan, cudaStream_t s, int* launches) {
+  const int64_t nodes = g.nodes ? g.nnodes : g.nn;
+  const int64_t nbr = g.R_u ? (nodes * 3 + 255) / 256 : 0, nbk = (plan.nslots + SLOTS - 1) / SLOTS;
+  if (nbr + nbk == 0) return cudaSuccess;
+  if (nbr + nbk > int64_t(0x7fffffff)) return cudaErrorInvalidValue;
+  pair_gather_kernel<<<unsigned(nbr + nbk), 256, 0, s>>>(g, plan, block, unsigned(nbr));
+  ++*launches;
+  return cudaGetLastError();
+}
+
+}  // namespace fec
