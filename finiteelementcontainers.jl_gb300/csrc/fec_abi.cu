@@ -289,13 +289,20 @@ bool tc_closure(const Block& B, int precision) {
 int num_fields_of(int physics) { return physics == FEC_PHYS_POISSON ? 1 : 3; }
 int num_states_of(int physics) { return (physics == FEC_PHYS_J2 || physics == FEC_PHYS_J2_MLP) ? 7 : 0; }
 
-// U[bc_dofs[i]-1] = vals[i]
-__global__ void set_dirichlet_kernel(double* U, int64_t n, const int64_t* dofs, const double* vals) {
+// U[bc_dofs[i]-1] = vals[i], then U[unknown_dofs[k]] = Uu[k] (unknown_dofs 0-based), in
+// one launch: a Dirichlet entry whose dof is an unknown loses to it.
+__global__ void update_field_kernel(double* U, int64_t nbc, const int64_t* bc_dofs, const double* bc_vals, int64_t n,
+                                    const int64_t* unknown_dofs, const int64_t* dtu, const double* Uu) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) U[dofs[i] - 1] = vals[i];
+  if (i < n) {
+    U[unknown_dofs[i]] = Uu[i];
+  } else if (i < n + nbc) {
+    const int64_t d = bc_dofs[i - n] - 1;
+    if (n == 0 || dtu[d] < 0) U[d] = bc_vals[i - n];
+  }
 }
 
-// U[unknown_dofs[k]] = Uu[k]  (unknown_dofs 0-based here)
+// U[unknown_dofs[k]] = Uu[k]
 __global__ void set_unknowns_kernel(double* U, int64_t n, const int64_t* unknown_dofs, const double* Uu) {
   const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k < n) U[unknown_dofs[k]] = Uu[k];
@@ -1146,14 +1153,12 @@ int fec_update_field(fec_ctx* c, double* U, const double* Uu, int64_t num_bc, co
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   c->n_timed = 0;
   LaunchTimer timer(c, s, "update_field");
-  if (num_bc > 0) {
-    set_dirichlet_kernel<<<unsigned((num_bc + 255) / 256), 256, 0, s>>>(U, num_bc, bc_dofs, bc_vals);
-    FEC_CUDA(c, cudaGetLastError());
-  }
-  if (c->n_unknowns > 0) {
-    if (!Uu) return fail(c, FEC_ERR_ARG, "Uu is NULL");
-    set_unknowns_kernel<<<unsigned((c->n_unknowns + 255) / 256), 256, 0, s>>>(
-        U, c->n_unknowns, static_cast<const int64_t*>(c->d_unknown_dofs.p), Uu);
+  if (c->n_unknowns > 0 && !Uu) return fail(c, FEC_ERR_ARG, "Uu is NULL");
+  const int64_t total = num_bc + c->n_unknowns;
+  if (total > 0) {
+    update_field_kernel<<<unsigned((total + 255) / 256), 256, 0, s>>>(
+        U, num_bc, bc_dofs, bc_vals, c->n_unknowns, static_cast<const int64_t*>(c->d_unknown_dofs.p),
+        static_cast<const int64_t*>(c->d_dtu.p), Uu);
     FEC_CUDA(c, cudaGetLastError());
   }
   return ok(c);
@@ -1265,6 +1270,7 @@ int fec_assemble(fec_ctx* c, int want, int precision, double t, double dt, const
     ea.closure = c->d_cl_args.p;
     ea.affine = affine_table(c, b, precision, mixed);
     ea.hex8_general = general_table(c, b, precision, mixed);
+    ea.hex8_tensor = B.tensor_rule ? 1 : 0;
     ea.ke_pairs = fp64_pairs(c, b, precision, want_k, mixed) ? 1 : 0;
     if (B.physics == FEC_PHYS_J2_MLP && !ea.closure)
       return fail(c, FEC_ERR_STATE, "block %d uses the learned closure but fec_closure_set was not called", int(b) + 1);
@@ -1839,6 +1845,7 @@ int fec_assemble_noalloc(fec_ctx* c, int want, int precision, double t, double d
     ea.closure = c->d_cl_args.p;
     ea.affine = affine_table(c, b, precision, false);
     ea.hex8_general = general_table(c, b, precision, false);
+    ea.hex8_tensor = B.tensor_rule ? 1 : 0;
     ea.ke_pairs = fp64_pairs(c, b, precision, want_k, false) ? 1 : 0;
     if (B.physics == FEC_PHYS_J2_MLP && !ea.closure)
       return fail(c, FEC_ERR_STATE, "block %d uses the learned closure but fec_closure_set was not called", int(b) + 1);

@@ -80,8 +80,11 @@ constexpr int T_SIG = W_BYTES;
 constexpr int T_G = T_SIG + NPAD * 4;
 constexpr int T_JXW = T_G + NQ * 24 * 8;
 constexpr int T_TEN = T_JXW + NQ * 8;           // TEN_N doubles, see tensor_gradient
-constexpr int TEN_N = 10 + 2 + NQ * 9;          // coefficients, diagonal flag (+ pad), Ji [q][k][j]
-constexpr int T_BYTES = T_TEN + TEN_N * 8;
+constexpr int TEN_N = 10 + 2 + NQ * 9;          // coefficients, box flag, separable-point flag, Ji [q][k][j]
+constexpr int T_OFF = T_TEN + TEN_N * 8;        // X_q - X_0 [q][3]
+constexpr int T_N = T_OFF + NQ * 24;            // shape functions [q][a]
+constexpr int T_K = T_N + NQ * 64;              // Poisson's element matrix [a][b]
+constexpr int T_BYTES = T_K + 64 * 8;
 static_assert(T_BYTES % 16 == 0 && T_G % 8 == 0, "table layout");
 constexpr int TMEM_COLS = 512;
 constexpr int TM_ENT = NLEV * NPAD;  // 96 columns after the accumulators: the slicers' scaled tangent entries (hi, lo)
@@ -502,20 +505,21 @@ __device__ __forceinline__ double signed_by(double d, unsigned bit) {
 // clocks per warp instruction.  Differences of values come first, so the
 // result is no further from the exact gradient.  co: I_x (own, across), I_y, then
 // I_y, I_z, I_z with the scales of gz, gy, gx folded in.
+__device__ __forceinline__ void tensor_gradient1(const double* co, int q, double v, double& gx, double& gy, double& gz) {
+  const double vx = __shfl_xor_sync(0xffffffffu, v, 1);
+  const double A = fma(co[0], v, mul_rn(co[1], vx)), B = signed_by(v - vx, q & 1);
+  const double Ay = __shfl_xor_sync(0xffffffffu, A, 2), By = __shfl_xor_sync(0xffffffffu, B, 2);
+  const double C = fma(co[4], A, mul_rn(co[5], Ay)), D = signed_by(A - Ay, q & 2);
+  const double E = fma(co[2], B, mul_rn(co[3], By));
+  const double Cz = __shfl_xor_sync(0xffffffffu, C, 4), Dz = __shfl_xor_sync(0xffffffffu, D, 4),
+               Ez = __shfl_xor_sync(0xffffffffu, E, 4);
+  gx = fma(co[8], E, mul_rn(co[9], Ez));
+  gy = fma(co[6], D, mul_rn(co[7], Dz));
+  gz = signed_by(C - Cz, q & 4);
+}
 __device__ __forceinline__ void tensor_gradient(const double* co, int q, const double (&v)[3], double (&g)[3][3]) {
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const double vx = __shfl_xor_sync(0xffffffffu, v[i], 1);
-    const double A = fma(co[0], v[i], mul_rn(co[1], vx)), B = signed_by(v[i] - vx, q & 1);
-    const double Ay = __shfl_xor_sync(0xffffffffu, A, 2), By = __shfl_xor_sync(0xffffffffu, B, 2);
-    const double C = fma(co[4], A, mul_rn(co[5], Ay)), D = signed_by(A - Ay, q & 2);
-    const double E = fma(co[2], B, mul_rn(co[3], By));
-    const double Cz = __shfl_xor_sync(0xffffffffu, C, 4), Dz = __shfl_xor_sync(0xffffffffu, D, 4),
-                 Ez = __shfl_xor_sync(0xffffffffu, E, 4);
-    g[i][0] = fma(co[8], E, mul_rn(co[9], Ez));
-    g[i][1] = fma(co[6], D, mul_rn(co[7], Dz));
-    g[i][2] = signed_by(C - Cz, q & 4);
-  }
+  for (int i = 0; i < 3; ++i) tensor_gradient1(co, q, v[i], g[i][0], g[i][1], g[i][2]);
 }
 
 // Point phase of quadrature point q of element e (FP64): the displacement gradient
@@ -1050,6 +1054,74 @@ __global__ void __launch_bounds__(R_EPB * NQ) hex8_action_kernel(ElemArgs g, con
   }
 }
 
+// Poisson on a block of translated elements (test/poisson/TestPoissonCommon.jl:75-107):
+// its element matrix is the block's constant, read from the table; the residual is
+// the transpose of the gradient applied to JxW grad u, less the source f(X_q) N_a JxW.
+// A box's points have two coordinates per direction, so its eight lanes share six
+// sines instead of forming 24.  FP64-pipe bound as before (about 70 instead of 460
+// FP64 operations a point with the matrix): 36 x 32 x 34 elements element
+// kernel 263 -> 48 us.
+template <bool WANT_R, bool WANT_K>
+__global__ void __launch_bounds__(R_EPB * NQ) hex8_poisson_kernel(ElemArgs g, const unsigned char* __restrict__ tab) {
+  __shared__ double s_ten[TEN_N], s_jxw[NQ], s_off[NQ * 3], s_n[NQ * 8];
+  __shared__ float2 s_k[64];
+  const int tid = threadIdx.x, el = tid >> 3, q = tid & 7, lane = tid & 31, l0 = lane & ~7;
+  const double* t = reinterpret_cast<const double*>(tab);
+  for (int i = tid; i < TEN_N; i += blockDim.x) s_ten[i] = __ldg(t + T_TEN / 8 + i);
+  if (tid < NQ) s_jxw[tid] = __ldg(t + T_JXW / 8 + tid);
+  if (tid < NQ * 3) s_off[tid] = __ldg(t + T_OFF / 8 + tid);
+  if (tid < NQ * 8) {
+    s_n[tid] = __ldg(t + T_N / 8 + tid);
+    s_k[tid] = df64_split(__ldg(t + T_K / 8 + tid));
+  }
+  __syncthreads();
+  const int64_t e = int64_t(blockIdx.x) * R_EPB + el;
+  const bool live = e < g.ne;
+  if (WANT_K && live) {  // row q of K_e
+    float4* dst = reinterpret_cast<float4*>(static_cast<float2*>(g.Ke) + (e * 8 + q) * 8);
+#pragma unroll
+    for (int b = 0; b < 8; b += 2)
+      dst[b / 2] = make_float4(s_k[q * 8 + b].x, s_k[q * 8 + b].y, s_k[q * 8 + b + 1].x, s_k[q * 8 + b + 1].y);
+  }
+  if (!WANT_R) return;
+  const int a = corner_node(q);
+  double u = 0.0, X0[3] = {0.0, 0.0, 0.0};
+  if (live) {
+    u = __ldg(&g.U[g.conn[e * 8 + a]]);
+    const int64_t n0 = g.conn[e * 8];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) X0[d] = __ldg(&g.coords[n0 * 3 + d]);
+  }
+  // source at the lane's point
+  double f = g.props[0] * s_jxw[q];
+  if (s_ten[11] != 0.0) {
+    const int d = q >> 1 < 3 ? q >> 1 : 2;  // lane 2d + side: the sine of that coordinate
+    const double sn = sinpi((d == 0 ? X0[0] : d == 1 ? X0[1] : X0[2]) + s_off[((q & 1) ? 7 : 0) * 3 + d]);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) f *= __shfl_sync(0xffffffffu, sn, l0 + 2 * k + (q >> k & 1));
+  } else {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) f *= sinpi(X0[d] + s_off[q * 3 + d]);
+  }
+  const double v = u - __shfl_sync(0xffffffffu, u, l0);
+  double g0, g1, g2;
+  tensor_gradient1(s_ten, q, v, g0, g1, g2);
+  const double* Ji = s_ten + 12 + q * 9;
+  const double w = s_jxw[q];
+  if (s_ten[10] == 0.0) {  // (dxi/dX)(dxi/dX)^T of the reference gradient
+    double p[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) p[j] = fma(g0, Ji[j], fma(g1, Ji[3 + j], mul_rn(g2, Ji[6 + j])));
+    g0 = fma(Ji[0], p[0], fma(Ji[1], p[1], mul_rn(Ji[2], p[2])));
+    g1 = fma(Ji[3], p[0], fma(Ji[4], p[1], mul_rn(Ji[5], p[2])));
+    g2 = fma(Ji[6], p[0], fma(Ji[7], p[1], mul_rn(Ji[8], p[2])));
+  }
+  double R = tensor_spread(s_ten, q, mul_rn(w, g0), mul_rn(w, g1), mul_rn(w, g2));
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) R = fma(-s_n[k * 8 + a], __shfl_sync(0xffffffffu, f, l0 + k), R);
+  if (live) static_cast<double*>(g.Re)[e * 8 + a] = R;
+}
+
 template <class Model>
 cudaError_t launch_act(const ElemArgs& a, const void* tab, const double* V, cudaStream_t s, int* launches) {
   const int64_t nb = (a.ne + R_EPB - 1) / R_EPB;
@@ -1114,7 +1186,8 @@ cudaError_t launch_hex8_affine_tc(int physics, bool want_r, bool want_k, const E
 }
 
 // Whether the reference tables are trilinear gradients at points (-+t_0, -+t_1,
-// -+t_2), x fastest (2 x 2 x 2 Gauss, Lobatto): c[d] = (1 + t_d) / 2 then.
+// -+t_2), x fastest (2 x 2 x 2 Gauss, Lobatto): c[d] = (1 + t_d) / 2 then.  (And the
+// shape functions sum to one: Poisson's points are offsets from node 0.)
 bool hex8_tensor_rule(const double* ref, double c[3]) {
   using L = RefLayout<1>;
   const double* dN = ref + L::DN_OFF;
@@ -1126,6 +1199,11 @@ bool hex8_tensor_rule(const double* ref, double c[3]) {
     for (int a = 0; a < 8; ++a)
       if ((corner(a) >> d & 1) && (corner(a) >> k & 1)) s += dN[(7 * 8 + a) * 3 + k];
     c[d] = 2.0 * s;
+  }
+  for (int q = 0; q < 8; ++q) {
+    double sum = 0.0;
+    for (int a = 0; a < 8; ++a) sum += ref[L::N_OFF + q * 8 + a];
+    if (!(std::fabs(sum - 1.0) <= 1e-14)) return false;
   }
   for (int q = 0; q < 8; ++q)
     for (int a = 0; a < 8; ++a)
@@ -1179,6 +1257,21 @@ cudaError_t launch_hex8_action(int physics, const ElemArgs& a, const double* V, 
   if (physics == 3 && a.affine) return aff::launch_act<aff::AffJ2>(a, a.affine, V, s, launches);
   if (physics == 2 && a.hex8_general) return aff::launch_act<aff::GenNeoHookean>(a, a.hex8_general, V, s, launches);
   return cudaErrorNotSupported;
+}
+
+cudaError_t launch_hex8_poisson(bool want_r, bool want_k, const ElemArgs& a, cudaStream_t s, int* launches) {
+  const int64_t nb = (a.ne + aff::R_EPB - 1) / aff::R_EPB;
+  if (nb == 0 || (!want_r && !want_k)) return cudaSuccess;
+  const unsigned char* tab = static_cast<const unsigned char*>(a.affine);
+  constexpr int T = aff::R_EPB * aff::NQ;
+  if (want_r && want_k)
+    aff::hex8_poisson_kernel<true, true><<<unsigned(nb), T, 0, s>>>(a, tab);
+  else if (want_r)
+    aff::hex8_poisson_kernel<true, false><<<unsigned(nb), T, 0, s>>>(a, tab);
+  else
+    aff::hex8_poisson_kernel<false, true><<<unsigned(nb), T, 0, s>>>(a, tab);
+  if (launches) ++*launches;
+  return cudaGetLastError();
 }
 
 // The operand of the reference element itself (the cube [-1, 1]^3).
@@ -1270,6 +1363,33 @@ bool hex8_affine_table(const double* x0, const double* ref, std::vector<unsigned
     ten[2 * k] = own[k];
     ten[2 * k + 1] = across[k];
   }
+  // Poisson: the points' offsets from node 0, shape functions, element matrix
+  double off[8][3], K[8][8] = {{0.0}};
+  const double* N = ref + L::N_OFF;
+  for (int q = 0; q < 8; ++q) {
+    for (int d = 0; d < 3; ++d) {
+      double s = 0.0;
+      for (int a = 1; a < 8; ++a) s = std::fma(N[q * 8 + a], x0[a * 3 + d] - x0[d], s);
+      off[q][d] = s;
+    }
+    for (int a = 0; a < 8; ++a)
+      for (int b = 0; b < 8; ++b) {
+        double s = 0.0;
+        for (int d = 0; d < 3; ++d) s = std::fma(dNX[q][a][d] * jxw[q], dNX[q][b][d], s);
+        K[a][b] += s;
+      }
+  }
+  bool separable = true;  // coordinate d of a point only depends on its bit d
+  for (int q = 0; q < 8; ++q) {
+    for (int d = 0; d < 3; ++d) {
+      const double h = std::fabs(off[7][d]) + std::fabs(off[0][d]);
+      separable = separable && std::fabs(off[q][d] - off[(q >> d & 1) ? 7 : 0][d]) <= 4e-16 * h;
+    }
+  }
+  ten[11] = separable ? 1.0 : 0.0;
+  std::memcpy(out.data() + aff::T_OFF, off, sizeof off);
+  std::memcpy(out.data() + aff::T_N, N, 64 * sizeof(double));
+  std::memcpy(out.data() + aff::T_K, K, sizeof K);
   std::memcpy(out.data() + aff::T_TEN, ten, sizeof ten);
   std::memcpy(out.data() + aff::T_SIG, sig, sizeof sig);
   std::memcpy(out.data() + aff::T_G, dNX, sizeof dNX);

@@ -69,6 +69,7 @@ struct ElemArgs {
   const void* hex8_general; // FP64 hex8 Neo-Hookean blocks of any shape: the reference element's operand table (or null)
   int* wait_err;            // set to 1 by a bounded wait that gave up (device flag; may be null)
   long long wait_budget;    // SM clocks a bounded wait allows before giving up (0: the default, ~1 s)
+  int hex8_tensor;          // affine: and the block's tables are a symmetric rule's (hex8_tensor_rule)
   int ke_pairs;             // the element kernel writes KE_PAIRS (FP64 hex8 tensor-core, FP64 hex27 kernels)
 };
 
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(EPB * Elem<ET>::NNPE) poisson_element_kernel(E
       if (WANT_R) {
         double f = g.props[0];
 #pragma unroll
-        for (int d = 0; d < D; ++d) f *= sin(M_PI * Xq[d]);
+        for (int d = 0; d < D; ++d) f *= sinpi(Xq[d]);
         s_f_all[ty][q] = Real(jxw * f);
 #pragma unroll
         for (int d = 0; d < D; ++d) {

@@ -123,6 +123,8 @@ cudaError_t launch_hex8_general_tc(bool want_r, bool want_k, const ElemArgs& arg
 // The FP64 matrix-free action on such blocks (args.affine: Neo-Hookean and J2;
 // args.hex8_general: Neo-Hookean), as launch_action.
 cudaError_t launch_hex8_action(int physics, const ElemArgs& args, const double* V, cudaStream_t stream, int* launches);
+// FP64 Poisson on a block of translated hex8 elements (args.affine) with such tables.
+cudaError_t launch_hex8_poisson(bool want_r, bool want_k, const ElemArgs& args, cudaStream_t stream, int* launches);
 bool hex8_general_table(const double* ref, std::vector<unsigned char>& out);
 bool hex8_general_enabled();
 // Tet10 (7) / hex27 (8) Neo-Hookean (2) or J2 (3) for a block whose element e is
