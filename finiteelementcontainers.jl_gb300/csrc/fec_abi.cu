@@ -82,6 +82,10 @@ struct fec_ctx {
   // pattern
   bool pattern_ready = false;
   int64_t nnz = 0;
+  // neighbour lists and column offsets: their total, and the host copies (after a build
+  // on the device fetched when first asked for)
+  int64_t n_nbr = 0;
+  bool lists_on_host = false, lists_on_device = false;
   std::vector<int64_t> nbr_ptr;
   std::vector<int32_t> nbr;
   std::vector<int64_t> col_base;
@@ -101,6 +105,7 @@ struct fec_ctx {
   fec::PcgHost cg_host;                // linear solve: where the host reads the stopping test
   DevBuf d_flag;                       // non-finite scan result
   DevBuf d_nbr_ptr, d_nbr;             // neighbour lists on the device (device symbolic phase, CSC fill)
+  DevBuf d_pat, d_rowoff;              // device symbolic phase: scratch, kept for the next pattern of the mesh
   DevBuf d_tile_counter;               // single launch of mixed element blocks: next work tile
   // node gather of a mesh of mixed element sizes: the nodes grouped by the element
   // size of their adjacent elements (built on first use, per pattern)
@@ -164,10 +169,14 @@ bool fp64_native_env() {
 }
 
 int upload(fec_ctx* c, DevBuf& b, const void* src, size_t bytes) {
-  b.release();
+  if (bytes == 0 || c->device < 0 || b.bytes < bytes || b.bytes / 2 > bytes) b.release();
   if (bytes == 0 || c->device < 0) return FEC_OK;
-  FEC_CUDA(c, cudaMalloc(&b.p, bytes));
-  b.bytes = bytes;
+  if (b.p) {  // the buffer of the last upload: nothing may still read it (as a release would wait)
+    FEC_CUDA(c, cudaDeviceSynchronize());
+  } else {
+    FEC_CUDA(c, cudaMalloc(&b.p, bytes));
+    b.bytes = bytes;
+  }
   FEC_CUDA(c, cudaMemcpy(b.p, src, bytes, cudaMemcpyHostToDevice));
   return FEC_OK;
 }
@@ -401,7 +410,7 @@ int pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s, fec::P
   const Block& B = c->blocks[b];
   // at most: a pair of neighbours once, a pair of element nodes once
   const int64_t np = int64_t(B.nnpe) * (B.nnpe + 1) / 2, max_list = B.ne * np;
-  const int64_t max_slots = std::min(max_list, (c->nbr_ptr.empty() ? max_list : (c->nbr_ptr.back() + c->nn) / 2));
+  const int64_t max_slots = std::min(max_list, (c->n_nbr + c->nn) / 2);
   const size_t slot_bytes = sizeof(int4) * size_t(max_slots), count_bytes = (2 * size_t(max_slots) + 15) / 16 * 16;
   DevBuf& d = c->d_plan[b];  // slots, counts, list
   if (c->plan_state[b] == 0) {
@@ -480,13 +489,36 @@ void invalidate_pattern(fec_ctx* c) {
   c->nnz = 0;
   c->d_colptr0.release();
   c->d_rowval32.release();
-  c->d_nadj_ptr.release();
-  c->d_nadj.release();
-  c->d_epos.release();
-  c->d_col_base.release();
-  c->d_col_len.release();
-  c->d_nbr_ptr.release();
-  c->d_nbr.release();
+  c->lists_on_host = c->lists_on_device = false;
+  // the pattern's device arrays are kept for the next one (the same mesh with other
+  // Dirichlet dofs: the same sizes but for the columns); nothing may still read them
+  if (c->device >= 0) cudaDeviceSynchronize();
+}
+
+// ... and given back when the mesh changes.
+void release_pattern(fec_ctx* c) {
+  for (DevBuf* b : {&c->d_nadj_ptr, &c->d_nadj, &c->d_epos, &c->d_col_base, &c->d_col_len, &c->d_nbr_ptr, &c->d_nbr,
+                    &c->d_pat, &c->d_rowoff})
+    b->release();
+}
+
+// The neighbour lists, column offsets and lengths on the host.
+int lists_to_host(fec_ctx* c) {
+  if (c->lists_on_host) return FEC_OK;
+  cudaSetDevice(c->device);
+  c->nbr_ptr.resize(size_t(c->nn + 1));
+  c->nbr.resize(size_t(c->n_nbr));
+  c->col_base.resize(size_t(c->nn));
+  c->col_len.resize(size_t(c->nn));
+  FEC_CUDA(c, cudaMemcpy(c->nbr_ptr.data(), c->d_nbr_ptr.p, sizeof(int64_t) * size_t(c->nn + 1), cudaMemcpyDeviceToHost));
+  if (c->n_nbr > 0)
+    FEC_CUDA(c, cudaMemcpy(c->nbr.data(), c->d_nbr.p, sizeof(int32_t) * size_t(c->n_nbr), cudaMemcpyDeviceToHost));
+  if (c->nn > 0) {
+    FEC_CUDA(c, cudaMemcpy(c->col_base.data(), c->d_col_base.p, sizeof(int64_t) * size_t(c->nn), cudaMemcpyDeviceToHost));
+    FEC_CUDA(c, cudaMemcpy(c->col_len.data(), c->d_col_len.p, sizeof(int32_t) * size_t(c->nn), cudaMemcpyDeviceToHost));
+  }
+  c->lists_on_host = true;
+  return FEC_OK;
 }
 
 }  // namespace
@@ -525,7 +557,8 @@ int fec_ctx_destroy(fec_ctx* c) {
   for (DevBuf* b : {&c->d_coords, &c->d_conn, &c->d_ref, &c->d_nadj_ptr, &c->d_nadj, &c->d_epos, &c->d_umask,
                     &c->d_col_base, &c->d_col_len, &c->d_dtu, &c->d_unknown_dofs, &c->d_Ke, &c->d_Re, &c->d_cl_w,
                     &c->d_cl_norm, &c->d_cl_cnt, &c->d_cl_args, &c->d_cl_img, &c->d_cl_table, &c->d_V, &c->d_colptr0, &c->d_rowval32,
-                    &c->d_cg, &c->d_flag, &c->d_nbr_ptr, &c->d_nbr, &c->d_tile_counter, &c->d_node_groups})
+                    &c->d_cg, &c->d_flag, &c->d_nbr_ptr, &c->d_nbr, &c->d_tile_counter, &c->d_node_groups, &c->d_pat,
+                    &c->d_rowoff})
     b->release();
   for (DevBuf& b : c->d_affine) b.release();
   for (DevBuf& b : c->d_plan) b.release();
@@ -702,6 +735,7 @@ int fec_mesh_set(fec_ctx* c, int dim, int64_t nn, const double* coords, int nblo
   c->n_unknowns = -1;
   c->nf = 0;
   invalidate_pattern(c);
+  release_pattern(c);
   return ok(c);
 }
 
@@ -817,8 +851,7 @@ int fec_pattern_build(fec_ctx* c, int64_t* nnz_out) {
   if (!c) return FEC_ERR_ARG;
   if (c->n_unknowns < 0) return fail(c, FEC_ERR_STATE, "fec_pattern_build before fec_dofs_set");
   if (c->device >= 0) cudaSetDevice(c->device);
-  c->d_nbr_ptr.release();  // device copies of the neighbour lists go with the pattern
-  c->d_nbr.release();
+  c->lists_on_device = false;  // device copies of the neighbour lists go with the pattern
   const int64_t nn = c->nn;
   // node -> (element, local node) adjacency, elements ascending
   std::vector<int64_t> nadj_ptr(nn + 1, 0);
@@ -948,6 +981,8 @@ int fec_pattern_build(fec_ctx* c, int64_t* nnz_out) {
       if (fullnbr[n]) um2[n] |= uint8_t(fec::UMASK_FULL_NBR);
     if ((rc = upload(c, c->d_umask, um2.data(), um2.size()))) return rc;
   }
+  c->n_nbr = nbr_ptr[nn];
+  c->lists_on_host = true;
   c->nbr_ptr = std::move(nbr_ptr);
   c->nbr = std::move(nbr);
   c->col_base = std::move(col_base);
@@ -991,32 +1026,22 @@ int fec_pattern_build_device(fec_ctx* c, int64_t* nnz_out, void* stream) {
     PB.epos_off[b] = B.epos_off;
     epos_total += (B.ne * B.nnpe * B.nnpe + 3) & ~int64_t(3);
   }
-  // scratch: counts/cursors (int32 nn), scan partials, flags
-  DevBuf t_cnt, t_cur, t_scan, t_flags, t_w, t_rowoff, t_um;
-  struct Frees {
-    DevBuf* b[7];
-    ~Frees() {
-      for (DevBuf* x : b) x->release();
-    }
-  } frees{{&t_cnt, &t_cur, &t_scan, &t_flags, &t_w, &t_rowoff, &t_um}};
+  // scratch: column sizes, scan partials, counts and cursors per node, flags, masks
   const size_t scan_n = fec::pattern_scan_scratch(nn + 1);
-  FEC_CUDA(c, cudaMalloc(&t_cnt.p, sizeof(int32_t) * size_t(nn + 1)));
-  FEC_CUDA(c, cudaMalloc(&t_cur.p, sizeof(int32_t) * size_t(nn + 1)));
-  FEC_CUDA(c, cudaMalloc(&t_scan.p, sizeof(int64_t) * scan_n));
-  FEC_CUDA(c, cudaMalloc(&t_flags.p, sizeof(int) * 4));
-  FEC_CUDA(c, cudaMalloc(&t_w.p, sizeof(int64_t) * size_t(nn + 1)));
-  FEC_CUDA(c, cudaMalloc(&t_um.p, size_t(nn + 1)));
-  int32_t* cnt = static_cast<int32_t*>(t_cnt.p);
-  int32_t* cur = static_cast<int32_t*>(t_cur.p);
-  int64_t* scan = static_cast<int64_t*>(t_scan.p);
-  int* flags = static_cast<int*>(t_flags.p);  // [0] overflow, [1] max column length, [2] max entries of a node
+  int rc;
+  if ((rc = ensure(c, c->d_pat, 8 * (size_t(nn + 1) + scan_n) + 4 * (2 * size_t(nn + 1) + 4) + size_t(nn + 1)))) return rc;
+  int64_t* w = static_cast<int64_t*>(c->d_pat.p);
+  int64_t* scan = w + nn + 1;
+  int32_t* cnt = reinterpret_cast<int32_t*>(scan + scan_n);
+  int32_t* cur = cnt + nn + 1;
+  int* flags = cur + nn + 1;  // [0] overflow, [1] max column length, [2] max entries of a node
+  uint8_t* um2 = reinterpret_cast<uint8_t*>(flags + 4);
   const uint8_t* um = static_cast<const uint8_t*>(c->d_umask.p);
   const int32_t* conn = static_cast<const int32_t*>(c->d_conn.p);
   FEC_CUDA(c, cudaMemsetAsync(flags, 0, sizeof(int) * 4, s));
   // node -> (element, local node) adjacency, elements ascending
   FEC_CUDA(c, cudaMemsetAsync(cnt, 0, sizeof(int32_t) * size_t(nn + 1), s));
   FEC_CUDA(c, fec::pattern_count_adjacency(conn, nent, cnt, s));
-  int rc;
   if ((rc = ensure(c, c->d_nadj_ptr, sizeof(int64_t) * size_t(nn + 1)))) return rc;
   if ((rc = ensure(c, c->d_nadj, sizeof(uint32_t) * size_t(nent > 0 ? nent : 1)))) return rc;
   int64_t* adj_ptr = static_cast<int64_t*>(c->d_nadj_ptr.p);
@@ -1041,12 +1066,11 @@ int fec_pattern_build_device(fec_ctx* c, int64_t* nnz_out, void* stream) {
     return fail(c, FEC_ERR_UNSUPPORTED, "a node gathers more than %d element nodes; use fec_pattern_build",
                 fec::PATTERN_CAND_CAP);
   if ((rc = ensure(c, c->d_nbr, sizeof(int32_t) * size_t(n_nbr > 0 ? n_nbr : 1)))) return rc;
-  FEC_CUDA(c, cudaMalloc(&t_rowoff.p, sizeof(int32_t) * size_t(n_nbr > 0 ? n_nbr : 1)));
+  if ((rc = ensure(c, c->d_rowoff, sizeof(int32_t) * size_t(n_nbr > 0 ? n_nbr : 1)))) return rc;
   int32_t* nbr = static_cast<int32_t*>(c->d_nbr.p);
-  int32_t* rowoff = static_cast<int32_t*>(t_rowoff.p);
+  int32_t* rowoff = static_cast<int32_t*>(c->d_rowoff.p);
   FEC_CUDA(c, fec::pattern_neighbours(PB, conn, adj_ptr, nadj, nn, um, cnt, col_len, nbr_ptr, nbr, rowoff, flags, s));
   // column sizes and offsets
-  int64_t* w = static_cast<int64_t*>(t_w.p);
   FEC_CUDA(c, fec::pattern_column_sizes(nn, um, col_len, w, flags + 1, flags + 2, s));
   if ((rc = ensure(c, c->d_col_base, sizeof(int64_t) * size_t(nn + 1)))) return rc;
   int64_t* col_base = static_cast<int64_t*>(c->d_col_base.p);
@@ -1066,21 +1090,11 @@ int fec_pattern_build_device(fec_ctx* c, int64_t* nnz_out, void* stream) {
   // element map and the full-neighbourhood flag
   if ((rc = ensure(c, c->d_epos, sizeof(uint16_t) * size_t(epos_total > 0 ? epos_total : 1)))) return rc;
   FEC_CUDA(c, fec::pattern_element_map(PB, conn, nbr_ptr, nbr, rowoff, static_cast<uint16_t*>(c->d_epos.p), s));
-  uint8_t* um2 = static_cast<uint8_t*>(t_um.p);
   FEC_CUDA(c, fec::pattern_full_neighbourhood(nn, c->nf, nbr_ptr, nbr, um, uint8_t(fec::UMASK_FULL_NBR), um2, s));
   if (nn > 0) FEC_CUDA(c, cudaMemcpyAsync(c->d_umask.p, um2, size_t(nn), cudaMemcpyDeviceToDevice, s));
-  // host copies for fec_pattern_get and the solver
-  c->nbr_ptr.resize(size_t(nn + 1));
-  c->nbr.resize(size_t(n_nbr));
-  c->col_base.resize(size_t(nn));
-  c->col_len.resize(size_t(nn));
-  FEC_CUDA(c, cudaMemcpyAsync(c->nbr_ptr.data(), nbr_ptr, sizeof(int64_t) * size_t(nn + 1), cudaMemcpyDeviceToHost, s));
-  if (n_nbr > 0)
-    FEC_CUDA(c, cudaMemcpyAsync(c->nbr.data(), nbr, sizeof(int32_t) * size_t(n_nbr), cudaMemcpyDeviceToHost, s));
-  if (nn > 0) {
-    FEC_CUDA(c, cudaMemcpyAsync(c->col_base.data(), col_base, sizeof(int64_t) * size_t(nn), cudaMemcpyDeviceToHost, s));
-    FEC_CUDA(c, cudaMemcpyAsync(c->col_len.data(), col_len, sizeof(int32_t) * size_t(nn), cudaMemcpyDeviceToHost, s));
-  }
+  c->n_nbr = n_nbr;
+  c->lists_on_host = false;  // (fetched when fec_pattern_get asks)
+  c->lists_on_device = true;
   FEC_CUDA(c, cudaStreamSynchronize(s));
   c->nnz = nnz;
   c->acc_stride = acc_stride;
@@ -1098,9 +1112,10 @@ int fec_pattern_get_device(const fec_ctx* cc, int64_t* colptr_dev, int64_t* rowv
   cudaSetDevice(c->device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int rc;
-  if (!c->d_nbr_ptr.p) {  // a host-built pattern: its neighbour lists go up once
+  if (!c->lists_on_device) {  // a host-built pattern: its neighbour lists go up once
     if ((rc = upload(c, c->d_nbr_ptr, c->nbr_ptr.data(), sizeof(int64_t) * c->nbr_ptr.size()))) return rc;
     if ((rc = upload(c, c->d_nbr, c->nbr.data(), sizeof(int32_t) * c->nbr.size()))) return rc;
+    c->lists_on_device = true;
   }
   FEC_CUDA(c, fec::pattern_csc(c->nn, c->nf, static_cast<const uint8_t*>(c->d_umask.p),
                                static_cast<const int64_t*>(c->d_dtu.p), static_cast<const int64_t*>(c->d_nbr_ptr.p),
@@ -1113,6 +1128,7 @@ int fec_pattern_get(const fec_ctx* cc, int64_t* colptr, int64_t* rowval) {
   fec_ctx* c = const_cast<fec_ctx*>(cc);
   if (!c) return FEC_ERR_ARG;
   if (!c->pattern_ready) return fail(c, FEC_ERR_STATE, "fec_pattern_get before fec_pattern_build");
+  if (int rc = lists_to_host(c)) return rc;
   const int nf = c->nf;
   if (colptr) {
     colptr[0] = 1;

@@ -41,4 +41,5 @@ def dirichlet_dofs(bcs, mesh, dof) -> np.ndarray:
     """unique(sort(all bc dofs)) (DirichletBCs.jl:396-398)."""
     if not bcs:
         return np.zeros(0, dtype=np.int64)
-    return np.unique(np.concatenate([bc.dofs_and_nodes(mesh, dof)[0] for bc in bcs]))
+    d = np.sort(np.concatenate([bc.dofs_and_nodes(mesh, dof)[0] for bc in bcs]))
+    return d[np.concatenate([[True], d[1:] != d[:-1]])] if d.size else d

@@ -42,17 +42,17 @@ class DofManager:
 
 def update_dofs(dof: DofManager, dirichlet_dofs) -> None:
     """update_dofs!(dof, dirichlet_dofs, [], []) (src/DofManagers.jl:227-298)."""
-    d = np.unique(np.asarray(dirichlet_dofs, dtype=np.int64))
+    d = np.asarray(dirichlet_dofs, dtype=np.int64).ravel()
     n = len(dof)
-    if d.size and (d[0] < 1 or d[-1] > n):
+    if d.size and (d.min() < 1 or d.max() > n):
         raise IndexError("Dirichlet dof out of range")
-    mask = np.ones(n, dtype=bool)
-    mask[d - 1] = False
-    dof.dirichlet_dofs = d
-    dof.unknown_dofs = np.nonzero(mask)[0].astype(np.int64) + 1
-    dtu = np.full(n, DIRICHLET_DOF, dtype=np.int64)
-    dtu[dof.unknown_dofs - 1] = np.arange(1, dof.unknown_dofs.size + 1, dtype=np.int64)
-    dof.dof_to_unknown = dtu
+    free = np.ones(n, dtype=bool)
+    free[d - 1] = False
+    fixed = ~free
+    dof.dirichlet_dofs = np.flatnonzero(fixed) + 1   # sorted, unique
+    dof.unknown_dofs = np.flatnonzero(free) + 1
+    dof.dof_to_unknown = np.cumsum(free, dtype=np.int64)
+    dof.dof_to_unknown[fixed] = DIRICHLET_DOF
 
 
 def create_unknowns(dof: DofManager, device=None):
