@@ -117,6 +117,7 @@ struct fec_ctx {
   std::vector<DevBuf> d_plan;
   std::vector<int64_t> plan_nslots;
   std::vector<int> plan_state;
+  std::vector<DevBuf> d_general;       // per block: the reference element's operand table of a tet10 block
   std::vector<DevBuf> d_affine;        // per block: the tensor-core operand table of a congruent hex8 block
                                        // or of a tet10/hex27 block of translation classes
   bool single_launch = false;          // FP64 mechanics: every element block in one launch
@@ -186,13 +187,17 @@ int upload(fec_ctx* c, DevBuf& b, const void* src, size_t bytes) {
 // host-only context, or for a degenerate first element.
 int build_affine(fec_ctx* c, size_t b) {
   if (c->d_affine.size() != c->blocks.size()) c->d_affine.resize(c->blocks.size());
+  if (c->d_general.size() != c->blocks.size()) c->d_general.resize(c->blocks.size());
   DevBuf& d = c->d_affine[b];
   d.release();
+  c->d_general[b].release();
   Block& B = c->blocks[b];
   double t[3];
   B.tensor_rule = B.elem_type == FEC_HEX8 && fec::hex8_tensor_rule(c->ref_host.data() + c->ref_off[b], t);
   if (c->device < 0) return FEC_OK;
   std::vector<unsigned char> tab;
+  if (B.elem_type == FEC_TET10 && fec::tet10_general_table(c->ref_host.data() + c->ref_off[b], tab))
+    if (int rc = upload(c, c->d_general[b], tab.data(), tab.size())) return rc;
   if (B.elem_type == FEC_HEX8 && !B.congruent) {
     if (!B.tensor_rule || !fec::hex8_general_table(c->ref_host.data() + c->ref_off[b], tab)) return FEC_OK;
   } else if (B.congruent) {
@@ -224,14 +229,19 @@ const void* affine_table(const fec_ctx* c, size_t b, int precision, bool mixed, 
   return (precision == FEC_FP32_ELEMENT || precision == FEC_FP64) ? c->d_affine[b].p : nullptr;
 }
 
-// The table of a Neo-Hookean hex8 block of elements of any shape on its own launch
-// (FP64, a symmetric rule), unless FEC_HEX8_GENERAL=0 or FEC_HEX8_DF64=tile.  A block
-// of translated elements has its own; with FEC_HEX8_AFFINE=0 it takes the per-element
-// kernels.
+// The table of a Neo-Hookean block of elements of any shape on its own launch (FP64, a
+// symmetric rule): hex8, unless FEC_HEX8_GENERAL=0 or FEC_HEX8_DF64=tile (a block of
+// translated elements has its own table; with FEC_HEX8_AFFINE=0 it takes the
+// per-element kernels), and tet10, unless FEC_TET10_GENERAL=0 (translation classes as
+// well, unless FEC_CLASS_TC=0).
 const void* general_table(const fec_ctx* c, size_t b, int precision, bool mixed) {
   const Block& B = c->blocks[b];
-  if (mixed || b >= c->d_affine.size() || B.elem_type != FEC_HEX8 || B.congruent || precision != FEC_FP64 ||
-      B.physics != FEC_PHYS_NEOHOOKEAN || fec::hex8_df64_tile_kernel() || !fec::hex8_general_enabled())
+  if (mixed || b >= c->d_affine.size() || precision != FEC_FP64 || B.physics != FEC_PHYS_NEOHOOKEAN) return nullptr;
+  if (B.elem_type == FEC_TET10)
+    return fp64_native_env() || !fec::tet10_general_enabled() || (B.nclass > 0 && !fec::class_tc_enabled())
+               ? nullptr
+               : c->d_general[b].p;
+  if (B.elem_type != FEC_HEX8 || B.congruent || fec::hex8_df64_tile_kernel() || !fec::hex8_general_enabled())
     return nullptr;
   return c->d_affine[b].p;
 }
@@ -256,14 +266,15 @@ bool hex27_pairs_enabled() {
 
 // Whether an assembly of block b with the stiffness runs an FP64 element kernel
 // that writes the symmetric half of K_e (KE_PAIRS): the hex8 tensor-core kernel
-// (instead of node rows, unless FEC_HEX8_PAIRS=0) and the hex27 double-float
-// kernel (on its own launch, unless FEC_HEX27_PAIRS=0).
+// (instead of node rows, unless FEC_HEX8_PAIRS=0), the tet10 one, and the hex27
+// double-float kernel (on its own launch, unless FEC_HEX27_PAIRS=0).
 bool fp64_pairs(const fec_ctx* c, size_t b, int precision, bool want_k, bool mixed) {
   const Block& B = c->blocks[b];
   if (!want_k || precision != FEC_FP64 || fp64_native_env() ||
       !(B.physics == FEC_PHYS_NEOHOOKEAN || B.physics == FEC_PHYS_J2))
     return false;
   if (B.elem_type == FEC_HEX27) return !mixed && hex27_pairs_enabled();
+  if (B.elem_type == FEC_TET10) return general_table(c, b, precision, mixed) != nullptr;
   return B.elem_type == FEC_HEX8 && fec::hex8_pairs_enabled() &&
          (affine_table(c, b, precision, mixed) || general_table(c, b, precision, mixed));
 }
@@ -561,6 +572,7 @@ int fec_ctx_destroy(fec_ctx* c) {
                     &c->d_rowoff})
     b->release();
   for (DevBuf& b : c->d_affine) b.release();
+  for (DevBuf& b : c->d_general) b.release();
   for (DevBuf& b : c->d_plan) b.release();
   c->cg_host.release();
   delete c;
@@ -730,6 +742,8 @@ int fec_mesh_set(fec_ctx* c, int dim, int64_t nn, const double* coords, int nblo
   c->ref_host = std::move(ref);
   for (DevBuf& d : c->d_affine) d.release();
   c->d_affine.assign(c->blocks.size(), DevBuf());
+  for (DevBuf& d : c->d_general) d.release();
+  c->d_general.assign(c->blocks.size(), DevBuf());
   for (size_t b = 0; b < c->blocks.size(); ++b)
     if ((rc = build_affine(c, b))) return rc;
   c->n_unknowns = -1;
@@ -1285,7 +1299,7 @@ int fec_assemble(fec_ctx* c, int want, int precision, double t, double dt, const
     ea.Re = want_r ? static_cast<char*>(c->d_Re.p) + rsz * size_t(re_off) : nullptr;
     ea.closure = c->d_cl_args.p;
     ea.affine = affine_table(c, b, precision, mixed);
-    ea.hex8_general = general_table(c, b, precision, mixed);
+    ea.general = general_table(c, b, precision, mixed);
     ea.hex8_tensor = B.tensor_rule ? 1 : 0;
     ea.ke_pairs = fp64_pairs(c, b, precision, want_k, mixed) ? 1 : 0;
     if (B.physics == FEC_PHYS_J2_MLP && !ea.closure)
@@ -1449,8 +1463,8 @@ int fec_assemble_action(fec_ctx* c, int precision, double t, double dt, const do
     // FP64 hex8 mechanics with the tables of a symmetric rule: the tensor-core kernel's
     // point phase; else blocks of translated elements: their constant gradients and JxW
     if (B.elem_type == FEC_HEX8 && B.physics != FEC_PHYS_POISSON) ea.affine = affine_table(c, b, precision, false);
-    ea.hex8_general = general_table(c, b, precision, false);
-    const bool tensor = ea.affine || ea.hex8_general;
+    ea.general = general_table(c, b, precision, false);
+    const bool tensor = ea.affine || ea.general;
     if (!tensor && B.elem_type == FEC_HEX8 && precision == FEC_FP64 && B.congruent)
       if (const void* tab = affine_table(c, b, precision, false, true))
         ea.affine = static_cast<const unsigned char*>(tab) + fec::hex8_affine_grad_offset();
@@ -1812,9 +1826,11 @@ int fec_assemble_noalloc(fec_ctx* c, int want, int precision, double t, double d
   int64_t ke_total = 0, ke_limit = 0, re_total = 0;
   for (size_t b = 0; b < c->blocks.size(); ++b) {
     ke_total += ke_entries(c, b, precision, want_k, false);
-    // (hex8 blocks of any shape count their whole element matrices against the limit,
-    // which the per-element kernels they may run write)
-    if (general_table(c, b, precision, false)) ke_limit += pad4(c->blocks[b].ne * 576);
+    // (blocks of any shape count their whole element matrices against the limit, which
+    // the per-element kernels they may run write)
+    const Block& B = c->blocks[b];
+    if (general_table(c, b, precision, false) && !(B.elem_type == FEC_TET10 && B.nclass > 0))
+      ke_limit += pad4(B.ne * (int64_t(9) * B.nnpe * B.nnpe));
     else ke_limit += ke_entries(c, b, precision, want_k, false);
     re_total += c->blocks[b].ne * c->nf * c->blocks[b].nnpe;
   }
@@ -1860,7 +1876,7 @@ int fec_assemble_noalloc(fec_ctx* c, int want, int precision, double t, double d
     ea.Re = want_r ? static_cast<char*>(Re) + rsz * size_t(re_off) : nullptr;
     ea.closure = c->d_cl_args.p;
     ea.affine = affine_table(c, b, precision, false);
-    ea.hex8_general = general_table(c, b, precision, false);
+    ea.general = general_table(c, b, precision, false);
     ea.hex8_tensor = B.tensor_rule ? 1 : 0;
     ea.ke_pairs = fp64_pairs(c, b, precision, want_k, false) ? 1 : 0;
     if (B.physics == FEC_PHYS_J2_MLP && !ea.closure)

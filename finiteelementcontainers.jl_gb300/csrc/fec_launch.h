@@ -115,18 +115,26 @@ size_t hex8_affine_grad_offset();
 // the KE_PAIRS layout, 36 * 9 entries per element) unless FEC_HEX8_PAIRS=0
 // (the node rows of the whole K_e, KE_NODE_ROWS).
 bool hex8_pairs_enabled();
-// FP64 hex8 Neo-Hookean on elements of any shape (args.hex8_general: the table
+// FP64 hex8 Neo-Hookean on elements of any shape (args.general: the table
 // hex8_general_table built): the same tensor-core contraction in reference
 // coordinates, whose constant operand is the reference element's.  Needs the tables
 // of a symmetric 2 x 2 x 2 rule.  FEC_HEX8_GENERAL=0 keeps the per-element kernels.
 cudaError_t launch_hex8_general_tc(bool want_r, bool want_k, const ElemArgs& args, cudaStream_t stream, int* launches);
 // The FP64 matrix-free action on such blocks (args.affine: Neo-Hookean and J2;
-// args.hex8_general: Neo-Hookean), as launch_action.
+// args.general: Neo-Hookean), as launch_action.
 cudaError_t launch_hex8_action(int physics, const ElemArgs& args, const double* V, cudaStream_t stream, int* launches);
 // FP64 Poisson on a block of translated hex8 elements (args.affine) with such tables.
 cudaError_t launch_hex8_poisson(bool want_r, bool want_k, const ElemArgs& args, cudaStream_t stream, int* launches);
 bool hex8_general_table(const double* ref, std::vector<unsigned char>& out);
 bool hex8_general_enabled();
+// FP64 tet10 Neo-Hookean on elements of any shape (args.general: the table
+// tet10_general_table built, for the quadratic tet at the symmetric 4-point rule):
+// with the stiffness on the tensor cores, written as KE_PAIRS; residual-only calls run
+// the same point phase and residual arithmetic.  FEC_TET10_GENERAL=0 keeps the other
+// kernels.
+cudaError_t launch_tet10_general(bool want_r, bool want_k, const ElemArgs& args, cudaStream_t stream, int* launches);
+bool tet10_general_table(const double* ref, std::vector<unsigned char>& out);
+bool tet10_general_enabled();
 // Tet10 (7) / hex27 (8) Neo-Hookean (2) or J2 (3) for a block whose element e is
 // a translate of element e mod P (args.affine: the table class_tc_table built):
 // the stiffness contraction on the tensor cores against each class's constant

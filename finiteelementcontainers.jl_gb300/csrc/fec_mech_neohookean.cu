@@ -204,7 +204,7 @@ cudaError_t launch_mech_neohookean(int elem_type, int precision, bool want_r, bo
         if (a.ne <= 0 || (!want_r && !want_k)) return cudaSuccess;
         return launch_hex8_affine_tc(2, want_r, want_k, a, s, launches);
       }
-      if (precision == 0 && a.hex8_general && !fp64_native()) {
+      if (precision == 0 && a.general && !fp64_native()) {
         if (a.ne <= 0 || (!want_r && !want_k)) return cudaSuccess;
         return launch_hex8_general_tc(want_r, want_k, a, s, launches);
       }
@@ -215,6 +215,7 @@ cudaError_t launch_mech_neohookean(int elem_type, int precision, bool want_r, bo
       return cudaErrorNotSupported;
     case 6: return tuned<6>(precision, want_r, want_k, a, s, launches);
     case 7:
+      if (precision == 0 && a.general) return launch_tet10_general(want_r, want_k, a, s, launches);
       if (class_tc_runs(2, 7, precision, want_r, want_k, a.affine != nullptr))
         return launch_class_tc(2, 7, precision, want_r, want_k, a, s, launches);
       return tuned<7>(precision, want_r, want_k, a, s, launches);
