@@ -117,7 +117,7 @@ struct fec_ctx {
   std::vector<DevBuf> d_plan;
   std::vector<int64_t> plan_nslots;
   std::vector<int> plan_state;
-  std::vector<DevBuf> d_general;       // per block: the reference element's operand table of a tet10 block
+  std::vector<DevBuf> d_general;       // per block: the reference element's table of a tet10 or hex27 block
   std::vector<DevBuf> d_affine;        // per block: the tensor-core operand table of a congruent hex8 block
                                        // or of a tet10/hex27 block of translation classes
   bool single_launch = false;          // FP64 mechanics: every element block in one launch
@@ -196,7 +196,9 @@ int build_affine(fec_ctx* c, size_t b) {
   B.tensor_rule = B.elem_type == FEC_HEX8 && fec::hex8_tensor_rule(c->ref_host.data() + c->ref_off[b], t);
   if (c->device < 0) return FEC_OK;
   std::vector<unsigned char> tab;
-  if (B.elem_type == FEC_TET10 && fec::tet10_general_table(c->ref_host.data() + c->ref_off[b], tab))
+  const double* ref = c->ref_host.data() + c->ref_off[b];
+  if ((B.elem_type == FEC_TET10 && fec::tet10_general_table(ref, tab)) ||
+      (B.elem_type == FEC_HEX27 && fec::hex27_general_table(ref, tab)))
     if (int rc = upload(c, c->d_general[b], tab.data(), tab.size())) return rc;
   if (B.elem_type == FEC_HEX8 && !B.congruent) {
     if (!B.tensor_rule || !fec::hex8_general_table(c->ref_host.data() + c->ref_off[b], tab)) return FEC_OK;
@@ -232,15 +234,15 @@ const void* affine_table(const fec_ctx* c, size_t b, int precision, bool mixed, 
 // The table of a Neo-Hookean block of elements of any shape on its own launch (FP64, a
 // symmetric rule): hex8, unless FEC_HEX8_GENERAL=0 or FEC_HEX8_DF64=tile (a block of
 // translated elements has its own table; with FEC_HEX8_AFFINE=0 it takes the
-// per-element kernels), and tet10, unless FEC_TET10_GENERAL=0 (translation classes as
-// well, unless FEC_CLASS_TC=0).
+// per-element kernels), and tet10 and hex27, unless FEC_TET10_GENERAL=0 or
+// FEC_HEX27_GENERAL=0 (translation classes as well, unless FEC_CLASS_TC=0).
 const void* general_table(const fec_ctx* c, size_t b, int precision, bool mixed) {
   const Block& B = c->blocks[b];
   if (mixed || b >= c->d_affine.size() || precision != FEC_FP64 || B.physics != FEC_PHYS_NEOHOOKEAN) return nullptr;
-  if (B.elem_type == FEC_TET10)
-    return fp64_native_env() || !fec::tet10_general_enabled() || (B.nclass > 0 && !fec::class_tc_enabled())
-               ? nullptr
-               : c->d_general[b].p;
+  if (B.elem_type == FEC_TET10 || B.elem_type == FEC_HEX27) {
+    const bool on = B.elem_type == FEC_TET10 ? fec::tet10_general_enabled() : fec::hex27_general_enabled();
+    return on && !fp64_native_env() && (B.nclass == 0 || fec::class_tc_enabled()) ? c->d_general[b].p : nullptr;
+  }
   if (B.elem_type != FEC_HEX8 || B.congruent || fec::hex8_df64_tile_kernel() || !fec::hex8_general_enabled())
     return nullptr;
   return c->d_affine[b].p;
@@ -1826,10 +1828,10 @@ int fec_assemble_noalloc(fec_ctx* c, int want, int precision, double t, double d
   int64_t ke_total = 0, ke_limit = 0, re_total = 0;
   for (size_t b = 0; b < c->blocks.size(); ++b) {
     ke_total += ke_entries(c, b, precision, want_k, false);
-    // (blocks of any shape count their whole element matrices against the limit, which
-    // the per-element kernels they may run write)
+    // (hex8 and tet10 blocks of any shape count their whole element matrices against the
+    // limit, which the per-element kernels they may run write)
     const Block& B = c->blocks[b];
-    if (general_table(c, b, precision, false) && !(B.elem_type == FEC_TET10 && B.nclass > 0))
+    if (B.elem_type != FEC_HEX27 && B.nclass == 0 && general_table(c, b, precision, false))
       ke_limit += pad4(B.ne * (int64_t(9) * B.nnpe * B.nnpe));
     else ke_limit += ke_entries(c, b, precision, want_k, false);
     re_total += c->blocks[b].ne * c->nf * c->blocks[b].nnpe;

@@ -135,6 +135,13 @@ bool hex8_general_enabled();
 cudaError_t launch_tet10_general(bool want_r, bool want_k, const ElemArgs& args, cudaStream_t stream, int* launches);
 bool tet10_general_table(const double* ref, std::vector<unsigned char>& out);
 bool tet10_general_enabled();
+// FP64 hex27 Neo-Hookean on elements of any shape (args.general: the table
+// hex27_general_table built, for tensor-product points numbered x fastest, the middle one at 0): the
+// stiffness by sum factorisation in double-float, the symmetric half (args.ke_pairs) or
+// whole (row-major).  FEC_HEX27_GENERAL=0 keeps the other kernels.
+cudaError_t launch_hex27_general(bool want_r, bool want_k, const ElemArgs& args, cudaStream_t stream, int* launches);
+bool hex27_general_table(const double* ref, std::vector<unsigned char>& out);
+bool hex27_general_enabled();
 // Tet10 (7) / hex27 (8) Neo-Hookean (2) or J2 (3) for a block whose element e is
 // a translate of element e mod P (args.affine: the table class_tc_table built):
 // the stiffness contraction on the tensor cores against each class's constant

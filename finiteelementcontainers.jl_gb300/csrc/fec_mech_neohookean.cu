@@ -220,6 +220,7 @@ cudaError_t launch_mech_neohookean(int elem_type, int precision, bool want_r, bo
         return launch_class_tc(2, 7, precision, want_r, want_k, a, s, launches);
       return tuned<7>(precision, want_r, want_k, a, s, launches);
     case 8:
+      if (precision == 0 && a.general) return launch_hex27_general(want_r, want_k, a, s, launches);
       if (class_tc_runs(2, 8, precision, want_r, want_k, a.affine != nullptr))
         return launch_class_tc(2, 8, precision, want_r, want_k, a, s, launches);
       if (precision == 1 && want_k && !hex27_on_cuda_cores())
