@@ -117,7 +117,7 @@ struct fec_ctx {
   std::vector<DevBuf> d_plan;
   std::vector<int64_t> plan_nslots;
   std::vector<int> plan_state;
-  std::vector<DevBuf> d_general;       // per block: the reference element's table of a tet10 or hex27 block
+  std::vector<DevBuf> d_general;       // per block: the reference element's table of a tet4, tet10 or hex27 block
   std::vector<DevBuf> d_affine;        // per block: the tensor-core operand table of a congruent hex8 block
                                        // or of a tet10/hex27 block of translation classes
   bool single_launch = false;          // FP64 mechanics: every element block in one launch
@@ -197,7 +197,8 @@ int build_affine(fec_ctx* c, size_t b) {
   if (c->device < 0) return FEC_OK;
   std::vector<unsigned char> tab;
   const double* ref = c->ref_host.data() + c->ref_off[b];
-  if ((B.elem_type == FEC_TET10 && fec::tet10_general_table(ref, tab)) ||
+  if ((B.elem_type == FEC_TET4 && fec::tet4_general_table(ref, tab)) ||
+      (B.elem_type == FEC_TET10 && fec::tet10_general_table(ref, tab)) ||
       (B.elem_type == FEC_HEX27 && fec::hex27_general_table(ref, tab)))
     if (int rc = upload(c, c->d_general[b], tab.data(), tab.size())) return rc;
   if (B.elem_type == FEC_HEX8 && !B.congruent) {
@@ -234,14 +235,18 @@ const void* affine_table(const fec_ctx* c, size_t b, int precision, bool mixed, 
 // The table of a Neo-Hookean block of elements of any shape on its own launch (FP64, a
 // symmetric rule): hex8, unless FEC_HEX8_GENERAL=0 or FEC_HEX8_DF64=tile (a block of
 // translated elements has its own table; with FEC_HEX8_AFFINE=0 it takes the
-// per-element kernels), and tet10 and hex27, unless FEC_TET10_GENERAL=0 or
-// FEC_HEX27_GENERAL=0 (translation classes as well, unless FEC_CLASS_TC=0).
+// per-element kernels), and tet4, tet10 and hex27, unless FEC_TET4_GENERAL=0,
+// FEC_TET10_GENERAL=0 or FEC_HEX27_GENERAL=0 (tet4 and translation classes: nor
+// FEC_CLASS_TC=0).
 const void* general_table(const fec_ctx* c, size_t b, int precision, bool mixed) {
   const Block& B = c->blocks[b];
   if (mixed || b >= c->d_affine.size() || precision != FEC_FP64 || B.physics != FEC_PHYS_NEOHOOKEAN) return nullptr;
-  if (B.elem_type == FEC_TET10 || B.elem_type == FEC_HEX27) {
-    const bool on = B.elem_type == FEC_TET10 ? fec::tet10_general_enabled() : fec::hex27_general_enabled();
-    return on && !fp64_native_env() && (B.nclass == 0 || fec::class_tc_enabled()) ? c->d_general[b].p : nullptr;
+  if (B.elem_type == FEC_TET4 || B.elem_type == FEC_TET10 || B.elem_type == FEC_HEX27) {
+    const bool on = B.elem_type == FEC_TET4    ? fec::tet4_general_enabled()
+                    : B.elem_type == FEC_TET10 ? fec::tet10_general_enabled()
+                                               : fec::hex27_general_enabled();
+    const bool classes = B.nclass > 0 || B.elem_type == FEC_TET4;
+    return on && !fp64_native_env() && (!classes || fec::class_tc_enabled()) ? c->d_general[b].p : nullptr;
   }
   if (B.elem_type != FEC_HEX8 || B.congruent || fec::hex8_df64_tile_kernel() || !fec::hex8_general_enabled())
     return nullptr;
@@ -268,15 +273,15 @@ bool hex27_pairs_enabled() {
 
 // Whether an assembly of block b with the stiffness runs an FP64 element kernel
 // that writes the symmetric half of K_e (KE_PAIRS): the hex8 tensor-core kernel
-// (instead of node rows, unless FEC_HEX8_PAIRS=0), the tet10 one, and the hex27
-// double-float kernel (on its own launch, unless FEC_HEX27_PAIRS=0).
+// (instead of node rows, unless FEC_HEX8_PAIRS=0), the tet4 and tet10 kernels for any
+// shape, and the hex27 ones (on their own launch, unless FEC_HEX27_PAIRS=0).
 bool fp64_pairs(const fec_ctx* c, size_t b, int precision, bool want_k, bool mixed) {
   const Block& B = c->blocks[b];
   if (!want_k || precision != FEC_FP64 || fp64_native_env() ||
       !(B.physics == FEC_PHYS_NEOHOOKEAN || B.physics == FEC_PHYS_J2))
     return false;
   if (B.elem_type == FEC_HEX27) return !mixed && hex27_pairs_enabled();
-  if (B.elem_type == FEC_TET10) return general_table(c, b, precision, mixed) != nullptr;
+  if (B.elem_type == FEC_TET4 || B.elem_type == FEC_TET10) return general_table(c, b, precision, mixed) != nullptr;
   return B.elem_type == FEC_HEX8 && fec::hex8_pairs_enabled() &&
          (affine_table(c, b, precision, mixed) || general_table(c, b, precision, mixed));
 }
@@ -1828,7 +1833,7 @@ int fec_assemble_noalloc(fec_ctx* c, int want, int precision, double t, double d
   int64_t ke_total = 0, ke_limit = 0, re_total = 0;
   for (size_t b = 0; b < c->blocks.size(); ++b) {
     ke_total += ke_entries(c, b, precision, want_k, false);
-    // (hex8 and tet10 blocks of any shape count their whole element matrices against the
+    // (hex8, tet4 and tet10 blocks of any shape count their whole element matrices against the
     // limit, which the per-element kernels they may run write)
     const Block& B = c->blocks[b];
     if (B.elem_type != FEC_HEX27 && B.nclass == 0 && general_table(c, b, precision, false))

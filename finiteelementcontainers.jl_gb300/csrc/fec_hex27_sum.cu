@@ -132,52 +132,18 @@ __device__ __forceinline__ double spread(const double* vd, const Lane& n, const 
   return r;
 }
 
-// A point's update in reference coordinates (GenNeoHookean's, c2 M formed), by way of
-// F = I + du/dX: a tenth less error in the residual than from dx/dxi, whose rounding the
-// element's condition multiplies, and no slower (0.65 ms both).
-struct Point {
-  double P[9], H[9], cM[6], a1h, a2;
-};
 __device__ __forceinline__ void point_phase(const ElemArgs& g, const double* vd, const Lane& n, double w, int node,
-                                            Point& m) {
-  double G[3][3], uo[3], Gi[3][3], gu[3][3], c[9];  // Gi = dxi/dX
+                                            RefPoint& m) {
+  double G[3][3], D[3][3], uo[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const double x = __ldg(&g.coords[int64_t(node) * 3 + d]);
     uo[d] = __ldg(&g.U[int64_t(node) * 3 + d]);
     gradient(vd, n, x, G[d]);
   }
-  GenNeoHookean::cofactors(G, c);
-  const double detG = fma(G[0][0], c[0], fma(G[0][1], c[1], mul_rn(G[0][2], c[2]))), rG = 1.0 / detG;
 #pragma unroll
-  for (int d = 0; d < 3; ++d)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) Gi[j][d] = mul_rn(c[d * 3 + j], rG);
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    double D[3];
-    gradient(vd, n, uo[d], D);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) gu[d][j] = fma(D[0], Gi[0][j], fma(D[1], Gi[1][j], mul_rn(D[2], Gi[2][j])));
-  }
-  AffNeoHookean::Mid s;
-  AffNeoHookean::point(g.props, gu, mul_rn(detG, w), nullptr, nullptr, s);
-#pragma unroll
-  for (int i = 0; i < 9; ++i) s.F[i] = fma(s.c2, s.F[i], -mul_rn(s.a2, s.H[i]));  // the stress
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      m.P[i * 3 + a] = fma(s.F[i * 3], Gi[a][0], fma(s.F[i * 3 + 1], Gi[a][1], mul_rn(s.F[i * 3 + 2], Gi[a][2])));
-      m.H[i * 3 + a] = fma(s.H[i * 3], Gi[a][0], fma(s.H[i * 3 + 1], Gi[a][1], mul_rn(s.H[i * 3 + 2], Gi[a][2])));
-    }
-  constexpr int A6[6] = {0, 1, 2, 1, 0, 0}, B6[6] = {0, 1, 2, 2, 2, 1};
-#pragma unroll
-  for (int k = 0; k < 6; ++k)
-    m.cM[k] = mul_rn(s.c2, fma(Gi[A6[k]][0], Gi[B6[k]][0],
-                               fma(Gi[A6[k]][1], Gi[B6[k]][1], mul_rn(Gi[A6[k]][2], Gi[B6[k]][2]))));
-  m.a1h = s.a1h;
-  m.a2 = s.a2;
+  for (int d = 0; d < 3; ++d) gradient(vd, n, uo[d], D[d]);
+  ref_point(g.props, G, D, w, m);
 }
 
 __device__ __forceinline__ Lane lane_place() {
@@ -361,7 +327,7 @@ __global__ void __launch_bounds__(NTHR, 1) hex27_sum_kernel(ElemArgs g, const do
     int64_t e = blockIdx.x + (tid - NCON) / 32 * G;
     int node = e < g.ne ? g.conn[e * A + n.l] : 0;
     for (int k = (tid - NCON) / 32; e < g.ne; e += NPROD * G, k += NPROD) {
-      Point m;
+      RefPoint m;
       const int at = node;
       if (e + NPROD * G < g.ne) node = g.conn[(e + NPROD * G) * A + n.l];
       point_phase(g, S.vd, n, w, at, m);
@@ -369,13 +335,12 @@ __global__ void __launch_bounds__(NTHR, 1) hex27_sum_kernel(ElemArgs g, const do
       if (use) wait_or_report(S.empty + slot, use - 1);  // its last element's entries are formed
       if (real) {
         float2* st = &S.stage[slot][0][n.l];
-        const float2 m23 = make_float2(-0.666666686534881591796875f, 1.98682155172491e-08f);  // -2/3 to 2^-50
-        const float2 b = df64_split(fma(-2.0 / 3.0, m.a2, m.a1h)), a2 = df64_split(m.a2);
+        const float2 b = df64_split(m.b), a2 = df64_split(m.a2);
 #pragma unroll
         for (int i = 0; i < 9; ++i) {
           const float2 h = df64_split(m.H[i]);
           st[i * NQ] = h;
-          st[(9 + i) * NQ] = df64_fma(b, h, df64_mul(m23, df64_split(m.P[i])));
+          st[(9 + i) * NQ] = tangent_z(b, h, m.P[i]);
           st[(18 + i) * NQ] = df64_mul(a2, h);
         }
 #pragma unroll
@@ -555,7 +520,7 @@ __global__ void __launch_bounds__(32 * R_WARPS) hex27_sum_r_kernel(ElemArgs g, c
   const int64_t e = int64_t(blockIdx.x) * R_WARPS + (threadIdx.x >> 5);
   if (e >= g.ne) return;
   const Lane n = lane_place();
-  Point m;
+  RefPoint m;
   point_phase(g, s_vd, n, __ldg(tab + T_W + n.l), g.conn[e * A + n.l], m);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {

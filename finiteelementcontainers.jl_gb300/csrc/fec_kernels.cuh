@@ -66,7 +66,7 @@ struct ElemArgs {
   void* Re;                 // block base, Real[ne][NDOF]
   const void* closure;      // learned-closure data (ClosureArgs) for the physics that uses one
   const void* affine;       // hex8 blocks of translated elements: the constant operand table (or null)
-  const void* general;      // FP64 hex8, tet10 and hex27 Neo-Hookean blocks of any shape: the reference element's table (or null)
+  const void* general;      // FP64 hex8, tet4, tet10 and hex27 Neo-Hookean blocks of any shape: the reference element's table (or null)
   int* wait_err;            // set to 1 by a bounded wait that gave up (device flag; may be null)
   long long wait_budget;    // SM clocks a bounded wait allows before giving up (0: the default, ~1 s)
   int hex8_tensor;          // affine: and the block's tables are a symmetric rule's (hex8_tensor_rule)

@@ -127,6 +127,11 @@ cudaError_t launch_hex8_action(int physics, const ElemArgs& args, const double* 
 cudaError_t launch_hex8_poisson(bool want_r, bool want_k, const ElemArgs& args, cudaStream_t stream, int* launches);
 bool hex8_general_table(const double* ref, std::vector<unsigned char>& out);
 bool hex8_general_enabled();
+// FP64 tet4 Neo-Hookean (args.general: the table tet4_general_table built), the stiffness
+// as KE_PAIRS.  FEC_TET4_GENERAL=0 keeps the per-element kernel.
+cudaError_t launch_tet4_general(bool want_r, bool want_k, const ElemArgs& args, cudaStream_t stream, int* launches);
+bool tet4_general_table(const double* ref, std::vector<unsigned char>& out);
+bool tet4_general_enabled();
 // FP64 tet10 Neo-Hookean on elements of any shape (args.general: the table
 // tet10_general_table built, for the quadratic tet at the symmetric 4-point rule):
 // with the stiffness on the tensor cores, written as KE_PAIRS; residual-only calls run

@@ -213,7 +213,9 @@ cudaError_t launch_mech_neohookean(int elem_type, int precision, bool want_r, bo
                              : hex8_df64<8>(want_r, want_k, a, s, launches);
       if (precision == 1) return hex8_f32<16>(want_r, want_k, a, s, launches);
       return cudaErrorNotSupported;
-    case 6: return tuned<6>(precision, want_r, want_k, a, s, launches);
+    case 6:
+      if (precision == 0 && a.general) return launch_tet4_general(want_r, want_k, a, s, launches);
+      return tuned<6>(precision, want_r, want_k, a, s, launches);
     case 7:
       if (precision == 0 && a.general) return launch_tet10_general(want_r, want_k, a, s, launches);
       if (class_tc_runs(2, 7, precision, want_r, want_k, a.affine != nullptr))
