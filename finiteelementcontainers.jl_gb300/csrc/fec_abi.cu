@@ -1469,8 +1469,11 @@ int fec_assemble_action(fec_ctx* c, int precision, double t, double dt, const do
     ea.Re = static_cast<char*>(c->d_Re.p) + rsz * size_t(re_off);
     // FP64 hex8 mechanics with the tables of a symmetric rule: the tensor-core kernel's
     // point phase; else blocks of translated elements: their constant gradients and JxW
-    if (B.elem_type == FEC_HEX8 && B.physics != FEC_PHYS_POISSON) ea.affine = affine_table(c, b, precision, false);
-    ea.general = general_table(c, b, precision, false);
+    // (the tables of the other element types are their assembly kernels' alone)
+    if (B.elem_type == FEC_HEX8 && B.physics != FEC_PHYS_POISSON) {
+      ea.affine = affine_table(c, b, precision, false);
+      ea.general = general_table(c, b, precision, false);
+    }
     const bool tensor = ea.affine || ea.general;
     if (!tensor && B.elem_type == FEC_HEX8 && precision == FEC_FP64 && B.congruent)
       if (const void* tab = affine_table(c, b, precision, false, true))
