@@ -43,8 +43,9 @@ __global__ void __launch_bounds__(EPB) tet4_kernel(ElemArgs g, const double* __r
                   uint32_t(i == k ? S_M + t / 9 : 63) << 16;
     }
   if (e < g.ne) {
-    const int4 c = __ldg(reinterpret_cast<const int4*>(g.conn) + e);
-    const int node[4] = {c.x, c.y, c.z, c.w};
+    int node[4];  // (a block's connectivity starts at any multiple of 4 bytes)
+#pragma unroll
+    for (int a = 0; a < 4; ++a) node[a] = __ldg(g.conn + e * 4 + a);
     double G[3][3], D[3][3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {

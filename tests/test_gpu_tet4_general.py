@@ -67,3 +67,18 @@ def test_calls_agree_bitwise(fec):
     K.nzval.fill_(float("nan"))
     fec.assemble_stiffness(asm, fec.stiffness, Uu, p)
     assert torch.equal(fec.stiffness(asm).nzval, nz)
+
+
+def test_block_after_one_of_odd_size(fec, orc):
+    """27 node numbers before the block's: its connectivity is not 16-byte aligned."""
+    import torch
+    from fec_gb300.meshes import box_hex27, merge_meshes
+    t = _mesh(fec, (3, 2, 2), 70)
+    mesh = merge_meshes([box_hex27((2, 2, 2)), t])
+    asm, p, U, Uu = _setup(fec, mesh)
+    R, K = fec.assemble_residual_and_stiffness(asm, Uu, p)
+    torch.cuda.synchronize()
+    args = (blocks_of(mesh), mesh.nodal_coords, "neohookean", p.physics[0].create_properties(), U)
+    Ro, _, _, nzo = orc.assembled_system(*args, asm.dof.dof_to_unknown, asm.dof.unknown_dofs)
+    assert max(rel_err(K.nzval.cpu().numpy(), nzo)) <= TOL64
+    assert max(rel_err(R.cpu().numpy(), Ro)[:2]) <= TOL64
