@@ -1550,6 +1550,7 @@ int fec_cg_solve(fec_ctx* c, const double* nzval, const double* b, double* x, in
   if ((rc = ensure(c, c->d_cg, sizeof(double) * fec::pcg_scratch_doubles(n)))) return rc;
   fec::CscSym A;
   A.n = n;
+  A.nnz = c->nnz;
   A.colptr = static_cast<const int64_t*>(c->d_colptr0.p);
   A.rowval = static_cast<const int32_t*>(c->d_rowval32.p);
   A.val = nzval;

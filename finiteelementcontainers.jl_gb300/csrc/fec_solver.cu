@@ -3,7 +3,8 @@
 // IterativeLinearSolver, src/Solvers.jl:88-152, which hands K and R to a Krylov
 // CG), on the device.
 //
-// K is symmetric, so its CSC columns are its rows.  An iteration is three
+// K is symmetric, so its CSC columns are its rows.  A matrix that fits the SMs' shared
+// memory is solved in one cooperative launch (cg_solve_kernel); else an iteration is three
 // kernels: y = K p with the partial sums of p.y, x and r updated with the
 // partial sums of r.z and r.r, and the new direction.  The partial sums of a
 // kernel (one per CTA) are added by every CTA of the next one in the same fixed
@@ -22,8 +23,9 @@
 // the host reads one batch of iterations behind, so the stream never runs dry and
 // the kernels of a batch that follow the converged iteration return at once.
 // Per iteration, Poisson: 36 x 32 x 34 elements 55 -> 15 us (product 7, update 4,
-// direction 4), 70^3 elements 59 us (product 44: 2.5 TB/s of matrix).
+// direction 4; 12 in one launch), 70^3 elements 59 us (product 44: 2.5 TB/s of matrix).
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include "fec_launch.h"
 #include "fec_solver.h"
@@ -317,6 +319,181 @@ __global__ void __launch_bounds__(THREADS) cg_test_kernel(CgScalars* sc, const d
   }
 }
 
+// The whole solve in one cooperative launch, for matrices that fit the SMs' shared
+// memory.  A CTA keeps its rows' entries there and their vectors in registers (KR rows a
+// thread); only p, which other rows read, and the partial sums go through memory.  An
+// iteration is three barriers over the grid -- the sums of p.y, those of r.z and r.r,
+// the new p -- and the arithmetic of the three kernels above.  A barrier is one atomic a
+// CTA and a bounded wait; a CTA that gives up reports through sc->done.
+//
+// What bounds it: latency -- three barriers, the FP64 sums on their way (a dozen dependent
+// additions each) and the gathers of p from L2 -- and the FP64 pipe in the product.  Whole
+// solves, three kernels an iteration against this: 60 elements 365 -> 312 us, 36 x 32 x 34
+// (35,805 unknowns) 2.05 -> 1.75 ms, 44 x 45 x 46 3.88 -> 2.91 ms: faster wherever it
+// applies.
+constexpr int KR = 4, COOP_CAP = 16384;  // entries of a CTA (one with more reads them from memory)
+constexpr size_t COOP_SMEM = size_t(COOP_CAP) * 12;
+constexpr long long COOP_BUDGET = 2000000000LL;
+struct CoopShape {
+  int64_t rows;  // of a CTA
+  unsigned grid;
+};
+__global__ void __launch_bounds__(THREADS, 1) cg_solve_kernel(CscSym A, int64_t rows, const double* __restrict__ b,
+                                                              double* x, double* p, int jacobi, double* parts,
+                                                              CgScalars* sc, unsigned long long* bar, int max_iter,
+                                                              int check_every, double rtol) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ SumBuf buf;
+  __shared__ double slot[2];
+  __shared__ int s_fail;
+  const int tid = threadIdx.x;
+  const int64_t r0 = int64_t(blockIdx.x) * rows, r1 = r0 + rows < A.n ? r0 + rows : A.n;
+  const int64_t base = A.colptr[r0];
+  const int cnt = int(A.colptr[r1] - base);
+  const double* val = A.val + base;
+  const int32_t* col = A.rowval + base;
+  if (cnt <= COOP_CAP) {
+    double* v = reinterpret_cast<double*>(sm);
+    int32_t* c = reinterpret_cast<int32_t*>(sm + size_t(COOP_CAP) * 8);
+    for (int i = tid; i < cnt; i += THREADS) {
+      v[i] = val[i];
+      c[i] = col[i];
+    }
+    val = v;
+    col = c;
+  }
+  if (tid == 0) s_fail = 0;
+  __syncthreads();
+  double* part_py = parts;
+  double* part_rz = parts + MAX_CTAS;
+  double* part_rr = parts + 2 * MAX_CTAS;
+  unsigned long long target = 0;
+  // false: a wait gave up, here or elsewhere
+  auto barrier = [&] {
+    target += gridDim.x;
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      atomicAdd(bar, 1ull);
+      const long long t0 = clock64();
+      while (*reinterpret_cast<volatile unsigned long long*>(bar) < target) {
+        if (clock64() - t0 > COOP_BUDGET) {
+          s_fail = 1;
+          atomicExch(&sc->done, -1);
+          break;
+        }
+      }
+      __threadfence();
+    }
+    __syncthreads();
+    return s_fail == 0;
+  };
+  int lo[KR], hi[KR];
+  double xk[KR], rk[KR], pk[KR], yk[KR], mk[KR];
+  // sum over row k of this thread of K_jc src_c; d: its diagonal entry
+  auto product = [&](const double* src, int k, double& d) {
+    const int64_t j = r0 + tid + k * THREADS;
+    double s = 0.0;
+    constexpr int U = 9;
+    for (int i = lo[k]; i < hi[k]; i += U) {
+      double xv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int cc = i + u < hi[k] ? col[i + u] : -1;
+        xv[u] = cc >= 0 ? __ldcg(src + cc) : 0.0;
+        if (cc == j) d = val[i + u];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (i + u < hi[k]) s = fma(val[i + u], xv[u], s);
+    }
+    return s;
+  };
+  double rz = 0.0, bb = 0.0;
+#pragma unroll
+  for (int k = 0; k < KR; ++k) {
+    const int64_t j = r0 + tid + k * THREADS;
+    lo[k] = hi[k] = 0;
+    xk[k] = rk[k] = pk[k] = yk[k] = 0.0;
+    mk[k] = 1.0;
+    if (j >= r1) continue;
+    lo[k] = int(A.colptr[j] - base);
+    hi[k] = int(A.colptr[j + 1] - base);
+    double d = 0.0;
+    const double bj = b[j];
+    rk[k] = bj - product(x, k, d);
+    xk[k] = x[j];
+    if (jacobi) mk[k] = d != 0.0 ? 1.0 / d : 1.0;
+    pk[k] = mk[k] * rk[k];
+    p[j] = pk[k];
+    rz = fma(rk[k], pk[k], rz);
+    bb = fma(bj, bj, bb);
+  }
+  cta_sums(buf, rz, bb, part_rz + blockIdx.x, part_rr + blockIdx.x);
+  if (!barrier()) return;
+  rz = total(part_rz, int(gridDim.x), slot);
+  bb = total(part_rr, int(gridDim.x), slot + 1);
+  double rr_test = 0.0;
+  int it_test = 0, done = bb == 0.0;
+  for (int it = 0; it < max_iter && !done;) {
+    double py = 0.0;
+#pragma unroll
+    for (int k = 0; k < KR; ++k) {
+      if (r0 + tid + k * THREADS >= r1) continue;
+      double d = 0.0;
+      yk[k] = product(p, k, d);
+      py = fma(pk[k], yk[k], py);
+    }
+    buf.a[tid] = py;
+    __syncthreads();
+    if (tid < 32) {
+      const double t = warp_total(buf.a);
+      if (tid == 0) part_py[blockIdx.x] = t;
+    }
+    if (!barrier()) return;
+    const double alpha = rz / total(part_py, int(gridDim.x), slot);
+    double rz1 = 0.0, rr = 0.0;
+    double zk[KR];
+#pragma unroll
+    for (int k = 0; k < KR; ++k) {
+      xk[k] = fma(alpha, pk[k], xk[k]);
+      rk[k] = fma(-alpha, yk[k], rk[k]);
+      zk[k] = mk[k] * rk[k];
+      rz1 = fma(rk[k], zk[k], rz1);
+      rr = fma(rk[k], rk[k], rr);
+    }
+    cta_sums(buf, rz1, rr, part_rz + blockIdx.x, part_rr + blockIdx.x);
+    if (!barrier()) return;
+    rz1 = total(part_rz, int(gridDim.x), slot);
+    ++it;
+    if (it % check_every == 0 || it == max_iter) {  // the stopping test
+      rr_test = total(part_rr, int(gridDim.x), slot + 1);
+      it_test = it;
+      done = sqrt(rr_test) / sqrt(bb) <= rtol;
+      if (done || it == max_iter) break;
+    }
+    const double beta = rz1 / rz;
+    rz = rz1;
+#pragma unroll
+    for (int k = 0; k < KR; ++k) {
+      const int64_t j = r0 + tid + k * THREADS;
+      pk[k] = fma(beta, pk[k], zk[k]);
+      if (j < r1) p[j] = pk[k];
+    }
+    if (!barrier()) return;
+  }
+#pragma unroll
+  for (int k = 0; k < KR; ++k) {
+    const int64_t j = r0 + tid + k * THREADS;
+    if (j < r1) x[j] = xk[k];
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    sc->bb = bb;
+    sc->rr = rr_test;
+    sc->it = it_test;
+  }
+}
+
 // A launch that may start while the kernel before it on the stream drains; its
 // kernels wait (grid_wait) before they read what that one wrote.
 template <typename... P, typename... Q>
@@ -355,7 +532,45 @@ void PcgHost::release() {
   }
 }
 
-size_t pcg_scratch_doubles(int64_t n) { return size_t(5) * size_t(n) + 3 * MAX_CTAS + SC_DOUBLES; }
+// Where the one-launch solve applies: the entries in the SMs' shared memory, at most KR
+// rows a thread.  FEC_CG_COOP=0 keeps the three kernels an iteration.
+static bool coop_shape(const CscSym& A, CoopShape* out) {
+  const char* v = std::getenv("FEC_CG_COOP");
+  const int64_t sms = num_sms() < MAX_CTAS ? num_sms() : MAX_CTAS;
+  const int64_t by_rows = (A.n + THREADS - 1) / THREADS, by_nnz = A.nnz / (COOP_CAP / 10 * 9) + 1;
+  int64_t grid = by_rows > by_nnz ? by_rows : by_nnz;
+  if (grid > sms) grid = sms;
+  if ((v && v[0] == '0') || A.nnz > grid * COOP_CAP || A.n > grid * KR * THREADS) return false;
+  int dev = 0, coop = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) {
+    cudaGetLastError();
+    return false;
+  }
+  out->rows = (A.n + grid - 1) / grid;
+  out->grid = unsigned((A.n + out->rows - 1) / out->rows);
+  return true;
+}
+
+size_t pcg_scratch_doubles(int64_t n) { return size_t(5) * size_t(n) + 3 * MAX_CTAS + SC_DOUBLES + 1; }
+
+// Reads the scalars of a finished solve.
+static cudaError_t finish(CgScalars& st, const CgScalars* sc, PcgHost& host, double* x, int64_t n, int max_iter,
+                          int* iterations, double* rel_residual, cudaStream_t s) {
+  cudaError_t e;
+  if ((e = cudaMemcpyAsync(host.pinned, sc, sizeof(CgScalars), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+  if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+  memcpy(&st, host.pinned, sizeof st);
+  if (st.done < 0) return cudaErrorLaunchTimeout;  // a barrier of the one-launch solve gave up
+  if (st.bb == 0.0) {  // x = 0 solves it
+    *iterations = 0;
+    *rel_residual = 0.0;
+    return cudaMemsetAsync(x, 0, sizeof(double) * size_t(n), s);
+  }
+  *iterations = st.it;
+  *rel_residual = max_iter > 0 ? std::sqrt(st.rr) / std::sqrt(st.bb) : 0.0;
+  return cudaSuccess;
+}
 
 cudaError_t pcg(const CscSym& A, const double* b, double* x, double* scratch, int max_iter, double rtol,
                 int check_every, bool jacobi, PcgHost& host, int* iterations, double* rel_residual, cudaStream_t s) {
@@ -380,6 +595,28 @@ cudaError_t pcg(const CscSym& A, const double* b, double* x, double* scratch, in
   if ((e = host.ensure()) != cudaSuccess || (e = ensure_smem<cg_init_kernel>(ROWS_SMEM)) != cudaSuccess ||
       (e = ensure_smem<cg_product_kernel>(ROWS_SMEM)) != cudaSuccess)
     return e;
+  CgScalars st;
+  CoopShape shape;
+  if (coop_shape(A, &shape)) {
+    unsigned long long* bar = reinterpret_cast<unsigned long long*>(sc) + SC_DOUBLES;
+    if ((e = ensure_smem<cg_solve_kernel>(COOP_SMEM)) != cudaSuccess ||
+        (e = cudaMemsetAsync(sc, 0, 8 * (SC_DOUBLES + 1), s)) != cudaSuccess)
+      return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(shape.grid);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = COOP_SMEM;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, cg_solve_kernel, A, shape.rows, b, x, p, jacobi ? 1 : 0, part_py, sc, bar, max_iter,
+                           check_every, rtol);
+    if (e != cudaSuccess) return e;
+    return finish(st, sc, host, x, n, max_iter, iterations, rel_residual, s);
+  }
   cg_init_kernel<<<gm, THREADS, ROWS_SMEM, s>>>(A, b, x, r, z, p, inv_diag, part_rz, part_py);
   cg_start_kernel<<<1, THREADS, 0, s>>>(part_rz, part_py, int(gm), sc);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -394,7 +631,6 @@ cudaError_t pcg(const CscSym& A, const double* b, double* x, double* scratch, in
     if (e1 == cudaSuccess) memcpy(out, static_cast<char*>(host.pinned) + (k & 1) * PcgHost::SLOT, sizeof(CgScalars));
     return e1;
   };
-  CgScalars st;
   int it = 0, batch = 0;
   while (it < max_iter) {
     const int end = max_iter - it < check_every ? max_iter : it + check_every;
@@ -417,17 +653,7 @@ cudaError_t pcg(const CscSym& A, const double* b, double* x, double* scratch, in
     ++batch;
   }
   // (after a break the batch just enqueued changed nothing)
-  if ((e = cudaMemcpyAsync(host.pinned, sc, sizeof(CgScalars), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
-  if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-  memcpy(&st, host.pinned, sizeof st);
-  if (st.bb == 0.0) {  // x = 0 solves it
-    *iterations = 0;
-    *rel_residual = 0.0;
-    return cudaMemsetAsync(x, 0, sizeof(double) * size_t(n), s);
-  }
-  *iterations = st.it;
-  *rel_residual = max_iter > 0 ? std::sqrt(st.rr) / std::sqrt(st.bb) : 0.0;
-  return cudaSuccess;
+  return finish(st, sc, host, x, n, max_iter, iterations, rel_residual, s);
 }
 
 }  // namespace fec

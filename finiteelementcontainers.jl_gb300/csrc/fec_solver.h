@@ -8,7 +8,7 @@ namespace fec {
 
 // Symmetric matrix in CSC over the unknowns (0-based), values on the device.
 struct CscSym {
-  int64_t n;
+  int64_t n, nnz;
   const int64_t* colptr;  // n + 1
   const int32_t* rowval;  // nnz
   const double* val;      // nnz
