@@ -113,7 +113,7 @@ struct fec_ctx {
   std::vector<fec::NodeGroup> node_groups;
   bool groups_ready = false;
   // per block: the plan of the gather by output entry (built on first use, per pattern);
-  // plan_state 0: not tried, 1: built, 2: the mesh has none
+  // plan_state 0: not assembled yet, 1: built, 2: the mesh has none, 3: assembled once, not tried
   std::vector<DevBuf> d_plan;
   std::vector<int64_t> plan_nslots;
   std::vector<int> plan_state;
@@ -412,11 +412,13 @@ bool stores_pairs(const fec_ctx* c, size_t b, int precision, bool want_r, bool w
                                        affine_table(c, b, precision, mixed) != nullptr));
 }
 
-// The plan of block b's gather by output entry (fec_pairgather.cu), built on first use
-// on stream s, before the element kernels: their workspace is its scratch.  slots null
-// where the block has none: nodes shared with other blocks or with very many elements,
-// indices that do not fit, no memory for it, or a first use under stream capture (the
-// per-node gathers then give the same bits).
+// The plan of block b's gather by output entry (fec_pairgather.cu), built at the second
+// assembly with a pattern on stream s, before the element kernels: their workspace is its
+// scratch.  (Building takes several times what an assembly then saves -- 128^3 hex8: 7 ms
+// against 0.9 -- so a pattern that is assembled once does without: first pass there 20.0 ->
+// 13.4 ms.)  slots null where the block has none: nodes shared with other blocks or with
+// very many elements, indices that do not fit, no memory for it, or a second use under
+// stream capture (the per-node gathers then give the same bits).
 int pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s, fec::PairPlan* out) {
   *out = fec::PairPlan{nullptr, nullptr, nullptr, 0};
   if (c->plan_state.size() != c->blocks.size()) {
@@ -432,6 +434,10 @@ int pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s, fec::P
   const size_t slot_bytes = sizeof(int4) * size_t(max_slots), count_bytes = (2 * size_t(max_slots) + 15) / 16 * 16;
   DevBuf& d = c->d_plan[b];  // slots, counts, list
   if (c->plan_state[b] == 0) {
+    c->plan_state[b] = 3;
+    return FEC_OK;
+  }
+  if (c->plan_state[b] == 3) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
       cudaGetLastError();
