@@ -2,7 +2,9 @@
 // (fec_hex8_affine_tc.cu, fec_tet10_tc.cu; the scheme is described in the former): the
 // Neo-Hookean update and its tangent entries, the accumulators' levels, barriers.
 #pragma once
+#include <cmath>
 #include <cstdint>
+#include <cstring>
 
 #include "fec_df64.cuh"
 #include "fec_kernels.cuh"
@@ -24,6 +26,21 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 }
 // 2^k as a float for k in [-126, 127]
 __device__ __forceinline__ float pow2f(int k) { return __uint_as_float(uint32_t(k + 127) << 23); }
+
+// Host: the seven digits of w, |w| < 2^e, at their place values 2^(-8s), as BF16 (each
+// exact).  Rounding by adding and subtracting 1.5 2^52: a table has 18,000 digits, whose
+// nearbyint and ldexp calls took 0.2 ms of setting a mesh.
+inline void bf16_digits(double w, int e, uint16_t (&out)[ND]) {
+  double y = std::ldexp(w, 7 - e), place = 1.0;  // |y| < 128, exact
+  for (int s = 0; s < ND; ++s, place *= 0x1p-8) {
+    const double d = (y + 0x1.8p52) - 0x1.8p52;
+    y = (y - d) * 256.0;
+    const float f = float(d * place);
+    uint32_t u;
+    std::memcpy(&u, &f, 4);
+    out[s] = uint16_t(u >> 16);
+  }
+}
 
 // Seven 4-column loads (the seven levels of one column chunk) under one wait.
 // NPAD: columns of a level.

@@ -1021,16 +1021,10 @@ bool hex8_affine_table(const double* x0, const double* ref, std::vector<unsigned
       if (e < -119 || e > 134) return false;  // the epilogue scales by 2^(e - 7) in FP32
       sig[n] = e;
       for (int r = 0; r < aff::KR; ++r) {
-        double y = std::ldexp(w[r], 7 - e);  // |y| < 128, exact
-        for (int s = 0; s < aff::ND; ++s) {
-          const double d = std::nearbyint(y);
-          y = (y - d) * 256.0;
-          const float fd = float(std::ldexp(d, -8 * s));  // digits at their place value
-          uint32_t u;
-          std::memcpy(&u, &fd, 4);
-          const uint16_t bits = uint16_t(u >> 16);
-          std::memcpy(out.data() + aff::T_W + s * aff::W_SLICE + aff::op_off(n, r % 9 * 8 + r / 9), &bits, 2);
-        }
+        uint16_t bits[aff::ND];
+        aff::bf16_digits(w[r], e, bits);
+        for (int s = 0; s < aff::ND; ++s)
+          std::memcpy(out.data() + aff::T_W + s * aff::W_SLICE + aff::op_off(n, r % 9 * 8 + r / 9), &bits[s], 2);
       }
     }
   // tensor_gradient's coefficients, with the scales dxi/dX folded in for a box

@@ -569,16 +569,9 @@ bool tet10_general_table(const double* ref, std::vector<unsigned char>& out) {
       if (e < -119 || e > 134) return false;  // the epilogue scales by 2^(e - 7) in FP32
       sig[n] = e;
       for (int r = 0; r < KR; ++r) {
-        double y = std::ldexp(w[r], 7 - e);  // |y| < 128, exact
-        for (int s = 0; s < ND; ++s) {
-          const double d = std::nearbyint(y);
-          y = (y - d) * 256.0;
-          const float fd = float(std::ldexp(d, -8 * s));  // digits at their place value
-          uint32_t u;
-          std::memcpy(&u, &fd, 4);
-          const uint16_t bits = uint16_t(u >> 16);
-          std::memcpy(out.data() + T_W + s * W_SLICE + op_off(n, r), &bits, 2);
-        }
+        uint16_t bits[ND];
+        bf16_digits(w[r], e, bits);
+        for (int s = 0; s < ND; ++s) std::memcpy(out.data() + T_W + s * W_SLICE + op_off(n, r), &bits[s], 2);
       }
     }
   double co[6] = {4.0 * b, 4.0 * (1.0 - 4.0 * b), wq[point[0]], wq[point[1]], wq[point[2]], wq[point[3]]};
