@@ -112,7 +112,7 @@ struct fec_ctx {
   DevBuf d_node_groups;
   std::vector<fec::NodeGroup> node_groups;
   bool groups_ready = false;
-  // per block: the plan of the gather by output entry (built on first use, per pattern);
+  // per block: the plan of the gather by output entry (built at the second assembly with a pattern);
   // plan_state 0: not assembled yet, 1: built, 2: the mesh has none, 3: assembled once, not tried
   std::vector<DevBuf> d_plan;
   std::vector<int64_t> plan_nslots;

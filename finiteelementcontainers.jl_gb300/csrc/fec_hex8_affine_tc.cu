@@ -44,10 +44,10 @@
 // What bounds it: every role is near the tile period (about 14k SM clocks a tile of
 // 12 elements), and straight-line code is what they all pay for -- five warps of a
 // sub-partition run different code, which does not fit the instruction cache, at
-// about five clocks an instruction (ncu: no-instruction stalls 3.3 per issue against
-// 1.2 for memory).  So the loops that can be small are kept small: one entry's digits
-// (four at once: 9.0 ms instead of 8.05), the MMA issue (unrolled: 9.4), one residual
-// component (three: 8.7).  128^3 Neo-Hookean: 8.05 ms; 64 x 56 x 60 J2: 0.84 ms.
+// about five clocks an instruction.  So the loops that can be small are kept small: one
+// entry's digits (four at once: 9.0 ms instead of 8.1), the MMA issue (unrolled: 9.4), one
+// residual component (three: 8.7); ncu's no-instruction stalls went from 3.3 to 0.9 per
+// issue.  Now FP64 pipe 49%, 2.3 instructions a clock, tensor pipe 23%.  128^3 Neo-Hookean: 8.2 ms; 64 x 56 x 60 J2: 0.85 ms.
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
