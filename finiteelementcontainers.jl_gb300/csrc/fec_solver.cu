@@ -23,7 +23,7 @@
 // the host reads one batch of iterations behind, so the stream never runs dry and
 // the kernels of a batch that follow the converged iteration return at once.
 // Per iteration, Poisson: 36 x 32 x 34 elements 55 -> 15 us (product 7, update 4,
-// direction 4; 12 in one launch), 70^3 elements 59 us (product 44: 2.5 TB/s of matrix).
+// direction 4; 11 in one launch), 70^3 elements 59 us (product 44: 2.5 TB/s of matrix).
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -56,14 +56,28 @@ __device__ __forceinline__ void grid_next() { asm volatile("griddepcontrol.launc
 struct SumBuf {
   double a[THREADS], b[THREADS];
 };
-__device__ __forceinline__ double warp_total(const double* v) {
-  const int lane = threadIdx.x & 31;
-  double t = v[lane];
+// (in pairs: a dependent FP64 addition takes over a hundred clocks, and these sums are a
+// third of an iteration)
+template <int N>
+__device__ __forceinline__ double pair_sum(double (&t)[N]) {
+  static_assert((N & (N - 1)) == 0, "pairs");
 #pragma unroll
-  for (int k = 1; k < THREADS / 32; ++k) t += v[lane + 32 * k];
+  for (int h = N / 2; h > 0; h /= 2)
+#pragma unroll
+    for (int k = 0; k < h; ++k) t[k] += t[k + h];
+  return t[0];
+}
+__device__ __forceinline__ double lanes_total(double t) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
   return t;
+}
+__device__ __forceinline__ double warp_total(const double* v) {
+  const int lane = threadIdx.x & 31;
+  double t[THREADS / 32];
+#pragma unroll
+  for (int k = 0; k < THREADS / 32; ++k) t[k] = v[lane + 32 * k];
+  return lanes_total(pair_sum(t));
 }
 __device__ __forceinline__ void cta_sums(SumBuf& buf, double a, double b, double* out_a, double* out_b) {
   buf.a[threadIdx.x] = a;
@@ -81,10 +95,18 @@ __device__ __forceinline__ void cta_sums(SumBuf& buf, double a, double b, double
 // every thread.
 __device__ __forceinline__ double total(const double* part, int count, double* slot) {
   if (threadIdx.x < 32) {
-    double s = 0.0;
-    for (int i = threadIdx.x; i < count; i += 32) s += __ldcg(part + i);
+    // (every load before the first addition)
+    double v[8], w[2] = {0.0, 0.0};
+    static_assert(MAX_CTAS <= 320, "ten a lane");
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    for (int i = 0; i < 8; ++i) v[i] = int(threadIdx.x) + 32 * i < count ? __ldcg(part + threadIdx.x + 32 * i) : 0.0;
+    if (count > 256)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (int(threadIdx.x) + 32 * (8 + i) < count) w[i] = __ldcg(part + threadIdx.x + 32 * (8 + i));
+    double s = pair_sum(v);
+    if (count > 256) s += w[0] + w[1];
+    s = lanes_total(s);
     if (threadIdx.x == 0) *slot = s;
   }
   __syncthreads();
@@ -326,10 +348,11 @@ __global__ void __launch_bounds__(THREADS) cg_test_kernel(CgScalars* sc, const d
 // the new p -- and the arithmetic of the three kernels above.  A barrier is one atomic a
 // CTA and a bounded wait; a CTA that gives up reports through sc->done.
 //
-// What bounds it: latency -- three barriers, the FP64 sums on their way (a dozen dependent
-// additions each) and the gathers of p from L2 -- and the FP64 pipe in the product.  Whole
-// solves, three kernels an iteration against this: 60 elements 365 -> 312 us, 36 x 32 x 34
-// (35,805 unknowns) 2.05 -> 1.75 ms, 44 x 45 x 46 3.88 -> 2.91 ms: faster wherever it
+// What bounds it: latency -- three barriers (2,500 clocks each), the FP64 sums on their way
+// (eight dependent additions each) and the gathers of p from L2 -- and the FP64 pipe in the
+// product.  (The next nine gathers in flight during the additions: no faster.)  Whole
+// solves, three kernels an iteration against this: 60 elements 364 -> 308 us, 36 x 32 x 34
+// (35,805 unknowns) 1.98 -> 1.61 ms, 44 x 45 x 46 3.77 -> 2.77 ms: faster wherever it
 // applies.
 constexpr int KR = 4, COOP_CAP = 16384;  // entries of a CTA (one with more reads them from memory)
 constexpr size_t COOP_SMEM = size_t(COOP_CAP) * 12;
@@ -373,17 +396,18 @@ __global__ void __launch_bounds__(THREADS, 1) cg_solve_kernel(CscSym A, int64_t 
     target += gridDim.x;
     __syncthreads();
     if (tid == 0) {
-      __threadfence();
-      atomicAdd(bar, 1ull);
+      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(bar), "l"(1ull) : "memory");
       const long long t0 = clock64();
-      while (*reinterpret_cast<volatile unsigned long long*>(bar) < target) {
+      for (;;) {
+        unsigned long long seen;
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(bar) : "memory");
+        if (seen >= target) break;
         if (clock64() - t0 > COOP_BUDGET) {
           s_fail = 1;
           atomicExch(&sc->done, -1);
           break;
         }
       }
-      __threadfence();
     }
     __syncthreads();
     return s_fail == 0;
@@ -456,6 +480,8 @@ __global__ void __launch_bounds__(THREADS, 1) cg_solve_kernel(CscSym A, int64_t 
     double zk[KR];
 #pragma unroll
     for (int k = 0; k < KR; ++k) {
+      zk[k] = 0.0;
+      if (k * THREADS >= rows) continue;  // (an FP64 instruction costs the same with no lane active)
       xk[k] = fma(alpha, pk[k], xk[k]);
       rk[k] = fma(-alpha, yk[k], rk[k]);
       zk[k] = mk[k] * rk[k];
@@ -477,6 +503,7 @@ __global__ void __launch_bounds__(THREADS, 1) cg_solve_kernel(CscSym A, int64_t 
 #pragma unroll
     for (int k = 0; k < KR; ++k) {
       const int64_t j = r0 + tid + k * THREADS;
+      if (k * THREADS >= rows) continue;
       pk[k] = fma(beta, pk[k], zk[k]);
       if (j < r1) p[j] = pk[k];
     }
