@@ -784,7 +784,9 @@ int fec_block_reference_set(fec_ctx* c, int block, int num_q, const double* N, c
   std::copy(w, w + NQ, t.begin() + size_t(NQ) * A * (1 + D));
   for (size_t i = 0; i < t.size(); ++i)
     if (!std::isfinite(t[i])) return fail(c, FEC_ERR_ARG, "block %d: table entry %zu is not finite", block, i);
-  std::copy(t.begin(), t.end(), c->ref_host.begin() + c->ref_off[block - 1]);
+  double* cur = c->ref_host.data() + c->ref_off[block - 1];
+  if (std::memcmp(cur, t.data(), sizeof(double) * t.size()) == 0) return ok(c);  // (the built-in rule handed over)
+  std::copy(t.begin(), t.end(), cur);
   if (c->device >= 0) {
     cudaSetDevice(c->device);
     // other blocks share the buffer: rewrite only this block's slice (kernels read it in stream order,
