@@ -641,8 +641,9 @@ cudaError_t pcg(const CscSym& A, const double* b, double* x, double* scratch, in
     cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, cg_solve_kernel, A, shape.rows, b, x, p, jacobi ? 1 : 0, part_py, sc, bar, max_iter,
                            check_every, rtol);
-    if (e != cudaSuccess) return e;
-    return finish(st, sc, host, x, n, max_iter, iterations, rel_residual, s);
+    if (e == cudaSuccess) return finish(st, sc, host, x, n, max_iter, iterations, rel_residual, s);
+    if (e != cudaErrorCooperativeLaunchTooLarge) return e;
+    cudaGetLastError();  // (a share of the device: fewer CTAs resident than SMs) the three kernels
   }
   cg_init_kernel<<<gm, THREADS, ROWS_SMEM, s>>>(A, b, x, r, z, p, inv_diag, part_rz, part_py);
   cg_start_kernel<<<1, THREADS, 0, s>>>(part_rz, part_py, int(gm), sc);
