@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(Roles<Model>::NTHR, 1) hex8_affine_tc_kernel(E
   int* s_taust = reinterpret_cast<int*>(sm + Lay::TAUST);
   uint32_t* s_code = reinterpret_cast<uint32_t*>(sm + Lay::CODE);
   uint64_t* bar_sl = reinterpret_cast<uint64_t*>(sm + Lay::BAR);  // slices of a tile written
-  uint64_t* bar_mma = bar_sl + 1;                                  // a tile's MMAs complete
+  uint64_t* bar_mma = bar_sl + 1;                                  // a tile's MMAs complete (and their issuer saw its slices)
   uint64_t* bar_tfree = bar_sl + 2;                                // the epilogue read a tile's accumulators
   float2* s_P = reinterpret_cast<float2*>(sm + Lay::P);
   float2* s_scr = reinterpret_cast<float2*>(sm + Lay::SCR);
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(Roles<Model>::NTHR, 1) hex8_affine_tc_kernel(E
   }
   if (tid == 0) {
     mbar_init(bar_sl, NSL);
-    mbar_init(bar_mma, 1);
+    mbar_init(bar_mma, 2);
     mbar_init(bar_tfree, 32 * EP_W);
     mbar_fence_init();
   }
@@ -539,14 +539,14 @@ __global__ void __launch_bounds__(Roles<Model>::NTHR, 1) hex8_affine_tc_kernel(E
     for (int k = 0;; ++k) {
       const int64_t tile = blockIdx.x + int64_t(k) * gridDim.x;
       if (tile >= ntiles) break;
-      const uint32_t par = uint32_t(k & 1);
-      wait_or_report(bar_sl, par);
       const int64_t e0 = tile * EPT;
       const bool live = used && e0 + el < g.ne;
-      const int tau = s_tau[(k & 1) * 16 + el];
-      const float f1 = pow2f(tau - 7);
-      wait_or_report(bar_mma, par);
+      // (bar_mma alone: its next phase needs this warp's arrival at bar_tfree.  The slicers'
+      // barrier may complete another phase as soon as the MMAs are done, and a warp that
+      // came that late would wait by parity for the phase after)
+      wait_or_report(bar_mma, uint32_t(k & 1));
       tc_fence_after();
+      const float f1 = pow2f(s_tau[(k & 1) * 16 + el] - 7);
 #pragma unroll 1
       for (int n0 = 0; n0 < NPAIR; n0 += 4) {
         float v[NLEV][4];
@@ -608,6 +608,7 @@ __global__ void __launch_bounds__(Roles<Model>::NTHR, 1) hex8_affine_tc_kernel(E
                        (t == 0 && kk == 0) ? 0u : 1u);
           }
         mma_commit(bar_mma);
+        mbar_arrive(bar_mma);  // (passes on what the slicers wrote before the slices: the scales)
       }
       __syncwarp();
     }

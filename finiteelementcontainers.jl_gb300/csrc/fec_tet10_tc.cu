@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(NTHR, 1) tet10_tc_kernel(ElemArgs g, const uns
   int* s_tau = reinterpret_cast<int*>(sm + Lay::TAU);
   uint32_t* s_code = reinterpret_cast<uint32_t*>(sm + Lay::CODE);
   uint64_t* bar_sl = reinterpret_cast<uint64_t*>(sm + Lay::BAR);  // slices of a half tile written
-  uint64_t* bar_mma = bar_sl + 1;                                  // its MMAs complete
+  uint64_t* bar_mma = bar_sl + 1;                                  // its MMAs complete (and their issuer saw its slices)
   uint64_t* bar_tfree = bar_sl + 2;                                // the epilogue read its accumulators
   uint64_t* bar_full = bar_sl + 3;                                 // per producer: a unit staged
   uint64_t* bar_empty = bar_full + NPROD;                          // and read by the slicers
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(NTHR, 1) tet10_tc_kernel(ElemArgs g, const uns
   }
   if (tid == 0) {
     mbar_init(bar_sl, NSL);
-    mbar_init(bar_mma, 1);
+    mbar_init(bar_mma, 2);
     mbar_init(bar_tfree, 32 * EP_W);
     for (int i = 0; i < NPROD; ++i) {
       mbar_init(bar_full + i, 32);
@@ -385,12 +385,11 @@ __global__ void __launch_bounds__(NTHR, 1) tet10_tc_kernel(ElemArgs g, const uns
       const int nh = halves(tile);
       for (int h = 0; h < nh; ++h, ++hh) {
         const uint32_t par = uint32_t(hh & 1);
-        wait_or_report(bar_sl, par);
         const int64_t e = tile * EPT + h * HALF_EL + el;
         const bool live = used && e < g.ne;
-        const float f1 = pow2f(s_tau[par * HALF_EL + el] - 7);
-        wait_or_report(bar_mma, par);
+        wait_or_report(bar_mma, par);  // (alone, as in the hex8 kernel)
         tc_fence_after();
+        const float f1 = pow2f(s_tau[par * HALF_EL + el] - 7);
         float2* dst = static_cast<float2*>(g.Ke) + e * (NPAIR * 9) + ik;
 #pragma unroll 1
         for (int n0 = 0; n0 < NPAIR; n0 += 4) {
@@ -435,6 +434,7 @@ __global__ void __launch_bounds__(NTHR, 1) tet10_tc_kernel(ElemArgs g, const uns
                          (t == 0 && kk == 0) ? 0u : 1u);
             }
           mma_commit(bar_mma);
+          mbar_arrive(bar_mma);  // (passes on what the slicers wrote before the slices: the scales)
         }
         __syncwarp();
       }
