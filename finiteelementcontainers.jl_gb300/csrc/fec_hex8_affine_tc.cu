@@ -52,6 +52,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "fec_digits.cuh"
@@ -263,20 +264,24 @@ __device__ __forceinline__ void point_phase(const ElemArgs& g, const double* s_t
   if (live) Model::point(g.props, gu, s_jxw[q], st, sn, m);
 }
 
-// The same on an element of any shape, X: its corner node's coordinates; s_ten: the
-// reference element's coefficients, w: the quadrature weight.
+// Its inputs on an element of any shape, X: its corner node's coordinates; s_ten: the
+// reference element's coefficients: dX/dxi and du/dxi at point q.
+__device__ __forceinline__ void general_gradients(const double* s_ten, int q, const double (&X)[3], const double (&uo)[3],
+                                                  double (&G)[3][3], double (&D)[3][3]) {
+  const int l0 = threadIdx.x & 24;
+  double v[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) v[d] = X[d] - __shfl_sync(0xffffffffu, X[d], l0);
+  tensor_gradient(s_ten, q, v, G);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) v[d] = uo[d] - __shfl_sync(0xffffffffu, uo[d], l0);
+  tensor_gradient(s_ten, q, v, D);
+}
 __device__ __forceinline__ void general_point(const ElemArgs& g, const double* s_ten, double w, int q, bool live,
-                                              const double (&X)[3], const double (&uo)[3], GenNeoHookean::Mid& m) {
-  const int lane = threadIdx.x & 31;
-  double v[3], G[3][3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) v[d] = X[d] - __shfl_sync(0xffffffffu, X[d], lane & ~7);
-  tensor_gradient(s_ten, q, v, G);
-  const double detG = GenNeoHookean::metric(G, m.M);
-#pragma unroll
-  for (int d = 0; d < 3; ++d) v[d] += uo[d] - __shfl_sync(0xffffffffu, uo[d], lane & ~7);
-  tensor_gradient(s_ten, q, v, G);
-  if (live) GenNeoHookean::point(g.props, G, detG, w, m);
+                                              const double (&X)[3], const double (&uo)[3], RefPoint& m) {
+  double G[3][3], D[3][3];
+  general_gradients(s_ten, q, X, uo, G, D);
+  if (live) ref_point(g.props, G, D, w, m);
 }
 
 // node pair n = (a, b), a <= b, as a << 4 | b
@@ -701,12 +706,15 @@ __global__ void __launch_bounds__(R_EPB * NQ) hex8_action_kernel(ElemArgs g, con
       if (Model::GENERAL) X[d] = __ldg(&g.coords[node * 3 + d]);
     }
   }
-  typename Model::Mid mid;
-  if constexpr (Model::GENERAL)
-    general_point(g, s_ten, s_jxw[q], q, live, X, uo, mid);
-  else
-    point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
   double D[3][3], out[3][3];
+  std::conditional_t<Model::GENERAL, PointUpdate, typename Model::Mid> mid;
+  if constexpr (Model::GENERAL) {
+    double G[3][3];
+    general_gradients(s_ten, q, X, uo, G, D);
+    if (live) point_update(g.props, G, D, s_jxw[q], mid);
+  } else {
+    point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
+  }
 #pragma unroll
   for (int d = 0; d < 3; ++d) v[d] -= __shfl_sync(0xffffffffu, v[d], lane & ~7);
   tensor_gradient(s_ten, q, v, D);

@@ -116,23 +116,15 @@ __device__ __forceinline__ void gradient_of(const Coef& k, int q, const double (
 }
 
 // Point phase of point q of an element; X, uo: coordinates and displacements of the
-// lane's four nodes (0 where not live).  The displacement has its own gradient: the
-// rounding of dX/dxi then is common to dx/dxi and cancels from the strain.  Every lane of
-// the warp calls it.
+// lane's four nodes (0 where not live).  Every lane of the warp calls it.
 __device__ __forceinline__ void point_phase(const ElemArgs& g, const Coef& k, double w, int q, bool live,
                                             const double (&X)[3][4], const double (&uo)[3][4], Model::Mid& m) {
-  double G[3][3];
+  double G[3][3], D[3][3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) gradient_of(k, q, X[d], G[d]);
-  const double detG = Model::metric(G, m.M);
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    double D[3];
-    gradient_of(k, q, uo[d], D);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) G[d][j] += D[j];
-  }
-  if (live) Model::point(g.props, G, detG, w, m);
+  for (int d = 0; d < 3; ++d) gradient_of(k, q, uo[d], D[d]);
+  if (live) ref_point(g.props, G, D, w, m);
 }
 
 // Component i of the element's residual from row i of JxW P at the lane's point, in FP64
@@ -300,7 +292,7 @@ __global__ void __launch_bounds__(NTHR, 1) tet10_tc_kernel(ElemArgs g, const uns
 #pragma unroll
         for (int i = 0; i < 9; ++i) {
           s_P[sp * 9 + i] = P2[i];
-          P[i] = fma(mid.c2s, mid.Q[i], -mul_rn(mid.a2, mid.H[i]));
+          P[i] = mid.P[i];
         }
       }
       // the element's scale 2^tau > |every tangent entry|
@@ -475,7 +467,7 @@ __global__ void __launch_bounds__(R_THR) tet10_r_kernel(ElemArgs g, const unsign
     double p[3] = {0.0, 0.0, 0.0};
     if (live)
 #pragma unroll
-      for (int j = 0; j < 3; ++j) p[j] = fma(mid.c2s, mid.Q[i * 3 + j], -mul_rn(mid.a2, mid.H[i * 3 + j]));
+      for (int j = 0; j < 3; ++j) p[j] = mid.P[i * 3 + j];
     residual_row(co, q, live, p, Re + i);
   }
 }
