@@ -50,6 +50,17 @@ struct CgScalars {
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// The step length, and the factor of the old direction in the new one: a / b, and 0 where b
+// is.  That is where the residual has become exactly zero (r.z = 0; p = 0 an iteration
+// later): x stays.  (Compared as an integer: off the FP64 pipe.)
+__device__ __forceinline__ double quotient(double a, double b) {
+  return (__double_as_longlong(b) << 1) == 0 ? 0.0 : a / b;
+}
+// The stopping test (rtol 0: none, every iteration asked for).
+__device__ __forceinline__ bool converged(double rr, double bb, double rtol) {
+  return rtol > 0.0 && sqrt(rr) / sqrt(bb) <= rtol;
+}
+
 // Sums over the CTA of a and b (fixed order), to thread 0 (a) and thread 32 (b).
 // Through shared memory: a shuffle tree in every warp would issue three times the
 // FP64 instructions.
@@ -282,7 +293,7 @@ __global__ void __launch_bounds__(THREADS) cg_update_kernel(int64_t n, const CgS
     if (inv_diag) mi = inv_diag[i];
   };
   load();
-  const double alpha = __ldcg(&sc->rz[parity]) / total(part_py, count, &slot);
+  const double alpha = quotient(__ldcg(&sc->rz[parity]), total(part_py, count, &slot));
   double rz = 0.0, rr = 0.0;
   while (i < n) {
     const int64_t k = i;
@@ -315,7 +326,7 @@ __global__ void __launch_bounds__(THREADS) cg_direction_kernel(int64_t n, CgScal
   };
   load();
   const double rz = total(part_rz, count, &slot);
-  const double beta = rz / __ldcg(&sc->rz[parity]);
+  const double beta = quotient(rz, __ldcg(&sc->rz[parity]));
   if (blockIdx.x == 0 && threadIdx.x == 0) sc->rz[parity ^ 1] = rz;
   while (i < n) {
     const int64_t k = i;
@@ -337,7 +348,7 @@ __global__ void __launch_bounds__(THREADS) cg_test_kernel(CgScalars* sc, const d
   if (threadIdx.x == 0) {
     sc->rr = rr;
     sc->it = it;
-    if (sqrt(rr) / sqrt(sc->bb) <= rtol) sc->done = 1;
+    if (converged(rr, sc->bb, rtol)) sc->done = 1;
   }
 }
 
@@ -475,7 +486,7 @@ __global__ void __launch_bounds__(THREADS, 1) cg_solve_kernel(CscSym A, int64_t 
       if (tid == 0) part_py[blockIdx.x] = t;
     }
     if (!barrier()) return;
-    const double alpha = rz / total(part_py, int(gridDim.x), slot);
+    const double alpha = quotient(rz, total(part_py, int(gridDim.x), slot));
     double rz1 = 0.0, rr = 0.0;
     double zk[KR];
 #pragma unroll
@@ -495,10 +506,10 @@ __global__ void __launch_bounds__(THREADS, 1) cg_solve_kernel(CscSym A, int64_t 
     if (it % check_every == 0 || it == max_iter) {  // the stopping test
       rr_test = total(part_rr, int(gridDim.x), slot + 1);
       it_test = it;
-      done = sqrt(rr_test) / sqrt(bb) <= rtol;
+      done = converged(rr_test, bb, rtol);
       if (done || it == max_iter) break;
     }
-    const double beta = rz1 / rz;
+    const double beta = quotient(rz1, rz);
     rz = rz1;
 #pragma unroll
     for (int k = 0; k < KR; ++k) {

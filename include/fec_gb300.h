@@ -197,7 +197,9 @@ int fec_assemble_action(fec_ctx* ctx, int precision, double t, double dt, const 
  * stiffness over the unknowns (nzval from fec_assemble; symmetric), K x = b,
  * starting from x.  preconditioner 0: none (the reference's Krylov CG), 1:
  * Jacobi.  Stops at ||b - K x|| <= rtol ||b|| (checked every 10 iterations) or
- * after max_iter; reports the iterations and the final relative residual.
+ * after max_iter (rtol 0: after max_iter); reports the iterations and the final
+ * relative residual.  A residual that reaches exactly zero in between leaves x as it
+ * is for the rest of them.
  * Bitwise repeatable.  Synchronises the stream.  Replaces the Krylov solve of
  * IterativeLinearSolver (src/Solvers.jl:88-152). */
 int fec_cg_solve(fec_ctx* ctx, const double* nzval_dev, const double* b_dev, double* x_dev, int max_iter,
