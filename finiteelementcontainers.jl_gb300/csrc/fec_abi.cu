@@ -1565,7 +1565,7 @@ int fec_cg_solve(fec_ctx* c, const double* nzval, const double* b, double* x, in
   int it = 0;
   double rr = 0.0;
   const cudaError_t e = fec::pcg(A, b, x, static_cast<double*>(c->d_cg.p), max_iter, rtol, 10, preconditioner == 1,
-                                 c->cg_host, &it, &rr, s);
+                                 g_wait_budget, c->cg_host, &it, &rr, s);
   if (iterations) *iterations = it;
   if (rel_residual) *rel_residual = rr;
   if (e != cudaSuccess) return fail(c, FEC_ERR_CUDA, "conjugate gradients: %s", cudaGetErrorString(e));

@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(THREADS) cg_test_kernel(CgScalars* sc, const d
 // applies.
 constexpr int KR = 4, COOP_CAP = 16384;  // entries of a CTA (one with more reads them from memory)
 constexpr size_t COOP_SMEM = size_t(COOP_CAP) * 12;
-constexpr long long COOP_BUDGET = 2000000000LL;
+constexpr long long COOP_BUDGET = 2000000000LL;  // clocks a barrier waits when no budget is set
 struct CoopShape {
   int64_t rows;  // of a CTA
   unsigned grid;
@@ -375,7 +375,7 @@ struct CoopShape {
 __global__ void __launch_bounds__(THREADS, 1) cg_solve_kernel(CscSym A, int64_t rows, const double* __restrict__ b,
                                                               double* x, double* p, int jacobi, double* parts,
                                                               CgScalars* sc, unsigned long long* bar, int max_iter,
-                                                              int check_every, double rtol) {
+                                                              int check_every, double rtol, long long budget) {
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ SumBuf buf;
   __shared__ double slot[2];
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(THREADS, 1) cg_solve_kernel(CscSym A, int64_t 
         unsigned long long seen;
         asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(bar) : "memory");
         if (seen >= target) break;
-        if (clock64() - t0 > COOP_BUDGET) {
+        if (clock64() - t0 > budget) {
           s_fail = 1;
           atomicExch(&sc->done, -1);
           break;
@@ -611,7 +611,8 @@ static cudaError_t finish(CgScalars& st, const CgScalars* sc, PcgHost& host, dou
 }
 
 cudaError_t pcg(const CscSym& A, const double* b, double* x, double* scratch, int max_iter, double rtol,
-                int check_every, bool jacobi, PcgHost& host, int* iterations, double* rel_residual, cudaStream_t s) {
+                int check_every, bool jacobi, long long wait_budget, PcgHost& host, int* iterations,
+                double* rel_residual, cudaStream_t s) {
   static_assert(sizeof(CgScalars) <= PcgHost::SLOT, "host slot");
   *iterations = 0;
   *rel_residual = 0.0;
@@ -651,7 +652,7 @@ cudaError_t pcg(const CscSym& A, const double* b, double* x, double* scratch, in
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, cg_solve_kernel, A, shape.rows, b, x, p, jacobi ? 1 : 0, part_py, sc, bar, max_iter,
-                           check_every, rtol);
+                           check_every, rtol, wait_budget > 0 ? wait_budget : COOP_BUDGET);
     if (e == cudaSuccess) return finish(st, sc, host, x, n, max_iter, iterations, rel_residual, s);
     if (e != cudaErrorCooperativeLaunchTooLarge) return e;
     cudaGetLastError();  // (a share of the device: fewer CTAs resident than SMs) the three kernels

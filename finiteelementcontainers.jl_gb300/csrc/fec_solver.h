@@ -27,8 +27,11 @@ struct PcgHost {
 size_t pcg_scratch_doubles(int64_t n);
 // Conjugate gradients for A x = b from the x passed in (Jacobi-preconditioned if
 // asked); stops when ||b - A x|| <= rtol ||b|| (tested every check_every
-// iterations) or after max_iter.  Synchronises the stream.
+// iterations) or after max_iter.  wait_budget: clocks a barrier of the one-launch solve
+// waits before the solve gives up with cudaErrorLaunchTimeout (0: the default, ~1 s).
+// Synchronises the stream.
 cudaError_t pcg(const CscSym& A, const double* b, double* x, double* scratch, int max_iter, double rtol,
-                int check_every, bool jacobi, PcgHost& host, int* iterations, double* rel_residual, cudaStream_t s);
+                int check_every, bool jacobi, long long wait_budget, PcgHost& host, int* iterations,
+                double* rel_residual, cudaStream_t s);
 
 }  // namespace fec

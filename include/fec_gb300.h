@@ -331,11 +331,12 @@ int fec_autotune_report(char* buf, size_t len);
  * clears the flag.  fec_check_finite reports the same flag.  Synchronous.  No
  * counterpart in the reference. */
 int fec_tensor_core_status(int reset);
-/* SM clocks the element kernels' bounded waits allow before they give up:
- * the main waits of the hex27 tensor-core kernel (hex27 FP32-element) and the
- * hex8 kernels' wait on their bulk table copy (FEC_HEX8_DF64=tile and the
- * FP32-element hex8 kernel).  0 (the default) is about one second.  The drain
- * that follows a timeout always allows the full second.  Process-wide; for
+/* SM clocks the kernels' bounded waits allow before they give up: the main waits
+ * of the tensor-core element kernels, the hex8 kernels' wait on their bulk table
+ * copy (FEC_HEX8_DF64=tile and the FP32-element hex8 kernel), and the barriers of
+ * fec_cg_solve in one launch, which then returns FEC_ERR_CUDA (x is not to be
+ * used).  0 (the default) is about one second.  The drain that follows a timeout
+ * of an element kernel always allows the full second.  Process-wide; for
  * testing the timeout path on operations that complete anyway.  No
  * counterpart in the reference. */
 int fec_set_wait_budget(long long clocks);
