@@ -216,19 +216,14 @@ int build_affine(fec_ctx* c, size_t b) {
 
 // The table a launch of block b may use: FP64 assemblies of congruent hex8
 // blocks on their own launch (the single launch across blocks keeps the
-// per-element kernels), unless FEC_HEX8_AFFINE=0.  The mechanics kernel also
-// wants the tables of a symmetric rule; `gradients`: a kernel that only reads the
-// block's gradients and JxW (Poisson, the action) takes any.
+// per-element kernels), unless FEC_HEX8_AFFINE=0.
 // Assemblies of tet10/hex27 blocks of translation classes get theirs: FP32-element
 // and FP64 (tet10: the tensor-core kernels; hex27 FP64: the class gradients).
-const void* affine_table(const fec_ctx* c, size_t b, int precision, bool mixed, bool gradients = false) {
+const void* affine_table(const fec_ctx* c, size_t b, int precision, bool mixed) {
   if (mixed || b >= c->d_affine.size()) return nullptr;
   const Block& B = c->blocks[b];
   if (B.elem_type == FEC_HEX8)
-    return B.congruent && precision == FEC_FP64 && fec::hex8_affine_enabled() &&
-                   (B.tensor_rule || gradients || B.physics == FEC_PHYS_POISSON)
-               ? c->d_affine[b].p
-               : nullptr;
+    return B.congruent && precision == FEC_FP64 && fec::hex8_affine_enabled() ? c->d_affine[b].p : nullptr;
   return (precision == FEC_FP32_ELEMENT || precision == FEC_FP64) ? c->d_affine[b].p : nullptr;
 }
 
@@ -1478,13 +1473,13 @@ int fec_assemble_action(fec_ctx* c, int precision, double t, double dt, const do
     // FP64 hex8 mechanics with the tables of a symmetric rule: the tensor-core kernel's
     // point phase; else blocks of translated elements: their constant gradients and JxW
     // (the tables of the other element types are their assembly kernels' alone)
-    if (B.elem_type == FEC_HEX8 && B.physics != FEC_PHYS_POISSON) {
+    if (B.elem_type == FEC_HEX8 && B.tensor_rule && B.physics != FEC_PHYS_POISSON) {
       ea.affine = affine_table(c, b, precision, false);
       ea.general = general_table(c, b, precision, false);
     }
     const bool tensor = ea.affine || ea.general;
     if (!tensor && B.elem_type == FEC_HEX8 && precision == FEC_FP64 && B.congruent)
-      if (const void* tab = affine_table(c, b, precision, false, true))
+      if (const void* tab = affine_table(c, b, precision, false))
         ea.affine = static_cast<const unsigned char*>(tab) + fec::hex8_affine_grad_offset();
     cudaError_t e;
     {

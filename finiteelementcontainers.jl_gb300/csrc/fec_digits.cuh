@@ -109,6 +109,7 @@ struct AffNeoHookean {
   static constexpr int NS = 0, SCR2 = 12;  // H, b, a2, c2
   static constexpr bool TANGENT_P = true;  // the slicers read the stress
   static constexpr bool GENERAL = false;
+  static constexpr bool TENSOR = true;     // hex8: the tables of a symmetric rule (AnyRule: any others)
   static constexpr int PROD_GROUPS = 2, STAGES = 2;  // of the hex8 kernel
   struct Mid {
     double F[9], H[9], a1h, a2, c2;
@@ -298,7 +299,7 @@ __device__ __forceinline__ void ref_point(const double* props, const double (&G)
 
 struct GenNeoHookean {
   static constexpr int NS = 0, SCR2 = 17;  // H, b, a2, c2 M (6)
-  static constexpr bool GENERAL = true, TANGENT_P = true;
+  static constexpr bool GENERAL = true, TANGENT_P = true, TENSOR = true;
   static constexpr int PROD_GROUPS = 3, STAGES = 1;
   using Mid = RefPoint;
   __device__ static void stress(const Mid& m, float2* P) {

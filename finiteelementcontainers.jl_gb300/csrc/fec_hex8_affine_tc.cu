@@ -122,7 +122,7 @@ __host__ __device__ __forceinline__ int quarter_start(int quarter) { return 3 * 
 struct AffJ2 {
   static constexpr int NS = J2::NS, SCR2 = J2::SCR2;
   static constexpr bool TANGENT_P = false;
-  static constexpr bool GENERAL = false;
+  static constexpr bool GENERAL = false, TENSOR = true;
   static constexpr int PROD_GROUPS = 3, STAGES = 3;
   struct Mid {
     double P[9], scr[J2::SCR];
@@ -153,6 +153,15 @@ struct AffJ2 {
   __device__ static float2 entry(const Tangent& t, int i, int J, int k, int L) {
     return J2::aentry_df64(t.s, i, J, k, L);
   }
+};
+
+// The same on a block of translated elements with 8-point tables that are not a symmetric
+// rule's (points in another order, any other points): gradients and residual by sums over
+// the block's own dNX, read from its table.  An assembly of 128^3 such elements 17.2 ms
+// (11.6 with a symmetric rule's tables, 25.4 with the per-element kernels).
+template <class Model>
+struct AnyRule : Model {
+  static constexpr bool TENSOR = false;
 };
 
 template <class Model>
@@ -235,10 +244,11 @@ __device__ __forceinline__ void tensor_gradient(const double* co, int q, const d
 
 // Point phase of quadrature point q of element e (FP64): the displacement gradient
 // and the constitutive update.  Every lane of the warp calls it (the shuffles);
-// uo: the displacement of the lane's corner node (0 where not live).
+// uo: the displacement of the lane's corner node (0 where not live); dNX: the block's gradients.
 template <class Model>
-__device__ __forceinline__ void point_phase(const ElemArgs& g, const double* s_ten, const double* s_jxw, int64_t e,
-                                            int q, bool live, const double (&uo)[3], typename Model::Mid& m) {
+__device__ __forceinline__ void point_phase(const ElemArgs& g, const double* s_ten, const double* s_jxw,
+                                            const double* __restrict__ dNX, int64_t e, int q, bool live,
+                                            const double (&uo)[3], typename Model::Mid& m) {
   const int lane = threadIdx.x & 31;
   double st[Model::NS ? Model::NS : 1];
   double* sn = nullptr;
@@ -251,8 +261,24 @@ __device__ __forceinline__ void point_phase(const ElemArgs& g, const double* s_t
   double v[3], gu[3][3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) v[d] = uo[d] - __shfl_sync(0xffffffffu, uo[d], lane & ~7);
-  tensor_gradient(s_ten, q, v, gu);
-  if (s_ten[10] == 0.0) {  // not an axis-aligned box: reference gradient times dxi/dX
+  if constexpr (!Model::TENSOR) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) gu[i / 3][i % 3] = 0.0;
+#pragma unroll 1
+    for (int a = 1; a < 8; ++a) {
+      const double* ga = dNX + q * 24 + a * 3;
+      const int src = (lane & ~7) | corner_node(a);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const double t = __shfl_sync(0xffffffffu, v[i], src);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) gu[i][j] = fma(t, __ldg(ga + j), gu[i][j]);
+      }
+    }
+  } else {
+    tensor_gradient(s_ten, q, v, gu);
+  }
+  if (Model::TENSOR && s_ten[10] == 0.0) {  // not an axis-aligned box: reference gradient times dxi/dX
     const double* Ji = s_ten + 12 + q * 9;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -325,7 +351,22 @@ __device__ __forceinline__ float2 df64_spread(float2 v, int q, int bit) {
 // direction at a time across the element's eight lanes -- 150 FP32 operations per
 // entry instead of the 290 of the sum over points, and no gradient table.  Every
 // lane of the warp calls it.
-__device__ __forceinline__ double residual_entry(const double* ten, const float2* ten2, int q, float2 p0, float2 p1, float2 p2) {
+template <class Model>
+__device__ __forceinline__ double residual_entry(const double* ten, const float2* ten2, const double* __restrict__ dNX,
+                                                 int q, float2 p0, float2 p1, float2 p2) {
+  if constexpr (!Model::TENSOR) {  // the sum over points
+    const double* ga = dNX + corner_node(q) * 3;
+    const int l0 = threadIdx.x & 24;
+    auto at = [](float2 v, int l) {
+      return make_float2(__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l));
+    };
+    float2 R = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int k = 0; k < NQ; ++k)
+      R = df64_dot3_acc(R, df64_split(__ldg(ga + k * 24)), at(p0, l0 + k), df64_split(__ldg(ga + k * 24 + 1)),
+                        at(p1, l0 + k), df64_split(__ldg(ga + k * 24 + 2)), at(p2, l0 + k));
+    return widen(R.x) + widen(R.y);
+  }
   if (ten[10] == 0.0) {  // not a box: to the reference element
     float2 Ji[9];
 #pragma unroll
@@ -444,7 +485,7 @@ __global__ void __launch_bounds__(Roles<Model>::NTHR, 1) hex8_affine_tc_kernel(E
         general_point(g, s_ten, s_jxw[q], q, live, X, uo, mid);
       } else {
         node = node_of(tile + PG * G);
-        point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
+        point_phase<Model>(g, s_ten, s_jxw, reinterpret_cast<const double*>(tab + T_G), e, q, live, uo, mid);
       }
       if (k >= NB) named_sync(Ro::EMPTY + grp, N_SL);  // the buffer's last tile has been read
       float bnd = 0.f;
@@ -470,7 +511,7 @@ __global__ void __launch_bounds__(Roles<Model>::NTHR, 1) hex8_affine_tc_kernel(E
       if (WANT_R) {  // while the slicers work on the staging
 #pragma unroll 1
         for (int i = 0; i < 3; ++i) {
-          const double r = residual_entry(s_ten, s_ten2, q, P[0], P[1], P[2]);
+          const double r = residual_entry<Model>(s_ten, s_ten2, reinterpret_cast<const double*>(tab + T_G), q, P[0], P[1], P[2]);
           if (live) static_cast<double*>(g.Re)[e * 24 + corner_node(q) * 3 + i] = r;
 #pragma unroll
           for (int j = 0; j < 6; ++j) P[j] = P[j + 3];
@@ -657,14 +698,15 @@ __global__ void __launch_bounds__(R_EPB * NQ) hex8_affine_r_kernel(ElemArgs g, c
   if constexpr (Model::GENERAL)
     general_point(g, s_ten, s_jxw[q], q, live, X, uo, mid);
   else
-    point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
+    point_phase<Model>(g, s_ten, s_jxw, reinterpret_cast<const double*>(tab + T_G), e, q, live, uo, mid);
   float2 P[9];
 #pragma unroll
   for (int i = 0; i < 9; ++i) P[i] = make_float2(0.f, 0.f);
   if (live) Model::stress(mid, P);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const double r = residual_entry(s_ten, s_ten2, q, P[i * 3], P[i * 3 + 1], P[i * 3 + 2]);
+    const double r = residual_entry<Model>(s_ten, s_ten2, reinterpret_cast<const double*>(tab + T_G), q, P[i * 3], P[i * 3 + 1],
+                                           P[i * 3 + 2]);
     if (live) static_cast<double*>(g.Re)[e * 24 + corner_node(q) * 3 + i] = r;
   }
 }
@@ -713,7 +755,7 @@ __global__ void __launch_bounds__(R_EPB * NQ) hex8_action_kernel(ElemArgs g, con
     general_gradients(s_ten, q, X, uo, G, D);
     if (live) point_update(g.props, G, D, s_jxw[q], mid);
   } else {
-    point_phase<Model>(g, s_ten, s_jxw, e, q, live, uo, mid);
+    point_phase<Model>(g, s_ten, s_jxw, reinterpret_cast<const double*>(tab + T_G), e, q, live, uo, mid);
   }
 #pragma unroll
   for (int d = 0; d < 3; ++d) v[d] -= __shfl_sync(0xffffffffu, v[d], lane & ~7);
@@ -862,18 +904,21 @@ bool hex8_pairs_enabled() {
   return !(v && v[0] == '0');
 }
 
+template <class Model>
+static cudaError_t launch_affine(bool want_r, bool want_k, const ElemArgs& a, cudaStream_t s, int* launches) {
+  if (!want_k) return want_r ? aff::launch_r<Model>(a, s, launches) : cudaSuccess;
+  return want_r ? aff::launch1<Model, true>(a, s, launches) : aff::launch1<Model, false>(a, s, launches);
+}
+
 cudaError_t launch_hex8_affine_tc(int physics, bool want_r, bool want_k, const ElemArgs& a, cudaStream_t s,
                                   int* launches) {
   if (!a.affine || (want_k && !a.Ke) || (want_r && !a.Re)) return cudaErrorInvalidValue;
-  if (!want_k) {
-    if (!want_r) return cudaSuccess;
-    if (physics == 2) return aff::launch_r<aff::AffNeoHookean>(a, s, launches);
-    if (physics == 3) return aff::launch_r<aff::AffJ2>(a, s, launches);
-    return cudaErrorNotSupported;
-  }
   if (physics == 2)
-    return want_r ? aff::launch1<aff::AffNeoHookean, true>(a, s, launches) : aff::launch1<aff::AffNeoHookean, false>(a, s, launches);
-  if (physics == 3) return want_r ? aff::launch1<aff::AffJ2, true>(a, s, launches) : aff::launch1<aff::AffJ2, false>(a, s, launches);
+    return a.hex8_tensor ? launch_affine<aff::AffNeoHookean>(want_r, want_k, a, s, launches)
+                         : launch_affine<aff::AnyRule<aff::AffNeoHookean>>(want_r, want_k, a, s, launches);
+  if (physics == 3)
+    return a.hex8_tensor ? launch_affine<aff::AffJ2>(want_r, want_k, a, s, launches)
+                         : launch_affine<aff::AnyRule<aff::AffJ2>>(want_r, want_k, a, s, launches);
   return cudaErrorNotSupported;
 }
 

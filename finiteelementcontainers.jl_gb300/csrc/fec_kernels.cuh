@@ -69,7 +69,7 @@ struct ElemArgs {
   const void* general;      // FP64 hex8, tet4, tet10 and hex27 Neo-Hookean blocks of any shape: the reference element's table (or null)
   int* wait_err;            // set to 1 by a bounded wait that gave up (device flag; may be null)
   long long wait_budget;    // SM clocks a bounded wait allows before giving up (0: the default, ~1 s)
-  int hex8_tensor;          // affine: and the block's tables are a symmetric rule's (hex8_tensor_rule)
+  int hex8_tensor;          // affine: the block's tables are a symmetric rule's (hex8_tensor_rule)
   int ke_pairs;             // the element kernel writes KE_PAIRS (FP64 hex8 tensor-core, FP64 hex27 kernels)
 };
 
