@@ -859,6 +859,7 @@ int fec_dofs_set(fec_ctx* c, int nf, const int64_t* dtu, int64_t n_unknowns) {
   if (next - 1 != n_unknowns)
     return fail(c, FEC_ERR_ARG, "num_unknowns = %lld but dof_to_unknown numbers %lld unknowns", (long long)n_unknowns,
                 (long long)(next - 1));
+  if (c->device >= 0) cudaSetDevice(c->device);
   int rc;
   if ((rc = upload(c, c->d_dtu, d.data(), sizeof(int64_t) * d.size()))) return rc;
   if ((rc = upload(c, c->d_umask, um.data(), um.size()))) return rc;
