@@ -112,11 +112,13 @@ struct fec_ctx {
   DevBuf d_node_groups;
   std::vector<fec::NodeGroup> node_groups;
   bool groups_ready = false;
-  // per block: the plan of the gather by output entry (built at the second assembly with a pattern);
-  // plan_state 0: not assembled yet, 1: built, 2: the mesh has none, 3: assembled once, not tried
+  // per block: the mesh's plan of the gather by output entry (pair_plan), the assemblies that
+  // could have used one; plan_state 0: not tried, 1: built, 2: the mesh has none
   std::vector<DevBuf> d_plan;
   std::vector<int64_t> plan_nslots;
-  std::vector<int> plan_state;
+  std::vector<int> plan_state, plan_uses;
+  std::vector<int64_t> plan_pattern;   // the pattern (pattern_id) whose row offsets a plan holds
+  int64_t pattern_id = 0;
   std::vector<DevBuf> d_general;       // per block: the reference element's table of a tet4, tet10 or hex27 block
   std::vector<DevBuf> d_affine;        // per block: the tensor-core operand table of a congruent hex8 block
                                        // or of a tet10/hex27 block of translation classes
@@ -407,104 +409,131 @@ bool stores_pairs(const fec_ctx* c, size_t b, int precision, bool want_r, bool w
                                        affine_table(c, b, precision, mixed) != nullptr));
 }
 
-// The plan of block b's gather by output entry (fec_pairgather.cu), built at the second
-// assembly with a pattern on stream s, before the element kernels: their workspace is its
-// scratch.  (Building takes several times what an assembly then saves -- 128^3 hex8: 7 ms
-// against 0.9 -- so a pattern that is assembled once does without: first pass there 20.0 ->
-// 13.4 ms.)  slots null where the block has none: nodes shared with other blocks or with
-// very many elements, indices that do not fit, no memory for it, or a second use under
-// stream capture (the per-node gathers then give the same bits).
-int pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s, fec::PairPlan* out) {
-  *out = fec::PairPlan{nullptr, nullptr, nullptr, 0};
-  if (c->plan_state.size() != c->blocks.size()) {
-    c->plan_state.assign(c->blocks.size(), 0);
-    c->plan_nslots.assign(c->blocks.size(), 0);
-    for (DevBuf& x : c->d_plan) x.release();
-    c->d_plan.assign(c->blocks.size(), DevBuf());
-  }
+// The calling thread may allocate while another one captures a graph (whose capture an
+// allocation would otherwise end).
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Builds block b's plan of the gather by output entry on stream s, with d_Ke as scratch
+// where it is large enough; plan_state 2 where the block has none.
+int build_pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s) {
+  RelaxedCapture relaxed;
   const Block& B = c->blocks[b];
+  c->plan_state[b] = 2;
   // at most: a pair of neighbours once, a pair of element nodes once
-  const int64_t np = int64_t(B.nnpe) * (B.nnpe + 1) / 2, max_list = B.ne * np;
+  const int64_t max_list = B.ne * (int64_t(B.nnpe) * (B.nnpe + 1) / 2);
+  if (max_list <= 0 || max_list >= (int64_t(1) << 31) || c->nn >= (int64_t(1) << 31)) return FEC_OK;
   const int64_t max_slots = std::min(max_list, (c->n_nbr + c->nn) / 2);
-  const size_t slot_bytes = sizeof(int4) * size_t(max_slots), count_bytes = (2 * size_t(max_slots) + 15) / 16 * 16;
+  // scratch: sums, counts per node, flags; slots and counts in node order
+  const size_t n1 = size_t(c->nn) + 1, scan_n = fec::pattern_scan_scratch(c->nn + 1);
+  const size_t sums = (8 * (2 * n1 + scan_n) + 4 * 2 * n1 + 16 + 15) / 16 * 16;
+  const size_t need = sums + (sizeof(int4) + 4) * size_t(max_slots);
+  DevBuf own;
+  struct Free {
+    DevBuf* b;
+    ~Free() { b->release(); }
+  } free_own{&own};
+  char* t = static_cast<char*>(c->d_Ke.p);
+  if (c->d_Ke.bytes < need) {
+    if (cudaMalloc(&own.p, need) != cudaSuccess) {
+      cudaGetLastError();
+      own.p = nullptr;
+      return FEC_OK;
+    }
+    t = static_cast<char*>(own.p);
+  }
+  int64_t* slot0 = reinterpret_cast<int64_t*>(t);
+  int64_t* list0 = slot0 + n1;
+  int64_t* scan = list0 + n1;
+  int32_t* nslot = reinterpret_cast<int32_t*>(scan + scan_n);
+  int32_t* nlist = nslot + n1;
+  int* flags = nlist + n1;
+  FEC_CUDA(c, cudaMemsetAsync(flags, 0, 2 * sizeof(int), s));
+  FEC_CUDA(c, fec::pair_plan_count(ga, int(b), B.ne, nslot, nlist, flags, s));
+  FEC_CUDA(c, fec::pattern_scan(nslot, nullptr, c->nn, slot0, scan, s));
+  FEC_CUDA(c, fec::pattern_scan(nlist, nullptr, c->nn, list0, scan, s));
+  int64_t nslots = 0, nentries = 0;
+  int h[2];
+  FEC_CUDA(c, cudaMemcpyAsync(&nslots, slot0 + c->nn, 8, cudaMemcpyDeviceToHost, s));
+  FEC_CUDA(c, cudaMemcpyAsync(&nentries, list0 + c->nn, 8, cudaMemcpyDeviceToHost, s));
+  FEC_CUDA(c, cudaMemcpyAsync(h, flags, sizeof h, cudaMemcpyDeviceToHost, s));
+  FEC_CUDA(c, cudaStreamSynchronize(s));
+  if (h[0] || h[1] || nslots == 0 || nslots > max_slots || nentries > max_list) return FEC_OK;
   DevBuf& d = c->d_plan[b];  // slots, counts, list
-  if (c->plan_state[b] == 0) {
-    c->plan_state[b] = 3;
+  d.release();
+  const size_t bytes = (sizeof(int4) + 4) * size_t(nslots) + sizeof(uint32_t) * size_t(nentries);
+  if (cudaMalloc(&d.p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    d.p = nullptr;
     return FEC_OK;
   }
-  if (c->plan_state[b] == 3) {
+  d.bytes = bytes;
+  int4* slots = static_cast<int4*>(d.p);
+  uint32_t* count = reinterpret_cast<uint32_t*>(slots + nslots);
+  int4* slots2 = reinterpret_cast<int4*>(t + sums);
+  FEC_CUDA(c, fec::pair_plan_fill(ga, int(b), B.ne, slot0, list0, slots2, slots,
+                                  reinterpret_cast<uint32_t*>(slots2 + nslots), count, count + nslots, flags, s));
+  if (own.p) FEC_CUDA(c, cudaStreamSynchronize(s));
+  c->plan_nslots[b] = nslots;
+  c->plan_state[b] = 1;
+  return FEC_OK;
+}
+
+// The plan of block b's gather by output entry (fec_pairgather.cu), which belongs to the
+// mesh: it outlives changes of the Dirichlet dofs, and only its row offsets are renewed at
+// the first assembly with a pattern (128^3 hex8: 0.4 ms).  Built at the assembly after
+// PLAN_AFTER that could have used it; both before the element kernels and outside stream
+// capture.  slots null where the block has none (yet): nodes shared with other blocks or with very
+// many elements, indices that do not fit, no memory for it; the per-node gathers then give
+// the same bits.
+// PLAN_AFTER: building takes what 1.6 to 9 assemblies then save (128^3 hex8 7.3 ms against
+// 0.80 ms an assembly, 61 x 53 x 47 hex8 0.74 against 0.17, 55k tet10 0.51 against 0.20,
+// tet4 + tet10 + hex27 of 22 x 24 x 26 cells 1.75 against 1.06, 40^3 hex8 0.38 against 0.05), so
+// a mesh that is assembled 8 times or fewer does not pay for it.
+constexpr int PLAN_AFTER = 8;
+int pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s, fec::PairPlan* out) {
+  *out = fec::PairPlan{nullptr, nullptr, nullptr, 0};
+  if (c->plan_state[b] == 2) return FEC_OK;
+  if (c->plan_state[b] == 0 || c->plan_pattern[b] != c->pattern_id) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
       cudaGetLastError();
       return FEC_OK;
     }
     if (cs != cudaStreamCaptureStatusNone) return FEC_OK;
-    c->plan_state[b] = 2;
-    if (max_list <= 0 || max_list >= (int64_t(1) << 31) || c->nn >= (int64_t(1) << 31)) return FEC_OK;
-    // scratch: sums, counts per node, flags, slots and counts in node order
-    const size_t n1 = size_t(c->nn) + 1, scan_n = fec::pattern_scan_scratch(c->nn + 1);
-    const size_t need = 8 * (2 * n1 + scan_n) + 4 * 2 * n1 + 16 + 16 + slot_bytes + count_bytes;
-    DevBuf own;
-    struct Free {
-      DevBuf* b;
-      ~Free() { b->release(); }
-    } free_own{&own};
-    void* t = c->d_Ke.p;
-    if (c->d_Ke.bytes < need) {
-      if (cudaMalloc(&own.p, need) != cudaSuccess) {
-        cudaGetLastError();
-        return FEC_OK;
-      }
-      t = own.p;
-    }
-    d.release();
-    if (cudaMalloc(&d.p, slot_bytes + count_bytes + sizeof(uint32_t) * size_t(max_list)) != cudaSuccess) {
-      cudaGetLastError();
-      d.p = nullptr;
-      return FEC_OK;
-    }
-    int4* slots2 = static_cast<int4*>(t);
-    uint16_t* count2 = reinterpret_cast<uint16_t*>(slots2 + max_slots);
-    int64_t* slot0 = reinterpret_cast<int64_t*>(reinterpret_cast<char*>(count2) + count_bytes);
-    int64_t* list0 = slot0 + n1;
-    int64_t* scan = list0 + n1;
-    int32_t* nslot = reinterpret_cast<int32_t*>(scan + scan_n);
-    int32_t* nlist = nslot + n1;
-    int* flags = nlist + n1;
-    char* base = static_cast<char*>(d.p);
-    FEC_CUDA(c, cudaMemsetAsync(flags, 0, 2 * sizeof(int), s));
-    FEC_CUDA(c, fec::pair_plan_count(ga, int(b), B.ne, nslot, nlist, flags, s));
-    FEC_CUDA(c, fec::pattern_scan(nslot, nullptr, c->nn, slot0, scan, s));
-    FEC_CUDA(c, fec::pattern_scan(nlist, nullptr, c->nn, list0, scan, s));
-    FEC_CUDA(c, fec::pair_plan_fill(ga, int(b), B.ne, slot0, list0, slots2, base, count2,
-                                    reinterpret_cast<uint16_t*>(base + slot_bytes),
-                                    reinterpret_cast<uint32_t*>(base + slot_bytes + count_bytes), flags, s));
-    int64_t total = 0;
-    int h[2];
-    FEC_CUDA(c, cudaMemcpyAsync(&total, slot0 + c->nn, 8, cudaMemcpyDeviceToHost, s));
-    FEC_CUDA(c, cudaMemcpyAsync(h, flags, sizeof h, cudaMemcpyDeviceToHost, s));
-    FEC_CUDA(c, cudaStreamSynchronize(s));
-    if (h[0] || h[1] || total == 0) {
-      d.release();
-      return FEC_OK;
-    }
-    c->plan_nslots[b] = total;
-    c->plan_state[b] = 1;
   }
-  if (c->plan_state[b] == 1) {
-    const char* base = static_cast<const char*>(d.p);
-    *out = fec::PairPlan{reinterpret_cast<const int4*>(base), reinterpret_cast<const uint16_t*>(base + slot_bytes),
-                         reinterpret_cast<const uint32_t*>(base + slot_bytes + count_bytes), c->plan_nslots[b]};
+  if (c->plan_state[b] == 0) {
+    if (c->plan_uses[b]++ < PLAN_AFTER) return FEC_OK;
+    if (int rc = build_pair_plan(c, ga, b, s)) return rc;
+    if (c->plan_state[b] != 1) return FEC_OK;
   }
+  int4* slots = static_cast<int4*>(c->d_plan[b].p);
+  const uint32_t* count = reinterpret_cast<const uint32_t*>(slots + c->plan_nslots[b]);
+  const fec::PairPlan plan = {slots, count, count + c->plan_nslots[b], c->plan_nslots[b]};
+  if (c->plan_pattern[b] != c->pattern_id) {
+    FEC_CUDA(c, fec::pair_plan_offsets(ga, int(b), plan, s));
+    c->plan_pattern[b] = c->pattern_id;
+  }
+  *out = plan;
   return FEC_OK;
+}
+
+void release_plans(fec_ctx* c) {
+  for (DevBuf& x : c->d_plan) x.release();
+  c->d_plan.assign(c->blocks.size(), DevBuf());
+  c->plan_nslots.assign(c->blocks.size(), 0);
+  c->plan_state.assign(c->blocks.size(), 0);
+  c->plan_uses.assign(c->blocks.size(), 0);
+  c->plan_pattern.assign(c->blocks.size(), -1);
 }
 
 void invalidate_pattern(fec_ctx* c) {
   c->pattern_ready = false;
   c->groups_ready = false;
   c->d_node_groups.release();
-  for (DevBuf& b : c->d_plan) b.release();
-  c->plan_state.assign(c->plan_state.size(), 0);
   c->nnz = 0;
   c->d_colptr0.release();
   c->d_rowval32.release();
@@ -758,6 +787,7 @@ int fec_mesh_set(fec_ctx* c, int dim, int64_t nn, const double* coords, int nblo
   c->nf = 0;
   invalidate_pattern(c);
   release_pattern(c);
+  release_plans(c);
   return ok(c);
 }
 
@@ -1015,6 +1045,7 @@ int fec_pattern_build(fec_ctx* c, int64_t* nnz_out) {
   c->nnz = nnz;
   c->acc_stride = acc_stride;
   c->pattern_ready = true;
+  ++c->pattern_id;
   if (nnz_out) *nnz_out = nnz;
   return ok(c);
 }
@@ -1124,6 +1155,7 @@ int fec_pattern_build_device(fec_ctx* c, int64_t* nnz_out, void* stream) {
   c->nnz = nnz;
   c->acc_stride = acc_stride;
   c->pattern_ready = true;
+  ++c->pattern_id;
   if (nnz_out) *nnz_out = nnz;
   return ok(c);
 }

@@ -50,19 +50,22 @@ cudaError_t launch_gather_groups(int precision, int nf, const GatherArgs& args, 
 // which writes the CSC values of every node of the block and, when R_u is set, the
 // residual of g.nodes (all nodes when null).  Bitwise launch_gather's results.
 struct PairPlan {
-  const int4* slots;
-  const uint16_t* count;
+  int4* slots;
+  const uint32_t* count;
   const uint32_t* list;
   int64_t nslots;
 };
+// Of the mesh, whatever its Dirichlet dofs.
 // Pairs and list entries per node (int32, nn); flags (int[2], zeroed by the caller):
-// [0] a node with too many rows or elements, [1] a node shared with another block.
+// [0] a node with too many neighbours or elements, [1] a node shared with another block.
 // unordered, unordered_count: scratch of the sizes of slots and count.
 cudaError_t pair_plan_count(const GatherArgs& g, int block, int64_t ne, int32_t* nslot, int32_t* nlist, int* flags,
                             cudaStream_t stream);
 cudaError_t pair_plan_fill(const GatherArgs& g, int block, int64_t ne, const int64_t* slot0, const int64_t* list0,
-                           void* unordered, void* slots, uint16_t* unordered_count, uint16_t* count, uint32_t* list,
+                           void* unordered, void* slots, uint32_t* unordered_count, uint32_t* count, uint32_t* list,
                            int* flags, cudaStream_t stream);
+// ... but for the pairs' row offsets, which belong to the pattern.
+cudaError_t pair_plan_offsets(const GatherArgs& g, int block, const PairPlan& plan, cudaStream_t stream);
 cudaError_t launch_pair_gather(const GatherArgs& g, int block, const PairPlan& plan, cudaStream_t stream,
                                int* launches);
 // FEC_GATHER_PAIRS=0 keeps the per-node gathers.

@@ -9,7 +9,8 @@
 // (m, i), columns (m, i) and row (n, k).  Every stored block is read once (the
 // per-node gathers read it for both nodes), nothing goes through shared memory, and
 // the loads of a thread do not depend on one another.  Nodes with Dirichlet dofs need
-// no path of their own.
+// no path of their own.  The plan is the mesh's: only the pairs' row offsets follow the
+// Dirichlet dofs (offsets_kernel).
 //
 // Bound: latency and issue, then DRAM.  A hex8 node of a box has 14 pairs with lists
 // of 8, 4, 2 or 1; the pairs of GROUP consecutive nodes are ordered by the length of
@@ -25,29 +26,26 @@
 namespace fec {
 namespace {
 
-constexpr int WPB = 8;      // warps per CTA of the plan kernel
-constexpr int MAXL = 1024;  // rows per column of a node
+constexpr int WPB = 4;      // warps per CTA of the plan kernel
+constexpr int MAXT = 512;   // places of a node's hash table: its neighbours m >= n
 constexpr int GROUP = 8;    // nodes whose pairs are ordered together (8: 128^3 3.40 ms; 32: 3.49, 128: 3.53)
 constexpr int CLASSES = 64; // list lengths told apart
 
-// One warp per node n: its elements' nodes m >= n with an unknown component, told
-// apart by their row offset in n's columns.  FILL = false: how many pairs and list
-// entries n has; FILL = true: writes them.  flags[0]: a node with too many rows or
-// elements; flags[1]: a node of this block shared with another.
+// One warp per node n: its elements' nodes m >= n, told apart by their place in a hash table.
+// FILL = false: how many pairs and list entries n has; FILL = true: writes
+// them.  flags[0]: a node with too many neighbours or elements; flags[1]: a node of this
+// block shared with another.  Nothing here depends on the Dirichlet dofs.
 struct PlanArgs {
-  int64_t nn, elem_start, ne, conn_off, epos_off;
+  int64_t nn, elem_start, ne, conn_off;
   int A;
   bool shared;                     // several blocks: nodes may be shared
   const int64_t* nadj_ptr;
   const uint32_t* nadj;
   const int32_t* conn;
-  const uint16_t* epos;
-  const uint8_t* umask;
-  const int32_t* col_len;
   int32_t *nslot, *nlist;          // per node (FILL = false)
   const int64_t *slot0, *list0;    // their exclusive sums (FILL = true)
-  int4* slots;                     // n, m, first list entry, row offsets of m in n's and of n in m's columns
-  uint16_t* count;                 // list entries of a slot
+  int4* slots;                     // n, m, first list entry, row offsets (offsets_kernel)
+  uint32_t* count;                 // list entries of a slot | n's and m's places in that element << 16, << 24
   uint32_t* list;                  // (element * pairs + pair) << 1 | transposed
   int* flags;
 };
@@ -59,15 +57,17 @@ __device__ __forceinline__ bool owned(const PlanArgs& a, int64_t n) {
 
 template <bool FILL>
 __global__ void __launch_bounds__(WPB * 32) plan_kernel(PlanArgs a) {
-  __shared__ uint16_t s_cnt[WPB][MAXL], s_at[WPB][FILL ? MAXL : 1], s_rank[WPB][FILL ? MAXL : 1];
+  __shared__ int32_t s_key[WPB][MAXT];
+  __shared__ int2 s_pair[WPB][FILL ? MAXT : 1];  // the neighbours and their list entries
+  __shared__ uint16_t s_cnt[WPB][MAXT], s_at[WPB][FILL ? MAXT : 1], s_rank[WPB][FILL ? MAXT : 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t n = int64_t(blockIdx.x) * WPB + warp;
   if (n >= a.nn) return;
+  int32_t* key = s_key[warp];
   uint16_t* cnt = s_cnt[warp];
-  const int64_t p0 = a.nadj_ptr[n], p1 = a.nadj_ptr[n + 1];
-  const int L = a.col_len[n];
-  bool use = (a.umask[n] & 7u) != 0 && (!a.shared || owned(a, n));
-  if (use && (L > MAXL || (p1 - p0) * a.A > 65535)) {
+  const int64_t p0 = a.nadj_ptr[n], p1 = a.nadj_ptr[n + 1], cand = (p1 - p0) * a.A;
+  bool use = p1 > p0 && (!a.shared || owned(a, n));
+  if (use && cand > 65535) {
     if (lane == 0) a.flags[0] = 1;
     use = false;
   }
@@ -75,43 +75,71 @@ __global__ void __launch_bounds__(WPB * 32) plan_kernel(PlanArgs a) {
     if (!FILL && lane == 0) a.nslot[n] = a.nlist[n] = 0;
     return;
   }
-  for (int i = lane; i < L; i += 32) cnt[i] = 0;
+  int T = 32;  // no more places than candidates
+  while (T < MAXT && T < cand) T <<= 1;
+  for (int i = lane; i < T; i += 32) {
+    key[i] = -1;
+    cnt[i] = 0;
+  }
   __syncwarp();
+  // the place of m, taken if it has none; -1 where the table is full
+  auto place = [&](int32_t m) {
+    unsigned h = uint32_t(m) * 2654435761u >> 16;
+    for (int tries = 0; tries < T; ++tries, ++h) {
+      const int i = int(h & unsigned(T - 1));
+      const int32_t was = atomicCAS(&key[i], -1, m);
+      if (was == -1 || was == m) return i;
+    }
+    return -1;
+  };
   // elements in order; an element's nodes are distinct, so its lanes are
   for (int64_t p = p0; p < p1; ++p) {
-    const uint32_t packed = a.nadj[p];
-    const int64_t le = int64_t(packed >> 5) - a.elem_start;
+    const int64_t le = int64_t(a.nadj[p] >> 5) - a.elem_start;
     if (lane < a.A) {
-      const int64_t m = a.conn[a.conn_off + le * a.A + lane];
+      const int32_t m = a.conn[a.conn_off + le * a.A + lane];
       if (!FILL && a.shared && !owned(a, m)) a.flags[1] = 1;
-      if (m >= n && (a.umask[m] & 7u)) ++cnt[a.epos[a.epos_off + (le * a.A + int(packed & 31u)) * a.A + lane]];
+      if (m >= n) {
+        const int i = place(m);
+        if (i >= 0)
+          ++cnt[i];
+        else
+          a.flags[0] = 1;
+      }
     }
     __syncwarp();
   }
-  // pairs and list entries before each row offset
   int slots = 0, entries = 0;
-  for (int i0 = 0; i0 < L; i0 += 32) {
-    const int i = i0 + lane, c = i < L ? cnt[i] : 0;
+  for (int i0 = 0; i0 < T; i0 += 32) {
+    const int i = i0 + lane, c = cnt[i];
     const unsigned mask = __ballot_sync(0xffffffffu, c > 0);
-    int inc = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += t;
-    }
-    if (FILL && i < L) {
-      s_rank[warp][i] = uint16_t(slots + __popc(mask & ((1u << lane) - 1u)));
-      s_at[warp][i] = uint16_t(entries + inc - c);
-    }
+    if (FILL && c > 0) s_pair[warp][slots + __popc(mask & ((1u << lane) - 1u))] = make_int2(key[i], c);
     slots += __popc(mask);
-    entries += __shfl_sync(0xffffffffu, inc, 31);
+    entries += c;
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) entries += __shfl_xor_sync(0xffffffffu, entries, o);
   if (!FILL) {
     if (lane == 0) {
       a.nslot[n] = slots;
       a.nlist[n] = entries;
     }
     return;
+  }
+  __syncwarp();
+  // pairs and list entries of the neighbours before each (ascending: rows of a column, and
+  // element nodes, are)
+  for (int i = lane; i < T; i += 32) {
+    if (cnt[i] == 0) continue;
+    int rank = 0, at = 0;
+    for (int j = 0; j < slots; ++j) {
+      const int2 o = s_pair[warp][j];
+      if (o.x < key[i]) {
+        ++rank;
+        at += o.y;
+      }
+    }
+    s_rank[warp][i] = uint16_t(rank);
+    s_at[warp][i] = uint16_t(at);
   }
   __syncwarp();
   const int np = a.A * (a.A + 1) / 2;
@@ -121,20 +149,19 @@ __global__ void __launch_bounds__(WPB * 32) plan_kernel(PlanArgs a) {
     const int la = int(packed & 31u), lb = lane;
     if (lb < a.A) {
       const int32_t m = a.conn[a.conn_off + le * a.A + lb];
-      if (m >= n && (a.umask[m] & 7u)) {
-        const uint16_t* ep = a.epos + a.epos_off + le * a.A * a.A;
-        const int off = ep[la * a.A + lb];
-        const int c = cnt[off];
+      const int i = m >= n ? place(m) : -1;
+      if (i >= 0) {  // (a full table: the plan is not used)
+        const int c = cnt[i];
         const int x = la < lb ? la : lb, y = la < lb ? lb : la;
-        const int64_t at = a.list0[n] + s_at[warp][off];
+        const int64_t at = a.list0[n] + s_at[warp][i];
         const int64_t block = le * np + x * (2 * a.A - x + 1) / 2 + y - x;
         a.list[at] = uint32_t(block) << 1 | (la > lb ? 1u : 0u);
-        ++s_at[warp][off];
+        ++s_at[warp][i];
         if (c != 0xffff) {  // the pair's first element (at is its first list entry)
-          const int64_t s = a.slot0[n] + s_rank[warp][off];
-          a.slots[s] = make_int4(int(n), m, int(uint32_t(at)), off | int(uint32_t(ep[lb * a.A + la]) << 16));
-          a.count[s] = uint16_t(c);
-          cnt[off] = 0xffff;
+          const int64_t s = a.slot0[n] + s_rank[warp][i];
+          a.slots[s] = make_int4(int(n), m, int(uint32_t(at)), 0);
+          a.count[s] = uint32_t(c) | uint32_t(la) << 16 | uint32_t(lb) << 24;
+          cnt[i] = 0xffff;
         }
       }
     }
@@ -144,11 +171,14 @@ __global__ void __launch_bounds__(WPB * 32) plan_kernel(PlanArgs a) {
 
 // The slots of GROUP consecutive nodes by descending list length (a CTA per group).
 __global__ void __launch_bounds__(256) order_kernel(int64_t nn, const int64_t* slot0, const int4* in,
-                                                    const uint16_t* cin, int4* out, uint16_t* cout) {
+                                                    const uint32_t* cin, int4* out, uint32_t* cout) {
   __shared__ int hist[CLASSES];
   const int64_t n0 = int64_t(blockIdx.x) * GROUP, n1 = n0 + GROUP < nn ? n0 + GROUP : nn;
   const int64_t s0 = slot0[n0], s1 = slot0[n1];
-  auto cls = [](int c) { return c < CLASSES ? CLASSES - 1 - c : 0; };
+  auto cls = [](uint32_t v) {
+    const int c = int(v & 0xffffu);
+    return c < CLASSES ? CLASSES - 1 - c : 0;
+  };
   for (int i = threadIdx.x; i < CLASSES; i += 256) hist[i] = 0;
   __syncthreads();
   for (int64_t s = s0 + threadIdx.x; s < s1; s += 256) atomicAdd(&hist[cls(cin[s])], 1);
@@ -163,11 +193,24 @@ __global__ void __launch_bounds__(256) order_kernel(int64_t nn, const int64_t* s
   }
   __syncthreads();
   for (int64_t s = s0 + threadIdx.x; s < s1; s += 256) {
-    const int c = cin[s];
-    const int64_t at = s0 + atomicAdd(&hist[cls(c)], 1);
+    const int64_t at = s0 + atomicAdd(&hist[cls(cin[s])], 1);
     out[at] = in[s];
-    cout[at] = uint16_t(c);
+    cout[at] = cin[s];
   }
+}
+
+// The row offsets of a slot's m in n's columns and of n in m's, by the pattern at hand: from
+// the element map at the pair's first element.
+__global__ void __launch_bounds__(256) offsets_kernel(GatherArgs g, int4* slots, const uint32_t* count,
+                                                      const uint32_t* list, int64_t nslots, int block) {
+  const int64_t s = int64_t(blockIdx.x) * 256 + threadIdx.x;
+  if (s >= nslots) return;
+  const BlockInfo& B = g.blk[block];
+  const int A = B.nnpe;
+  const uint32_t c = count[s], la = c >> 16 & 0xffu, lb = c >> 24;
+  const uint32_t le = (list[uint32_t(slots[s].z)] >> 1) / uint32_t(A * (A + 1) / 2);
+  const uint16_t* ep = g.epos + B.epos_off + int64_t(le) * A * A;
+  slots[s].w = int(uint32_t(ep[la * A + lb]) | uint32_t(ep[lb * A + la]) << 16);
 }
 
 // Row k of pair slot s per thread (85 slots a CTA); the first nbr CTAs form the residual.
@@ -181,7 +224,7 @@ __global__ void __launch_bounds__(256) pair_gather_kernel(GatherArgs g, PairPlan
   const int64_t s = int64_t(blockIdx.x - nbr) * SLOTS + sl;
   if (sl >= SLOTS || s >= plan.nslots) return;
   const int4 r = __ldg(plan.slots + s);
-  int left = __ldg(plan.count + s);
+  int left = int(__ldg(plan.count + s) & 0xffffu);
   const uint32_t* lp = plan.list + uint32_t(r.z);
   const unsigned un = g.umask[r.x], um = g.umask[r.y];
   const int64_t cn = g.col_base[r.x], cm = g.col_base[r.y];
@@ -229,57 +272,49 @@ __global__ void __launch_bounds__(256) pair_gather_kernel(GatherArgs g, PairPlan
 
 }  // namespace
 
-cudaError_t pair_plan_count(const GatherArgs& g, int block, int64_t ne, int32_t* nslot, int32_t* nlist, int* flags,
-                            cudaStream_t s) {
+static PlanArgs plan_args(const GatherArgs& g, int block, int64_t ne, int* flags) {
   PlanArgs a{};
   const BlockInfo& B = g.blk[block];
   a.nn = g.nn;
   a.elem_start = B.elem_start;
   a.ne = ne;
   a.conn_off = B.conn_off;
-  a.epos_off = B.epos_off;
   a.A = B.nnpe;
   a.shared = g.nblocks > 1;
   a.nadj_ptr = g.nadj_ptr;
   a.nadj = g.nadj;
   a.conn = g.conn;
-  a.epos = g.epos;
-  a.umask = g.umask;
-  a.col_len = g.col_len;
+  a.flags = flags;
+  return a;
+}
+
+cudaError_t pair_plan_count(const GatherArgs& g, int block, int64_t ne, int32_t* nslot, int32_t* nlist, int* flags,
+                            cudaStream_t s) {
+  PlanArgs a = plan_args(g, block, ne, flags);
   a.nslot = nslot;
   a.nlist = nlist;
-  a.flags = flags;
   plan_kernel<false><<<unsigned((g.nn + WPB - 1) / WPB), WPB * 32, 0, s>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t pair_plan_fill(const GatherArgs& g, int block, int64_t ne, const int64_t* slot0, const int64_t* list0,
-                           void* unordered, void* slots, uint16_t* count2, uint16_t* count, uint32_t* list, int* flags,
+                           void* unordered, void* slots, uint32_t* count2, uint32_t* count, uint32_t* list, int* flags,
                            cudaStream_t s) {
-  PlanArgs a{};
-  const BlockInfo& B = g.blk[block];
-  a.nn = g.nn;
-  a.elem_start = B.elem_start;
-  a.ne = ne;
-  a.conn_off = B.conn_off;
-  a.epos_off = B.epos_off;
-  a.A = B.nnpe;
-  a.shared = g.nblocks > 1;
-  a.nadj_ptr = g.nadj_ptr;
-  a.nadj = g.nadj;
-  a.conn = g.conn;
-  a.epos = g.epos;
-  a.umask = g.umask;
-  a.col_len = g.col_len;
+  PlanArgs a = plan_args(g, block, ne, flags);
   a.slot0 = slot0;
   a.list0 = list0;
   a.slots = static_cast<int4*>(unordered);
   a.count = count2;
   a.list = list;
-  a.flags = flags;
   plan_kernel<true><<<unsigned((g.nn + WPB - 1) / WPB), WPB * 32, 0, s>>>(a);
   order_kernel<<<unsigned((g.nn + GROUP - 1) / GROUP), 256, 0, s>>>(g.nn, slot0, a.slots, count2,
                                                                      static_cast<int4*>(slots), count);
+  return cudaGetLastError();
+}
+
+cudaError_t pair_plan_offsets(const GatherArgs& g, int block, const PairPlan& plan, cudaStream_t s) {
+  offsets_kernel<<<unsigned((plan.nslots + 255) / 256), 256, 0, s>>>(g, plan.slots, plan.count, plan.list, plan.nslots,
+                                                                     block);
   return cudaGetLastError();
 }
 
