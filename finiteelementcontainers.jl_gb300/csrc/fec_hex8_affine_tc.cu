@@ -1019,6 +1019,28 @@ bool hex8_general_table(const double* ref, std::vector<unsigned char>& out) {
   return hex8_affine_table(x, ref, out);
 }
 
+// Host: sums of products and 2 x 2 determinants as if in twice the precision (Ogita, Rump and
+// Oishi, SIAM J. Sci. Comput. 26 (2005) 1955-1988, Dot2).  The mapping of a block is a constant of
+// all its elements, so its rounding would be a common factor of their matrices that no sum
+// averages out: det J from rounded sums put 3 ulp on every entry.
+namespace {
+struct Dot2 {
+  double s = 0.0, c = 0.0;
+  void add(double a, double b) {
+    const double p = a * b, e = std::fma(a, b, -p), t = s + p, z = t - s;
+    c += e + ((s - (t - z)) + (p - z));
+    s = t;
+  }
+  double value() const { return s + c; }
+};
+double det2(double a, double b, double c, double d) {  // a d - b c
+  Dot2 t;
+  t.add(a, d);
+  t.add(-b, c);
+  return t.value();
+}
+}  // namespace
+
 // Host: the constant operand of a block whose elements are translates of its
 // first one.  x0: the first element's node coordinates [8][3]; ref: the block's
 // reference tables (RefLayout<1>: N, dN/dxi [q][a][3], weights).  Returns false
@@ -1028,27 +1050,48 @@ bool hex8_affine_table(const double* x0, const double* ref, std::vector<unsigned
   using L = RefLayout<1>;
   out.assign(aff::T_BYTES, 0);
   double dNX[8][8][3], jxw[8], ten[aff::TEN_N] = {0.0};
+  double cI[3] = {1.0, 1.0, 1.0}, sc[3];
+  const bool trilinear = hex8_tensor_rule(ref, cI), box = box_scales(x0, sc);
+  auto corner = [](int bits) { return bits ^ (bits >> 1 & 1); };
   for (int q = 0; q < 8; ++q) {
     const double* dN = ref + L::DN_OFF + q * 24;
-    double J[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    for (int a = 0; a < 8; ++a)
-      for (int d = 0; d < 3; ++d)
-        for (int k = 0; k < 3; ++k) J[d][k] = std::fma(x0[a * 3 + d], dN[a * 3 + k], J[d][k]);
-    const double c00 = J[1][1] * J[2][2] - J[1][2] * J[2][1], c01 = J[1][2] * J[2][0] - J[1][0] * J[2][2],
-                 c02 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
-    const double det = J[0][0] * c00 + J[0][1] * c01 + J[0][2] * c02;
+    double J[3][3], co[3][3], Ji[3][3];
+    for (int d = 0; d < 3; ++d)
+      for (int k = 0; k < 3; ++k) {
+        if (trilinear) {
+          // half the edges along k, interpolated: of a parallelepiped an edge, whatever the
+          // tables' rounding (a box is taken as one to 1e-13, see box_scales)
+          const int m = (k + 1) % 3, n = (k + 2) % 3;
+          const double fm = q >> m & 1 ? cI[m] : 1.0 - cI[m], fn = q >> n & 1 ? cI[n] : 1.0 - cI[n];
+          auto edge = [&](int bits) {
+            return x0[corner(bits | 1 << k) * 3 + d] - x0[corner(bits) * 3 + d];
+          };
+          const double e = edge(0), em = edge(1 << m) - e, en = edge(1 << n) - e,
+                       emn = edge(1 << m | 1 << n) - e - em - en;
+          Dot2 s;
+          s.add(e, 1.0);
+          s.add(em, fm);
+          s.add(en, fn);
+          s.add(emn, fm * fn);
+          J[d][k] = 0.5 * s.value();
+          if (box) J[d][k] = d == k ? 0.5 * (x0[18 + d] - x0[d]) : 0.0;
+        } else {
+          Dot2 s;
+          for (int a = 1; a < 8; ++a) s.add(x0[a * 3 + d] - x0[d], dN[a * 3 + k]);
+          J[d][k] = s.value();
+        }
+      }
+    for (int d = 0; d < 3; ++d)
+      for (int k = 0; k < 3; ++k) {
+        const int d1 = (d + 1) % 3, d2 = (d + 2) % 3, k1 = (k + 1) % 3, k2 = (k + 2) % 3;
+        co[d][k] = det2(J[d1][k1], J[d1][k2], J[d2][k1], J[d2][k2]);
+      }
+    Dot2 sum;
+    for (int k = 0; k < 3; ++k) sum.add(J[0][k], co[0][k]);
+    const double det = sum.value();
     if (!(det > 0.0)) return false;
-    const double r = 1.0 / det;
-    double Ji[3][3];
-    Ji[0][0] = c00 * r;
-    Ji[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) * r;
-    Ji[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * r;
-    Ji[1][0] = c01 * r;
-    Ji[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * r;
-    Ji[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * r;
-    Ji[2][0] = c02 * r;
-    Ji[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * r;
-    Ji[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * r;
+    for (int k = 0; k < 3; ++k)
+      for (int d = 0; d < 3; ++d) Ji[k][d] = trilinear && box ? (d == k ? 2.0 * sc[d] : 0.0) : co[d][k] / det;
     for (int k = 0; k < 3; ++k)
       for (int d = 0; d < 3; ++d) ten[12 + q * 9 + k * 3 + d] = Ji[k][d];
     for (int a = 0; a < 8; ++a)
@@ -1082,9 +1125,6 @@ bool hex8_affine_table(const double* x0, const double* ref, std::vector<unsigned
       }
     }
   // tensor_gradient's coefficients, with the scales dxi/dX folded in for a box
-  double cI[3] = {1.0, 1.0, 1.0}, sc[3];
-  hex8_tensor_rule(ref, cI);
-  const bool box = box_scales(x0, sc);
   ten[10] = box ? 1.0 : 0.0;
   if (!box) sc[0] = sc[1] = sc[2] = 0.5;
   const double own[5] = {cI[0], cI[1], cI[1] * sc[2], cI[2] * sc[1], cI[2] * sc[0]};
