@@ -112,7 +112,7 @@ struct AffNeoHookean {
   static constexpr bool TENSOR = true;     // hex8: the tables of a symmetric rule (AnyRule: any others)
   static constexpr int PROD_GROUPS = 2, STAGES = 2;  // of the hex8 kernel
   struct Mid {
-    double F[9], H[9], a1h, a2, c2;
+    double F[9], H[9], a1h, a2, c2, J, I13, r2;  // (r2 = J^(-2/3))
   };
   // J^(-1/3): CUDA's FP32 rcbrtf and one third-order step from the expansion of
   // (1 - e)^(-1/3), e = 1 - J r^3 (e is below 2^-20, the dropped term below
@@ -145,7 +145,10 @@ struct AffNeoHookean {
     const double r3 = inv_cbrt(J);
     const double I13 = mul_rn(I1, 1.0 / 3.0);
     const double JJ = mul_rn(J, J), d = JJ - J;
-    m.c2 = mul_rn(mul_rn(r3, r3), Gj);
+    m.J = J;
+    m.I13 = I13;
+    m.r2 = mul_rn(r3, r3);
+    m.c2 = mul_rn(m.r2, Gj);
     m.a2 = fma(m.c2, I13, -mul_rn(0.5 * Kj, d - 1.0));
     m.a1h = fma(m.c2, mul_rn(I13, 1.0 / 3.0), mul_rn(0.25 * Kj, JJ + d));
 #pragma unroll
@@ -239,7 +242,7 @@ struct AffNeoHookean {
 // condition: errors of 6e-13 at an aspect ratio of 1000, where this has 4e-16.
 struct PointUpdate {
   AffNeoHookean::Mid s;
-  double Gi[3][3];
+  double Gi[3][3], jxw;
 };
 __device__ __forceinline__ void cofactors(const double (&F)[3][3], double (&c)[9]) {
 #pragma unroll
@@ -270,19 +273,30 @@ __device__ __forceinline__ void point_update(const double* props, const double (
 #pragma unroll
     for (int j = 0; j < 3; ++j) m.Gi[j][d] = mul_rn(c[d * 3 + j], rG);
   to_x(D, m.Gi, gu);
-  AffNeoHookean::point(props, gu, mul_rn(detG, w), nullptr, nullptr, m.s);
+  m.jxw = mul_rn(detG, w);
+  AffNeoHookean::point(props, gu, m.jxw, nullptr, nullptr, m.s);
 }
-// The point's stress, H, c2 M, b and a2 (times JxW) in reference coordinates.
+// The point's stress, H, c2 M, b and a2 (times JxW) in reference coordinates.  DEVIATOR: the
+// stress as JxW (c1 H + G r2 (F - I1/3 H)), 20 operations more, which rounds a tenth less: where an
+// element has one point, so that no sum averages that out.
 struct RefPoint {
   double P[9], H[9], cM[6], b, a2;
 };
+template <bool DEVIATOR = false>
 __device__ __forceinline__ void ref_point(const double* props, const double (&G)[3][3], const double (&D)[3][3],
                                           double w, RefPoint& m) {
   PointUpdate u;
   point_update(props, G, D, w, u);
   AffNeoHookean::Mid& s = u.s;
 #pragma unroll
-  for (int i = 0; i < 9; ++i) s.F[i] = fma(s.c2, s.F[i], -mul_rn(s.a2, s.H[i]));  // the stress
+  for (int i = 0; i < 9; ++i) {  // the stress
+    if (DEVIATOR) {
+      const double c1 = mul_rn(0.5 * props[0], fma(s.J, s.J, -s.J) - 1.0), c2 = mul_rn(props[1], s.r2);
+      s.F[i] = mul_rn(u.jxw, fma(c1, s.H[i], mul_rn(c2, fma(-s.I13, s.H[i], s.F[i]))));
+    } else {
+      s.F[i] = fma(s.c2, s.F[i], -mul_rn(s.a2, s.H[i]));
+    }
+  }
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll

@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(EPB) tet4_kernel(ElemArgs g, const double* __r
       }
     }
     RefPoint m;
-    ref_point(g.props, G, D, __ldg(tab), m);
+    ref_point<true>(g.props, G, D, __ldg(tab), m);
     double P0[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) P0[i] = -((m.P[i * 3] + m.P[i * 3 + 1]) + m.P[i * 3 + 2]);
