@@ -116,8 +116,8 @@ struct fec_ctx {
   // could have used one; plan_state 0: not tried, 1: built, 2: the mesh has none
   std::vector<DevBuf> d_plan;
   std::vector<int64_t> plan_nslots;
-  std::vector<int> plan_state, plan_uses;
-  std::vector<int64_t> plan_pattern;   // the pattern (pattern_id) whose row offsets a plan holds
+  std::vector<int> plan_state;
+  std::vector<int64_t> plan_uses, plan_pattern;  // (the pattern whose row offsets it holds: pattern_id)
   int64_t pattern_id = 0;
   std::vector<DevBuf> d_general;       // per block: the reference element's table of a tet4, tet10 or hex27 block
   std::vector<DevBuf> d_affine;        // per block: the tensor-core operand table of a congruent hex8 block
@@ -451,16 +451,21 @@ int build_pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s) 
   int32_t* nslot = reinterpret_cast<int32_t*>(scan + scan_n);
   int32_t* nlist = nslot + n1;
   int* flags = nlist + n1;
-  FEC_CUDA(c, cudaMemsetAsync(flags, 0, 2 * sizeof(int), s));
-  FEC_CUDA(c, fec::pair_plan_count(ga, int(b), B.ne, nslot, nlist, flags, s));
-  FEC_CUDA(c, fec::pattern_scan(nslot, nullptr, c->nn, slot0, scan, s));
-  FEC_CUDA(c, fec::pattern_scan(nlist, nullptr, c->nn, list0, scan, s));
   int64_t nslots = 0, nentries = 0;
-  int h[2];
-  FEC_CUDA(c, cudaMemcpyAsync(&nslots, slot0 + c->nn, 8, cudaMemcpyDeviceToHost, s));
-  FEC_CUDA(c, cudaMemcpyAsync(&nentries, list0 + c->nn, 8, cudaMemcpyDeviceToHost, s));
-  FEC_CUDA(c, cudaMemcpyAsync(h, flags, sizeof h, cudaMemcpyDeviceToHost, s));
-  FEC_CUDA(c, cudaStreamSynchronize(s));
+  int h[2] = {0, 0};
+  bool wide = false;
+  for (int k = 0; k < 2; ++k) {
+    wide = k > 0;
+    FEC_CUDA(c, cudaMemsetAsync(flags, 0, 2 * sizeof(int), s));
+    FEC_CUDA(c, fec::pair_plan_count(ga, int(b), B.ne, nslot, nlist, flags, wide, s));
+    FEC_CUDA(c, fec::pattern_scan(nslot, nullptr, c->nn, slot0, scan, s));
+    FEC_CUDA(c, fec::pattern_scan(nlist, nullptr, c->nn, list0, scan, s));
+    FEC_CUDA(c, cudaMemcpyAsync(&nslots, slot0 + c->nn, 8, cudaMemcpyDeviceToHost, s));
+    FEC_CUDA(c, cudaMemcpyAsync(&nentries, list0 + c->nn, 8, cudaMemcpyDeviceToHost, s));
+    FEC_CUDA(c, cudaMemcpyAsync(h, flags, sizeof h, cudaMemcpyDeviceToHost, s));
+    FEC_CUDA(c, cudaStreamSynchronize(s));
+    if (!h[0]) break;
+  }
   if (h[0] || h[1] || nslots == 0 || nslots > max_slots || nentries > max_list) return FEC_OK;
   DevBuf& d = c->d_plan[b];  // slots, counts, list
   d.release();
@@ -475,7 +480,7 @@ int build_pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s) 
   uint32_t* count = reinterpret_cast<uint32_t*>(slots + nslots);
   int4* slots2 = reinterpret_cast<int4*>(t + sums);
   FEC_CUDA(c, fec::pair_plan_fill(ga, int(b), B.ne, slot0, list0, slots2, slots,
-                                  reinterpret_cast<uint32_t*>(slots2 + nslots), count, count + nslots, flags, s));
+                                  reinterpret_cast<uint32_t*>(slots2 + nslots), count, count + nslots, flags, wide, s));
   if (own.p) FEC_CUDA(c, cudaStreamSynchronize(s));
   c->plan_nslots[b] = nslots;
   c->plan_state[b] = 1;
@@ -484,16 +489,21 @@ int build_pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s) 
 
 // The plan of block b's gather by output entry (fec_pairgather.cu), which belongs to the
 // mesh: it outlives changes of the Dirichlet dofs, and only its row offsets are renewed at
-// the first assembly with a pattern (128^3 hex8: 0.4 ms).  Built at the assembly after
-// PLAN_AFTER that could have used it; both before the element kernels and outside stream
+// the first assembly with a pattern (128^3 hex8: 0.4 ms).  Built at the assembly after plan_after
+// that could have used it; both before the element kernels and outside stream
 // capture.  slots null where the block has none (yet): nodes shared with other blocks or with very
 // many elements, indices that do not fit, no memory for it; the per-node gathers then give
 // the same bits.
-// PLAN_AFTER: building takes what 1.6 to 9 assemblies then save (128^3 hex8 7.3 ms against
-// 0.80 ms an assembly, 61 x 53 x 47 hex8 0.74 against 0.17, 55k tet10 0.51 against 0.20,
-// tet4 + tet10 + hex27 of 22 x 24 x 26 cells 1.75 against 1.06, 40^3 hex8 0.38 against 0.05), so
-// a mesh that is assembled 8 times or fewer does not pay for it.
-constexpr int PLAN_AFTER = 8;
+// The rule: building takes about 0.17 ms (launches, an allocation, a wait) and then what up
+// to four assemblies save (128^3 hex8 3.35 ms against 0.80 an assembly, 61 x 53 x 47 hex8
+// 0.43 against 0.17, 55k tet10 0.32 against 0.20, tet4 + tet10 + hex27 of 22 x 24 x 26 cells 1.25
+// against 1.06), and an assembly saves 0.03 ns or more per stored pair of element nodes (20^3
+// hex8 9 us, 40^3 50): it is built when the assemblies without it have lost as much as it costs.
+// FEC_GATHER_PAIRS=1: at the first.
+int64_t plan_after(int64_t pairs) {
+  const char* e = getenv("FEC_GATHER_PAIRS");
+  return e && e[0] == '1' ? 0 : 4 + int64_t(4000000) / std::max<int64_t>(pairs, 1);
+}
 int pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s, fec::PairPlan* out) {
   *out = fec::PairPlan{nullptr, nullptr, nullptr, 0};
   if (c->plan_state[b] == 2) return FEC_OK;
@@ -506,7 +516,8 @@ int pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s, fec::P
     if (cs != cudaStreamCaptureStatusNone) return FEC_OK;
   }
   if (c->plan_state[b] == 0) {
-    if (c->plan_uses[b]++ < PLAN_AFTER) return FEC_OK;
+    const Block& B = c->blocks[b];
+    if (c->plan_uses[b]++ < plan_after(B.ne * (int64_t(B.nnpe) * (B.nnpe + 1) / 2))) return FEC_OK;
     if (int rc = build_pair_plan(c, ga, b, s)) return rc;
     if (c->plan_state[b] != 1) return FEC_OK;
   }

@@ -57,18 +57,19 @@ struct PairPlan {
 };
 // Of the mesh, whatever its Dirichlet dofs.
 // Pairs and list entries per node (int32, nn); flags (int[2], zeroed by the caller):
-// [0] a node with too many neighbours or elements, [1] a node shared with another block.
+// [0] a node with too many neighbours (more than 128 after it in number; 512 if wide) or
+// elements, [1] a node shared with another block.
 // unordered, unordered_count: scratch of the sizes of slots and count.
 cudaError_t pair_plan_count(const GatherArgs& g, int block, int64_t ne, int32_t* nslot, int32_t* nlist, int* flags,
-                            cudaStream_t stream);
+                            bool wide, cudaStream_t stream);
 cudaError_t pair_plan_fill(const GatherArgs& g, int block, int64_t ne, const int64_t* slot0, const int64_t* list0,
                            void* unordered, void* slots, uint32_t* unordered_count, uint32_t* count, uint32_t* list,
-                           int* flags, cudaStream_t stream);
+                           int* flags, bool wide, cudaStream_t stream);
 // ... but for the pairs' row offsets, which belong to the pattern.
 cudaError_t pair_plan_offsets(const GatherArgs& g, int block, const PairPlan& plan, cudaStream_t stream);
 cudaError_t launch_pair_gather(const GatherArgs& g, int block, const PairPlan& plan, cudaStream_t stream,
                                int* launches);
-// FEC_GATHER_PAIRS=0 keeps the per-node gathers.
+// FEC_GATHER_PAIRS=0 keeps the per-node gathers (1: the plan at the first assembly).
 bool gather_pairs_enabled();
 // Matrix-free tangent action: element contributions K_e v_e (summed over points
 // in point order) into the residual workspace args.Re; V is the full direction

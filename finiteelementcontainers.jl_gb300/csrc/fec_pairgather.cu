@@ -27,7 +27,8 @@ namespace fec {
 namespace {
 
 constexpr int WPB = 4;      // warps per CTA of the plan kernel
-constexpr int MAXT = 512;   // places of a node's hash table: its neighbours m >= n
+// Places of a node's hash table (its neighbours m >= n): 128 unless a node has more (warps of
+// 512 leave an SM a third of its warps: 48^3 165 us to fill instead of 86)
 constexpr int GROUP = 8;    // nodes whose pairs are ordered together (8: 128^3 3.40 ms; 32: 3.49, 128: 3.53)
 constexpr int CLASSES = 64; // list lengths told apart
 
@@ -55,15 +56,19 @@ __device__ __forceinline__ bool owned(const PlanArgs& a, int64_t n) {
   return p1 > p0 && int64_t(a.nadj[p0] >> 5) >= a.elem_start && int64_t(a.nadj[p1 - 1] >> 5) < a.elem_start + a.ne;
 }
 
-template <bool FILL>
+template <bool FILL, int MAXT>
 __global__ void __launch_bounds__(WPB * 32) plan_kernel(PlanArgs a) {
+  // a place: a neighbour, its list entries so far, and which of the CHUNK elements at hand have it
   __shared__ int32_t s_key[WPB][MAXT];
-  __shared__ int2 s_pair[WPB][FILL ? MAXT : 1];  // the neighbours and their list entries
+  __shared__ uint32_t s_in[WPB][MAXT];
   __shared__ uint16_t s_cnt[WPB][MAXT], s_at[WPB][FILL ? MAXT : 1], s_rank[WPB][FILL ? MAXT : 1];
+  __shared__ int2 s_pair[WPB][FILL ? MAXT : 1];  // the neighbours; their list entries, places << 16
+  constexpr int CHUNK = 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t n = int64_t(blockIdx.x) * WPB + warp;
   if (n >= a.nn) return;
   int32_t* key = s_key[warp];
+  uint32_t* in = s_in[warp];
   uint16_t* cnt = s_cnt[warp];
   const int64_t p0 = a.nadj_ptr[n], p1 = a.nadj_ptr[n + 1], cand = (p1 - p0) * a.A;
   bool use = p1 > p0 && (!a.shared || owned(a, n));
@@ -80,6 +85,7 @@ __global__ void __launch_bounds__(WPB * 32) plan_kernel(PlanArgs a) {
   for (int i = lane; i < T; i += 32) {
     key[i] = -1;
     cnt[i] = 0;
+    in[i] = 0;
   }
   __syncwarp();
   // the place of m, taken if it has none; -1 where the table is full
@@ -92,27 +98,53 @@ __global__ void __launch_bounds__(WPB * 32) plan_kernel(PlanArgs a) {
     }
     return -1;
   };
-  // elements in order; an element's nodes are distinct, so its lanes are
-  for (int64_t p = p0; p < p1; ++p) {
-    const int64_t le = int64_t(a.nadj[p] >> 5) - a.elem_start;
-    if (lane < a.A) {
-      const int32_t m = a.conn[a.conn_off + le * a.A + lane];
-      if (!FILL && a.shared && !owned(a, m)) a.flags[1] = 1;
-      if (m >= n) {
-        const int i = place(m);
-        if (i >= 0)
-          ++cnt[i];
-        else
-          a.flags[0] = 1;
-      }
+  // f(element of the chunk, local element, local nodes of n and m, m): the lanes take the
+  // nodes of the chunk's elements, all at once
+  const unsigned by_A = 65536u / unsigned(a.A) + 1u;  // i / A = i by_A >> 16 for i < 32 * 27
+  auto nodes = [&](int64_t q, auto f) {
+    const int ne = int(p1 - q < CHUNK ? p1 - q : CHUNK);
+    for (int i = lane; i < ne * a.A; i += 32) {
+      const int j = int(unsigned(i) * by_A >> 16), b = i - j * a.A;
+      const uint32_t packed = a.nadj[q + j];
+      const int64_t le = int64_t(packed >> 5) - a.elem_start;
+      const int32_t m = a.conn[a.conn_off + le * a.A + b];
+      f(j, le, int(packed & 31u), b, m);
     }
+  };
+  // which elements of the chunk have m (an element's nodes are distinct)
+  auto mark = [&](int64_t q) {
+    nodes(q, [&](int j, int64_t, int, int, int32_t m) {
+      if (!FILL && a.shared && !owned(a, m)) a.flags[1] = 1;
+      if (m < n) return;
+      const int i = place(m);
+      if (i >= 0)
+        atomicOr(&in[i], 1u << j);
+      else
+        a.flags[0] = 1;
+    });
+    __syncwarp();
+  };
+  auto next = [&](uint16_t* to) {  // ... counted, and cleared for the next chunk
+    for (int i = lane; i < T; i += 32) {
+      to[i] = uint16_t(to[i] + __popc(in[i]));
+      in[i] = 0;
+    }
+    __syncwarp();
+  };
+  const bool once = p1 - p0 <= CHUNK;
+  for (int64_t q = p0; q < p1; q += CHUNK) {
+    mark(q);
+    if (!once) next(cnt);
+  }
+  if (once) {
+    for (int i = lane; i < T; i += 32) cnt[i] = uint16_t(__popc(in[i]));
     __syncwarp();
   }
   int slots = 0, entries = 0;
   for (int i0 = 0; i0 < T; i0 += 32) {
     const int i = i0 + lane, c = cnt[i];
     const unsigned mask = __ballot_sync(0xffffffffu, c > 0);
-    if (FILL && c > 0) s_pair[warp][slots + __popc(mask & ((1u << lane) - 1u))] = make_int2(key[i], c);
+    if (FILL && c > 0) s_pair[warp][slots + __popc(mask & ((1u << lane) - 1u))] = make_int2(key[i], c | i << 16);
     slots += __popc(mask);
     entries += c;
   }
@@ -128,44 +160,46 @@ __global__ void __launch_bounds__(WPB * 32) plan_kernel(PlanArgs a) {
   __syncwarp();
   // pairs and list entries of the neighbours before each (ascending: rows of a column, and
   // element nodes, are)
-  for (int i = lane; i < T; i += 32) {
-    if (cnt[i] == 0) continue;
-    int rank = 0, at = 0;
+  uint16_t* at = s_at[warp];
+  for (int e = lane; e < slots; e += 32) {
+    const int2 own = s_pair[warp][e];
+    int rank = 0, before = 0;
+#pragma unroll 4
     for (int j = 0; j < slots; ++j) {
       const int2 o = s_pair[warp][j];
-      if (o.x < key[i]) {
+      if (o.x < own.x) {
         ++rank;
-        at += o.y;
+        before += o.y & 0xffff;
       }
     }
-    s_rank[warp][i] = uint16_t(rank);
-    s_at[warp][i] = uint16_t(at);
+    s_rank[warp][own.y >> 16] = uint16_t(rank);
+    at[own.y >> 16] = uint16_t(before);
   }
   __syncwarp();
   const int np = a.A * (a.A + 1) / 2;
-  for (int64_t p = p0; p < p1; ++p) {
-    const uint32_t packed = a.nadj[p];
-    const int64_t le = int64_t(packed >> 5) - a.elem_start;
-    const int la = int(packed & 31u), lb = lane;
-    if (lb < a.A) {
-      const int32_t m = a.conn[a.conn_off + le * a.A + lb];
+  for (int64_t q = p0; q < p1; q += CHUNK) {
+    if (!once) mark(q);
+    nodes(q, [&](int j, int64_t le, int la, int lb, int32_t m) {
       const int i = m >= n ? place(m) : -1;
-      if (i >= 0) {  // (a full table: the plan is not used)
-        const int c = cnt[i];
-        const int x = la < lb ? la : lb, y = la < lb ? lb : la;
-        const int64_t at = a.list0[n] + s_at[warp][i];
-        const int64_t block = le * np + x * (2 * a.A - x + 1) / 2 + y - x;
-        a.list[at] = uint32_t(block) << 1 | (la > lb ? 1u : 0u);
-        ++s_at[warp][i];
-        if (c != 0xffff) {  // the pair's first element (at is its first list entry)
-          const int64_t s = a.slot0[n] + s_rank[warp][i];
-          a.slots[s] = make_int4(int(n), m, int(uint32_t(at)), 0);
-          a.count[s] = uint32_t(c) | uint32_t(la) << 16 | uint32_t(lb) << 24;
-          cnt[i] = 0xffff;
-        }
+      if (i < 0) return;  // (a full table: the plan is not used)
+      const int x = la < lb ? la : lb, y = la < lb ? lb : la;
+      const uint32_t first = in[i] & ((1u << j) - 1u);
+      const int64_t t = a.list0[n] + at[i] + __popc(first);
+      const int64_t block = le * np + x * (2 * a.A - x + 1) / 2 + y - x;
+      a.list[t] = uint32_t(block) << 1 | (la > lb ? 1u : 0u);
+      if (first == 0 && cnt[i] != 0) {  // the pair's first element (t is its first list entry)
+        const int64_t s = a.slot0[n] + s_rank[warp][i];
+        a.slots[s] = make_int4(int(n), m, int(uint32_t(t)), 0);
+        a.count[s] = uint32_t(cnt[i]) | uint32_t(la) << 16 | uint32_t(lb) << 24;
       }
-    }
+    });
     __syncwarp();
+    if (q + CHUNK < p1) {
+      for (int i = lane; i < T; i += 32)
+        if (in[i]) cnt[i] = 0;  // its slot is written
+      __syncwarp();
+      next(at);
+    }
   }
 }
 
@@ -289,24 +323,32 @@ static PlanArgs plan_args(const GatherArgs& g, int block, int64_t ne, int* flags
 }
 
 cudaError_t pair_plan_count(const GatherArgs& g, int block, int64_t ne, int32_t* nslot, int32_t* nlist, int* flags,
-                            cudaStream_t s) {
+                            bool wide, cudaStream_t s) {
   PlanArgs a = plan_args(g, block, ne, flags);
   a.nslot = nslot;
   a.nlist = nlist;
-  plan_kernel<false><<<unsigned((g.nn + WPB - 1) / WPB), WPB * 32, 0, s>>>(a);
+  const unsigned grid = unsigned((g.nn + WPB - 1) / WPB);
+  if (wide)
+    plan_kernel<false, 512><<<grid, WPB * 32, 0, s>>>(a);
+  else
+    plan_kernel<false, 128><<<grid, WPB * 32, 0, s>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t pair_plan_fill(const GatherArgs& g, int block, int64_t ne, const int64_t* slot0, const int64_t* list0,
                            void* unordered, void* slots, uint32_t* count2, uint32_t* count, uint32_t* list, int* flags,
-                           cudaStream_t s) {
+                           bool wide, cudaStream_t s) {
   PlanArgs a = plan_args(g, block, ne, flags);
   a.slot0 = slot0;
   a.list0 = list0;
   a.slots = static_cast<int4*>(unordered);
   a.count = count2;
   a.list = list;
-  plan_kernel<true><<<unsigned((g.nn + WPB - 1) / WPB), WPB * 32, 0, s>>>(a);
+  const unsigned grid = unsigned((g.nn + WPB - 1) / WPB);
+  if (wide)
+    plan_kernel<true, 512><<<grid, WPB * 32, 0, s>>>(a);
+  else
+    plan_kernel<true, 128><<<grid, WPB * 32, 0, s>>>(a);
   order_kernel<<<unsigned((g.nn + GROUP - 1) / GROUP), 256, 0, s>>>(g.nn, slot0, a.slots, count2,
                                                                      static_cast<int4*>(slots), count);
   return cudaGetLastError();
