@@ -23,10 +23,10 @@
 //               neighbours in r, and stores 8 bytes per digit;
 //   4 warps     the epilogue into the symmetric half (KE_PAIRS);
 //   1 warp      issues 30 MMAs a half tile.
-// What bounds it: the FP64 point phase, about 350 operations a point at 64 clocks a warp
+// What bounds it: the FP64 point phase, about 400 operations a point at 64 clocks a warp
 // instruction and sub-partition (two thirds of the time a tile takes); the epilogue, the
-// MMAs and the slicers each need about half of it.  55,062 distorted elements 0.229 ms
-// (the per-element kernel 1.37), 82,368 of six translation classes 0.32 (the class
+// MMAs and the slicers each need about half of it.  55,062 distorted elements 0.252 ms
+// (the per-element kernel 1.37), 82,368 of six translation classes 0.364 (the class
 // kernel 1.19).
 #include <cmath>
 #include <cstdint>
@@ -56,8 +56,8 @@ constexpr int T_BYTES = (T_B4 + 6 * 8 + 15) / 16 * 16;
 
 // Producer warps take units of 8 elements (32 points), three to a tile, whichever the
 // tile, and stage a unit in a buffer of their own.  Nine of them: with eight (two a
-// sub-partition) the FP64 pipe idles for latency (247 us on 55,062 elements against 229;
-// three groups of three warps, a tile each: 232).
+// sub-partition) the FP64 pipe idles for latency (8% longer on 55,062 elements;
+// three groups of three warps, a tile each: 1%).
 constexpr int NPROD = 9, UNITS = NPT / 32, UEL = EPT / UNITS, SL_W = 2 * UNITS, EP_W = 4;
 constexpr int T_SL = 32 * NPROD, NSL = 32 * SL_W, T_EP = T_SL + NSL, T_MMA = T_EP + 32 * EP_W, NTHR = T_MMA + 32;
 static_assert(NTHR <= 640, "roles");

@@ -9,8 +9,9 @@
 // (KE_PAIRS, 90 entries an element), in double-float, consecutive threads consecutive
 // entries.
 //
-// What bounds it: the FP64 operations of the update, about 300 an element.  82,368
-// elements 0.074 ms (0.369 with a thread per matrix row of FP64 products).
+// What bounds it: the FP64 operations of the update, about 320 an element.  82,368
+// elements 0.077 ms (0.369 with the per-element kernel: a thread per matrix row, entries of A
+// formed in FP64, then contracted in double-float over nine places each).
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
