@@ -119,6 +119,7 @@ struct fec_ctx {
   std::vector<int> plan_state;
   std::vector<int64_t> plan_uses, plan_pattern;  // (the pattern whose row offsets it holds: pattern_id)
   int64_t pattern_id = 0;
+  bool plan_first = false;             // built at the first assembly that can use it (fec_set_gather_plan)
   std::vector<DevBuf> d_general;       // per block: the reference element's table of a tet4, tet10 or hex27 block
   std::vector<DevBuf> d_affine;        // per block: the tensor-core operand table of a congruent hex8 block
                                        // or of a tet10/hex27 block of translation classes
@@ -499,7 +500,7 @@ int build_pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s) 
 // 0.43 against 0.17, 55k tet10 0.32 against 0.20, tet4 + tet10 + hex27 of 22 x 24 x 26 cells 1.25
 // against 1.06), and an assembly saves 0.03 ns or more per stored pair of element nodes (20^3
 // hex8 9 us, 40^3 50): it is built when the assemblies without it have lost as much as it costs.
-// FEC_GATHER_PAIRS=1: at the first.
+// FEC_GATHER_PAIRS=1 or fec_set_gather_plan: at the first.
 int64_t plan_after(int64_t pairs) {
   const char* e = getenv("FEC_GATHER_PAIRS");
   return e && e[0] == '1' ? 0 : 4 + int64_t(4000000) / std::max<int64_t>(pairs, 1);
@@ -517,7 +518,7 @@ int pair_plan(fec_ctx* c, const GatherArgs& ga, size_t b, cudaStream_t s, fec::P
   }
   if (c->plan_state[b] == 0) {
     const Block& B = c->blocks[b];
-    if (c->plan_uses[b]++ < plan_after(B.ne * (int64_t(B.nnpe) * (B.nnpe + 1) / 2))) return FEC_OK;
+    if (c->plan_uses[b]++ < plan_after(B.ne * (int64_t(B.nnpe) * (B.nnpe + 1) / 2)) && !c->plan_first) return FEC_OK;
     if (int rc = build_pair_plan(c, ga, b, s)) return rc;
     if (c->plan_state[b] != 1) return FEC_OK;
   }
@@ -1058,6 +1059,12 @@ int fec_pattern_build(fec_ctx* c, int64_t* nnz_out) {
   c->pattern_ready = true;
   ++c->pattern_id;
   if (nnz_out) *nnz_out = nnz;
+  return ok(c);
+}
+
+int fec_set_gather_plan(fec_ctx* c, int first) {
+  if (!c) return FEC_ERR_ARG;
+  c->plan_first = first != 0;
   return ok(c);
 }
 

@@ -167,6 +167,11 @@ class SparseMatrixAssembler:
         tet10, hex27 blocks) in one persistent launch (fec_set_single_launch)."""
         self._call("fec_set_single_launch", 1 if on else 0)
 
+    def set_gather_plan(self, first: bool = True) -> None:
+        """Build the mesh's plan of the gather by output entry at the next assembly that can
+        use it (fec_set_gather_plan): before a capture, whose graph keeps its gathers."""
+        self._call("fec_set_gather_plan", 1 if first else 0)
+
     def pattern_device(self):
         """1-based (colptr, rowval) of the CSC stiffness as int64 device tensors,
         filled by a kernel (for a CuSparse-style matrix on the device)."""

@@ -108,6 +108,8 @@ class NewtonLoop:
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         saved = [Uu.clone() for _, _, Uu, _ in self.systems]
+        for asm, _, _, _ in self.systems:
+            asm.set_gather_plan()  # in the warm-up: the graph keeps the gathers it is captured with
         with torch.cuda.stream(side):  # warm-up outside the graph (allocations, attributes)
             self._body()
         torch.cuda.current_stream().wait_stream(side)

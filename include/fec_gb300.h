@@ -150,6 +150,11 @@ int fec_pattern_build_device(fec_ctx* ctx, int64_t* nnz_out, void* stream);
  * launch per block.  No counterpart in the reference, which launches one
  * kernel per block from foreach_block (src/Utils.jl:171-189). */
 int fec_set_single_launch(fec_ctx* ctx, int on);
+/* first != 0: the mesh's plan of the gather by output entry is built at the next
+ * assembly outside stream capture that can use it, not after some assemblies without it: for a
+ * caller about to capture an assembly, whose graph keeps the gathers it was captured
+ * with.  Results are the same bits.  No counterpart in the reference. */
+int fec_set_gather_plan(fec_ctx* ctx, int first);
 /* 1-based colptr (n_unknowns + 1) and rowval (nnz) written into DEVICE buffers
  * on `stream` (the colptr/rowval of sparse!, SparsityPatterns.jl:301-308). */
 int fec_pattern_get_device(const fec_ctx* ctx, int64_t* colptr_dev, int64_t* rowval_dev, void* stream);
